@@ -6,6 +6,7 @@
 
 #include "common.h"
 #include "krylov.h"
+#include "samg.h"
 
 namespace pb {
 
@@ -90,6 +91,9 @@ struct Amg {
     // extra coarse-level launches cost more than that saved)
     void forPressure();
     bool kLevel(size_t l) const;
+    // the smoothed-aggregation hierarchy of flexible CG (fcgMode picks it); this struct's own
+    // levels then stay unbuilt
+    std::unique_ptr<SaAmg> sa;
 
     // Build the hierarchy (first call) or refresh its values (later calls) for
     // the matrix A, whose CSR pattern (device rowptr/col) lists each row's

@@ -748,23 +748,26 @@ void iterateEager(const SellMatrix& A, const T* M, Vecs<T> V, Amg* amg, T* y, T*
 }
 
 // Krylov method of a solve: BiCGSTAB, or flexible CG preconditioned by an FP64
-// cycle (with the K-cycle levels) or by an FP32 V-cycle
-enum { KM_BICGSTAB = 0, KM_FCG = 1, KM_FCG_PRE32 = 2 };
+// cycle (with the K-cycle levels), by an FP32 V-cycle of the same hierarchy, or by the
+// FP32 V-cycle of smoothed aggregation
+enum { KM_BICGSTAB = 0, KM_FCG = 1, KM_FCG_PRE32 = 2, KM_FCG_SA = 3 };
+inline bool precondIn32(int mode) { return mode == KM_FCG_PRE32 || mode == KM_FCG_SA; }
 
 // `count` flexible-CG iterations (FP64 recurrences), launched one kernel at a time.
-// Vectors: x = V.x, r = V.r, d = V.p, q = V.v, u = V.t; z = y (KM_FCG) or, for
-// KM_FCG_PRE32, the FP32 pair r32 = w.y32 -> z32 = w.z32.
+// Vectors: x = V.x, r = V.r, d = V.p, q = V.v, u = V.t; z = y (KM_FCG) or, with an FP32
+// cycle, the FP32 pair r32 = w.y32 -> z32 = w.z32.
 void iterateFcgEager(const SellMatrix& A, const double* M, Vecs<double> V, Amg* amg, double* y, int mode,
                      long long count, bool sample, KrylovWork& w, cudaStream_t s) {
     KState* S = w.state.p;
     const int n = A.n, vg = vecGrid(n);
-    const bool p32 = mode == KM_FCG_PRE32;
+    const bool p32 = precondIn32(mode);
     auto k64 = fcg_spmv_kernel<4, 6, double>;
     auto k32 = fcg_spmv_kernel<4, 6, float>;
     const int sg = p32 ? waveGrid(k32, ceil_div(A.nslices, WARPS)) : waveGrid(k64, ceil_div(A.nslices, WARPS));
     for (long long it = 0; it < count; ++it) {
         if (p32) {
-            amg->apply32(w.y32.p, w.z32.p, S, s, true, sample);
+            if (mode == KM_FCG_SA) amg->sa->apply(w.y32.p, w.z32.p, S, s, sample);
+            else amg->apply32(w.y32.p, w.z32.p, S, s, true, sample);
             const int slot = sample ? profBegin(PROF_FCG_SPMV, false, fcgSpmvBytes(A, 4), s) : -1;
             launchPdl(k32, sg, BS, s, A.nslices, n, A.sl_off, A.col, M, (const float*)w.z32.p, V.t,
                       (const double*)V.v, (const double*)V.r, w.partials.p, w.counter.p, S);
@@ -819,7 +822,7 @@ void iterate(const SellMatrix& A, const T* M, Vecs<T> V, Amg* amg, T* y, T* z, l
     std::vector<uintptr_t> key = {(uintptr_t)mode, (uintptr_t)sizeof(T), (uintptr_t)A.sl_off, (uintptr_t)A.col, (uintptr_t)A.nslices,
                                   (uintptr_t)A.n, (uintptr_t)M, (uintptr_t)V.x, (uintptr_t)V.r, (uintptr_t)V.r0,
                                   (uintptr_t)V.p, (uintptr_t)V.v, (uintptr_t)V.s, (uintptr_t)V.t, (uintptr_t)amg,
-                                  (uintptr_t)(amg ? amg->generation : 0), (uintptr_t)y, (uintptr_t)z,
+                                  (uintptr_t)(!amg ? 0 : mode == KM_FCG_SA ? amg->sa->generation : amg->generation), (uintptr_t)y, (uintptr_t)z,
                                   (uintptr_t)w.state.p, (uintptr_t)w.partials.p, (uintptr_t)w.counter.p,
                                   (uintptr_t)w.y32.p, (uintptr_t)w.z32.p};
     constexpr size_t MAX_GRAPHS = 8;
@@ -885,7 +888,7 @@ KrylovOut runBicgstab(const SellMatrix& A, const T* M, const T* rhs, Vecs<T> V, 
         if constexpr (sizeof(T) == 8) {
             if (flex) {
                 if (zero) fail(PRISM_INTERNAL, "flexible CG starts from A x");
-                fcg_init_kernel<<<vg, BS, 0, s>>>(n, V.r, rhs, V.p, V.v, mode == KM_FCG_PRE32 ? w.y32.p : nullptr, tol,
+                fcg_init_kernel<<<vg, BS, 0, s>>>(n, V.r, rhs, V.p, V.v, precondIn32(mode) ? w.y32.p : nullptr, tol,
                                                   w.partials.p, w.counter.p, S); countLaunch();
             }
         }
@@ -943,8 +946,26 @@ namespace {
 // flexible CG's preconditioner: an FP32 V-cycle (half the bytes of the FP64 one; the
 // recurrences stay FP64) unless the hierarchy has K-cycle levels (FP64 only) or
 // PRISM_FCG_PREC=fp64
-int fcgMode(const Amg* amg) { return fcgPre32(amg) ? KM_FCG_PRE32 : KM_FCG; }
+int fcgMode(const Amg* amg, const SellMatrix& A) {
+    return fcgSmoothed(amg, A) ? KM_FCG_SA : fcgPre32(amg) ? KM_FCG_PRE32 : KM_FCG;
+}
+// values of the cycle's hierarchy from the current matrix (built on first use)
+void setupCycle(Amg* amg, int mode, const SellMatrix& A, const int* rowptr, const int* col, bool pre32,
+                cudaStream_t s) {
+    if (mode != KM_FCG_SA) {
+        amg->setup(A, rowptr, col, pre32, s);
+        return;
+    }
+    if (!amg->sa) amg->sa = std::make_unique<SaAmg>();
+    amg->sa->setup(A, rowptr, col, amg->values_current, s);
+}
 }  // namespace
+
+// Smoothed aggregation up to 2^28 matrix entries (38M rows of a hex mesh): its setup sorts
+// about three 64-bit keys per entry and numbers them with 32-bit ints.
+bool fcgSmoothed(const Amg* amg, const SellMatrix& A) {
+    return fcgPre32(amg) && A.nnz_csr < (int64_t(1) << 28);
+}
 
 bool fcgPre32(const Amg* amg) {
     static const bool p64 = [] {
@@ -959,8 +980,8 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
                    bool flexible) {
     const bool mixed = precision == PRISM_PREC_MIXED;
     if (flexible && (mixed || !amg)) fail(PRISM_INTERNAL, "flexible CG runs FP64 with AMG only");
-    const int mode = flexible ? fcgMode(amg) : KM_BICGSTAB;
-    const bool pre32 = mixed || mode == KM_FCG_PRE32;  // FP32 copy of the hierarchy
+    const int mode = flexible ? fcgMode(amg, A) : KM_BICGSTAB;
+    const bool pre32 = mixed || precondIn32(mode);  // FP32 copy of the hierarchy
     w.ensure(A.nslices * 32, A.nnz_padded, mixed);
     const int n = A.n;
     const int gn = ceil_div(n, BS);
@@ -985,7 +1006,7 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
         if (!rowptr || !col) fail(PRISM_INTERNAL, "AMG preconditioner without a CSR pattern");
         w.ensurePrec(pre32);
         VerboseTimer vt("amg setup", s);
-        amg->setup(A, rowptr, col, pre32, s);
+        setupCycle(amg, mode, A, rowptr, col, pre32, s);
         M32 = amg->vals32();
     }
     VerboseTimer vt_solve(mixed ? "bicgstab fp32+fp64" : flexible ? "fcg fp64" : "bicgstab fp64", s);
@@ -1421,7 +1442,7 @@ void emitBicgstab(const SellMatrix& A, const double* b, double* x, double tol, l
                   cudaStream_t s, Amg* amg, const int* rowptr, const int* col, SolveCtl* ctl, CaptureStreams& cs,
                   int depth, bool flexible) {
     if (flexible && !amg) fail(PRISM_INTERNAL, "flexible CG runs with AMG only");
-    const int mode = flexible ? fcgMode(amg) : KM_BICGSTAB;
+    const int mode = flexible ? fcgMode(amg, A) : KM_BICGSTAB;
     w.ensure(A.nslices * 32, A.nnz_padded, false);
     const int n = A.n, gn = ceil_div(n, BS);
     const bool scaled = amg == nullptr;
@@ -1435,8 +1456,8 @@ void emitBicgstab(const SellMatrix& A, const double* b, double* x, double tol, l
         X = w.xs.p;
     } else {
         if (!rowptr || !col) fail(PRISM_INTERNAL, "AMG preconditioner without a CSR pattern");
-        w.ensurePrec(mode == KM_FCG_PRE32);
-        amg->setup(A, rowptr, col, mode == KM_FCG_PRE32, s);
+        w.ensurePrec(precondIn32(mode));
+        setupCycle(amg, mode, A, rowptr, col, precondIn32(mode), s);
     }
     KState* S = w.state.p;
     Vecs<double> V{X, w.r.p, w.r0.p, w.p.p, w.v.p, w.s.p, w.t.p};
@@ -1453,7 +1474,7 @@ void emitBicgstab(const SellMatrix& A, const double* b, double* x, double tol, l
     spmv_kernel<double, 0><<<sg, BS, 0, sub>>>(A.nslices, n, A.sl_off, A.col, A64.vals, V.x, V.r, nullptr, nullptr,
                                                nullptr, nullptr); countLaunch();
     if (flexible) {
-        fcg_init_kernel<<<vg, BS, 0, sub>>>(n, V.r, b, V.p, V.v, mode == KM_FCG_PRE32 ? w.y32.p : nullptr, tol,
+        fcg_init_kernel<<<vg, BS, 0, sub>>>(n, V.r, b, V.p, V.v, precondIn32(mode) ? w.y32.p : nullptr, tol,
                                             w.partials.p, w.counter.p, S); countLaunch();
     } else {
         init_kernel<double><<<vg, BS, 0, sub>>>(n, V.r, b, V.r0, V.p, V.v, 0, tol, w.partials.p, w.counter.p, S); countLaunch();

@@ -92,6 +92,8 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
                    const int* col = nullptr, bool flexible = false);
 // flexible CG with amg preconditions with an FP32 V-cycle (else with the FP64 cycle)
 bool fcgPre32(const Amg* amg);
+// that V-cycle is smoothed aggregation's (samg.h)
+bool fcgSmoothed(const Amg* amg, const SellMatrix& A);
 // x <- x + D^-1 (b - A x)   (numerics/jacobi.cpp:5-9)
 void jacobiStep(const SellMatrix& A, const double* b, double* x, KrylovWork& w, cudaStream_t s);
 // max|A x - b| / (max|diag(A) x| + eps)   (numerics/solver.cpp:8-24); returns NaN if non-finite values met

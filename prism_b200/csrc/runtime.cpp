@@ -1343,7 +1343,10 @@ bool graphReady(const Transport& eq, const PrismSolveOpts& o) {
         pc = eq.auto_pc;
     }
     if (pc == PRISM_PC_AMG) {
-        if (!eq.amg || !eq.amg->built || !m.kw.y) return false;
+        if (!eq.amg || !m.kw.y) return false;
+        if (flexibleFor(eq, o, eq.amg.get()) && fcgSmoothed(eq.amg.get(), m.matrix(eq.A.p)))
+            return eq.amg->sa && eq.amg->sa->built && m.kw.y32;
+        if (!eq.amg->built) return false;
         for (auto& L : eq.amg->levels)
             if (!L->b || !L->dinv) return false;
         if (eq.amg->k_levels > 0 && !eq.amg->kscal) return false;
