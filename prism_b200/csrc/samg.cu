@@ -42,6 +42,7 @@ constexpr int WARPS = BS / 32;
 constexpr int COARSE_MAX = 96;  // rows solved by a dense inverse
 constexpr int MAX_LEVELS = 12;
 constexpr int MIS_ROUNDS = 24;   // 6-9 rounds leave nothing undecided on the meshes seen
+constexpr int MIS_BATCH = 8;     // rounds between two looks at the number left
 constexpr double STRONG = 0.25;
 
 inline int grid(int64_t n) { return std::max(1, ceil_div(n, BS)); }
@@ -179,34 +180,19 @@ __global__ void p_keys_kernel(int n, const int* rowptr, const int* col, const in
         keys[k] = i * nc + (a >= 0 ? a : agg[i] >= 0 ? agg[i] : 0);
     }
 }
-// products of row i of A P
-__global__ void ap_count_kernel(int n, const int* rowptr, const int* col, const int* p_rowptr, long long* count) {
-    const int i = blockIdx.x * BS + threadIdx.x;
-    if (i >= n) return;
-    long long c = 0;
-    for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) c += p_rowptr[col[k] + 1] - p_rowptr[col[k]];
-    count[i] = c;
+// keys of a row product's pattern, one left entry per thread: the output row of entry k
+// with every column of row idx[k] of the right matrix
+__global__ void product_count_kernel(int64_t m, const int* idx, const int* b_rowptr, long long* count) {
+    const int64_t k = blockIdx.x * (int64_t)BS + threadIdx.x;
+    if (k < m) count[k] = b_rowptr[idx[k] + 1] - b_rowptr[idx[k]];
 }
-__global__ void ap_keys_kernel(int n, const int* rowptr, const int* col, const int* p_rowptr, const int* p_col,
-                               const long long* off, long long nc, long long* keys) {
-    const int i = blockIdx.x * BS + threadIdx.x;
-    if (i >= n) return;
-    long long o = off[i];
-    for (int k = rowptr[i]; k < rowptr[i + 1]; ++k)
-        for (int q = p_rowptr[col[k]]; q < p_rowptr[col[k] + 1]; ++q) keys[o++] = i * nc + p_col[q];
-}
-// products of P^T (A P), generated by fine row: (column of P row i) x (column of A P row i)
-__global__ void ac_count_kernel(int n, const int* p_rowptr, const int* q_rowptr, long long* count) {
-    const int i = blockIdx.x * BS + threadIdx.x;
-    if (i < n) count[i] = (long long)(p_rowptr[i + 1] - p_rowptr[i]) * (q_rowptr[i + 1] - q_rowptr[i]);
-}
-__global__ void ac_keys_kernel(int n, const int* p_rowptr, const int* p_col, const int* q_rowptr, const int* q_col,
-                               const long long* off, long long nc, long long* keys) {
-    const int i = blockIdx.x * BS + threadIdx.x;
-    if (i >= n) return;
-    long long o = off[i];
-    for (int p = p_rowptr[i]; p < p_rowptr[i + 1]; ++p)
-        for (int q = q_rowptr[i]; q < q_rowptr[i + 1]; ++q) keys[o++] = p_col[p] * nc + q_col[q];
+__global__ void product_keys_kernel(int64_t m, const int* orow, const int* idx, const int* b_rowptr, const int* b_col,
+                                    const long long* off, long long nc, long long* keys) {
+    const int64_t k = blockIdx.x * (int64_t)BS + threadIdx.x;
+    if (k >= m) return;
+    long long o = off[k];
+    const long long r = orow[k] * nc;
+    for (int e = b_rowptr[idx[k]]; e < b_rowptr[idx[k] + 1]; ++e) keys[o++] = r + b_col[e];
 }
 // CSR of the sorted distinct keys: columns, and each row's start by binary search
 __global__ void key_cols_kernel(int64_t m, const long long* keys, long long nc, int* col) {
@@ -819,19 +805,6 @@ int readInt(const int* d, cudaStream_t s) {
     return v;
 }
 
-// exclusive offsets of count[0, n) (count[n] is overwritten); returns the total
-long long offsets(TmpBuf<long long>& count, TmpBuf<long long>& off, int n, cudaStream_t s) {
-    PB_CUDA(cudaMemsetAsync(count.p + n, 0, sizeof(long long), s));
-    size_t tb = 0;
-    PB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, count.p, off.p, n + 1, s));
-    TmpBuf<unsigned char> tmp(std::max<size_t>(tb, 1), s);
-    PB_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, count.p, off.p, n + 1, s));
-    long long total = 0;
-    PB_CUDA(cudaMemcpyAsync(&total, off.p + n, sizeof(long long), cudaMemcpyDeviceToHost, s));
-    PB_CUDA(cudaStreamSynchronize(s));
-    return total;
-}
-
 // CSR pattern (sorted columns) of the distinct keys row * ncols + col among keys[0, m); keys is overwritten
 int64_t patternOf(DevArena& ar, long long* keys, int64_t m, int nrows, long long ncols, ArenaBuf<int>& rowptr,
                   ArenaBuf<int>& col, cudaStream_t s) {
@@ -852,6 +825,24 @@ int64_t patternOf(DevArena& ar, long long* keys, int64_t m, int nrows, long long
     key_cols_kernel<<<grid(nnz), BS, 0, s>>>(nnz, keys, ncols, col.p); countLaunch();
     key_rows_kernel<<<grid(nrows + 1), BS, 0, s>>>(nrows, nnz, keys, ncols, rowptr.p); countLaunch();
     return nnz;
+}
+
+// Pattern of the row product of m left entries (output row orow[k], right row idx[k]) with B
+int64_t productPattern(DevArena& ar, int64_t m, const int* orow, const int* idx, const int* b_rowptr, const int* b_col,
+                       int nrows, long long ncols, ArenaBuf<int>& rowptr, ArenaBuf<int>& col, cudaStream_t s) {
+    TmpBuf<long long> count(m + 1, s), off(m + 1, s);
+    product_count_kernel<<<grid(m), BS, 0, s>>>(m, idx, b_rowptr, count.p); countLaunch();
+    PB_CUDA(cudaMemsetAsync(count.p + m, 0, sizeof(long long), s));
+    size_t tb = 0;
+    PB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, count.p, off.p, m + 1, s));
+    TmpBuf<unsigned char> tmp(std::max<size_t>(tb, 1), s);
+    PB_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, count.p, off.p, m + 1, s));
+    long long total = 0;
+    PB_CUDA(cudaMemcpyAsync(&total, off.p + m, sizeof(long long), cudaMemcpyDeviceToHost, s));
+    PB_CUDA(cudaStreamSynchronize(s));
+    TmpBuf<long long> keys(std::max<long long>(total, 1), s);
+    product_keys_kernel<<<grid(m), BS, 0, s>>>(m, orow, idx, b_rowptr, b_col, off.p, ncols, keys.p); countLaunch();
+    return patternOf(ar, keys.p, total, nrows, ncols, rowptr, col, s);
 }
 
 // Transpose of the pattern (n rows, nc columns): row starts, the row of every entry, and
@@ -890,6 +881,7 @@ int aggregate(DevArena& ar, SaLevel& L, cudaStream_t s) {
     for (int r = 0; r < MIS_ROUNDS; ++r) {
         mis_near_kernel<<<grid(n), BS, 0, s>>>(n, L.rowptr, strong.p, key.p, near.p, left.p + r); countLaunch();
         mis_decide_kernel<<<grid(n), BS, 0, s>>>(n, L.rowptr, strong.p, key.p, near.p, left.p + r, left.p + r + 1); countLaunch();
+        if (r % MIS_BATCH == MIS_BATCH - 1 && readInt(left.p + r + 1, s) == 0) break;
     }
     PB_CUDA(cudaMemsetAsync(root.p + n, 0, sizeof(int), s));
     mis_root_kernel<<<grid(n), BS, 0, s>>>(n, key.p, root.p); countLaunch();
@@ -1032,14 +1024,11 @@ void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, cudaSt
         }
         L.p_val.alloc(arena, std::max<int64_t>(L.p_nnz, 1), s);
         transposeOf(arena, L.n, nc, L.p_nnz, L.p_rowptr.p, L.p_col.p, L.pt_rowptr, L.pt_row, &L.pt_src, nullptr, s);
-        TmpBuf<long long> count(L.n + 1, s), off(L.n + 1, s);
         // A P, the pattern of Q
-        ap_count_kernel<<<grid(L.n), BS, 0, s>>>(L.n, L.rowptr, L.col, L.p_rowptr.p, count.p); countLaunch();
-        int64_t m = offsets(count, off, L.n, s);
         {
-            TmpBuf<long long> keys(std::max<int64_t>(m, 1), s);
-            ap_keys_kernel<<<grid(L.n), BS, 0, s>>>(L.n, L.rowptr, L.col, L.p_rowptr.p, L.p_col.p, off.p, nc, keys.p); countLaunch();
-            L.q_nnz = patternOf(arena, keys.p, m, L.n, nc, L.q_rowptr, L.q_col, s);
+            TmpBuf<int> erow(std::max<int64_t>(L.nnz, 1), s);
+            entry_rows_kernel<<<grid(L.n), BS, 0, s>>>(L.n, L.rowptr, erow.p); countLaunch();
+            L.q_nnz = productPattern(arena, L.nnz, erow.p, L.col, L.p_rowptr.p, L.p_col.p, L.n, nc, L.q_rowptr, L.q_col, s);
         }
         L.ap_val.alloc(arena, std::max<int64_t>(L.q_nnz, 1), s);
         L.q_val.alloc(arena, std::max<int64_t>(L.q_nnz, 1), s);
@@ -1050,13 +1039,11 @@ void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, cudaSt
         L.lpr_t = lanesFor(nc, L.q_nnz);
         // P^T A P
         auto C = std::make_unique<SaLevel>();
-        ac_count_kernel<<<grid(L.n), BS, 0, s>>>(L.n, L.p_rowptr.p, L.q_rowptr.p, count.p); countLaunch();
-        m = offsets(count, off, L.n, s);
         {
-            TmpBuf<long long> keys(std::max<int64_t>(m, 1), s);
-            ac_keys_kernel<<<grid(L.n), BS, 0, s>>>(L.n, L.p_rowptr.p, L.p_col.p, L.q_rowptr.p, L.q_col.p, off.p, nc,
-                                                    keys.p); countLaunch();
-            C->nnz = patternOf(arena, keys.p, m, nc, nc, C->o_rowptr, C->o_col, s);
+            TmpBuf<int> erow(std::max<int64_t>(L.p_nnz, 1), s);
+            entry_rows_kernel<<<grid(L.n), BS, 0, s>>>(L.n, L.p_rowptr.p, erow.p); countLaunch();
+            C->nnz = productPattern(arena, L.p_nnz, L.p_col.p, erow.p, L.q_rowptr.p, L.q_col.p, nc, nc, C->o_rowptr,
+                                    C->o_col, s);
         }
         C->n = nc;
         C->rowptr = C->o_rowptr.p;
