@@ -43,6 +43,63 @@ __global__ void __launch_bounds__(256) ls_grad_kernel(const MeshView m, ScalarVi
     }
 }
 
+// pinv = (D^T D)^-1 D^T per cell and the weighted distance vectors w per cell face
+// (LeastSquares::setPseudoInvMatrices, least_squares.cpp:12-61), one thread per cell, in the
+// reference's operation order. One pass over the mesh's geometry (about 270 bytes per cell and
+// 50 per cell face, HBM-bound): 2.1M cells took 331 ms of a first pass on one host core.
+__global__ void __launch_bounds__(256) ls_operator_kernel(const MeshView m, double* __restrict__ pinv,
+                                                          double* __restrict__ w, int64_t nk) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= m.nc) return;
+    double D[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    const D3 xc = cellCenter(m, c);
+    for (int q = m.cf_off[c]; q < m.cf_off[c + 1]; ++q) {
+        const int f = m.cf_face[q];
+        D3 r;
+        if (f >= m.nb) {
+            const int o = m.owner[f];
+            r = cellCenter(m, o == c ? m.nbr[f] : o) - xc;
+        } else {
+            r = D3{m.fx[f], m.fy[f], m.fz[f]} - xc;
+        }
+        const double wk = 1 / (sqrt((r.x * r.x + r.y * r.y) + r.z * r.z) + EPSILON);
+        const double rv[3] = {r.x, r.y, r.z};
+        const double wd[3] = {r.x * wk, r.y * wk, r.z * wk};
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) D[i][j] += wd[i] * rv[j];
+        w[q] = wd[0];
+        w[nk + q] = wd[1];
+        w[2 * nk + q] = wd[2];
+    }
+    double P[3][3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) P[i][j] = (D[0][i] * D[0][j] + D[1][i] * D[1][j]) + D[2][i] * D[2][j];
+    const double c00 = P[1][1] * P[2][2] - P[1][2] * P[2][1];
+    const double c10 = P[1][2] * P[2][0] - P[1][0] * P[2][2];
+    const double c20 = P[1][0] * P[2][1] - P[1][1] * P[2][0];
+    const double det = (P[0][0] * c00 + P[0][1] * c10) + P[0][2] * c20;
+    double I[3][3];
+    I[0][0] = c00 / det;
+    I[1][0] = c10 / det;
+    I[2][0] = c20 / det;
+    I[0][1] = (P[0][2] * P[2][1] - P[0][1] * P[2][2]) / det;
+    I[1][1] = (P[0][0] * P[2][2] - P[0][2] * P[2][0]) / det;
+    I[2][1] = (P[0][1] * P[2][0] - P[0][0] * P[2][1]) / det;
+    I[0][2] = (P[0][1] * P[1][2] - P[0][2] * P[1][1]) / det;
+    I[1][2] = (P[0][2] * P[1][0] - P[0][0] * P[1][2]) / det;
+    I[2][2] = (P[0][0] * P[1][1] - P[0][1] * P[1][0]) / det;
+    const int64_t n = m.nc;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)  // (I * D^T)(i,j) = sum_k I(i,k) D(j,k)
+            pinv[(3 * i + j) * n + c] = (I[i][0] * D[j][0] + I[i][1] * D[j][1]) + I[i][2] * D[j][2];
+}
+
 // GreenGauss::computeGradAtCell (green_gauss.cpp:47-76) for the cells of one dependency
 // level, GG_LPC lanes per cell: each lane evaluates one face's term (phi_b S_f on a
 // boundary face of a non-empty patch, S_f^out phi_f with the skewness correction on an
@@ -111,6 +168,12 @@ __global__ void __launch_bounds__(256) gg_level_kernel(const MeshView m, ScalarV
         s.g[s.gstride + c] = grad.y;
         s.g[2 * s.gstride + c] = grad.z;
     }
+}
+
+void launchLeastSquaresOperators(const MeshView& m, double* pinv, double* w, int64_t nk, cudaStream_t st) {
+    if (m.nc == 0) return;
+    ls_operator_kernel<<<ceil_div(m.nc, 256), 256, 0, st>>>(m, pinv, w, nk); countLaunch();
+    PB_LAUNCH("ls_operator_kernel");
 }
 
 void launchLeastSquares(const MeshView& m, const ScalarView& s, const double* pinv, const double* w, int64_t nk,

@@ -10,6 +10,7 @@ namespace pb {
 
 void launchLeastSquares(const MeshView& m, const ScalarView& s, const double* pinv, const double* w, int64_t nk,
                         cudaStream_t st);
+void launchLeastSquaresOperators(const MeshView& m, double* pinv, double* w, int64_t nk, cudaStream_t st);
 void launchGreenGauss(const MeshView& m, const ScalarView& s, const int* level_cells,
                       const std::vector<int>& level_off, cudaStream_t st);
 void launchScalarFaces(const MeshView& m, const ScalarView& s, double* out, cudaStream_t st);

@@ -18,13 +18,6 @@ namespace pb {
 
 namespace {
 
-struct H3 {
-    double x, y, z;
-    double operator[](int i) const { return i == 0 ? x : (i == 1 ? y : z); }
-};
-inline H3 hsub(H3 a, H3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
-inline double hdot(H3 a, H3 b) { return (a.x * b.x + a.y * b.y) + a.z * b.z; }
-
 template <typename T>
 void upload(DevBuf<T>& d, const std::vector<T>& h, cudaStream_t s) {
     d.alloc(h.size());
@@ -253,57 +246,13 @@ void reorderMesh(Mesh& m, bool reverse) {
     setupDevice(m);
 }
 
-// LeastSquares::setPseudoInvMatrices (least_squares.cpp:12-61): pinv = (D^T D)^-1 D^T
+// LeastSquares::setPseudoInvMatrices (least_squares.cpp:12-61), once per mesh
 void Mesh::ensureLeastSquares() {
     if (ls_ready) return;
-    const HostMesh& H = *h;
-    const int64_t nk = (int64_t)H.cf_face.size();
-    std::vector<double> pinv(9 * (size_t)nc), w(3 * (size_t)nk, 0.0);
-    for (int c = 0; c < nc; ++c) {
-        double D[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-        H3 xc{H.cc[0][c], H.cc[1][c], H.cc[2][c]};
-        for (int64_t q = H.cf_off[c]; q < H.cf_off[c + 1]; ++q) {
-            int f = H.cf_face[q];
-            H3 r;
-            if (f >= nb) {
-                int o = H.owner[f];
-                int n = (o == c) ? H.nbr[f] : o;
-                r = hsub(H3{H.cc[0][n], H.cc[1][n], H.cc[2][n]}, xc);
-            } else {
-                r = hsub(H3{H.fc[0][f], H.fc[1][f], H.fc[2][f]}, xc);
-            }
-            double wk = 1 / (std::sqrt(hdot(r, r)) + EPSILON);
-            H3 wd{r.x * wk, r.y * wk, r.z * wk};
-            for (int i = 0; i < 3; ++i)
-                for (int j = 0; j < 3; ++j) D[i][j] += wd[i] * r[j];
-            w[q] = wd.x;
-            w[nk + q] = wd.y;
-            w[2 * nk + q] = wd.z;
-        }
-        double P[3][3];
-        for (int i = 0; i < 3; ++i)
-            for (int j = 0; j < 3; ++j) P[i][j] = (D[0][i] * D[0][j] + D[1][i] * D[1][j]) + D[2][i] * D[2][j];
-        double c00 = P[1][1] * P[2][2] - P[1][2] * P[2][1];
-        double c10 = P[1][2] * P[2][0] - P[1][0] * P[2][2];
-        double c20 = P[1][0] * P[2][1] - P[1][1] * P[2][0];
-        double det = (P[0][0] * c00 + P[0][1] * c10) + P[0][2] * c20;
-        double I[3][3];
-        I[0][0] = c00 / det;
-        I[1][0] = c10 / det;
-        I[2][0] = c20 / det;
-        I[0][1] = (P[0][2] * P[2][1] - P[0][1] * P[2][2]) / det;
-        I[1][1] = (P[0][0] * P[2][2] - P[0][2] * P[2][0]) / det;
-        I[2][1] = (P[0][1] * P[2][0] - P[0][0] * P[2][1]) / det;
-        I[0][2] = (P[0][1] * P[1][2] - P[0][2] * P[1][1]) / det;
-        I[1][2] = (P[0][2] * P[1][0] - P[0][0] * P[1][2]) / det;
-        I[2][2] = (P[0][0] * P[1][1] - P[0][1] * P[1][0]) / det;
-        for (int i = 0; i < 3; ++i)
-            for (int j = 0; j < 3; ++j)  // (I * D^T)(i,j) = sum_k I(i,k) D(j,k)
-                pinv[(3 * i + j) * (size_t)nc + c] = (I[i][0] * D[j][0] + I[i][1] * D[j][1]) + I[i][2] * D[j][2];
-    }
-    upload(ls_pinv, pinv, stream);
-    upload(ls_w, w, stream);
-    PB_CUDA(cudaStreamSynchronize(stream));
+    const int64_t nk = (int64_t)h->cf_face.size();
+    ls_pinv.alloc(9 * (size_t)nc);
+    ls_w.alloc(3 * (size_t)nk);
+    launchLeastSquaresOperators(view(), ls_pinv.p, ls_w.p, nk, stream);
     ls_ready = true;
 }
 
@@ -1281,7 +1230,7 @@ PrismSolveResult fromCtl(const SolveCtl& c) {
 // into one graph, launches it (updating the previous call's executable graph
 // in place when only parameters changed) and reads the solves' records back.
 int runAsGraph(Mesh& m, const std::function<void()>& f) {
-    // least-squares operators are built on the host at first use: build them now, outside the capture
+    // least-squares operators are allocated and built at first use: build them now, outside the capture
     m.ensureLeastSquares();
     if (!m.graph_ctl) m.graph_ctl.alloc(GRAPH_SLOTS);
     if (!m.graph_host) PB_CUDA(cudaMallocHost(&m.graph_host, GRAPH_SLOTS * sizeof(SolveCtl)));
