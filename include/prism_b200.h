@@ -124,10 +124,13 @@ extern "C" {
 #define PRISM_PREC_FP64 0  /* FP64 Krylov */
 #define PRISM_PREC_MIXED 1 /* FP32 BiCGSTAB (FP64 dots) with FP64 reliable updates */
 
-#define PRISM_PC_AUTO 0   /* library choice: AMG from PRISM_PC_AUTO_MIN_ROWS rows, Jacobi below */
+#define PRISM_PC_AUTO 0   /* library choice: AMG from PRISM_PC_AUTO_MIN_ROWS rows (PRISM_PC_AUTO_MIN_ROWS_SYM
+                             where the matrix is symmetric by construction: diffusion without convection),
+                             Jacobi below and for strongly diagonally dominant matrices */
 #define PRISM_PC_JACOBI 1 /* diagonal (column scaling), the cheapest iteration */
 #define PRISM_PC_AMG 2    /* aggregation AMG V-cycle; hierarchy kept per equation, values refreshed per solve */
-#define PRISM_PC_AUTO_MIN_ROWS 32768
+#define PRISM_PC_AUTO_MIN_ROWS 12288
+#define PRISM_PC_AUTO_MIN_ROWS_SYM 8192
 
 /* ---- handles ------------------------------------------------------------ */
 typedef struct PrismMesh PrismMesh;

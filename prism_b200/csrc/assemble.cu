@@ -376,26 +376,16 @@ void launchRelax(double* A, double* b, const int* diag_pos, const double* phi, d
     PB_LAUNCH("relax_kernel");
 }
 
-// reference-cell pin (numerics/solver.cpp:50-57)
-__global__ void pin_kernel(double* A, double* b, int pos, int row, double ref_value) {
-    double diag = A[pos];
-    A[pos] += diag;
-    b[row] += diag * ref_value;
-}
-void launchPin(double* A, double* b, int pos, int row, double ref_value, cudaStream_t s) {
-    pin_kernel<<<1, 1, 0, s>>>(A, b, pos, row, ref_value); countLaunch();
-    PB_LAUNCH("pin_kernel");
-}
-// the same, with the diagonal's position read on the device (for graph capture)
-__global__ void pin_dev_kernel(double* A, double* b, const int* diag_pos, int row, double ref_value) {
+// reference-cell pin (numerics/solver.cpp:50-57); the diagonal's position is read on the device
+__global__ void pin_kernel(double* A, double* b, const int* diag_pos, int row, double ref_value) {
     const int pos = diag_pos[row];
     double diag = A[pos];
     A[pos] += diag;
     b[row] += diag * ref_value;
 }
-void launchPinDev(double* A, double* b, const int* diag_pos, int row, double ref_value, cudaStream_t s) {
-    pin_dev_kernel<<<1, 1, 0, s>>>(A, b, diag_pos, row, ref_value); countLaunch();
-    PB_LAUNCH("pin_dev_kernel");
+void launchPin(double* A, double* b, const int* diag_pos, int row, double ref_value, cudaStream_t s) {
+    pin_kernel<<<1, 1, 0, s>>>(A, b, diag_pos, row, ref_value); countLaunch();
+    PB_LAUNCH("pin_kernel");
 }
 
 }  // namespace pb

@@ -841,7 +841,12 @@ API int prism_solve_csr(int64_t n, const int64_t* rowptr, const int64_t* col, co
             const bool fcg = o->method == PRISM_SOLVER_FCG;
             if (fcg && (o->precision != PRISM_PREC_FP64 || o->preconditioner == PRISM_PC_JACOBI))
                 fail(PRISM_BAD_ARG, "flexible CG runs in FP64 with the AMG preconditioner");
-            const bool use_amg = fcg || choosePreconditioner(o->preconditioner, n) == PRISM_PC_AMG;
+            // a hierarchy built for one solve pays later than one kept with an equation: the
+            // one-launch solve takes 9.7 ms at 26^3 rows, building and using AMG the same
+            constexpr int64_t ONE_OFF_AMG = 32768;
+            const bool use_amg = fcg || (o->preconditioner == PRISM_PC_AUTO
+                                             ? n >= ONE_OFF_AMG
+                                             : choosePreconditioner(o->preconditioner, n) == PRISM_PC_AMG);
             if (use_amg) {
                 std::vector<int> rp32(rowptr, rowptr + n + 1), col32(col, col + rowptr[n]);
                 d_rp.upload(rp32, s);

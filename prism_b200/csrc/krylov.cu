@@ -606,6 +606,12 @@ KrylovWork::~KrylovWork() {
     for (auto& g : graphs)
         if (g.exec) cudaGraphExecDestroy(g.exec);
     if (host_state) cudaFreeHost(host_state);
+    if (host_ctl) cudaFreeHost(host_ctl);
+}
+SolveCtl* KrylovWork::ctlRecord() {
+    if (!host_ctl) PB_CUDA(cudaMallocHost(&host_ctl, sizeof(SolveCtl)));
+    if (!ctl) ctl.alloc(sizeof(SolveCtl));
+    return reinterpret_cast<SolveCtl*>(ctl.p);
 }
 
 void spmv(const SellMatrix& A, const double* x, double* y, cudaStream_t s) {
@@ -975,9 +981,29 @@ bool fcgPre32(const Amg* amg) {
     return !p64 && amg->k_levels == 0;
 }
 
+const SolveCtl& runSmall(const SellMatrix& A, const double* b, double* x, long long n_iter, double eps, double tol,
+                         long long maxit, bool symmetric, KrylovWork& w, cudaStream_t s) {
+    SolveCtl* d = w.ctlRecord();
+    smallSolve(A, b, x, n_iter, eps, tol, maxit, symmetric, d, s);
+    PB_CUDA(cudaMemcpyAsync(w.host_ctl, d, sizeof(SolveCtl), cudaMemcpyDeviceToHost, s));
+    PB_CUDA(cudaStreamSynchronize(s));
+    if (verbose())
+        std::fprintf(stderr, "[prism] one-launch solve n=%d: %lld iterations, rel residual %.3e, status %d\n", A.n,
+                     w.host_ctl->krylov_iterations, w.host_ctl->krylov_rel, w.host_ctl->status);
+    return *w.host_ctl;
+}
+
 KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, int precision,
                    double inner_tol, KrylovWork& w, cudaStream_t s, Amg* amg, const int* rowptr, const int* col,
-                   bool flexible) {
+                   bool flexible, bool symmetric) {
+    if (!amg && smallSolveFits(A, maxit)) {
+        const SolveCtl& c = runSmall(A, b, x, 1, 0.0, tol, maxit, symmetric, w, s);
+        KrylovOut out;
+        out.iterations = c.krylov_iterations;
+        out.status = c.status;
+        out.rel_residual = c.krylov_rel;
+        return out;
+    }
     const bool mixed = precision == PRISM_PREC_MIXED;
     if (flexible && (mixed || !amg)) fail(PRISM_INTERNAL, "flexible CG runs FP64 with AMG only");
     const int mode = flexible ? fcgMode(amg, A) : KM_BICGSTAB;

@@ -31,6 +31,7 @@ int profBegin(int kind, bool fp32, double bytes, cudaStream_t s);
 void profEnd(int slot, cudaStream_t s);
 
 struct Amg;
+struct SolveCtl;
 
 // Device-resident solver state (one per BiCGSTAB run).
 struct KState {
@@ -59,6 +60,9 @@ struct KrylovWork {
     DevBuf<double> partials, scal;
     DevBuf<unsigned int> counter;
     DevBuf<KState> state;
+    DevBuf<unsigned char> ctl;        // SolveCtl of a one-launch solve, and its pinned copy
+    SolveCtl* host_ctl = nullptr;
+    SolveCtl* ctlRecord();            // device record (allocated on first use)
     KState* host_state = nullptr;  // pinned
     // one BiCGSTAB iteration captured as a CUDA graph, kept per operand set (key:
     // precision, matrix, vectors, preconditioner), least recently used last out
@@ -86,10 +90,11 @@ struct KrylovOut {
 // flexible: FP64 with amg only -- flexible conjugate gradients (Notay 2000, one
 // previous direction kept) preconditioned by amg->applyK(), for symmetric
 // positive (semi-)definite A (the pressure-correction equation), in place of
-// BiCGSTAB; same stopping rule, passes and statuses.
+// BiCGSTAB; same stopping rule, passes and statuses. symmetric: A is symmetric by construction
+// (the one-launch solve of a small system may then run conjugate gradients).
 KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, int precision,
                    double inner_tol, KrylovWork& w, cudaStream_t s, Amg* amg = nullptr, const int* rowptr = nullptr,
-                   const int* col = nullptr, bool flexible = false);
+                   const int* col = nullptr, bool flexible = false, bool symmetric = false);
 // flexible CG with amg preconditions with an FP32 V-cycle (else with the FP64 cycle)
 bool fcgPre32(const Amg* amg);
 // that V-cycle is smoothed aggregation's (samg.h)
@@ -122,6 +127,17 @@ struct SolveCtl {
     int phase, pass, restarts, kstatus;
     long long guard;  // controller passes of the current BiCGSTAB solve
 };
+
+// A whole ISolver::solve of a small system with Jacobi-preconditioned FP64 BiCGSTAB in one
+// launch (small.cu): the record lands in *out (device), x is updated in place. It fits up to
+// 32,768 rows; a cap beyond 2^20 iterations keeps to the ordinary path, whose launches stay short.
+bool smallSolveFits(const SellMatrix& A, long long maxit);
+void smallSolve(const SellMatrix& A, const double* b, double* x, long long n_iter, double eps, double tol,
+                long long maxit, bool symmetric, SolveCtl* out, cudaStream_t s);
+
+// the same, waited for: the record on the host (valid until the workspace's next solve)
+const SolveCtl& runSmall(const SellMatrix& A, const double* b, double* x, long long n_iter, double eps, double tol,
+                         long long maxit, bool symmetric, KrylovWork& w, cudaStream_t s);
 
 // Helper streams for the bodies of nested conditional nodes (one per depth).
 struct CaptureStreams {

@@ -479,8 +479,14 @@ void solveDefaults(PrismSolveOpts* o) {
     o->clear_coeffs = 1;
 }
 
-int choosePreconditioner(int pc, int64_t n) {
-    if (pc == PRISM_PC_AUTO) return n >= PRISM_PC_AUTO_MIN_ROWS ? PRISM_PC_AMG : PRISM_PC_JACOBI;
+// PRISM_PC_AUTO by size: AMG pays from where the one-launch Jacobi solve (small.cu) falls
+// behind it. Measured per solve, one-launch / multigrid: symmetric (conjugate gradients
+// against smoothed aggregation, 2-D Poisson) 64^2 rows 0.79 / 0.94 ms, 90^2 1.57 / 1.11,
+// 128^2 2.40 / 1.30; BiCGSTAB on 3-D MUSCL transport 18^3 3.56 / 3.17, 22^3 4.91 / 3.55, 26^3
+// 9.71 / 4.36, where building the hierarchy on a first solve costs another 4-5 ms.
+int choosePreconditioner(int pc, int64_t n, bool symmetric) {
+    if (pc == PRISM_PC_AUTO)
+        return n >= (symmetric ? PRISM_PC_AUTO_MIN_ROWS_SYM : PRISM_PC_AUTO_MIN_ROWS) ? PRISM_PC_AMG : PRISM_PC_JACOBI;
     if (pc != PRISM_PC_JACOBI && pc != PRISM_PC_AMG) fail(PRISM_BAD_ARG, "unknown preconditioner");
     return pc;
 }
@@ -509,16 +515,24 @@ static double autoJacobiRatio() {
     return v;
 }
 
+// The assembled matrix is symmetric: diffusion (one coefficient per face, in both rows),
+// with at most diagonal terms besides (time derivative, boundaries, relaxation, reference cell)
+static bool symmetricMatrix(const Transport& eq) { return eq.has_diff && !eq.has_conv && !eq.symmetry; }
+
 // preconditioner of a solve of eq (A: its assembled matrix); measures and records the
 // automatic choice on the first solve (a host round trip, never inside a capture)
 static int pcFor(Transport& eq, const PrismSolveOpts& o, const SellMatrix& A) {
-    const int c = choosePreconditioner(o.preconditioner, A.n);
+    const int c = choosePreconditioner(o.preconditioner, A.n, symmetricMatrix(eq));
     if (o.preconditioner != PRISM_PC_AUTO || c != PRISM_PC_AMG || eq.spd || autoJacobiRatio() <= 0.0) return c;
     if (eq.auto_pc == 0) {
         Mesh& m = *eq.phi->m;
         if (capturing(m.stream)) fail(PRISM_INTERNAL, "automatic preconditioner not chosen before capture");
         const double t = offDiagonalRatio(A, m.kw, m.stream);
-        eq.auto_pc = t <= autoJacobiRatio() ? PRISM_PC_JACOBI : PRISM_PC_AMG;
+        // a one-launch iteration costs a tenth of an AMG one: at those sizes Jacobi keeps every
+        // matrix that a time term or relaxation makes at all dominant (implicit convection-
+        // diffusion, 29,478 tetrahedra: 0.4 ms a solve against 1.4 ms)
+        const double limit = smallSolveFits(A, 1) ? std::max(autoJacobiRatio(), 0.98) : autoJacobiRatio();
+        eq.auto_pc = t <= limit ? PRISM_PC_JACOBI : PRISM_PC_AMG;
         if (verbose())
             std::fprintf(stderr, "[prism] automatic preconditioner of %s: %s (off-diagonal ratio %.3f)\n",
                          eq.phi->name.c_str(), eq.auto_pc == PRISM_PC_AMG ? "AMG" : "Jacobi", t);
@@ -526,15 +540,37 @@ static int pcFor(Transport& eq, const PrismSolveOpts& o, const SellMatrix& A) {
     return eq.auto_pc;
 }
 
-// FP64 AMG solves of an spd equation run flexible CG; PRISM_PRESSURE_SOLVER=bicgstab
-// keeps BiCGSTAB with the V-cycle for them
+// Transport::matrix_unchanged for one solve (cleared however the solve ends)
+struct MatrixUnchanged {
+    Transport& e;
+    MatrixUnchanged(Transport& t, bool on) : e(t) { e.matrix_unchanged = on; }
+    ~MatrixUnchanged() { e.matrix_unchanged = false; }
+};
+
+// set while a SIMPLE/PRIME/PISO step runs its solves
+static thread_local bool g_in_step = false;
+struct InStep {
+    bool before = g_in_step;
+    InStep() { g_in_step = true; }
+    ~InStep() { g_in_step = before; }
+};
+
+// AMG solves of the spd pressure correction run flexible CG (FP64 recurrences), and so do
+// those of a user's symmetric equation, which go back to BiCGSTAB should it fail
+// (symmetricFallback); PRISM_PRESSURE_SOLVER=bicgstab keeps BiCGSTAB with the V-cycle
 static bool flexibleFor(const Transport& eq, const PrismSolveOpts& o, const Amg* amg) {
     static const bool on = [] {
         const char* e = std::getenv("PRISM_PRESSURE_SOLVER");
         return !(e && std::strcmp(e, "bicgstab") == 0);
     }();
     if (o.method == PRISM_SOLVER_FCG) return true;
-    return on && eq.spd && amg && o.method == PRISM_SOLVER_BICGSTAB && o.precision == PRISM_PREC_FP64;
+    if (!on || !amg || o.method != PRISM_SOLVER_BICGSTAB) return false;
+    if (eq.spd) return o.precision == PRISM_PREC_FP64;
+    return symmetricMatrix(eq) && !eq.no_flex && !g_in_step;
+}
+// flexible CG stands in for the BiCGSTAB that was asked for
+static bool flexibleStandIn(const Transport& eq, const PrismSolveOpts& o, const Amg* amg) {
+    return flexibleFor(eq, o, amg) && o.method != PRISM_SOLVER_FCG && !eq.spd;
 }
 
 // PRISM_SOLVER_FCG's requirements: FP64, and the AMG preconditioner (its own choice
@@ -543,6 +579,24 @@ static void checkFcg(const PrismSolveOpts& o) {
     if (o.method != PRISM_SOLVER_FCG) return;
     if (o.precision != PRISM_PREC_FP64) fail(PRISM_BAD_ARG, "flexible CG runs in FP64 (precision PRISM_PREC_FP64)");
     if (o.preconditioner == PRISM_PC_JACOBI) fail(PRISM_BAD_ARG, "flexible CG needs the AMG preconditioner");
+}
+
+// One step on a matrix symmetric by construction: flexible CG; should it fail (an indefinite
+// matrix), BiCGSTAB from the same guess, as for any other matrix, then and from then on (failed).
+// The guess waits in r0, which flexible CG does not use.
+static KrylovOut symmetricSolve(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, Mesh& m,
+                                Amg* amg, bool& failed) {
+    KrylovWork& w = m.kw;
+    w.ensure(A.nslices * 32, A.nnz_padded, false);
+    PB_CUDA(cudaMemcpyAsync(w.r0.p, x, A.n * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
+    KrylovOut k = bicgstab(A, b, x, tol, maxit, PRISM_PREC_FP64, 0.1, w, m.stream, amg, m.pat.rowptr.p, m.pat.col.p, true);
+    if (k.status == PRISM_OK || (k.status == PRISM_NOT_CONVERGED && k.iterations >= maxit)) return k;
+    failed = true;
+    PB_CUDA(cudaMemcpyAsync(x, w.r0.p, A.n * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
+    amg->values_current = false;
+    KrylovOut f = bicgstab(A, b, x, tol, maxit, PRISM_PREC_FP64, 0.1, w, m.stream, amg, m.pat.rowptr.p, m.pat.col.p);
+    f.iterations += k.iterations;
+    return f;
 }
 
 namespace {
@@ -554,22 +608,24 @@ struct GraphCapture {
 thread_local GraphCapture* g_capture = nullptr;
 constexpr int GRAPH_SLOTS = 256;  // captured solves per graph
 PrismSolveResult solveCaptured(Transport& eq, const PrismSolveOpts& o);
+
+PrismSolveResult fromCtl(const SolveCtl& c) {
+    PrismSolveResult r{};
+    r.iterations = c.outer;
+    r.initial_residual = c.init_res;
+    r.final_residual = c.cur_res;
+    r.converged = c.converged;
+    r.status = c.status;
+    r.krylov_iterations = c.krylov_iterations;
+    r.krylov_rel_residual = c.krylov_rel;
+    return r;
+}
 }  // namespace
 
-// ISolver::solve (numerics/solver.cpp:27-82)
-PrismSolveResult solve(Transport& eq, const PrismSolveOpts& o) {
-    checkFcg(o);
-    if (g_capture) return solveCaptured(eq, o);
+// the steps of ISolver::solve on the assembled, relaxed and pinned system of eq
+static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o) {
     Scalar& phi = *eq.phi;
     Mesh& m = *phi.m;
-    updateCoeffs(eq);
-    relax(eq);
-    if (o.ref_cell >= 0 && o.ref_cell < m.nc) {
-        int pos = 0;
-        PB_CUDA(cudaMemcpyAsync(&pos, m.pat.diag_pos.p + o.ref_cell, sizeof(int), cudaMemcpyDeviceToHost, m.stream));
-        PB_CUDA(cudaStreamSynchronize(m.stream));
-        launchPin(eq.A.p, eq.b.p, pos, (int)o.ref_cell, o.ref_value, m.stream);
-    }
     SellMatrix A = m.matrix(eq.A.p);
     const double ktol = o.krylov_tol > 0 ? o.krylov_tol : 1e-12;
     const long long kmax = o.krylov_max_iter > 0 ? o.krylov_max_iter : 2LL * m.nc;
@@ -578,6 +634,12 @@ PrismSolveResult solve(Transport& eq, const PrismSolveOpts& o) {
     if (o.method == PRISM_SOLVER_FCG || (o.method != PRISM_SOLVER_JACOBI && pcFor(eq, o, A) == PRISM_PC_AMG)) {
         if (!eq.amg) eq.amg = std::make_shared<Amg>();
         amg = eq.amg.get();
+    }
+    if (o.method == PRISM_SOLVER_BICGSTAB && !amg && smallSolveFits(A, kmax)) {
+        const SolveCtl& c = runSmall(A, eq.b.p, phi.v.p, std::max<int64_t>(o.n_iter, 0), o.eps, ktol, kmax,
+                                     symmetricMatrix(eq), m.kw, m.stream);
+        phi.event += c.outer > 0 ? 1 + 3 * c.outer : 0;
+        return fromCtl(c);
     }
     PrismSolveResult r{};
     r.status = PRISM_OK;
@@ -594,8 +656,12 @@ PrismSolveResult solve(Transport& eq, const PrismSolveOpts& o) {
             jacobiStep(A, eq.b.p, phi.v.p, m.kw, m.stream);
         } else {
             const HoldAmgValues hold(amg, eq.matrix_unchanged || iter > 0);  // A is fixed within one solve
-            KrylovOut k = bicgstab(A, eq.b.p, phi.v.p, ktol, kmax, o.precision, itol, m.kw, m.stream, amg,
-                                   m.pat.rowptr.p, m.pat.col.p, flexibleFor(eq, o, amg));
+            KrylovOut k;
+            if (flexibleStandIn(eq, o, amg))
+                k = symmetricSolve(A, eq.b.p, phi.v.p, ktol, kmax, m, amg, eq.no_flex);
+            else
+                k = bicgstab(A, eq.b.p, phi.v.p, ktol, kmax, o.precision, itol, m.kw, m.stream, amg, m.pat.rowptr.p,
+                             m.pat.col.p, flexibleFor(eq, o, amg), symmetricMatrix(eq));
             r.krylov_iterations += k.iterations;
             r.krylov_rel_residual = k.rel_residual;
             if (k.status != PRISM_OK && r.status == PRISM_OK) r.status = k.status;
@@ -609,11 +675,25 @@ PrismSolveResult solve(Transport& eq, const PrismSolveOpts& o) {
             break;
         }
     }
-    if (o.clear_coeffs) zeroOutCoeffs(eq);
     r.iterations = iter;
     r.initial_residual = init_res;
     r.final_residual = cur;
     r.converged = conv ? 1 : 0;
+    return r;
+}
+
+// ISolver::solve (numerics/solver.cpp:27-82)
+PrismSolveResult solve(Transport& eq, const PrismSolveOpts& o) {
+    checkFcg(o);
+    if (g_capture) return solveCaptured(eq, o);
+    Scalar& phi = *eq.phi;
+    Mesh& m = *phi.m;
+    updateCoeffs(eq);
+    relax(eq);
+    if (o.ref_cell >= 0 && o.ref_cell < m.nc)
+        launchPin(eq.A.p, eq.b.p, m.pat.diag_pos.p, (int)o.ref_cell, o.ref_value, m.stream);
+    PrismSolveResult r = solveAssembled(eq, o);
+    if (o.clear_coeffs) zeroOutCoeffs(eq);
     return r;
 }
 
@@ -813,11 +893,7 @@ PressureResult solvePressureEquation(PrismSIMPLEControls c, std::vector<Transpor
         PhaseTimer pt("pressure corrector " + std::to_string(i), m.stream);
         // the correctors re-assemble the same matrix (D and the mesh are fixed; only the
         // explicit non-orthogonal part of b changes)
-        struct Unchanged {
-            Transport& e;
-            Unchanged(Transport& t, bool on) : e(t) { e.matrix_unchanged = on; }
-            ~Unchanged() { e.matrix_unchanged = false; }
-        } unchanged(pEqn, i > 0);
+        const MatrixUnchanged unchanged(pEqn, i > 0);
         auto r = solve(pEqn, inner(so, c.pressure_max_iter, c.pressure_residual, c.p_ref_cell, c.p_ref_value, true));
         rep.push_back({pp->name + "_corr_" + std::to_string(i), r.iterations, r.initial_residual, r.final_residual,
                        r.converged != 0});
@@ -864,6 +940,7 @@ void simpleStep(const PrismSIMPLEControls& c, std::vector<Transport*>& mom, Vect
                 const PrismSolveOpts& so, std::vector<Report>& rep) {
     if (mom.size() != 2 && mom.size() != 3) fail(PRISM_BAD_ARG, "SIMPLE expects 2 or 3 momentum predictors");
     PhaseTimer pt("SIMPLE step", p.m->stream);
+    const InStep in_step;
     solveImplicitMomentum(c, mom, so, rep);
     auto r = solvePressureEquation(c, mom, U, mdot, p, so, rep);
     PhaseTimer pc("correct fields", p.m->stream);
@@ -873,6 +950,7 @@ void simpleStep(const PrismSIMPLEControls& c, std::vector<Transport*>& mom, Vect
 void primeStep(const PrismSIMPLEControls& pc, std::vector<Transport*>& mom, Vector& U, Vector& mdot, Scalar& p,
                const PrismSolveOpts& so, std::vector<Report>& rep) {
     if (mom.size() != 2 && mom.size() != 3) fail(PRISM_BAD_ARG, "PRIME expects 2 or 3 momentum predictors");
+    const InStep in_step;
     solveExplicitMomentum(mom);
     PrismSIMPLEControls c;
     simpleDefaults(&c);
@@ -920,6 +998,8 @@ FixedPointOut steadySolve(Transport& eq, const PrismSolveOpts& o, int max_outer,
     double h[2];
     for (int it = 0; it < max_outer; ++it) {
         PB_CUDA(cudaMemcpyAsync(prev.p, phi.v.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
+        // without convection and time terms the matrix does not depend on phi
+        const MatrixUnchanged unchanged(eq, it > 0 && symmetricMatrix(eq) && !eq.has_temporal);
         PrismSolveResult r = solve(eq, o);
         out.krylov += r.krylov_iterations;
         ++out.outer;
@@ -993,7 +1073,7 @@ FixedPointOut adjointBackward(Transport& eq, const double* dJ, double* gk, doubl
     d_dJ.upload(dJ, m.nc, s);
 
     Amg* amg = nullptr;
-    if (choosePreconditioner(o.preconditioner, m.nc) == PRISM_PC_AMG) {
+    if (choosePreconditioner(o.preconditioner, m.nc, true) == PRISM_PC_AMG) {  // diffusion only: A^T = A
         if (!eq.amg_adj) eq.amg_adj = std::make_shared<Amg>();
         amg = eq.amg_adj.get();
     }
@@ -1004,8 +1084,11 @@ FixedPointOut adjointBackward(Transport& eq, const double* dJ, double* gk, doubl
         adjointCorrection(P, lam.p, u.p, d.p, np, s);
         adjointRhs(P, d_dJ.p, lam.p, u.p, d.p, np, rhs.p, s);
         PB_CUDA(cudaMemcpyAsync(lam_prev.p, lam.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        KrylovOut k = bicgstab(AT, rhs.p, lam.p, ktol, kmax, PRISM_PREC_FP64, 0.1, m.kw, s, amg, m.pat.rowptr.p,
-                               m.pat.col.p);
+        const HoldAmgValues hold(amg, it > 0);
+        KrylovOut k = amg && !eq.no_flex
+                          ? symmetricSolve(AT, rhs.p, lam.p, ktol, kmax, m, amg, eq.no_flex)
+                          : bicgstab(AT, rhs.p, lam.p, ktol, kmax, PRISM_PREC_FP64, 0.1, m.kw, s, amg, m.pat.rowptr.p,
+                                     m.pat.col.p, false, true);
         out.krylov += k.iterations;
         ++out.outer;
         if (k.status != PRISM_OK && out.status == PRISM_OK) out.status = k.status;
@@ -1181,7 +1264,7 @@ PrismSolveResult solveCaptured(Transport& eq, const PrismSolveOpts& o) {
     updateCoeffs(eq);
     relax(eq);
     if (o.ref_cell >= 0 && o.ref_cell < m.nc)
-        launchPinDev(eq.A.p, eq.b.p, m.pat.diag_pos.p, (int)o.ref_cell, o.ref_value, s);
+        launchPin(eq.A.p, eq.b.p, m.pat.diag_pos.p, (int)o.ref_cell, o.ref_value, s);
     SellMatrix A = m.matrix(eq.A.p);
     const double ktol = o.krylov_tol > 0 ? o.krylov_tol : 1e-12;
     const long long kmax = o.krylov_max_iter > 0 ? o.krylov_max_iter : 2LL * m.nc;
@@ -1191,6 +1274,18 @@ PrismSolveResult solveCaptured(Transport& eq, const PrismSolveOpts& o) {
         amg = eq.amg.get();
     }
     const long long n_iter = std::max<long long>(o.n_iter, 0);
+    // a stand-in's guess is kept in case it fails (solveAsGraph, which then needs the system too)
+    const bool stand_in = flexibleStandIn(eq, o, amg);
+    if (stand_in)
+        PB_CUDA(cudaMemcpyAsync(m.kw.r0.p, phi.v.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    if (o.method == PRISM_SOLVER_BICGSTAB && !amg && smallSolveFits(A, kmax)) {
+        smallSolve(A, eq.b.p, phi.v.p, n_iter, o.eps, ktol, kmax, symmetricMatrix(eq), ctl, s);
+        if (n_iter > 0) phi.event += 4;
+        if (o.clear_coeffs) zeroOutCoeffs(eq);
+        PrismSolveResult r{};
+        r.iterations = -(slot + 1);
+        return r;
+    }
     cudaGraphConditionalHandle outer = createConditional(s, 0);
     emitSolveBegin(ctl, n_iter, o.eps, kmax, ktol, outer, s);
     if (n_iter > 0) {
@@ -1208,21 +1303,9 @@ PrismSolveResult solveCaptured(Transport& eq, const PrismSolveOpts& o) {
         emitOuterStep(ctl, m.kw, outer, body);
         endConditional(body);
     }
-    if (o.clear_coeffs) zeroOutCoeffs(eq);
+    if (o.clear_coeffs && !stand_in) zeroOutCoeffs(eq);
     PrismSolveResult r{};
     r.iterations = -(slot + 1);  // the device record of this solve, read after the launch
-    return r;
-}
-
-PrismSolveResult fromCtl(const SolveCtl& c) {
-    PrismSolveResult r{};
-    r.iterations = c.outer;
-    r.initial_residual = c.init_res;
-    r.final_residual = c.cur_res;
-    r.converged = c.converged;
-    r.status = c.status;
-    r.krylov_iterations = c.krylov_iterations;
-    r.krylov_rel_residual = c.krylov_rel;
     return r;
 }
 
@@ -1284,13 +1367,16 @@ bool graphReady(const Transport& eq, const PrismSolveOpts& o) {
     const Mesh& m = *eq.phi->m;
     if ((o.method != PRISM_SOLVER_BICGSTAB && o.method != PRISM_SOLVER_FCG) || o.precision != PRISM_PREC_FP64)
         return false;
-    if (!eq.A || !eq.b || m.kw.n != m.n_pad) return false;
-    int pc = o.method == PRISM_SOLVER_FCG ? PRISM_PC_AMG : choosePreconditioner(o.preconditioner, m.nc);
+    if (!eq.A || !eq.b) return false;
+    int pc = o.method == PRISM_SOLVER_FCG ? PRISM_PC_AMG : choosePreconditioner(o.preconditioner, m.nc, symmetricMatrix(eq));
+    const long long kmax = o.krylov_max_iter > 0 ? o.krylov_max_iter : 2LL * m.nc;
     if (o.method != PRISM_SOLVER_FCG && o.preconditioner == PRISM_PC_AUTO && pc == PRISM_PC_AMG && !eq.spd &&
         autoJacobiRatio() > 0.0) {
         if (eq.auto_pc == 0) return false;  // chosen on an ordinary solve first
         pc = eq.auto_pc;
     }
+    if (pc == PRISM_PC_JACOBI && smallSolveFits(m.matrix(eq.A.p), kmax)) return true;
+    if (m.kw.n != m.n_pad) return false;
     if (pc == PRISM_PC_AMG) {
         if (!eq.amg || !m.kw.y) return false;
         if (flexibleFor(eq, o, eq.amg.get()) && fcgSmoothed(eq.amg.get(), m.matrix(eq.A.p)))
@@ -1311,6 +1397,7 @@ bool graphReady(const Transport& eq, const PrismSolveOpts& o) {
 bool stepGraphReady(const std::vector<Transport*>& mom, const Vector& U, const Scalar& p, const PrismSolveOpts& so,
                     bool momentum_solved) {
     const Mesh& m = *p.m;
+    const InStep in_step;
     for (auto* eq : mom) {
         if (momentum_solved && !graphReady(*eq, so)) return false;
         if (!eq->A || !eq->b) return false;
@@ -1325,7 +1412,17 @@ PrismSolveResult solveAsGraph(Transport& eq, const PrismSolveOpts& o) {
     PrismSolveResult out{};
     const int used = runAsGraph(m, [&] { out = solve(eq, o); });
     if (used != 1) fail(PRISM_INTERNAL, "graph solve recorded no solve");
-    return fromCtl(m.graph_host[0]);
+    out = fromCtl(m.graph_host[0]);
+    if (flexibleStandIn(eq, o, eq.amg.get()) && pcFor(eq, o, m.matrix(eq.A.p)) == PRISM_PC_AMG) {
+        if (out.status != PRISM_OK && !(out.status == PRISM_NOT_CONVERGED && out.krylov_iterations >= m.graph_host[0].kmax)) {
+            eq.no_flex = true;
+            eq.amg->values_current = false;
+            PB_CUDA(cudaMemcpyAsync(eq.phi->v.p, m.kw.r0.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
+            out = solveAssembled(eq, o);
+        }
+        if (o.clear_coeffs) zeroOutCoeffs(eq);
+    }
+    return out;
 }
 
 void stepAsGraph(Mesh& m, const std::function<void()>& step, std::vector<Report>& rep) {

@@ -143,6 +143,9 @@ struct Transport {
     // PRISM_PC_AUTO at AMG sizes, decided on the equation's first solve: Jacobi when
     // its matrix is diagonally dominant enough (offDiagonalRatio), else AMG (0: not yet)
     int auto_pc = 0;
+    // flexible CG failed on this symmetric equation (an indefinite matrix: negative
+    // diffusivities): it keeps BiCGSTAB
+    bool no_flex = false;
     // the next solves assemble the same matrix as the last one (only b changes):
     // its AMG hierarchy keeps its values
     bool matrix_unchanged = false;
@@ -224,6 +227,6 @@ void simpleDefaults(PrismSIMPLEControls* c);
 void pisoDefaults(PrismPISOControls* c);
 void solveDefaults(PrismSolveOpts* o);
 // PRISM_PC_AUTO resolved for an n-row system
-int choosePreconditioner(int pc, int64_t n);
+int choosePreconditioner(int pc, int64_t n, bool symmetric = false);
 
 }  // namespace pb

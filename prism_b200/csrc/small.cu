@@ -1,0 +1,450 @@
+// small.cu -- a whole ISolver::solve of a small system in one launch of one thread-block
+// cluster: the scaled residuals, the outer steps, and in each of them Jacobi-preconditioned
+// BiCGSTAB with its restarts and accurate-residual passes (bicgstab() in krylov.cu, whose
+// control flow and statuses these are).
+//
+// Systems of a few thousand rows are bound by launches, not by bytes: an iteration as five
+// kernels takes 17 us whatever the size (32^2 to 31^3 rows), and a solve that has nothing to
+// do still 130 us. Here a thread owns two or four rows: their vectors stay in registers, the
+// matrix in L1, and only the two preconditioned directions pass through shared memory, read
+// by the cluster's other blocks as distributed shared memory. An iteration is five barriers,
+// three of them carrying a reduction (each block sends its partial sums to every other block
+// before it arrives, and all add them in block order, so results repeat bit for bit).
+#include <cooperative_groups.h>
+
+#include <cmath>
+
+#include "krylov.h"
+
+namespace cg = cooperative_groups;
+
+namespace pb {
+
+namespace {
+
+constexpr int MAX_CTAS = 16;
+constexpr int NV = 5;  // values of one reduction, at most
+
+struct SmallParams {
+    int n;
+    const int* sl_off;
+    const int* col;
+    const double* vals;
+    const int* diag_pos;
+    const double* b;
+    double* x;
+    long long n_iter, maxit;
+    double eps, tol;
+    int symmetric;  // the matrix is symmetric by construction
+    SolveCtl* out;
+};
+
+// THREADS threads of K rows each per block; CL: more than one block
+template <int THREADS, int K, bool CL>
+__global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallParams P) {
+    constexpr int ROWS = THREADS * K;  // rows per block
+    __shared__ double ph[ROWS], sh[ROWS];  // the gathered vectors: M^-1 p (or x), M^-1 s
+    constexpr int NW = THREADS / 32;
+    __shared__ double red[2][NV][NW];
+    __shared__ double xch[2][MAX_CTAS][NV];
+    cg::cluster_group cl = cg::this_cluster();
+    const int ctas = CL ? (int)cl.num_blocks() : 1, rank = CL ? (int)cl.block_rank() : 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int parity = 0;
+
+    auto barrier = [&] {
+        if constexpr (CL) cl.sync();
+        else __syncthreads();
+    };
+    // sums (or maxima of magnitudes) of v over all rows, in every thread; also a barrier.
+    // The buffers alternate: the next reduction never writes what a slow thread still reads.
+    auto reduce = [&](auto count, bool maxima, double (&v)[NV]) {
+        constexpr int N = decltype(count)::value;
+        auto join = [&](double a, double c) { return maxima ? fmax(a, c) : a + c; };
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int k = 0; k < N; ++k) v[k] = join(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+        if (lane == 0)
+#pragma unroll
+            for (int k = 0; k < N; ++k) red[parity][k][warp] = v[k];
+        __syncthreads();
+        if constexpr (!CL) {
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                double u[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+                for (int w = 0; w < NW; ++w) u[w & 3] = join(u[w & 3], red[parity][k][w]);
+                v[k] = join(join(u[0], u[1]), join(u[2], u[3]));
+            }
+        } else {
+            if (warp == 0) {
+                double u[N];
+#pragma unroll
+                for (int k = 0; k < N; ++k) u[k] = red[parity][k][lane % NW];
+#pragma unroll
+                for (int o = NW / 2; o > 0; o >>= 1)
+#pragma unroll
+                    for (int k = 0; k < N; ++k) u[k] = join(u[k], __shfl_xor_sync(0xffffffffu, u[k], o));
+                if (lane < ctas) {
+                    double* to = cl.map_shared_rank(&xch[parity][rank][0], lane);
+#pragma unroll
+                    for (int k = 0; k < N; ++k) to[k] = u[k];
+                }
+            }
+            barrier();
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                double u = xch[parity][0][k];
+                for (int c = 1; c < ctas; ++c) u = join(u, xch[parity][c][k]);
+                v[k] = u;
+            }
+        }
+        parity ^= 1;
+    };
+    using One = std::integral_constant<int, 1>;
+    using Two = std::integral_constant<int, 2>;
+    using Three = std::integral_constant<int, 3>;
+    using Five = std::integral_constant<int, 5>;
+
+    int row[K], at[K], width[K];
+    double dinv[K], x[K], r[K], r0[K], p[K], v[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        row[k] = rank * ROWS + k * THREADS + threadIdx.x;
+        const bool in = row[k] < P.n;
+        const int s0 = in ? P.sl_off[row[k] >> 5] : 0;
+        width[k] = in ? (P.sl_off[(row[k] >> 5) + 1] - s0) >> 5 : 0;
+        at[k] = s0 + (row[k] & 31);
+        const double d = in ? P.vals[P.diag_pos[row[k]]] : 1.0;
+        dinv[k] = d != 0.0 ? 1.0 / d : 1.0;
+        x[k] = in ? P.x[row[k]] : 0.0;
+        r[k] = r0[k] = p[k] = v[k] = 0.0;
+    }
+    auto rhs = [&](int k) { return row[k] < P.n ? __ldg(P.b + row[k]) : 0.0; };
+    auto own = [&](int k) { return k * THREADS + (int)threadIdx.x; };
+    auto gather = [&](double* a, int j) -> double {
+        if constexpr (CL) return *cl.map_shared_rank(a + (j & (ROWS - 1)), j / ROWS);
+        else return a[j];
+    };
+    // (A y)_row with y spread over the blocks' shared array a; up to 4 entries in flight
+    auto rowOf = [&](int k, double* a) {
+        double sum = 0.0;
+        for (int j0 = 0; j0 < width[k]; j0 += 4) {
+            int c[4];
+            double m[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j0 + j < width[k]) {
+                    c[j] = __ldg(P.col + at[k] + 32 * (j0 + j));
+                    m[j] = __ldg(P.vals + at[k] + 32 * (j0 + j));
+                }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j0 + j < width[k]) sum += m[j] * gather(a, c[j]);
+        }
+        return sum;
+    };
+    // ax := A x
+    double ax[K];
+    auto applyToX = [&] {
+#pragma unroll
+        for (int k = 0; k < K; ++k) ph[own(k)] = x[k];
+        barrier();
+#pragma unroll
+        for (int k = 0; k < K; ++k) ax[k] = row[k] < P.n ? rowOf(k, ph) : 0.0;
+    };
+    // max|A x - b| / (max|diag x| + eps) from ax; NaN if a term is not finite
+    auto scaledResidual = [&] {
+        double m[NV] = {};
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            if (row[k] >= P.n) continue;
+            const double e = fabs(ax[k] - rhs(k)), d = fabs(P.vals[P.diag_pos[row[k]]] * x[k]);
+            if (!isfinite(e) || !isfinite(d)) {
+                m[2] = 1.0;
+            } else {
+                m[0] = fmax(m[0], e);
+                m[1] = fmax(m[1], d);
+            }
+        }
+        reduce(Three{}, true, m);
+        return m[2] != 0.0 ? __longlong_as_double(0x7ff8000000000000LL) : m[0] / (m[1] + EPSILON);
+    };
+
+    double init_res = 0.0, cur_res = 0.0, krylov_rel = 0.0;
+    int status = PRISM_OK, converged = 0;
+    long long outer = 0, total = 0;
+    if (P.n_iter > 0) {
+        applyToX();
+        init_res = scaledResidual();
+    }
+    // conjugate gradients where the matrix is symmetric and, by its signs and row sums,
+    // positive semi-definite: half the products and a third of the reductions of BiCGSTAB
+    bool cg_ok = P.symmetric != 0;
+    if (cg_ok && P.n_iter > 0) {
+        double bad[NV] = {};
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            double sum = 0.0, d = 0.0;
+            for (int j = 0; j < width[k]; ++j) {
+                const double a = __ldg(P.vals + at[k] + 32 * j);
+                if (__ldg(P.col + at[k] + 32 * j) == row[k]) d += a;
+                else if (a > 0.0) bad[0] = 1.0;
+                sum += a;
+            }
+            if (row[k] < P.n && !(d > 0.0 && sum >= -1e-12 * d)) bad[0] = 1.0;
+        }
+        reduce(One{}, true, bad);
+        cg_ok = bad[0] == 0.0;
+    }
+    while (outer < P.n_iter) {
+        long long left = P.maxit;
+        int kstatus = PRISM_OK;
+        for (int pass = 0; pass < 4; ++pass) {
+            long long iter = 0;
+            int restarts = 0, done = 0;
+            kstatus = PRISM_OK;
+            while (true) {
+                applyToX();
+                double d[NV] = {};
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    const double bk = rhs(k);
+                    r[k] = r0[k] = bk - ax[k];
+                    p[k] = v[k] = 0.0;
+                    d[0] += r[k] * r[k];
+                    d[1] += bk * bk;
+                }
+                reduce(Two{}, false, d);
+                const double r0sq = d[0], tol2 = P.tol * P.tol * d[1];
+                double rho = d[0], beta = d[0], w = 1.0;
+                long long iter_cg = 0;
+                done = !isfinite(d[0]) || !isfinite(d[1]) ? 5 : d[1] == 0.0 ? 4 : d[0] <= tol2 ? 1 : 0;
+                if (cg_ok) {
+                    // Chronopoulos and Gear 1989: one reduction per iteration; q = A p is carried in v
+                    double gamma_old = 1.0, alpha = 1.0;
+                    beta = 0.0;
+                    while (done == 0) {
+                        double z[K], az[K];
+#pragma unroll
+                        for (int k = 0; k < K; ++k) {
+                            z[k] = dinv[k] * r[k];
+                            ph[own(k)] = z[k];
+                        }
+                        barrier();
+                        d[0] = d[1] = d[2] = 0.0;
+#pragma unroll
+                        for (int k = 0; k < K; ++k) {
+                            az[k] = rowOf(k, ph);
+                            d[0] += r[k] * z[k];
+                            d[1] += az[k] * z[k];
+                            d[2] += r[k] * r[k];
+                        }
+                        reduce(Three{}, false, d);
+                        if (!isfinite(d[0]) || !isfinite(d[1]) || !isfinite(d[2])) done = 5;
+                        else if (d[2] <= tol2) done = 1;
+                        else if (iter >= left) done = 2;
+                        if (done) break;
+                        beta = iter_cg > 0 ? d[0] / gamma_old : 0.0;
+                        const double pq = d[1] - (iter_cg > 0 ? beta * d[0] / alpha : 0.0);
+                        alpha = d[0] / pq;
+                        if (!(pq > 0.0) || !isfinite(alpha)) {
+                            done = 3;
+                            cg_ok = false;
+                            break;
+                        }
+                        gamma_old = d[0];
+#pragma unroll
+                        for (int k = 0; k < K; ++k) {
+                            p[k] = z[k] + beta * p[k];
+                            v[k] = az[k] + beta * v[k];
+                            x[k] += alpha * p[k];
+                            r[k] -= alpha * v[k];
+                        }
+                        ++iter_cg;
+                        ++iter;
+                    }
+                }
+                while (done == 0) {
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        p[k] = r[k] + beta * (p[k] - w * v[k]);
+                        ph[own(k)] = dinv[k] * p[k];
+                    }
+                    barrier();
+                    d[0] = 0.0;
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        v[k] = rowOf(k, ph);
+                        d[0] += r0[k] * v[k];
+                    }
+                    reduce(One{}, false, d);
+                    const double alpha = rho / d[0];
+                    if (d[0] == 0.0 || !isfinite(alpha)) {  // breakdown: restart from the current x
+                        done = isfinite(d[0]) ? 3 : 5;
+                        break;
+                    }
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        r[k] -= alpha * v[k];  // s
+                        sh[own(k)] = dinv[k] * r[k];
+                    }
+                    barrier();
+                    // t = A M^-1 s; the dots of r = s - w t follow from those of s and t, so the
+                    // update needs no reduction of its own
+                    double t[K];
+                    d[0] = d[1] = d[2] = d[3] = d[4] = 0.0;
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        t[k] = rowOf(k, sh);
+                        d[0] += t[k] * r[k];
+                        d[1] += t[k] * t[k];
+                        d[2] += r0[k] * r[k];
+                        d[3] += r0[k] * t[k];
+                        d[4] += r[k] * r[k];
+                    }
+                    reduce(Five{}, false, d);
+                    w = d[1] > 0.0 ? d[0] / d[1] : 0.0;
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        x[k] += alpha * (dinv[k] * p[k]) + w * (dinv[k] * r[k]);
+                        r[k] -= w * t[k];
+                    }
+                    ++iter;
+                    const double rho_new = d[2] - w * d[3], rr = d[4] - w * d[0];
+                    if (!isfinite(rho_new) || !isfinite(rr)) done = 5;
+                    else if (rr <= tol2) done = 1;
+                    else if (iter >= left) done = 2;
+                    else if (w == 0.0 || fabs(rho_new) < EPSILON * EPSILON * r0sq) done = 3;
+                    else {
+                        beta = (rho_new / rho) * (alpha / w);
+                        rho = rho_new;
+                    }
+                }
+                if (done != 3) break;
+                if (++restarts > 20) {
+                    kstatus = PRISM_BREAKDOWN;
+                    break;
+                }
+            }
+            if (done == 2) kstatus = PRISM_NOT_CONVERGED;
+            if (done == 5) kstatus = PRISM_NONFINITE;
+            if (done == 4) {  // b = 0: x = 0
+#pragma unroll
+                for (int k = 0; k < K; ++k) x[k] = 0.0;
+            }
+            total += iter;
+            left -= iter;
+            // accurate residual: the recursive one drifts from b - A x
+            applyToX();
+            double d[NV] = {};
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const double bk = rhs(k), e = bk - ax[k];
+                d[0] += e * e;
+                d[1] += bk * bk;
+            }
+            reduce(Two{}, false, d);
+            krylov_rel = d[1] > 0 ? sqrt(d[0] / d[1]) : 0.0;
+            if (kstatus != PRISM_OK || krylov_rel <= 10 * P.tol || left <= 0 || d[1] == 0) break;
+        }
+        cur_res = scaledResidual();
+        ++outer;
+        if (kstatus != PRISM_OK && status == PRISM_OK) status = kstatus;
+        if (isnan(cur_res)) status = PRISM_NONFINITE;
+        if (cur_res < P.eps) {
+            converged = 1;
+            break;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (row[k] < P.n) P.x[row[k]] = x[k];
+    if (rank == 0 && threadIdx.x == 0) {
+        SolveCtl z{};
+        z.n_iter = P.n_iter;
+        z.outer = outer;
+        z.eps = P.eps;
+        z.init_res = init_res;
+        z.cur_res = cur_res;
+        z.converged = converged;
+        z.status = status;
+        z.kmax = P.maxit;
+        z.krylov_iterations = total;
+        z.tol = P.tol;
+        z.krylov_rel = krylov_rel;
+        *P.out = z;
+    }
+}
+
+// largest cluster the device places (16 is a non-portable size; 8 is always allowed)
+template <int T, int K>
+bool placed() {
+    auto kernel = small_solve_kernel<T, K, true>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return false;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(MAX_CTAS);
+    cfg.blockDim = dim3(T);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = MAX_CTAS;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    return cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n >= 1;
+}
+int maxCtas() {
+    static const int c = [] {
+        const bool ok = placed<256, 1>() && placed<512, 2>() && placed<512, 4>();
+        cudaGetLastError();  // a refused query leaves no sticky error
+        return ok ? MAX_CTAS : 8;
+    }();
+    return c;
+}
+
+template <int T, int K>
+void launchSmall(const SmallParams& P, cudaStream_t s) {
+    const int ctas = ceil_div(P.n, T * K);
+    if (ctas == 1) {
+        small_solve_kernel<T, K, false><<<1, T, 0, s>>>(P);
+        return;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(T);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    PB_CUDA(cudaLaunchKernelEx(&cfg, small_solve_kernel<T, K, true>, P));
+}
+
+}  // namespace
+
+bool smallSolveFits(const SellMatrix& A, long long maxit) {
+    return A.n > 0 && A.n <= maxCtas() * 2048 && maxit <= (1LL << 20);
+}
+
+// Rows per block: one block up to 1,024 rows, whose barriers cost a fraction of a cluster's;
+// then as few rows per block as 16 blocks allow.
+void smallSolve(const SellMatrix& A, const double* b, double* x, long long n_iter, double eps, double tol,
+                long long maxit, bool symmetric, SolveCtl* out, cudaStream_t s) {
+    const SmallParams P{A.n, A.sl_off, A.col, A.vals, A.diag_pos, b, x, n_iter, maxit, eps, tol, symmetric ? 1 : 0, out};
+    const int max = maxCtas();
+    if (A.n <= 256) launchSmall<256, 1>(P, s);
+    else if (A.n <= 1024) launchSmall<512, 2>(P, s);
+    else if (A.n <= max * 256) launchSmall<256, 1>(P, s);
+    else if (A.n <= max * 1024) launchSmall<512, 2>(P, s);
+    else launchSmall<512, 4>(P, s);
+    countLaunch();
+    PB_LAUNCH("small_solve_kernel");
+}
+
+}  // namespace pb
