@@ -107,10 +107,10 @@ __device__ __forceinline__ T sliceRow(const int* __restrict__ col, const T* __re
     return sum;
 }
 
-template <typename T, int STAGE, int W = 8, int MINB = 5>
+template <typename T, int STAGE, int W = 8, int MINB = 5, typename TX = T>
 __global__ void __launch_bounds__(BS, MINB) spmv_kernel(int nslices, int n, const int* __restrict__ sl_off,
                                                   const int* __restrict__ col, const T* __restrict__ val,
-                                                  const T* __restrict__ x, T* __restrict__ y,
+                                                  const TX* __restrict__ x, T* __restrict__ y,
                                                   const T* __restrict__ u, double* partials,
                                                   unsigned int* counter, KState* S) {
     pdlEnter();
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(BS, MINB) spmv_kernel(int nslices, int n, cons
     for (int sl = blockIdx.x * WARPS + warp; sl < nslices; sl += gridDim.x * WARPS) {
         const int b = sl_off[sl];
         const int width = (sl_off[sl + 1] - b) >> 5;
-        const T sum = sliceRow<T, W>(col, val, x, b, width, lane);
+        const T sum = sliceRow<T, W, TX>(col, val, x, b, width, lane);
         const int r = sl * 32 + lane;
         y[r] = sum;
         if (STAGE != 0 && r < n) {
@@ -145,30 +145,37 @@ __global__ void __launch_bounds__(BS, MINB) spmv_kernel(int nslices, int n, cons
     }
 }
 
+// c32 (optional): the FP32 copy that an FP32 preconditioner of an FP64 iteration reads
 template <typename T>
 __global__ void __launch_bounds__(BS) p_kernel(int n, T* __restrict__ p, const T* __restrict__ r,
-                                               const T* __restrict__ v, const KState* S) {
+                                               const T* __restrict__ v, float* __restrict__ c32, const KState* S) {
     pdlEnter();
     if (S->done) return;
     const double beta = S->beta, w = S->w;
-    for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS)
-        p[i] = (T)((double)r[i] + beta * ((double)p[i] - w * (double)v[i]));
+    for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
+        const T pi = (T)((double)r[i] + beta * ((double)p[i] - w * (double)v[i]));
+        p[i] = pi;
+        if (c32) c32[i] = (float)pi;
+    }
 }
 
 template <typename T>
 __global__ void __launch_bounds__(BS) s_kernel(int n, T* __restrict__ s, const T* __restrict__ r,
-                                               const T* __restrict__ v, const KState* S) {
+                                               const T* __restrict__ v, float* __restrict__ c32, const KState* S) {
     pdlEnter();
     if (S->done) return;
     const double alpha = S->alpha;
-    for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS)
-        s[i] = (T)((double)r[i] - alpha * (double)v[i]);
+    for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
+        const T si = (T)((double)r[i] - alpha * (double)v[i]);
+        s[i] = si;
+        if (c32) c32[i] = (float)si;
+    }
 }
 
 // x += alpha p + w q ; r = s - w t  (q = s without a preconditioner pass, else q = M^-1 s, p = M^-1 p)
-template <typename T>
-__global__ void __launch_bounds__(BS) xr_kernel(int n, T* __restrict__ x, T* __restrict__ r, const T* __restrict__ p,
-                                                const T* __restrict__ q, const T* __restrict__ s,
+template <typename T, typename TQ = T>
+__global__ void __launch_bounds__(BS) xr_kernel(int n, T* __restrict__ x, T* __restrict__ r, const TQ* __restrict__ p,
+                                                const TQ* __restrict__ q, const T* __restrict__ s,
                                                 const T* __restrict__ t, const T* __restrict__ r0, double* partials,
                                                 unsigned int* counter, KState* S) {
     pdlEnter();
@@ -368,6 +375,9 @@ template <typename T>
 __global__ void scale_kernel(int64_t nnz, const int* col, const double* vals, const double* dinv, T* out) {
     for (int64_t k = blockIdx.x * (int64_t)BS + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * BS)
         out[k] = (T)(vals[k] * dinv[col[k]]);
+}
+__global__ void to_float_kernel(int64_t nnz, const double* vals, float* out) {
+    for (int64_t k = blockIdx.x * (int64_t)BS + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * BS) out[k] = (float)vals[k];
 }
 __global__ void unscale_kernel(int n, const double* dinv, const double* xs, double* x) {
     int i = blockIdx.x * BS + threadIdx.x;
@@ -719,10 +729,23 @@ void withSpmvShape(F&& f) {
     }
 }
 
+// Krylov method of a solve: BiCGSTAB (Jacobi or amg's V-cycle), flexible CG preconditioned
+// by an FP64 cycle (with the K-cycle levels), by an FP32 V-cycle of the same hierarchy, or by
+// the FP32 V-cycle of smoothed aggregation, and BiCGSTAB with the latter
+enum { KM_BICGSTAB = 0, KM_FCG = 1, KM_FCG_PRE32 = 2, KM_FCG_SA = 3, KM_BICGSTAB_SA = 4 };
+inline bool precondIn32(int mode) { return mode == KM_FCG_PRE32 || mode == KM_FCG_SA || mode == KM_BICGSTAB_SA; }
+inline bool smoothedMode(int mode) { return mode == KM_FCG_SA || mode == KM_BICGSTAB_SA; }
+inline bool flexMode(int mode) { return mode == KM_FCG || mode == KM_FCG_PRE32 || mode == KM_FCG_SA; }
+
 template <typename T>
 void iterateEager(const SellMatrix& A, const T* M, Vecs<T> V, Amg* amg, T* y, T* z, long long count, bool sample,
-                  KrylovWork& w, cudaStream_t s) {
+                  int mode, KrylovWork& w, cudaStream_t s) {
     KState* S = w.state.p;
+    auto cycle = [&](const T* r, T* out) {
+        if constexpr (sizeof(T) == 4)
+            if (mode == KM_BICGSTAB_SA) return amg->sa->apply(r, out, S, s, sample);
+        precApply(amg, r, out, S, s, sample);
+    };
     const int n = A.n, vg = vecGrid(n);
     decltype(&spmv_kernel<T, 1>) k1 = nullptr;
     decltype(&spmv_kernel<T, 2>) k2 = nullptr;
@@ -731,33 +754,55 @@ void iterateEager(const SellMatrix& A, const T* M, Vecs<T> V, Amg* amg, T* y, T*
     const int sg1 = waveGrid(k1, ceil_div(A.nslices, WARPS));
     const int sg2 = waveGrid(k2, ceil_div(A.nslices, WARPS));
     for (long long it = 0; it < count; ++it) {
-        launchPdl(p_kernel<T>, vg, BS, s, n, V.p, V.r, V.v, S);
+        launchPdl(p_kernel<T>, vg, BS, s, n, V.p, V.r, V.v, (float*)nullptr, S);
         const T* dp = V.p;
         if (amg) {
-            precApply(amg, V.p, y, S, s, sample);
+            cycle(V.p, y);
             dp = y;
         }
         const int slot = sample ? profBegin(PROF_SPMV, sizeof(T) == 4, spmvBytes<T>(A), s) : -1;
         launchPdl(k1, sg1, BS, s, A.nslices, n, A.sl_off, A.col, M, dp, V.v, V.r0, w.partials.p,
                   w.counter.p, S);
         profEnd(slot, s);
-        launchPdl(s_kernel<T>, vg, BS, s, n, V.s, V.r, V.v, S);
+        launchPdl(s_kernel<T>, vg, BS, s, n, V.s, V.r, V.v, (float*)nullptr, S);
         const T* ds = V.s;
         if (amg) {
-            precApply(amg, V.s, z, S, s, sample);
+            cycle(V.s, z);
             ds = z;
         }
         launchPdl(k2, sg2, BS, s, A.nslices, n, A.sl_off, A.col, M, ds, V.t, V.s, w.partials.p,
                   w.counter.p, S);
-        launchPdl(xr_kernel<T>, vg, BS, s, n, V.x, V.r, dp, ds, V.s, V.t, V.r0, w.partials.p, w.counter.p, S);
+        launchPdl(xr_kernel<T, T>, vg, BS, s, n, V.x, V.r, dp, ds, V.s, V.t, V.r0, w.partials.p, w.counter.p, S);
     }
 }
 
-// Krylov method of a solve: BiCGSTAB, or flexible CG preconditioned by an FP64
-// cycle (with the K-cycle levels), by an FP32 V-cycle of the same hierarchy, or by the
-// FP32 V-cycle of smoothed aggregation
-enum { KM_BICGSTAB = 0, KM_FCG = 1, KM_FCG_PRE32 = 2, KM_FCG_SA = 3 };
-inline bool precondIn32(int mode) { return mode == KM_FCG_PRE32 || mode == KM_FCG_SA; }
+// `count` FP64 BiCGSTAB iterations with the FP32 cycle of smoothed aggregation: p and s go to
+// the cycle as FP32 copies (w.y32), M^-1 p and M^-1 s stay FP32 (w.z32, and w.z's memory)
+void iterateSmoothed(const SellMatrix& A, const double* M, Vecs<double> V, Amg* amg, long long count, bool sample,
+                     KrylovWork& w, cudaStream_t s) {
+    KState* S = w.state.p;
+    const int n = A.n, vg = vecGrid(n);
+    auto k1 = spmv_kernel<double, 1, 4, 6, float>;
+    auto k2 = spmv_kernel<double, 2, 4, 6, float>;
+    const int sg1 = waveGrid(k1, ceil_div(A.nslices, WARPS)), sg2 = waveGrid(k2, ceil_div(A.nslices, WARPS));
+    float* in = w.y32.p;
+    float* ph = w.z32.p;
+    float* sh = reinterpret_cast<float*>(w.z.p);
+    for (long long it = 0; it < count; ++it) {
+        launchPdl(p_kernel<double>, vg, BS, s, n, V.p, V.r, V.v, in, S);
+        amg->sa->apply(in, ph, S, s, sample);
+        const int slot = sample ? profBegin(PROF_SPMV, false, spmvBytes<double>(A) - 4.0 * A.n, s) : -1;
+        launchPdl(k1, sg1, BS, s, A.nslices, n, A.sl_off, A.col, M, (const float*)ph, V.v, V.r0, w.partials.p,
+                  w.counter.p, S);
+        profEnd(slot, s);
+        launchPdl(s_kernel<double>, vg, BS, s, n, V.s, V.r, V.v, in, S);
+        amg->sa->apply(in, sh, S, s);
+        launchPdl(k2, sg2, BS, s, A.nslices, n, A.sl_off, A.col, M, (const float*)sh, V.t, V.s, w.partials.p,
+                  w.counter.p, S);
+        launchPdl(xr_kernel<double, float>, vg, BS, s, n, V.x, V.r, (const float*)ph, (const float*)sh, V.s, V.t, V.r0,
+                  w.partials.p, w.counter.p, S);
+    }
+}
 
 // `count` flexible-CG iterations (FP64 recurrences), launched one kernel at a time.
 // Vectors: x = V.x, r = V.r, d = V.p, q = V.v, u = V.t; z = y (KM_FCG) or, with an FP32
@@ -810,12 +855,16 @@ template <typename T>
 void iterateAny(const SellMatrix& A, const T* M, Vecs<T> V, Amg* amg, T* y, T* z, long long count, bool sample,
                 int mode, KrylovWork& w, cudaStream_t s) {
     if constexpr (sizeof(T) == 8) {
-        if (mode != KM_BICGSTAB) {
+        if (flexMode(mode)) {
             iterateFcgEager(A, M, V, amg, y, mode, count, sample, w, s);
             return;
         }
+        if (mode == KM_BICGSTAB_SA) {
+            iterateSmoothed(A, M, V, amg, count, sample, w, s);
+            return;
+        }
     }
-    iterateEager<T>(A, M, V, amg, y, z, count, sample, w, s);
+    iterateEager<T>(A, M, V, amg, y, z, count, sample, mode, w, s);
 }
 
 template <typename T>
@@ -828,7 +877,7 @@ void iterate(const SellMatrix& A, const T* M, Vecs<T> V, Amg* amg, T* y, T* z, l
     std::vector<uintptr_t> key = {(uintptr_t)mode, (uintptr_t)sizeof(T), (uintptr_t)A.sl_off, (uintptr_t)A.col, (uintptr_t)A.nslices,
                                   (uintptr_t)A.n, (uintptr_t)M, (uintptr_t)V.x, (uintptr_t)V.r, (uintptr_t)V.r0,
                                   (uintptr_t)V.p, (uintptr_t)V.v, (uintptr_t)V.s, (uintptr_t)V.t, (uintptr_t)amg,
-                                  (uintptr_t)(!amg ? 0 : mode == KM_FCG_SA ? amg->sa->generation : amg->generation), (uintptr_t)y, (uintptr_t)z,
+                                  (uintptr_t)(!amg ? 0 : smoothedMode(mode) ? amg->sa->generation : amg->generation), (uintptr_t)y, (uintptr_t)z,
                                   (uintptr_t)w.state.p, (uintptr_t)w.partials.p, (uintptr_t)w.counter.p,
                                   (uintptr_t)w.y32.p, (uintptr_t)w.z32.p};
     constexpr size_t MAX_GRAPHS = 8;
@@ -877,7 +926,7 @@ template <typename T>
 KrylovOut runBicgstab(const SellMatrix& A, const T* M, const T* rhs, Vecs<T> V, bool from_zero, double tol,
                       long long maxit, KrylovWork& w, cudaStream_t s, Amg* amg, T* y, T* z,
                       int mode = KM_BICGSTAB) {
-    const bool flex = mode != KM_BICGSTAB;
+    const bool flex = flexMode(mode);
     KrylovOut out;
     KState* S = w.state.p;
     KState init{};
@@ -952,26 +1001,27 @@ namespace {
 // flexible CG's preconditioner: an FP32 V-cycle (half the bytes of the FP64 one; the
 // recurrences stay FP64) unless the hierarchy has K-cycle levels (FP64 only) or
 // PRISM_FCG_PREC=fp64
-int fcgMode(const Amg* amg, const SellMatrix& A) {
+int solveMode(int kind, const Amg* amg, const SellMatrix& A) {
+    if (kind == SOLVE_SMOOTHED) return KM_BICGSTAB_SA;
+    if (kind == SOLVE_PLAIN) return KM_BICGSTAB;
     return fcgSmoothed(amg, A) ? KM_FCG_SA : fcgPre32(amg) ? KM_FCG_PRE32 : KM_FCG;
 }
 // values of the cycle's hierarchy from the current matrix (built on first use)
 void setupCycle(Amg* amg, int mode, const SellMatrix& A, const int* rowptr, const int* col, bool pre32,
                 cudaStream_t s) {
-    if (mode != KM_FCG_SA) {
+    if (!smoothedMode(mode)) {
         amg->setup(A, rowptr, col, pre32, s);
         return;
     }
     if (!amg->sa) amg->sa = std::make_unique<SaAmg>();
-    amg->sa->setup(A, rowptr, col, amg->values_current, s);
+    amg->sa->setup(A, rowptr, col, mode == KM_FCG_SA, amg->values_current, s);
 }
 }  // namespace
 
 // Smoothed aggregation up to 2^28 matrix entries (38M rows of a hex mesh): its setup sorts
 // about three 64-bit keys per entry and numbers them with 32-bit ints.
-bool fcgSmoothed(const Amg* amg, const SellMatrix& A) {
-    return fcgPre32(amg) && A.nnz_csr < (int64_t(1) << 28);
-}
+bool smoothedFits(const SellMatrix& A) { return A.nnz_csr < (int64_t(1) << 28); }
+bool fcgSmoothed(const Amg* amg, const SellMatrix& A) { return fcgPre32(amg) && smoothedFits(A); }
 
 bool fcgPre32(const Amg* amg) {
     static const bool p64 = [] {
@@ -995,7 +1045,7 @@ const SolveCtl& runSmall(const SellMatrix& A, const double* b, double* x, long l
 
 KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, int precision,
                    double inner_tol, KrylovWork& w, cudaStream_t s, Amg* amg, const int* rowptr, const int* col,
-                   bool flexible, bool symmetric) {
+                   int kind, bool symmetric) {
     if (!amg && smallSolveFits(A, maxit)) {
         const SolveCtl& c = runSmall(A, b, x, 1, 0.0, tol, maxit, symmetric, w, s);
         KrylovOut out;
@@ -1005,8 +1055,10 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
         return out;
     }
     const bool mixed = precision == PRISM_PREC_MIXED;
+    const bool flexible = kind == SOLVE_FLEXIBLE;
     if (flexible && (mixed || !amg)) fail(PRISM_INTERNAL, "flexible CG runs FP64 with AMG only");
-    const int mode = flexible ? fcgMode(amg, A) : KM_BICGSTAB;
+    if (kind == SOLVE_SMOOTHED && !amg) fail(PRISM_INTERNAL, "smoothed aggregation without its hierarchy");
+    const int mode = solveMode(kind, amg, A);
     const bool pre32 = mixed || precondIn32(mode);  // FP32 copy of the hierarchy
     w.ensure(A.nslices * 32, A.nnz_padded, mixed);
     const int n = A.n;
@@ -1034,6 +1086,11 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
         VerboseTimer vt("amg setup", s);
         setupCycle(amg, mode, A, rowptr, col, pre32, s);
         M32 = amg->vals32();
+        if (mixed && mode == KM_BICGSTAB_SA) {  // the FP32 iteration's matrix
+            to_float_kernel<<<std::min<int64_t>((A.nnz_padded + BS - 1) / BS, NUM_SMS * 32), BS, 0, s>>>(A.nnz_padded, A.vals,
+                                                                                                    w.As32.p); countLaunch();
+            M32 = w.As32.p;
+        }
     }
     VerboseTimer vt_solve(mixed ? "bicgstab fp32+fp64" : flexible ? "fcg fp64" : "bicgstab fp64", s);
     auto finish = [&] {
@@ -1105,7 +1162,7 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
     Vecs<float> V32{w.x32.p, w.r32.p, w.r032.p, w.p32.p, w.v32.p, w.s32.p, w.t32.p};
     bool first = true;
     while (done == 0) {
-        iterate<float>(A, M32, V32, amg, w.y32.p, w.z32.p, batch, first, w, s);
+        iterate<float>(A, M32, V32, amg, w.y32.p, w.z32.p, batch, first, w, s, mode);
         first = false;
         PB_LAUNCH("bicgstab fp32 iteration");
         PB_CUDA(cudaMemcpyAsync(w.host_state, S, sizeof(KState), cudaMemcpyDeviceToHost, s));
@@ -1466,9 +1523,10 @@ void emitOuterStep(SolveCtl* ctl, KrylovWork& w, cudaGraphConditionalHandle oute
 // The kernels and their order are those of the eager path, so the results are the same.
 void emitBicgstab(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, KrylovWork& w,
                   cudaStream_t s, Amg* amg, const int* rowptr, const int* col, SolveCtl* ctl, CaptureStreams& cs,
-                  int depth, bool flexible) {
-    if (flexible && !amg) fail(PRISM_INTERNAL, "flexible CG runs with AMG only");
-    const int mode = flexible ? fcgMode(amg, A) : KM_BICGSTAB;
+                  int depth, int kind) {
+    const bool flexible = kind == SOLVE_FLEXIBLE;
+    if (kind != SOLVE_PLAIN && !amg) fail(PRISM_INTERNAL, "a multigrid solve without its hierarchy");
+    const int mode = solveMode(kind, amg, A);
     w.ensure(A.nslices * 32, A.nnz_padded, false);
     const int n = A.n, gn = ceil_div(n, BS);
     const bool scaled = amg == nullptr;

@@ -82,23 +82,27 @@ struct KrylovOut {
     double rel_residual = 0.0;
 };
 
+enum { SOLVE_PLAIN = 0, SOLVE_FLEXIBLE = 1, SOLVE_SMOOTHED = 2 };
 // x <- BiCGSTAB solve of A x = b from the guess x, stopping at ||b - A x|| <= tol ||b||.
 // precision: PRISM_PREC_FP64 or PRISM_PREC_MIXED. Right preconditioning: Jacobi
 // (column scaling) when amg is null, else one V-cycle of amg, whose hierarchy is
 // built on first use from the device CSR pattern (rowptr, col) of A and refreshed
 // with A's values on every call.
-// flexible: FP64 with amg only -- flexible conjugate gradients (Notay 2000, one
+// kind, with amg: SOLVE_PLAIN (BiCGSTAB with amg's own V-cycle), SOLVE_SMOOTHED (BiCGSTAB with
+// the FP32 cycle of smoothed aggregation), or SOLVE_FLEXIBLE: FP64 only -- flexible conjugate gradients (Notay 2000, one
 // previous direction kept) preconditioned by amg->applyK(), for symmetric
 // positive (semi-)definite A (the pressure-correction equation), in place of
 // BiCGSTAB; same stopping rule, passes and statuses. symmetric: A is symmetric by construction
 // (the one-launch solve of a small system may then run conjugate gradients).
 KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, int precision,
                    double inner_tol, KrylovWork& w, cudaStream_t s, Amg* amg = nullptr, const int* rowptr = nullptr,
-                   const int* col = nullptr, bool flexible = false, bool symmetric = false);
+                   const int* col = nullptr, int kind = SOLVE_PLAIN, bool symmetric = false);
 // flexible CG with amg preconditions with an FP32 V-cycle (else with the FP64 cycle)
 bool fcgPre32(const Amg* amg);
 // that V-cycle is smoothed aggregation's (samg.h)
 bool fcgSmoothed(const Amg* amg, const SellMatrix& A);
+// smoothed aggregation takes matrices of this size
+bool smoothedFits(const SellMatrix& A);
 // x <- x + D^-1 (b - A x)   (numerics/jacobi.cpp:5-9)
 void jacobiStep(const SellMatrix& A, const double* b, double* x, KrylovWork& w, cudaStream_t s);
 // max|A x - b| / (max|diag(A) x| + eps)   (numerics/solver.cpp:8-24); returns NaN if non-finite values met
@@ -170,6 +174,6 @@ void emitOuterStep(SolveCtl* ctl, KrylovWork& w, cudaGraphConditionalHandle oute
 // the FP64 bicgstab() of one step, as device-controlled nodes (streams: helpers for the bodies)
 void emitBicgstab(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, KrylovWork& w,
                   cudaStream_t s, Amg* amg, const int* rowptr, const int* col, SolveCtl* ctl, CaptureStreams& cs,
-                  int depth, bool flexible = false);
+                  int depth, int kind = SOLVE_PLAIN);
 
 }  // namespace pb

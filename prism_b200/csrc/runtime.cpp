@@ -555,22 +555,32 @@ struct InStep {
     ~InStep() { g_in_step = before; }
 };
 
-// AMG solves of the spd pressure correction run flexible CG (FP64 recurrences), and so do
-// those of a user's symmetric equation, which go back to BiCGSTAB should it fail
-// (symmetricFallback); PRISM_PRESSURE_SOLVER=bicgstab keeps BiCGSTAB with the V-cycle
-static bool flexibleFor(const Transport& eq, const PrismSolveOpts& o, const Amg* amg) {
+// How an AMG solve of eq runs. The spd pressure correction: flexible CG (FP64 recurrences).
+// A user's equation: flexible CG where its matrix is symmetric, else BiCGSTAB with the cycle of
+// smoothed aggregation, which takes a third of the iterations of amg's own hierarchy; both go
+// back to the latter should they fail (standInSolve). Inside a step the momentum predictors
+// keep amg's cycle: nothing could step in for a solve that failed in a captured step.
+// PRISM_PRESSURE_SOLVER=bicgstab keeps BiCGSTAB with amg's cycle everywhere.
+static int kindFor(const Transport& eq, const PrismSolveOpts& o, const Amg* amg, const SellMatrix& A) {
     static const bool on = [] {
         const char* e = std::getenv("PRISM_PRESSURE_SOLVER");
         return !(e && std::strcmp(e, "bicgstab") == 0);
     }();
-    if (o.method == PRISM_SOLVER_FCG) return true;
-    if (!on || !amg || o.method != PRISM_SOLVER_BICGSTAB) return false;
-    if (eq.spd) return o.precision == PRISM_PREC_FP64;
-    return symmetricMatrix(eq) && !eq.no_flex && !g_in_step;
+    if (o.method == PRISM_SOLVER_FCG) return SOLVE_FLEXIBLE;
+    if (!on || !amg || o.method != PRISM_SOLVER_BICGSTAB) return SOLVE_PLAIN;
+    if (eq.spd) return o.precision == PRISM_PREC_FP64 ? SOLVE_FLEXIBLE : SOLVE_PLAIN;
+    if (eq.no_stand_in || g_in_step || !smoothedFits(A)) return SOLVE_PLAIN;
+    return symmetricMatrix(eq) ? SOLVE_FLEXIBLE : SOLVE_SMOOTHED;
 }
-// flexible CG stands in for the BiCGSTAB that was asked for
-static bool flexibleStandIn(const Transport& eq, const PrismSolveOpts& o, const Amg* amg) {
-    return flexibleFor(eq, o, amg) && o.method != PRISM_SOLVER_FCG && !eq.spd;
+// that kind stands in for the BiCGSTAB with amg's cycle that was asked for
+static bool standsIn(const Transport& eq, const PrismSolveOpts& o, int kind) {
+    return kind != SOLVE_PLAIN && o.method != PRISM_SOLVER_FCG && !eq.spd;
+}
+constexpr long long STAND_IN_MAX = 500;  // iterations (20-60 are usual) after which it has failed
+// a stand-in's end that has to be mended: anything but success or the caller's own iteration cap
+static bool standInFailed(const PrismSolveOpts& o, int status, long long iterations) {
+    return status != PRISM_OK &&
+           !(status == PRISM_NOT_CONVERGED && o.krylov_max_iter > 0 && iterations >= o.krylov_max_iter);
 }
 
 // PRISM_SOLVER_FCG's requirements: FP64, and the AMG preconditioner (its own choice
@@ -581,20 +591,21 @@ static void checkFcg(const PrismSolveOpts& o) {
     if (o.preconditioner == PRISM_PC_JACOBI) fail(PRISM_BAD_ARG, "flexible CG needs the AMG preconditioner");
 }
 
-// One step on a matrix symmetric by construction: flexible CG; should it fail (an indefinite
-// matrix), BiCGSTAB from the same guess, as for any other matrix, then and from then on (failed).
-// The guess waits in r0, which flexible CG does not use.
-static KrylovOut symmetricSolve(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, Mesh& m,
-                                Amg* amg, bool& failed) {
+// One step by a stand-in (kindFor); should it fail, BiCGSTAB with amg's cycle from the same
+// guess, then and from then on (failed). The guess waits in xs, which AMG solves do not use.
+static KrylovOut standInSolve(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, int kind,
+                              const PrismSolveOpts& o, Mesh& m, Amg* amg, bool& failed) {
     KrylovWork& w = m.kw;
     w.ensure(A.nslices * 32, A.nnz_padded, false);
-    PB_CUDA(cudaMemcpyAsync(w.r0.p, x, A.n * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
-    KrylovOut k = bicgstab(A, b, x, tol, maxit, PRISM_PREC_FP64, 0.1, w, m.stream, amg, m.pat.rowptr.p, m.pat.col.p, true);
-    if (k.status == PRISM_OK || (k.status == PRISM_NOT_CONVERGED && k.iterations >= maxit)) return k;
+    const double itol = o.inner_tol > 0 ? o.inner_tol : 0.1;
+    PB_CUDA(cudaMemcpyAsync(w.xs.p, x, A.n * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
+    KrylovOut k = bicgstab(A, b, x, tol, std::min(maxit, STAND_IN_MAX), kind == SOLVE_FLEXIBLE ? PRISM_PREC_FP64 : o.precision,
+                           itol, w, m.stream, amg, m.pat.rowptr.p, m.pat.col.p, kind);
+    if (!standInFailed(o, k.status, k.iterations)) return k;
     failed = true;
-    PB_CUDA(cudaMemcpyAsync(x, w.r0.p, A.n * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
+    PB_CUDA(cudaMemcpyAsync(x, w.xs.p, A.n * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
     amg->values_current = false;
-    KrylovOut f = bicgstab(A, b, x, tol, maxit, PRISM_PREC_FP64, 0.1, w, m.stream, amg, m.pat.rowptr.p, m.pat.col.p);
+    KrylovOut f = bicgstab(A, b, x, tol, maxit, o.precision, itol, w, m.stream, amg, m.pat.rowptr.p, m.pat.col.p);
     f.iterations += k.iterations;
     return f;
 }
@@ -656,12 +667,11 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o) {
             jacobiStep(A, eq.b.p, phi.v.p, m.kw, m.stream);
         } else {
             const HoldAmgValues hold(amg, eq.matrix_unchanged || iter > 0);  // A is fixed within one solve
-            KrylovOut k;
-            if (flexibleStandIn(eq, o, amg))
-                k = symmetricSolve(A, eq.b.p, phi.v.p, ktol, kmax, m, amg, eq.no_flex);
-            else
-                k = bicgstab(A, eq.b.p, phi.v.p, ktol, kmax, o.precision, itol, m.kw, m.stream, amg, m.pat.rowptr.p,
-                             m.pat.col.p, flexibleFor(eq, o, amg), symmetricMatrix(eq));
+            const int kind = kindFor(eq, o, amg, A);
+            KrylovOut k = standsIn(eq, o, kind)
+                              ? standInSolve(A, eq.b.p, phi.v.p, ktol, kmax, kind, o, m, amg, eq.no_stand_in)
+                              : bicgstab(A, eq.b.p, phi.v.p, ktol, kmax, o.precision, itol, m.kw, m.stream, amg,
+                                         m.pat.rowptr.p, m.pat.col.p, kind, symmetricMatrix(eq));
             r.krylov_iterations += k.iterations;
             r.krylov_rel_residual = k.rel_residual;
             if (k.status != PRISM_OK && r.status == PRISM_OK) r.status = k.status;
@@ -1079,16 +1089,19 @@ FixedPointOut adjointBackward(Transport& eq, const double* dJ, double* gk, doubl
     }
     const double ktol = o.krylov_tol > 0 ? o.krylov_tol : 1e-12;
     const long long kmax = o.krylov_max_iter > 0 ? o.krylov_max_iter : 2LL * m.nc;
+    PrismSolveOpts fp64 = o;
+    fp64.precision = PRISM_PREC_FP64;
+    fp64.inner_tol = 0.0;
     double h[2];
     for (int it = 0; it < max_outer; ++it) {
         adjointCorrection(P, lam.p, u.p, d.p, np, s);
         adjointRhs(P, d_dJ.p, lam.p, u.p, d.p, np, rhs.p, s);
         PB_CUDA(cudaMemcpyAsync(lam_prev.p, lam.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, s));
         const HoldAmgValues hold(amg, it > 0);
-        KrylovOut k = amg && !eq.no_flex
-                          ? symmetricSolve(AT, rhs.p, lam.p, ktol, kmax, m, amg, eq.no_flex)
+        KrylovOut k = amg && !eq.no_stand_in && smoothedFits(AT)
+                          ? standInSolve(AT, rhs.p, lam.p, ktol, kmax, SOLVE_FLEXIBLE, fp64, m, amg, eq.no_stand_in)
                           : bicgstab(AT, rhs.p, lam.p, ktol, kmax, PRISM_PREC_FP64, 0.1, m.kw, s, amg, m.pat.rowptr.p,
-                                     m.pat.col.p, false, true);
+                                     m.pat.col.p, SOLVE_PLAIN, true);
         out.krylov += k.iterations;
         ++out.outer;
         if (k.status != PRISM_OK && out.status == PRISM_OK) out.status = k.status;
@@ -1275,9 +1288,10 @@ PrismSolveResult solveCaptured(Transport& eq, const PrismSolveOpts& o) {
     }
     const long long n_iter = std::max<long long>(o.n_iter, 0);
     // a stand-in's guess is kept in case it fails (solveAsGraph, which then needs the system too)
-    const bool stand_in = flexibleStandIn(eq, o, amg);
+    const int kind = kindFor(eq, o, amg, A);
+    const bool stand_in = standsIn(eq, o, kind);
     if (stand_in)
-        PB_CUDA(cudaMemcpyAsync(m.kw.r0.p, phi.v.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        PB_CUDA(cudaMemcpyAsync(m.kw.xs.p, phi.v.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, s));
     if (o.method == PRISM_SOLVER_BICGSTAB && !amg && smallSolveFits(A, kmax)) {
         smallSolve(A, eq.b.p, phi.v.p, n_iter, o.eps, ktol, kmax, symmetricMatrix(eq), ctl, s);
         if (n_iter > 0) phi.event += 4;
@@ -1286,8 +1300,9 @@ PrismSolveResult solveCaptured(Transport& eq, const PrismSolveOpts& o) {
         r.iterations = -(slot + 1);
         return r;
     }
+    const long long cap = stand_in ? std::min(kmax, STAND_IN_MAX) : kmax;
     cudaGraphConditionalHandle outer = createConditional(s, 0);
-    emitSolveBegin(ctl, n_iter, o.eps, kmax, ktol, outer, s);
+    emitSolveBegin(ctl, n_iter, o.eps, cap, ktol, outer, s);
     if (n_iter > 0) {
         ++phi.event;
         emitResidual(A, eq.b.p, phi.v.p, m.kw, s);
@@ -1296,8 +1311,7 @@ PrismSolveResult solveCaptured(Transport& eq, const PrismSolveOpts& o) {
         beginConditional(s, cudaGraphCondTypeWhile, outer, body);
         phi.event += 2;
         const HoldAmgValues hold(amg, eq.matrix_unchanged);
-        emitBicgstab(A, eq.b.p, phi.v.p, ktol, kmax, m.kw, body, amg, m.pat.rowptr.p, m.pat.col.p, ctl, m.cs, 1,
-                     flexibleFor(eq, o, amg));
+        emitBicgstab(A, eq.b.p, phi.v.p, ktol, cap, m.kw, body, amg, m.pat.rowptr.p, m.pat.col.p, ctl, m.cs, 1, kind);
         ++phi.event;
         emitResidual(A, eq.b.p, phi.v.p, m.kw, body);
         emitOuterStep(ctl, m.kw, outer, body);
@@ -1379,13 +1393,15 @@ bool graphReady(const Transport& eq, const PrismSolveOpts& o) {
     if (m.kw.n != m.n_pad) return false;
     if (pc == PRISM_PC_AMG) {
         if (!eq.amg || !m.kw.y) return false;
-        if (flexibleFor(eq, o, eq.amg.get()) && fcgSmoothed(eq.amg.get(), m.matrix(eq.A.p)))
-            return eq.amg->sa && eq.amg->sa->built && m.kw.y32;
+        const SellMatrix A = m.matrix(eq.A.p);
+        const int kind = kindFor(eq, o, eq.amg.get(), A);
+        if (kind == SOLVE_SMOOTHED || (kind == SOLVE_FLEXIBLE && fcgSmoothed(eq.amg.get(), A)))
+            return eq.amg->sa && eq.amg->sa->built && eq.amg->sa->symmetric == (kind == SOLVE_FLEXIBLE) && m.kw.y32;
         if (!eq.amg->built) return false;
         for (auto& L : eq.amg->levels)
             if (!L->b || !L->dinv) return false;
         if (eq.amg->k_levels > 0 && !eq.amg->kscal) return false;
-        if (flexibleFor(eq, o, eq.amg.get()) && fcgPre32(eq.amg.get())) {
+        if (kind == SOLVE_FLEXIBLE && fcgPre32(eq.amg.get())) {
             if (!m.kw.y32 || (!eq.amg->coarse_inv32 && eq.amg->coarse_inv)) return false;
             for (auto& L : eq.amg->levels)
                 if (!L->b32 || !L->vals32) return false;
@@ -1413,11 +1429,13 @@ PrismSolveResult solveAsGraph(Transport& eq, const PrismSolveOpts& o) {
     const int used = runAsGraph(m, [&] { out = solve(eq, o); });
     if (used != 1) fail(PRISM_INTERNAL, "graph solve recorded no solve");
     out = fromCtl(m.graph_host[0]);
-    if (flexibleStandIn(eq, o, eq.amg.get()) && pcFor(eq, o, m.matrix(eq.A.p)) == PRISM_PC_AMG) {
-        if (out.status != PRISM_OK && !(out.status == PRISM_NOT_CONVERGED && out.krylov_iterations >= m.graph_host[0].kmax)) {
-            eq.no_flex = true;
+    const SellMatrix A = m.matrix(eq.A.p);
+    const bool with_amg = o.method == PRISM_SOLVER_FCG || pcFor(eq, o, A) == PRISM_PC_AMG;
+    if (with_amg && standsIn(eq, o, kindFor(eq, o, eq.amg.get(), A))) {
+        if (standInFailed(o, out.status, out.krylov_iterations)) {
+            eq.no_stand_in = true;
             eq.amg->values_current = false;
-            PB_CUDA(cudaMemcpyAsync(eq.phi->v.p, m.kw.r0.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
+            PB_CUDA(cudaMemcpyAsync(eq.phi->v.p, m.kw.xs.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
             out = solveAssembled(eq, o);
         }
         if (o.clear_coeffs) zeroOutCoeffs(eq);

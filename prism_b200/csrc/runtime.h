@@ -143,9 +143,9 @@ struct Transport {
     // PRISM_PC_AUTO at AMG sizes, decided on the equation's first solve: Jacobi when
     // its matrix is diagonally dominant enough (offDiagonalRatio), else AMG (0: not yet)
     int auto_pc = 0;
-    // flexible CG failed on this symmetric equation (an indefinite matrix: negative
-    // diffusivities): it keeps BiCGSTAB
-    bool no_flex = false;
+    // the method standing in for BiCGSTAB with amg's cycle failed on this equation (kindFor):
+    // it keeps the latter
+    bool no_stand_in = false;
     // the next solves assemble the same matrix as the last one (only b changes):
     // its AMG hierarchy keeps its values
     bool matrix_unchanged = false;

@@ -1,5 +1,6 @@
 // samg.cu -- smoothed-aggregation multigrid (Vanek, Mandel and Brezina 1996): the FP32
-// V-cycle that preconditions flexible CG on symmetric positive (semi-)definite systems.
+// V-cycle that preconditions flexible CG on symmetric positive (semi-)definite systems and
+// BiCGSTAB on convection-diffusion.
 //
 //   * Aggregates: a maximal independent set at distance two of the strong couplings
 //     (w_ij = |a_ij| / sqrt(a_ii a_jj) >= 0.25 of the larger of both rows' strongest),
@@ -10,18 +11,18 @@
 //     prolongation needs about half the iterations of a piecewise-constant one and its
 //     aggregates of 7-11 rows leave fewer, smaller levels (2.1M-cell cavity: 5 levels
 //     against 7), which matters as much: the coarse levels are latency-bound.
-//   * Cycle: V(1,1) with damped Jacobi. With S = I - omega A D^-1 and Q = S^T P, the whole
-//     cycle of a level is two passes:
+//   * Cycle: V(1,1) with damped Jacobi. With Q = (I - omega D^-1 A) P, the whole cycle of a level is two passes:
 //       down   b_next = Q^T b          (pre-smoothing from zero, residual, restriction)
 //              y = omega D^-1 (2 b - A omega D^-1 b)   (both smoothing steps of b itself)
 //       up     x = y + Q x_next        (prolongation and its post-smoothing)
-//     because for symmetric A the post-smoothed prolongation (I - omega D^-1 A) P is Q.
+//     because the post-smoothed prolongation (I - omega D^-1 A) P is Q.
 //     The two halves of `down` share a launch; A is stored scaled by omega D^-1, so its
 //     pass gathers one vector. Q^T and Q hold fewer entries than A on 2-D meshes.
 //   * The smallest levels (TAIL_ROWS, TAIL_NNZ) run in one launch of a thread-block cluster.
 // The structure is built once per pattern (sorted 64-bit keys); every new matrix refreshes
-// the values by gathers in a fixed order. Matrices are taken as symmetric: (A P)^T stands
-// for P^T A.
+// the values by gathers in a fixed order. For a symmetric matrix (A P)^T stands for P^T A;
+// otherwise the restriction is smoothed with A^T's values: R^T = (I - omega_p D^-1 A^T) P0
+// takes P^T's place and (S R^T)^T, S with A^T, that of Q^T (Sala and Tuminaro 2008).
 #include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
@@ -49,7 +50,9 @@ inline int grid(int64_t n) { return std::max(1, ceil_div(n, BS)); }
 
 // ---------------------------------------------------------------- structure
 __device__ __forceinline__ double valueAt(const double* vals, const int* csr_pos, int k) {
-    return csr_pos ? vals[csr_pos[k]] : vals[k];
+    if (!csr_pos) return vals[k];
+    const int at = csr_pos[k];
+    return at >= 0 ? vals[at] : 0.0;
 }
 
 __global__ void csr_pos_kernel(int n, const int* rowptr, const int* sl_off, int* csr_pos) {
@@ -72,32 +75,60 @@ __global__ void scaling_kernel(int n, const int* rowptr, const int* col, const i
     wd[i] = (float)(omega * di);
 }
 
-__device__ __forceinline__ float coupling(double a, double di, double dj) {
-    return (float)(fabs(a) * sqrt(fabs(di * dj)));
+// |a_ij| / sqrt(a_ii a_jj), a_ij averaged with a_ji where the matrix is not symmetric
+__device__ __forceinline__ float coupling(const int* csr_pos, const int* tr_pos, const double* vals, int k, double di,
+                                          double dj) {
+    double a = fabs(valueAt(vals, csr_pos, k));
+    if (tr_pos) a = 0.5 * (a + (tr_pos[k] >= 0 ? fabs(vals[tr_pos[k]]) : 0.0));
+    return (float)(a * sqrt(fabs(di * dj)));
 }
 
-__global__ void strongest_kernel(int n, const int* rowptr, const int* col, const int* csr_pos, const double* vals,
-                                 const double* dinv, float* wmax) {
+// place in vals of the transposed entry of every CSR entry (-1: none)
+__global__ void transposed_kernel(int n, const int* rowptr, const int* col, const int* csr_pos, int* tr_pos) {
+    const int i = blockIdx.x * BS + threadIdx.x;
+    if (i >= n) return;
+    for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) {
+        const int j = col[k];
+        int at = -1;
+        if (csr_pos) {  // level 0: columns in the mesh's order
+            for (int q = rowptr[j]; q < rowptr[j + 1]; ++q)
+                if (col[q] == i) at = csr_pos[q];
+        } else {
+            int lo = rowptr[j], hi = rowptr[j + 1];
+            const int end = hi;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (col[mid] < i) lo = mid + 1;
+                else hi = mid;
+            }
+            if (lo < end && col[lo] == i) at = lo;
+        }
+        tr_pos[k] = at;
+    }
+}
+
+__global__ void strongest_kernel(int n, const int* rowptr, const int* col, const int* csr_pos, const int* tr_pos,
+                                 const double* vals, const double* dinv, float* wmax) {
     const int i = blockIdx.x * BS + threadIdx.x;
     if (i >= n) return;
     float best = 0.f;
     const double di = dinv[i];
     for (int k = rowptr[i]; k < rowptr[i + 1]; ++k)
-        if (col[k] != i) best = fmaxf(best, coupling(valueAt(vals, csr_pos, k), di, dinv[col[k]]));
+        if (col[k] != i) best = fmaxf(best, coupling(csr_pos, tr_pos, vals, k, di, dinv[col[k]]));
     wmax[i] = best;
 }
 
 // strong[k] = the column of a strong entry, else the row itself (which every neighbour
 // maximum below includes anyway)
-__global__ void strong_kernel(int n, const int* rowptr, const int* col, const int* csr_pos, const double* vals,
-                              const double* dinv, const float* wmax, int* strong) {
+__global__ void strong_kernel(int n, const int* rowptr, const int* col, const int* csr_pos, const int* tr_pos,
+                              const double* vals, const double* dinv, const float* wmax, int* strong) {
     const int i = blockIdx.x * BS + threadIdx.x;
     if (i >= n) return;
     const double di = dinv[i];
     const float wi = wmax[i];
     for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) {
         const int j = col[k];
-        const float w = j == i ? 0.f : coupling(valueAt(vals, csr_pos, k), di, dinv[j]);
+        const float w = j == i ? 0.f : coupling(csr_pos, tr_pos, vals, k, di, dinv[j]);
         strong[k] = (w > 0.f && w >= (float)STRONG * fmaxf(wi, wmax[j])) ? j : i;
     }
 }
@@ -150,8 +181,8 @@ __global__ void root_label_kernel(int n, const int* root, const int* id, int* la
     if (i < n) label[i] = root[i] ? id[i] : -1;
 }
 // an unlabelled row joins its strongest labelled strong neighbour (ties: lower label)
-__global__ void join_kernel(int n, const int* rowptr, const int* col, const int* csr_pos, const double* vals,
-                            const double* dinv, const int* strong, const int* label, int* out) {
+__global__ void join_kernel(int n, const int* rowptr, const int* col, const int* csr_pos, const int* tr_pos,
+                            const double* vals, const double* dinv, const int* strong, const int* label, int* out) {
     const int i = blockIdx.x * BS + threadIdx.x;
     if (i >= n) return;
     int l = label[i];
@@ -161,7 +192,7 @@ __global__ void join_kernel(int n, const int* rowptr, const int* col, const int*
         for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) {
             const int j = strong[k];
             if (j == i || label[j] < 0) continue;
-            const float w = coupling(valueAt(vals, csr_pos, k), di, dinv[j]);
+            const float w = coupling(csr_pos, tr_pos, vals, k, di, dinv[j]);
             if (w > best || (w == best && label[j] < l)) {
                 best = w;
                 l = label[j];
@@ -284,20 +315,20 @@ struct Product {
     const double* l_val;
     const int *b_rowptr, *b_col;
     const double* b_val;
-    double* out;
-    // after A P: Q = P - omega D^-1 A P, written to q_val and, transposed, to t_val (null: none)
+    double* out;  // null: not kept
+    // where B is P: Q = P - omega D^-1 A P, written to q_val and, transposed, to t_val (null: none)
     double omega;
     const double* dinv;
     const int* q_tpos;
     float *q_val, *t_val;
 };
 __device__ __forceinline__ void storeProduct(const Product& P, int r, int e, double v) {
-    P.out[e] = v;
-    if (P.q_val) {
+    if (P.out) P.out[e] = v;
+    if (P.q_val || P.t_val) {
         const int own = findColumn(P.b_col, P.b_rowptr[r], P.b_rowptr[r + 1], P.out_col[e]);
         const float q = (float)((own >= 0 ? P.b_val[own] : 0.0) - P.omega * P.dinv[r] * v);
-        P.q_val[e] = q;
-        P.t_val[P.q_tpos[e]] = q;
+        if (P.q_val) P.q_val[e] = q;
+        if (P.t_val) P.t_val[P.q_tpos[e]] = q;
     }
 }
 
@@ -874,8 +905,8 @@ int aggregate(DevArena& ar, SaLevel& L, cudaStream_t s) {
     TmpBuf<float> wmax(n, s);
     TmpBuf<int> strong(std::max<int64_t>(L.nnz, 1), s), left(MIS_ROUNDS + 1, s), root(n + 1, s), id(n + 1, s), lab(n, s);
     TmpBuf<unsigned long long> key(n, s), near(n, s);
-    strongest_kernel<<<grid(n), BS, 0, s>>>(n, L.rowptr, L.col, L.csr_pos, L.vals, L.dinv.p, wmax.p); countLaunch();
-    strong_kernel<<<grid(n), BS, 0, s>>>(n, L.rowptr, L.col, L.csr_pos, L.vals, L.dinv.p, wmax.p, strong.p); countLaunch();
+    strongest_kernel<<<grid(n), BS, 0, s>>>(n, L.rowptr, L.col, L.csr_pos, L.tr_pos.p, L.vals, L.dinv.p, wmax.p); countLaunch();
+    strong_kernel<<<grid(n), BS, 0, s>>>(n, L.rowptr, L.col, L.csr_pos, L.tr_pos.p, L.vals, L.dinv.p, wmax.p, strong.p); countLaunch();
     PB_CUDA(cudaMemsetAsync(left.p, 0, (MIS_ROUNDS + 1) * sizeof(int), s));
     mis_init_kernel<<<grid(n), BS, 0, s>>>(n, key.p, left.p); countLaunch();
     for (int r = 0; r < MIS_ROUNDS; ++r) {
@@ -893,8 +924,8 @@ int aggregate(DevArena& ar, SaLevel& L, cudaStream_t s) {
     L.agg.alloc(ar, n, s);
     // the rows next to a root, then the rows next to those
     root_label_kernel<<<grid(n), BS, 0, s>>>(n, root.p, id.p, L.agg.p); countLaunch();
-    join_kernel<<<grid(n), BS, 0, s>>>(n, L.rowptr, L.col, L.csr_pos, L.vals, L.dinv.p, strong.p, L.agg.p, lab.p); countLaunch();
-    join_kernel<<<grid(n), BS, 0, s>>>(n, L.rowptr, L.col, L.csr_pos, L.vals, L.dinv.p, strong.p, lab.p, L.agg.p); countLaunch();
+    join_kernel<<<grid(n), BS, 0, s>>>(n, L.rowptr, L.col, L.csr_pos, L.tr_pos.p, L.vals, L.dinv.p, strong.p, L.agg.p, lab.p); countLaunch();
+    join_kernel<<<grid(n), BS, 0, s>>>(n, L.rowptr, L.col, L.csr_pos, L.tr_pos.p, L.vals, L.dinv.p, strong.p, lab.p, L.agg.p); countLaunch();
     PB_LAUNCH("smoothed aggregation: aggregates");
     return nc;
 }
@@ -935,12 +966,15 @@ void SaAmg::levelScaling(SaLevel& L, cudaStream_t s) {
 void SaAmg::levelValues(size_t l, cudaStream_t s) {
     SaLevel& L = *levels[l];
     SaLevel& C = *levels[l + 1];
-    withLanes(L.lpr_p, [&](auto c) {
-        constexpr int LP = decltype(c)::value;
-        p_values_kernel<LP><<<grid((int64_t)L.n * LP), BS, 0, s>>>(L.n, L.rowptr, L.col, L.csr_pos, L.vals, L.dinv.p,
-                                                                   L.agg.p, L.p_rowptr.p, L.p_col.p, L.omega_p,
-                                                                   L.p_val.p); countLaunch();
-    });
+    const bool sym = !L.tr_pos.p;
+    auto prolongation = [&](const int* pos, double* val) {
+        withLanes(L.lpr_p, [&](auto c) {
+            constexpr int LP = decltype(c)::value;
+            p_values_kernel<LP><<<grid((int64_t)L.n * LP), BS, 0, s>>>(L.n, L.rowptr, L.col, pos, L.vals, L.dinv.p,
+                                                                       L.agg.p, L.p_rowptr.p, L.p_col.p, L.omega_p, val); countLaunch();
+        });
+    };
+    prolongation(L.csr_pos, L.p_val.p);
     Product AP{};
     AP.rows = L.n;
     AP.out_rowptr = L.q_rowptr.p;
@@ -957,8 +991,18 @@ void SaAmg::levelValues(size_t l, cudaStream_t s) {
     AP.dinv = L.dinv.p;
     AP.q_tpos = L.q_tpos.p;
     AP.q_val = L.q_val.p;
-    AP.t_val = L.t_val.p;
+    AP.t_val = sym ? L.t_val.p : nullptr;
     launchProduct(AP, L.q_nnz, L.n, L.p_nnz, s);
+    if (!sym) {
+        // the restriction from A^T in A's place: R^T, and (S R^T) stored transposed
+        prolongation(L.tr_pos.p, L.r_val.p);
+        AP.l_src = L.tr_pos.p;
+        AP.b_val = L.r_val.p;
+        AP.out = nullptr;
+        AP.q_val = nullptr;
+        AP.t_val = L.t_val.p;
+        launchProduct(AP, L.q_nnz, L.n, L.p_nnz, s);
+    }
     Product AC{};
     AC.rows = C.n;
     AC.out_rowptr = C.rowptr;
@@ -966,7 +1010,7 @@ void SaAmg::levelValues(size_t l, cudaStream_t s) {
     AC.l_rowptr = L.pt_rowptr.p;
     AC.l_idx = L.pt_row.p;
     AC.l_src = L.pt_src.p;
-    AC.l_val = L.p_val.p;
+    AC.l_val = sym ? L.p_val.p : L.r_val.p;
     AC.b_rowptr = L.q_rowptr.p;
     AC.b_col = L.q_col.p;
     AC.b_val = L.ap_val.p;
@@ -974,7 +1018,8 @@ void SaAmg::levelValues(size_t l, cudaStream_t s) {
     launchProduct(AC, C.nnz, L.n, L.q_nnz, s);
 }
 
-void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, cudaStream_t s) {
+void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, bool sym, cudaStream_t s) {
+    symmetric = sym;
     levels.clear();
     arena.reset();  // stream order keeps earlier work on the old hierarchy ahead of its reuse
     coarse_a.release();
@@ -998,11 +1043,19 @@ void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, cudaSt
     while (true) {
         const size_t l = levels.size() - 1;
         SaLevel& L = *levels[l];
-        // smoother weights: the spectrum of D^-1 A reaches 2 on the finest level and 1.2-1.5
-        // on the Galerkin levels (measured on 2-D, 3-D and tetrahedral diffusion); omega_p is
-        // 4/3 over it, omega the largest that leaves the stiffest modes damped
-        L.omega = l == 0 ? 0.9 : 1.1;
-        L.omega_p = l == 0 ? 0.7 : 0.95;
+        // Smoother weights. Symmetric: the spectrum of D^-1 A reaches 2 on the finest level and
+        // 1.2-1.5 on the Galerkin levels (measured on 2-D, 3-D and tetrahedral diffusion);
+        // omega_p is 4/3 over it, omega the largest that leaves the stiffest modes damped. With
+        // convection the spectrum is complex and the larger weights diverge: a CPU model of the
+        // cycle took 22 BiCGSTAB iterations on 48^3 MUSCL transport with (0.8, 0.66) on every
+        // level against 64 with piecewise-constant aggregation, 26 / 54 at a cell Peclet number
+        // of 3,000, 30 / 68 on tetrahedra, and failed with (0.9, 0.95).
+        L.omega = !sym ? 0.8 : l == 0 ? 0.9 : 1.1;
+        L.omega_p = !sym ? 0.66 : l == 0 ? 0.7 : 0.95;
+        if (!sym) {
+            L.tr_pos.alloc(arena, std::max<int64_t>(L.nnz, 1), s);
+            transposed_kernel<<<grid(L.n), BS, 0, s>>>(L.n, L.rowptr, L.col, L.csr_pos, L.tr_pos.p); countLaunch();
+        }
         L.dinv.alloc(arena, L.n, s);
         L.wd.alloc(arena, L.n, s);
         L.as32.alloc(arena, std::max<int64_t>(std::max(L.nnz, L.sell_nnz), 1), s);
@@ -1023,6 +1076,7 @@ void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, cudaSt
             L.p_nnz = patternOf(arena, keys.p, L.nnz, L.n, nc, L.p_rowptr, L.p_col, s);
         }
         L.p_val.alloc(arena, std::max<int64_t>(L.p_nnz, 1), s);
+        if (!sym) L.r_val.alloc(arena, std::max<int64_t>(L.p_nnz, 1), s);
         transposeOf(arena, L.n, nc, L.p_nnz, L.p_rowptr.p, L.p_col.p, L.pt_rowptr, L.pt_row, &L.pt_src, nullptr, s);
         // A P, the pattern of Q
         {
@@ -1083,11 +1137,11 @@ void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, cudaSt
     }
 }
 
-void SaAmg::setup(const SellMatrix& A, const int* rowptr, const int* col, bool keep_values, cudaStream_t s) {
-    const bool same = built && !levels.empty() && levels[0]->n == A.n && levels[0]->sl_off == A.sl_off;
+void SaAmg::setup(const SellMatrix& A, const int* rowptr, const int* col, bool sym, bool keep_values, cudaStream_t s) {
+    const bool same = built && symmetric == sym && !levels.empty() && levels[0]->n == A.n && levels[0]->sl_off == A.sl_off;
     if (same && keep_values && levels[0]->vals == A.vals) return;
     if (!same) {
-        build(A, rowptr, col, s);
+        build(A, rowptr, col, sym, s);
     } else {
         levels[0]->vals = A.vals;
         levelScaling(*levels[0], s);

@@ -1,5 +1,5 @@
-// samg.h -- smoothed-aggregation multigrid, the preconditioner of flexible CG on
-// symmetric positive (semi-)definite systems.
+// samg.h -- smoothed-aggregation multigrid, the preconditioner of flexible CG on symmetric
+// positive (semi-)definite systems and of BiCGSTAB on other transport equations.
 #pragma once
 
 #include <memory>
@@ -12,8 +12,9 @@ namespace pb {
 
 // One level. Level 0 borrows the equation's SELL-32 matrix; coarser matrices are CSR.
 // For the transfer to the next level, P = (I - omega_p D^-1 A) P0 is the smoothed
-// prolongation, S = I - omega A D^-1 the residual operator of one damped-Jacobi step from
-// zero, and Q = S^T P: the down-sweep is b_next = Q^T b and the up-sweep adds Q e.
+// prolongation and Q = (I - omega D^-1 A) P: the up-sweep adds Q e, and for symmetric A the
+// down-sweep is b_next = Q^T b. Otherwise R^T is P made with A^T and the down-sweep's matrix
+// that Q^T made with A^T and R^T.
 struct SaLevel {
     int n = 0;
     int64_t nnz = 0;
@@ -23,6 +24,7 @@ struct SaLevel {
     const int* csr_pos = nullptr;
     const double* vals = nullptr;
     ArenaBuf<int> o_rowptr, o_col, o_csr_pos;
+    ArenaBuf<int> tr_pos;  // A not symmetric: place in vals of each entry's transpose (-1: none)
     ArenaBuf<double> o_vals;
     // level 0: the SELL-32 view
     int nslices = 0;
@@ -39,7 +41,7 @@ struct SaLevel {
     // transfer to the next level
     ArenaBuf<int> agg;
     ArenaBuf<int> p_rowptr, p_col;           // P
-    ArenaBuf<double> p_val;
+    ArenaBuf<double> p_val, r_val;           // r_val: R^T on P's pattern (A not symmetric)
     ArenaBuf<int> pt_rowptr, pt_row, pt_src; // P^T: fine row and P entry of each
     ArenaBuf<int> q_rowptr, q_col, q_tpos;   // Q (the pattern of A P); q_tpos: its place in Q^T
     ArenaBuf<double> ap_val;                 // A P
@@ -53,7 +55,7 @@ struct SaLevel {
 struct SaAmg {
     DevArena arena;  // declared first: released last
     std::vector<std::unique_ptr<SaLevel>> levels;
-    bool built = false;
+    bool built = false, symmetric = true;
     uint64_t generation = 0;
     int tail = -1;  // first level of the fused coarse tail (-1: none)
     int coarse_n = 0;
@@ -62,14 +64,14 @@ struct SaAmg {
 
     // Builds the hierarchy (first call on a pattern) or refreshes its values for the
     // matrix A, whose CSR pattern lists each row's entries in the order of its SELL slots.
-    // keep_values: the matrix is unchanged since the last call.
-    void setup(const SellMatrix& A, const int* rowptr, const int* col, bool keep_values, cudaStream_t s);
+    // sym: A is symmetric. keep_values: the matrix is unchanged since the last call.
+    void setup(const SellMatrix& A, const int* rowptr, const int* col, bool sym, bool keep_values, cudaStream_t s);
     // z = B r, one V(1,1) cycle in FP32; S (optional): skip the work once the solve has
     // stopped; sample: time the finest-level kernels when a profiling window is open
     void apply(const float* r, float* z, const KState* S, cudaStream_t s, bool sample = false);
 
 private:
-    void build(const SellMatrix& A, const int* rowptr, const int* col, cudaStream_t s);
+    void build(const SellMatrix& A, const int* rowptr, const int* col, bool sym, cudaStream_t s);
     void levelScaling(SaLevel& L, cudaStream_t s);
     void levelValues(size_t l, cudaStream_t s);
 };
