@@ -23,7 +23,6 @@
 // the values by gathers in a fixed order. For a symmetric matrix (A P)^T stands for P^T A;
 // otherwise the restriction is smoothed with A^T's values: R^T = (I - omega_p D^-1 A^T) P0
 // takes P^T's place and (S R^T)^T, S with A^T, that of Q^T (Sala and Tuminaro 2008).
-#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
 #include <atomic>
@@ -32,6 +31,7 @@
 #include <type_traits>
 
 #include "amg.h"
+#include "cluster.cuh"
 #include "samg.h"
 
 namespace pb {
@@ -411,7 +411,9 @@ __global__ void __launch_bounds__(BS) product_team_kernel(const Product P) {
 // nnz_out, nnz_b: entries of the product and of B (n_b rows)
 void launchProduct(const Product& P, int64_t nnz_out, int n_b, int64_t nnz_b, cudaStream_t s) {
     const double out = (double)nnz_out / std::max(P.rows, 1), right = (double)nnz_b / std::max(n_b, 1);
-    if (out <= 12.0 && right <= 4.0) {
+    // one thread per row only where the rows fill the chip: 2,309 rows take 86 us that way, 9 us
+    // with a block each
+    if (P.rows > 16384 && out <= 12.0 && right <= 4.0) {
         product_thread_kernel<12><<<grid(P.rows), BS, 0, s>>>(P);
     } else if (P.rows > 16384) {
         const int g = ceil_div(P.rows, BS / 32);
@@ -751,8 +753,7 @@ __device__ __forceinline__ void tailRows(int n, int g, int nthreads, const int* 
 __global__ void __launch_bounds__(TAIL_BS) tail_kernel(const __grid_constant__ TailParams P) {
     pdlEnter();
     if (P.S && P.S->done) return;  // uniform: the state does not change during this launch
-    namespace cg = cooperative_groups;
-    cg::cluster_group cl = cg::this_cluster();
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     const int nthreads = (int)cl.num_blocks() * TAIL_BS;
     const int g = (int)cl.block_rank() * TAIL_BS + threadIdx.x;
     const int lane = threadIdx.x & 31;
@@ -785,47 +786,10 @@ __global__ void __launch_bounds__(TAIL_BS) tail_kernel(const __grid_constant__ T
     }
 }
 
-// CTAs of the tail's cluster: 16 (a non-portable size) where the device can place it, else 8
+// CTAs of the tail's cluster: 16 where the device can place it, else 8
 int tailCluster() {
-    static const int c = [] {
-        int cl = 8;
-        if (cudaFuncSetAttribute(tail_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
-            cudaLaunchConfig_t cfg{};
-            cfg.gridDim = dim3(16);
-            cfg.blockDim = dim3(TAIL_BS);
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = 16;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, tail_kernel, &cfg) == cudaSuccess && n >= 1) cl = 16;
-        }
-        cudaGetLastError();  // a refused query leaves no sticky error
-        return cl;
-    }();
+    static const int c = clusterPlaced(tail_kernel, TAIL_BS) ? CLUSTER_MAX : 8;
     return c;
-}
-
-void launchTail(const TailParams& P, cudaStream_t s) {
-    const int cl = tailCluster();
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)cl);
-    cfg.blockDim = dim3(TAIL_BS);
-    cfg.stream = s;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)cl;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = pdlEnabled() ? 1 : 0;
-    cfg.attrs = at;
-    cfg.numAttrs = 2;
-    PB_CUDA(cudaLaunchKernelEx(&cfg, tail_kernel, P));
-    countLaunch();
 }
 
 // ---------------------------------------------------------------- host side of the structure
@@ -1196,7 +1160,7 @@ void SaAmg::apply(const float* r, float* z, const KState* S, cudaStream_t s, boo
             P.L[k] = TailLevel{L.n, L.rowptr, L.col, L.as32.p, L.wd.p, L.t_rowptr.p, L.t_col.p, L.t_val.p,
                                L.q_rowptr.p, L.q_col.p, L.q_val.p, L.b.p, L.x.p, L.y.p};
         }
-        launchTail(P, s);
+        launchCluster(tail_kernel, tailCluster(), TAIL_BS, s, true, P);
     } else if (coarse_inv32.p) {
         launchPdl(coarse_kernel, grid((int64_t)coarse_n * 32), BS, s, coarse_n, (const float*)coarse_inv32.p, rhs(last),
                   sol(last), S);

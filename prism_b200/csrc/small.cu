@@ -10,19 +10,15 @@
 // by the cluster's other blocks as distributed shared memory. An iteration is five barriers,
 // three of them carrying a reduction (each block sends its partial sums to every other block
 // before it arrives, and all add them in block order, so results repeat bit for bit).
-#include <cooperative_groups.h>
-
 #include <cmath>
 
+#include "cluster.cuh"
 #include "krylov.h"
-
-namespace cg = cooperative_groups;
 
 namespace pb {
 
 namespace {
 
-constexpr int MAX_CTAS = 16;
 constexpr int NV = 5;  // values of one reduction, at most
 
 struct SmallParams {
@@ -44,68 +40,9 @@ template <int THREADS, int K, bool CL>
 __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallParams P) {
     constexpr int ROWS = THREADS * K;  // rows per block
     __shared__ double ph[ROWS], sh[ROWS];  // the gathered vectors: M^-1 p (or x), M^-1 s
-    constexpr int NW = THREADS / 32;
-    __shared__ double red[2][NV][NW];
-    __shared__ double xch[2][MAX_CTAS][NV];
-    cg::cluster_group cl = cg::this_cluster();
-    const int ctas = CL ? (int)cl.num_blocks() : 1, rank = CL ? (int)cl.block_rank() : 0;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int parity = 0;
-
-    auto barrier = [&] {
-        if constexpr (CL) cl.sync();
-        else __syncthreads();
-    };
-    // sums (or maxima of magnitudes) of v over all rows, in every thread; also a barrier.
-    // The buffers alternate: the next reduction never writes what a slow thread still reads.
-    auto reduce = [&](auto count, bool maxima, double (&v)[NV]) {
-        constexpr int N = decltype(count)::value;
-        auto join = [&](double a, double c) { return maxima ? fmax(a, c) : a + c; };
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int k = 0; k < N; ++k) v[k] = join(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
-        if (lane == 0)
-#pragma unroll
-            for (int k = 0; k < N; ++k) red[parity][k][warp] = v[k];
-        __syncthreads();
-        if constexpr (!CL) {
-#pragma unroll
-            for (int k = 0; k < N; ++k) {
-                double u[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-                for (int w = 0; w < NW; ++w) u[w & 3] = join(u[w & 3], red[parity][k][w]);
-                v[k] = join(join(u[0], u[1]), join(u[2], u[3]));
-            }
-        } else {
-            if (warp == 0) {
-                double u[N];
-#pragma unroll
-                for (int k = 0; k < N; ++k) u[k] = red[parity][k][lane % NW];
-#pragma unroll
-                for (int o = NW / 2; o > 0; o >>= 1)
-#pragma unroll
-                    for (int k = 0; k < N; ++k) u[k] = join(u[k], __shfl_xor_sync(0xffffffffu, u[k], o));
-                if (lane < ctas) {
-                    double* to = cl.map_shared_rank(&xch[parity][rank][0], lane);
-#pragma unroll
-                    for (int k = 0; k < N; ++k) to[k] = u[k];
-                }
-            }
-            barrier();
-#pragma unroll
-            for (int k = 0; k < N; ++k) {
-                double u = xch[parity][0][k];
-                for (int c = 1; c < ctas; ++c) u = join(u, xch[parity][c][k]);
-                v[k] = u;
-            }
-        }
-        parity ^= 1;
-    };
-    using One = std::integral_constant<int, 1>;
-    using Two = std::integral_constant<int, 2>;
-    using Three = std::integral_constant<int, 3>;
-    using Five = std::integral_constant<int, 5>;
+    __shared__ ClusterShared<THREADS, NV> shared;
+    ClusterReduce<THREADS, CL, NV> R(shared);
+    const int rank = R.rank;
 
     int row[K], at[K], width[K];
     double dinv[K], x[K], r[K], r0[K], p[K], v[K];
@@ -124,7 +61,7 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
     auto rhs = [&](int k) { return row[k] < P.n ? __ldg(P.b + row[k]) : 0.0; };
     auto own = [&](int k) { return k * THREADS + (int)threadIdx.x; };
     auto gather = [&](double* a, int j) -> double {
-        if constexpr (CL) return *cl.map_shared_rank(a + (j & (ROWS - 1)), j / ROWS);
+        if constexpr (CL) return *R.cl.map_shared_rank(a + (j & (ROWS - 1)), j / ROWS);
         else return a[j];
     };
     // (A y)_row with y spread over the blocks' shared array a; up to 4 entries in flight
@@ -150,7 +87,7 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
     auto applyToX = [&] {
 #pragma unroll
         for (int k = 0; k < K; ++k) ph[own(k)] = x[k];
-        barrier();
+        R.barrier();
 #pragma unroll
         for (int k = 0; k < K; ++k) ax[k] = row[k] < P.n ? rowOf(k, ph) : 0.0;
     };
@@ -168,7 +105,7 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
                 m[1] = fmax(m[1], d);
             }
         }
-        reduce(Three{}, true, m);
+        R.template all<3, true>(m);
         return m[2] != 0.0 ? __longlong_as_double(0x7ff8000000000000LL) : m[0] / (m[1] + EPSILON);
     };
 
@@ -195,7 +132,7 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
             }
             if (row[k] < P.n && !(d > 0.0 && sum >= -1e-12 * d)) bad[0] = 1.0;
         }
-        reduce(One{}, true, bad);
+        R.template all<1, true>(bad);
         cg_ok = bad[0] == 0.0;
     }
     while (outer < P.n_iter) {
@@ -216,7 +153,7 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
                     d[0] += r[k] * r[k];
                     d[1] += bk * bk;
                 }
-                reduce(Two{}, false, d);
+                R.template all<2>(d);
                 const double r0sq = d[0], tol2 = P.tol * P.tol * d[1];
                 double rho = d[0], beta = d[0], w = 1.0;
                 long long iter_cg = 0;
@@ -232,7 +169,7 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
                             z[k] = dinv[k] * r[k];
                             ph[own(k)] = z[k];
                         }
-                        barrier();
+                        R.barrier();
                         d[0] = d[1] = d[2] = 0.0;
 #pragma unroll
                         for (int k = 0; k < K; ++k) {
@@ -241,7 +178,7 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
                             d[1] += az[k] * z[k];
                             d[2] += r[k] * r[k];
                         }
-                        reduce(Three{}, false, d);
+                        R.template all<3>(d);
                         if (!isfinite(d[0]) || !isfinite(d[1]) || !isfinite(d[2])) done = 5;
                         else if (d[2] <= tol2) done = 1;
                         else if (iter >= left) done = 2;
@@ -272,14 +209,14 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
                         p[k] = r[k] + beta * (p[k] - w * v[k]);
                         ph[own(k)] = dinv[k] * p[k];
                     }
-                    barrier();
+                    R.barrier();
                     d[0] = 0.0;
 #pragma unroll
                     for (int k = 0; k < K; ++k) {
                         v[k] = rowOf(k, ph);
                         d[0] += r0[k] * v[k];
                     }
-                    reduce(One{}, false, d);
+                    R.template all<1>(d);
                     const double alpha = rho / d[0];
                     if (d[0] == 0.0 || !isfinite(alpha)) {  // breakdown: restart from the current x
                         done = isfinite(d[0]) ? 3 : 5;
@@ -290,7 +227,7 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
                         r[k] -= alpha * v[k];  // s
                         sh[own(k)] = dinv[k] * r[k];
                     }
-                    barrier();
+                    R.barrier();
                     // t = A M^-1 s; the dots of r = s - w t follow from those of s and t, so the
                     // update needs no reduction of its own
                     double t[K];
@@ -304,7 +241,7 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
                         d[3] += r0[k] * t[k];
                         d[4] += r[k] * r[k];
                     }
-                    reduce(Five{}, false, d);
+                    R.template all<5>(d);
                     w = d[1] > 0.0 ? d[0] / d[1] : 0.0;
 #pragma unroll
                     for (int k = 0; k < K; ++k) {
@@ -345,7 +282,7 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
                 d[0] += e * e;
                 d[1] += bk * bk;
             }
-            reduce(Two{}, false, d);
+            R.template all<2>(d);
             krylov_rel = d[1] > 0 ? sqrt(d[0] / d[1]) : 0.0;
             if (kstatus != PRISM_OK || krylov_rel <= 10 * P.tol || left <= 0 || d[1] == 0) break;
         }
@@ -378,52 +315,21 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
     }
 }
 
-// largest cluster the device places (16 is a non-portable size; 8 is always allowed)
-template <int T, int K>
-bool placed() {
-    auto kernel = small_solve_kernel<T, K, true>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return false;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(MAX_CTAS);
-    cfg.blockDim = dim3(T);
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = MAX_CTAS;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int n = 0;
-    return cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n >= 1;
-}
+// blocks of the largest cluster the device places (8 is always allowed)
 int maxCtas() {
-    static const int c = [] {
-        const bool ok = placed<256, 1>() && placed<512, 2>() && placed<512, 4>();
-        cudaGetLastError();  // a refused query leaves no sticky error
-        return ok ? MAX_CTAS : 8;
-    }();
+    static const int c = clusterPlaced(small_solve_kernel<256, 1, true>, 256) &&
+                                 clusterPlaced(small_solve_kernel<512, 2, true>, 512) &&
+                                 clusterPlaced(small_solve_kernel<512, 4, true>, 512)
+                             ? CLUSTER_MAX
+                             : 8;
     return c;
 }
 
 template <int T, int K>
 void launchSmall(const SmallParams& P, cudaStream_t s) {
     const int ctas = ceil_div(P.n, T * K);
-    if (ctas == 1) {
-        small_solve_kernel<T, K, false><<<1, T, 0, s>>>(P);
-        return;
-    }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(T);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)ctas;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    PB_CUDA(cudaLaunchKernelEx(&cfg, small_solve_kernel<T, K, true>, P));
+    if (ctas == 1) launchCluster(small_solve_kernel<T, K, false>, 1, T, s, false, P);
+    else launchCluster(small_solve_kernel<T, K, true>, ctas, T, s, false, P);
 }
 
 }  // namespace
@@ -443,8 +349,6 @@ void smallSolve(const SellMatrix& A, const double* b, double* x, long long n_ite
     else if (A.n <= max * 256) launchSmall<256, 1>(P, s);
     else if (A.n <= max * 1024) launchSmall<512, 2>(P, s);
     else launchSmall<512, 4>(P, s);
-    countLaunch();
-    PB_LAUNCH("small_solve_kernel");
 }
 
 }  // namespace pb
