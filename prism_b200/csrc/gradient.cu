@@ -107,9 +107,16 @@ __global__ void __launch_bounds__(256) ls_operator_kernel(const MeshView m, doub
 // first lane adds the terms in the cell's face order, so the sum is the sequential
 // sweep's, term for term. The face terms' loads are in flight together instead of one
 // face after another.
+// A level is a chain of dependent loads (cell, faces, neighbours, their values) of a few
+// microseconds and little else, and 128^3 hexes have 382 of them. All of that chain but the
+// neighbours' gradients is fixed during a sweep, so it is loaded before the kernel waits for
+// the level below (programmatic dependent launch; the first level is launched plainly, after
+// everything that the sweep reads): the sweep on 128^3 jittered hexes went
+// from 3.53 to 1.37 ms, on 31^3 from 0.57 to 0.29.
 constexpr int GG_LPC = 8;
 __global__ void __launch_bounds__(256) gg_level_kernel(const MeshView m, ScalarView s, const int* __restrict__ cells,
                                                        int count) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     const int gt = blockIdx.x * blockDim.x + threadIdx.x;
     const int idx = gt / GG_LPC, sub = gt % GG_LPC;
     const int lane = threadIdx.x & 31, lead = lane & ~(GG_LPC - 1);
@@ -119,17 +126,19 @@ __global__ void __launch_bounds__(256) gg_level_kernel(const MeshView m, ScalarV
     const int nq = valid ? m.cf_off[c + 1] - q0 : 0;
     const int nq_max = __reduce_max_sync(0xffffffffu, (unsigned)nq);
     D3 xc{0, 0, 0}, gc{0, 0, 0};
-    double phic = 0.0;
+    double phic = 0.0, vol = 1.0;
     if (valid) {
         xc = cellCenter(m, c);
         phic = s.v[c];
-        gc = gradAt(s, c);
+        gc = gradAt(s, c);  // written by this level only
+        vol = m.vol[c];
     }
     D3 grad{0, 0, 0};
-    for (int base = 0; base < nq_max; base += GG_LPC) {
+    for (int base = 0; base < nq_max || base == 0; base += GG_LPC) {
         const int q = base + sub;
-        D3 term{0, 0, 0};
-        int has = 0;
+        D3 term{0, 0, 0}, Sf{0, 0, 0}, vec{0, 0, 0};
+        double face_phi = 0.0;
+        int has = 0, n = -1;
         if (q < nq) {
             const int f = m.cf_face[q0 + q];
             if (f < m.nb) {
@@ -141,16 +150,19 @@ __global__ void __launch_bounds__(256) gg_level_kernel(const MeshView m, ScalarV
             } else {
                 const int o = m.owner[f];
                 const bool own = (o == c);
-                const int n = own ? m.nbr[f] : o;
-                D3 Sf = areaVector(m, f);
+                n = own ? m.nbr[f] : o;
+                Sf = areaVector(m, f);
                 if (!own) Sf = D3{-Sf.x, -Sf.y, -Sf.z};
-                double face_phi = 0.5 * (phic + s.v[n]);
-                D3 grad_sum = gc + gradAt(s, n);
-                D3 vec = faceCenter(m, f) - (0.5 * (xc + cellCenter(m, n)));
-                face_phi += 0.5 * dot(grad_sum, vec);
-                term = Sf * face_phi;
+                face_phi = 0.5 * (phic + s.v[n]);
+                vec = faceCenter(m, f) - (0.5 * (xc + cellCenter(m, n)));
                 has = 1;
             }
+        }
+        if (base == 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+        if (n >= 0) {
+            D3 grad_sum = gc + gradAt(s, n);
+            face_phi += 0.5 * dot(grad_sum, vec);
+            term = Sf * face_phi;
         }
 #pragma unroll
         for (int k = 0; k < GG_LPC; ++k) {
@@ -163,7 +175,7 @@ __global__ void __launch_bounds__(256) gg_level_kernel(const MeshView m, ScalarV
         }
     }
     if (valid && sub == 0) {
-        grad = grad / m.vol[c];
+        grad = grad / vol;
         s.g[c] = grad.x;
         s.g[s.gstride + c] = grad.y;
         s.g[2 * s.gstride + c] = grad.z;
@@ -185,11 +197,17 @@ void launchLeastSquares(const MeshView& m, const ScalarView& s, const double* pi
 
 void launchGreenGauss(const MeshView& m, const ScalarView& s, const int* level_cells,
                       const std::vector<int>& level_off, cudaStream_t st) {
+    bool first = true;
     for (size_t l = 0; l + 1 < level_off.size(); ++l) {
         const int count = level_off[l + 1] - level_off[l];
         if (count == 0) continue;
-        gg_level_kernel<<<ceil_div((int64_t)count * GG_LPC, 256), 256, 0, st>>>(m, s, level_cells + level_off[l],
-                                                                                count); countLaunch();
+        const int blocks = ceil_div((int64_t)count * GG_LPC, 256);
+        if (first) {
+            gg_level_kernel<<<blocks, 256, 0, st>>>(m, s, level_cells + level_off[l], count); countLaunch();
+            first = false;
+        } else {
+            launchPdl(gg_level_kernel, blocks, 256, st, m, s, level_cells + level_off[l], count);
+        }
     }
     PB_LAUNCH("gg_level_kernel");
 }
