@@ -6,12 +6,15 @@
 // machine precision. Here each step runs BiCGSTAB (van der Vorst 1992, the
 // textbook recurrences Eigen uses) with Jacobi right preconditioning, applied
 // by scaling the columns once per step: A' = A D^-1, x' = D x, so every
-// iteration is five streaming kernels and no preconditioner pass:
-//   p = r + beta (p - w v)                      vector kernel
+// iteration is three streaming kernels and no preconditioner pass:
 //   v = A' p ; r0.v -> alpha                    SpMV + fused dot
-//   s = r - alpha v                             vector kernel
-//   t = A' s ; t.s, t.t -> w                    SpMV + fused dots
-//   x += alpha p + w s ; r = s - w t ; r0.r, r.r -> beta, convergence
+//   s = r - alpha v (formed where it is read, and kept) ; t = A' s ;
+//   t.s, t.t, r0.s, r0.t, s.s -> w, r0.r, r.r, beta, convergence    SpMV + fused dots
+//   x += alpha p + w s ; r = s - w t ; p = r + beta (p - w v)       vector kernel
+// (r0.r = r0.s - w r0.t and r.r = s.s - w t.s, so the update needs no reduction and can
+// carry the next direction. Five kernels, with s, the update and p each on its own, took 16.9
+// against 13.7 us an iteration on 66,748 seven-point rows, 25.5 against 21.8 us on 262,144
+// five-point rows and the same 104 us on 2.1M, where the bytes decide.)
 // Scalars live in device memory (KState); every reduction is a fixed-order
 // two-stage tree (block partials, then the last block to finish reduces them),
 // so results are bitwise reproducible run to run. The host launches batches of
@@ -84,7 +87,7 @@ int waveGrid(K kernel, int needed) {
 // y = A x for a SELL-32 matrix: a warp walks 32-row slices (one row per lane),
 // coalesced loads; the matrix is read with evict-first (streaming) loads so
 // that L2 keeps the gathered x.
-// STAGE 0: plain; 1: alpha = rho / (u.y); 2: w = (u.y)/(y.y)
+// STAGE 0: plain; 1: alpha = rho / (u.y)
 // The columns and values of up to 8 slots are loaded before their gathers, so
 // a row's loads are all in flight at once; the sum runs over the slots in order.
 template <typename T, int W = 8, typename TX = T>
@@ -114,51 +117,119 @@ __global__ void __launch_bounds__(BS, MINB) spmv_kernel(int nslices, int n, cons
                                                   const T* __restrict__ u, double* partials,
                                                   unsigned int* counter, KState* S) {
     pdlEnter();
-    if (STAGE != 0 && S->done) return;
+    if (STAGE != 0 && S->done) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) S->pending = 0;  // the last update has run
+        return;
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double d0 = 0.0, d1 = 0.0;
+    double d0 = 0.0;
     for (int sl = blockIdx.x * WARPS + warp; sl < nslices; sl += gridDim.x * WARPS) {
         const int b = sl_off[sl];
         const int width = (sl_off[sl + 1] - b) >> 5;
         const T sum = sliceRow<T, W, TX>(col, val, x, b, width, lane);
         const int r = sl * 32 + lane;
         y[r] = sum;
-        if (STAGE != 0 && r < n) {
-            d0 += (double)sum * (double)u[r];
-            if (STAGE == 2) d1 += (double)sum * (double)sum;
-        }
+        if (STAGE != 0 && r < n) d0 += (double)sum * (double)u[r];
     }
     if (STAGE == 0) return;
-    double v[2] = {d0, d1}, out[2];
-    if (reduceLast<2, false>(v, partials, counter, out) && threadIdx.x == 0) {
-        if (STAGE == 1) {
-            // r0.v = 0 (or a non-finite alpha) breaks the recurrence down: the host restarts
-            // from the current x (every later kernel of this iteration returns at once)
-            const double alpha = S->rho / out[0];
-            if (out[0] == 0.0 || !isfinite(alpha)) S->done = isfinite(out[0]) ? 3 : 5;
-            else S->alpha = alpha;
-        } else {
-            S->ts = out[0];
-            S->tt = out[1];
-            S->w = out[1] > 0.0 ? out[0] / out[1] : 0.0;
-        }
+    double v[1] = {d0}, out[1];
+    if (reduceLast<1, false>(v, partials, counter, out) && threadIdx.x == 0) {
+        // r0.v = 0 (or a non-finite alpha) breaks the recurrence down: the host restarts
+        // from the current x (every later kernel of this iteration returns at once)
+        const double alpha = S->rho / out[0];
+        if (out[0] == 0.0 || !isfinite(alpha)) S->done = isfinite(out[0]) ? 3 : 5;
+        else S->alpha = alpha;
     }
 }
 
-// c32 (optional): the FP32 copy that an FP32 preconditioner of an FP64 iteration reads
-template <typename T>
-__global__ void __launch_bounds__(BS) p_kernel(int n, T* __restrict__ p, const T* __restrict__ r,
-                                               const T* __restrict__ v, float* __restrict__ c32, const KState* S) {
+// t = A q with the dots t.s, t.t, r0.s, r0.t, s.s -> w, r0.r, r.r of r = s - w t, beta and the
+// convergence test. FORM: q = s = r - alpha v, formed from r and v where it is gathered and
+// written for this row; else q is given (M^-1 s of a preconditioner) and s read.
+template <typename T, bool FORM, int W, int MINB, typename TX = T>
+__global__ void __launch_bounds__(BS, MINB) spmv2_kernel(int nslices, int n, const int* __restrict__ sl_off,
+                                                   const int* __restrict__ col, const T* __restrict__ val,
+                                                   const TX* __restrict__ q, T* __restrict__ t, T* __restrict__ s,
+                                                   const T* __restrict__ r, const T* __restrict__ v,
+                                                   const T* __restrict__ r0, double* partials, unsigned int* counter,
+                                                   KState* S) {
     pdlEnter();
     if (S->done) return;
-    const double beta = S->beta, w = S->w;
-    for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
-        const T pi = (T)((double)r[i] + beta * ((double)p[i] - w * (double)v[i]));
-        p[i] = pi;
-        if (c32) c32[i] = (float)pi;
+    const double alpha = S->alpha;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double d[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int sl = blockIdx.x * WARPS + warp; sl < nslices; sl += gridDim.x * WARPS) {
+        const int b = sl_off[sl];
+        const int width = (sl_off[sl + 1] - b) >> 5;
+        const int i = sl * 32 + lane;
+        T sum, si;
+        if constexpr (FORM) {
+            auto form = [&](int c) { return (T)((double)__ldg(r + c) - alpha * (double)__ldg(v + c)); };
+            sum = 0;
+            for (int j0 = 0; j0 < width; j0 += W) {
+                int c[W];
+                T m[W];
+#pragma unroll
+                for (int k = 0; k < W; ++k)
+                    if (j0 + k < width) {
+                        c[k] = __ldcs(col + b + 32 * (j0 + k) + lane);
+                        m[k] = __ldcs(val + b + 32 * (j0 + k) + lane);
+                    }
+#pragma unroll
+                for (int k = 0; k < W; ++k)
+                    if (j0 + k < width) sum += m[k] * form(c[k]);
+            }
+            si = i < n ? form(i) : (T)0;
+            s[i] = si;
+        } else {
+            sum = sliceRow<T, W, TX>(col, val, q, b, width, lane);
+            si = s[i];
+        }
+        t[i] = sum;
+        if (i < n) {
+            const double sd = (double)si, td = (double)sum, r0i = (double)r0[i];
+            d[0] += td * sd;
+            d[1] += td * td;
+            d[2] += r0i * sd;
+            d[3] += r0i * td;
+            d[4] += sd * sd;
+        }
+    }
+    double out[5];
+    if (reduceLast<5, false>(d, partials, counter, out) && threadIdx.x == 0) {
+        const double w = out[1] > 0.0 ? out[0] / out[1] : 0.0;
+        const double rho_new = out[2] - w * out[3], rr = out[4] - w * out[0];
+        S->w = w;
+        S->ts = out[0];
+        S->tt = out[1];
+        S->rr = rr;
+        S->iter += 1;
+        int done = 0;
+        if (!isfinite(rho_new) || !isfinite(rr)) done = 5;
+        else if (S->reliable && (rr <= S->tol2 || rr < S->delta2 * S->rr_update)) done = 6;
+        else if (rr <= S->tol2) done = 1;
+        else if (S->iter >= S->maxit) done = 2;
+        else if (w == 0.0 || fabs(rho_new) < EPSILON * EPSILON * S->r0sq) done = 3;
+        else {
+            S->beta = (rho_new / S->rho) * (S->alpha / w);
+            S->rho = rho_new;
+        }
+        S->pending = done != 0;
+        S->done = done;
     }
 }
 
+// p = r + beta (p - w v): after a reliable update that continues the recurrence
+template <typename T>
+__global__ void __launch_bounds__(BS) p_kernel(int n, T* __restrict__ p, const T* __restrict__ r,
+                                               const T* __restrict__ v, const KState* S) {
+    if (S->done) return;
+    const double beta = S->beta, w = S->w;
+    for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS)
+        p[i] = (T)((double)r[i] + beta * ((double)p[i] - w * (double)v[i]));
+}
+
+// s = r - alpha v, ahead of a preconditioner; c32 (optional): the FP32 copy that an FP32
+// preconditioner of an FP64 iteration reads
 template <typename T>
 __global__ void __launch_bounds__(BS) s_kernel(int n, T* __restrict__ s, const T* __restrict__ r,
                                                const T* __restrict__ v, float* __restrict__ c32, const KState* S) {
@@ -172,47 +243,36 @@ __global__ void __launch_bounds__(BS) s_kernel(int n, T* __restrict__ s, const T
     }
 }
 
-// x += alpha p + w q ; r = s - w t  (q = s without a preconditioner pass, else q = M^-1 s, p = M^-1 p)
+// x += alpha y + w q ; r = s - w t ; p = r + beta (p - w v), with y = p and q = s, or M^-1 of
+// them (y null: y = p); c32 as in s_kernel, of p. The last direction of a solve that stops is
+// left as it was.
 template <typename T, typename TQ = T>
-__global__ void __launch_bounds__(BS) xr_kernel(int n, T* __restrict__ x, T* __restrict__ r, const TQ* __restrict__ p,
-                                                const TQ* __restrict__ q, const T* __restrict__ s,
-                                                const T* __restrict__ t, const T* __restrict__ r0, double* partials,
-                                                unsigned int* counter, KState* S) {
+__global__ void __launch_bounds__(BS) xrp_kernel(int n, T* __restrict__ x, T* __restrict__ r, T* __restrict__ p,
+                                                 const TQ* __restrict__ y, const TQ* __restrict__ q,
+                                                 const T* __restrict__ s, const T* __restrict__ t,
+                                                 const T* __restrict__ v, float* __restrict__ c32, const KState* S) {
     pdlEnter();
-    if (S->done) return;
-    const double alpha = S->alpha, w = S->w;
-    double d0 = 0.0, d1 = 0.0;
+    const bool done = S->done != 0;
+    if (done && !S->pending) return;
+    const double alpha = S->alpha, w = S->w, beta = S->beta;
     for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
-        double si = (double)s[i];
-        double xi = (double)x[i] + alpha * (double)p[i] + w * (double)q[i];
-        T ri = (T)(si - w * (double)t[i]);
-        x[i] = (T)xi;
+        const double pi = (double)p[i];
+        const T ri = (T)((double)s[i] - w * (double)t[i]);
+        x[i] = (T)((double)x[i] + alpha * (y ? (double)y[i] : pi) + w * (double)q[i]);
         r[i] = ri;
-        d0 += (double)r0[i] * (double)ri;
-        d1 += (double)ri * (double)ri;
-    }
-    double v[2] = {d0, d1}, out[2];
-    if (reduceLast<2, false>(v, partials, counter, out) && threadIdx.x == 0) {
-        S->rr = out[1];
-        S->iter += 1;
-        const double rho_new = out[0];
-        if (!isfinite(out[0]) || !isfinite(out[1])) S->done = 5;
-        else if (S->reliable && (out[1] <= S->tol2 || out[1] < S->delta2 * S->rr_update)) S->done = 6;
-        else if (out[1] <= S->tol2) S->done = 1;
-        else if (S->iter >= S->maxit) S->done = 2;
-        else if (w == 0.0 || fabs(rho_new) < EPSILON * EPSILON * S->r0sq) S->done = 3;
-        else {
-            S->beta = (rho_new / S->rho) * (alpha / w);
-            S->rho = rho_new;
+        if (!done) {
+            const T pn = (T)((double)ri + beta * (pi - w * (double)v[i]));
+            p[i] = pn;
+            if (c32) c32[i] = (float)pn;
         }
     }
 }
 
-// r = b - r (r holds A x) or r = b (x = 0); r0 = r; p = v = 0; set up the state.
+// r = b - r (r holds A x) or r = b (x = 0); r0 = p = r (c32: p's FP32 copy); v = 0; set up the state.
 template <typename T>
 __global__ void __launch_bounds__(BS) init_kernel(int n, T* __restrict__ r, const T* __restrict__ b,
                                                   T* __restrict__ r0, T* __restrict__ p, T* __restrict__ v,
-                                                  int from_zero, double tol, double* partials,
+                                                  float* __restrict__ c32, int from_zero, double tol, double* partials,
                                                   unsigned int* counter, KState* S) {
     double d0 = 0.0, d1 = 0.0;
     for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
@@ -220,7 +280,8 @@ __global__ void __launch_bounds__(BS) init_kernel(int n, T* __restrict__ r, cons
         T ri = from_zero ? b[i] : (T)(bi - (double)r[i]);
         r[i] = ri;
         r0[i] = ri;
-        p[i] = 0;
+        p[i] = ri;
+        if (c32) c32[i] = (float)ri;
         v[i] = 0;
         d0 += (double)ri * (double)ri;
         d1 += bi * bi;
@@ -235,6 +296,7 @@ __global__ void __launch_bounds__(BS) init_kernel(int n, T* __restrict__ r, cons
         S->beta = out[0];
         S->alpha = 1.0;
         S->w = 1.0;
+        S->pending = 0;
         if (!isfinite(out[0]) || !isfinite(out[1])) S->done = 5;
         else if (out[1] == 0.0) S->done = 4;
         else if (out[0] <= S->tol2) S->done = 1;
@@ -415,7 +477,7 @@ __global__ void flush_kernel(int n, double* __restrict__ xs, float* __restrict__
 }
 // Reliable update, part 2 (Ax = A' xs already in `ax`): r64 = b - ax, r32 = (float) r64,
 // rr = r64.r64, rho = r0.r32; continue the recurrence or declare convergence.
-// first != 0: (re)start -- r0 = r32, p = v = 0, fresh recurrence scalars.
+// first != 0: (re)start -- r0 = p = r32, v = 0, fresh recurrence scalars.
 __global__ void __launch_bounds__(BS) reliable_kernel(int n, const double* __restrict__ ax, const double* __restrict__ b,
                                                       double* __restrict__ r64, float* __restrict__ r32,
                                                       float* __restrict__ r032, float* __restrict__ p32,
@@ -429,7 +491,7 @@ __global__ void __launch_bounds__(BS) reliable_kernel(int n, const double* __res
         r32[i] = rf;
         if (first) {
             r032[i] = rf;
-            p32[i] = 0.0f;
+            p32[i] = rf;
             v32[i] = 0.0f;
         }
         d0 += ri * ri;
@@ -440,6 +502,7 @@ __global__ void __launch_bounds__(BS) reliable_kernel(int n, const double* __res
     if (reduceLast<3, false>(v, partials, counter, out) && threadIdx.x == 0) {
         S->rr = out[0];
         S->rr_update = out[0];
+        S->pending = 0;
         if (first) {
             S->bb = out[2];
             S->tol2 = tol * tol * out[2];
@@ -570,7 +633,7 @@ void KrylovWork::ensure(int n_pad, int64_t nnz_padded, bool mixed) {
         nnz = nnz_padded;
         for (auto* b : {&r, &r0, &p, &v, &s, &t, &xs, &dinv, &tmp}) b->alloc(n_pad);
         As.alloc(nnz_padded);
-        partials.alloc((size_t)std::max(ceil_div(n_pad / 32, WARPS), std::max(NUM_SMS, smCount()) * 16) * 4);
+        partials.alloc((size_t)std::max(ceil_div(n_pad / 32, WARPS), std::max(NUM_SMS, smCount()) * 16) * 5);
         counter.alloc(1);
         PB_CUDA(cudaMemset(counter.p, 0, sizeof(unsigned int)));
         scal.alloc(8);
@@ -710,7 +773,8 @@ inline void precApply(Amg* amg, const float* r, float* z, const KState* S, cudaS
 // blocks per SM. Measured on the 128^3 transport matrix (ncu, FP64): 4x6 (40 registers,
 // 71% warps active) 45 / 43 us for the two stages against 47 / 53 us for 8x5 (48
 // registers, 60%) and 52 / 50 us for 4x8 (32 registers, 97%). PRISM_SPMV_SHAPE = "WxMINB"
-// (4x6, 8x5, 4x8) overrides it.
+// (4x6, 8x5, 4x8) overrides it. The second stage sums five dots and takes 4 blocks per SM (64
+// registers; at 6 it spills).
 int spmvShape() {
     static const int v = [] {
         const char* e = std::getenv("PRISM_SPMV_SHAPE");
@@ -720,12 +784,13 @@ int spmvShape() {
     }();
     return v;
 }
-template <typename T, int STAGE, typename F>
+// f(first SpMV, second SpMV forming s, second SpMV given M^-1 s)
+template <typename T, typename F>
 void withSpmvShape(F&& f) {
     switch (spmvShape()) {
-        case 0: f(spmv_kernel<T, STAGE, 8, 5>); break;
-        case 1: f(spmv_kernel<T, STAGE, 4, 8>); break;
-        default: f(spmv_kernel<T, STAGE, 4, 6>); break;
+        case 0: f(spmv_kernel<T, 1, 8, 5>, spmv2_kernel<T, true, 8, 5>, spmv2_kernel<T, false, 8, 5>); break;
+        case 1: f(spmv_kernel<T, 1, 4, 8>, spmv2_kernel<T, true, 4, 8>, spmv2_kernel<T, false, 4, 8>); break;
+        default: f(spmv_kernel<T, 1, 4, 6>, spmv2_kernel<T, true, 4, 4>, spmv2_kernel<T, false, 4, 4>); break;
     }
 }
 
@@ -748,13 +813,12 @@ void iterateEager(const SellMatrix& A, const T* M, Vecs<T> V, Amg* amg, T* y, T*
     };
     const int n = A.n, vg = vecGrid(n);
     decltype(&spmv_kernel<T, 1>) k1 = nullptr;
-    decltype(&spmv_kernel<T, 2>) k2 = nullptr;
-    withSpmvShape<T, 1>([&](auto k) { k1 = k; });
-    withSpmvShape<T, 2>([&](auto k) { k2 = k; });
+    withSpmvShape<T>([&](auto k, auto, auto) { k1 = k; });
+    decltype(&spmv2_kernel<T, true, 4, 6>) k2 = nullptr;
+    withSpmvShape<T>([&](auto, auto form, auto plain) { k2 = amg ? plain : form; });
     const int sg1 = waveGrid(k1, ceil_div(A.nslices, WARPS));
     const int sg2 = waveGrid(k2, ceil_div(A.nslices, WARPS));
     for (long long it = 0; it < count; ++it) {
-        launchPdl(p_kernel<T>, vg, BS, s, n, V.p, V.r, V.v, (float*)nullptr, S);
         const T* dp = V.p;
         if (amg) {
             cycle(V.p, y);
@@ -764,15 +828,16 @@ void iterateEager(const SellMatrix& A, const T* M, Vecs<T> V, Amg* amg, T* y, T*
         launchPdl(k1, sg1, BS, s, A.nslices, n, A.sl_off, A.col, M, dp, V.v, V.r0, w.partials.p,
                   w.counter.p, S);
         profEnd(slot, s);
-        launchPdl(s_kernel<T>, vg, BS, s, n, V.s, V.r, V.v, (float*)nullptr, S);
         const T* ds = V.s;
         if (amg) {
+            launchPdl(s_kernel<T>, vg, BS, s, n, V.s, V.r, V.v, (float*)nullptr, S);
             cycle(V.s, z);
             ds = z;
         }
-        launchPdl(k2, sg2, BS, s, A.nslices, n, A.sl_off, A.col, M, ds, V.t, V.s, w.partials.p,
+        launchPdl(k2, sg2, BS, s, A.nslices, n, A.sl_off, A.col, M, ds, V.t, V.s, V.r, V.v, V.r0, w.partials.p,
                   w.counter.p, S);
-        launchPdl(xr_kernel<T, T>, vg, BS, s, n, V.x, V.r, dp, ds, V.s, V.t, V.r0, w.partials.p, w.counter.p, S);
+        launchPdl(xrp_kernel<T, T>, vg, BS, s, n, V.x, V.r, V.p, amg ? dp : (const T*)nullptr, ds, V.s, V.t, V.v,
+                  (float*)nullptr, S);
     }
 }
 
@@ -783,13 +848,12 @@ void iterateSmoothed(const SellMatrix& A, const double* M, Vecs<double> V, Amg* 
     KState* S = w.state.p;
     const int n = A.n, vg = vecGrid(n);
     auto k1 = spmv_kernel<double, 1, 4, 6, float>;
-    auto k2 = spmv_kernel<double, 2, 4, 6, float>;
+    auto k2 = spmv2_kernel<double, false, 4, 4, float>;
     const int sg1 = waveGrid(k1, ceil_div(A.nslices, WARPS)), sg2 = waveGrid(k2, ceil_div(A.nslices, WARPS));
     float* in = w.y32.p;
     float* ph = w.z32.p;
     float* sh = reinterpret_cast<float*>(w.z.p);
     for (long long it = 0; it < count; ++it) {
-        launchPdl(p_kernel<double>, vg, BS, s, n, V.p, V.r, V.v, in, S);
         amg->sa->apply(in, ph, S, s, sample);
         const int slot = sample ? profBegin(PROF_SPMV, false, spmvBytes<double>(A) - 4.0 * A.n, s) : -1;
         launchPdl(k1, sg1, BS, s, A.nslices, n, A.sl_off, A.col, M, (const float*)ph, V.v, V.r0, w.partials.p,
@@ -797,10 +861,10 @@ void iterateSmoothed(const SellMatrix& A, const double* M, Vecs<double> V, Amg* 
         profEnd(slot, s);
         launchPdl(s_kernel<double>, vg, BS, s, n, V.s, V.r, V.v, in, S);
         amg->sa->apply(in, sh, S, s);
-        launchPdl(k2, sg2, BS, s, A.nslices, n, A.sl_off, A.col, M, (const float*)sh, V.t, V.s, w.partials.p,
-                  w.counter.p, S);
-        launchPdl(xr_kernel<double, float>, vg, BS, s, n, V.x, V.r, (const float*)ph, (const float*)sh, V.s, V.t, V.r0,
+        launchPdl(k2, sg2, BS, s, A.nslices, n, A.sl_off, A.col, M, (const float*)sh, V.t, V.s, V.r, V.v, V.r0,
                   w.partials.p, w.counter.p, S);
+        launchPdl(xrp_kernel<double, float>, vg, BS, s, n, V.x, V.r, V.p, (const float*)ph, (const float*)sh, V.s, V.t,
+                  V.v, in, S);
     }
 }
 
@@ -848,7 +912,7 @@ bool graphsEnabled() {
 
 // A batch of iterations. The first batch of a solve runs kernel by kernel (and
 // feeds the SpMV timing samples); later batches replay one iteration captured
-// as a CUDA graph (~90 kernels with an AMG V-cycle on each side), re-captured
+// as a CUDA graph, re-captured
 // only when an operand changes. Kernels after convergence return at once, so
 // replays past the end of a batch change nothing.
 template <typename T>
@@ -921,6 +985,10 @@ void iterate(const SellMatrix& A, const T* M, Vecs<T> V, Amg* amg, T* y, T* z, l
     launchCounter().fetch_add(g.kernels * batch);
 }
 
+// iterations before the next look at the state, after `done` of them: the ones past the end of
+// a solve are launches for nothing, a look costs a few microseconds of an idle device
+long long nextBatch(long long done) { return std::min<long long>(std::max<long long>(8, done / 4), 64); }
+
 // BiCGSTAB iterations on (M, rhs) from the current x; returns iterations done.
 template <typename T>
 KrylovOut runBicgstab(const SellMatrix& A, const T* M, const T* rhs, Vecs<T> V, bool from_zero, double tol,
@@ -948,7 +1016,8 @@ KrylovOut runBicgstab(const SellMatrix& A, const T* M, const T* rhs, Vecs<T> V, 
             }
         }
         if (!flex) {
-            init_kernel<T><<<vg, BS, 0, s>>>(n, V.r, rhs, V.r0, V.p, V.v, zero ? 1 : 0, tol, w.partials.p, w.counter.p,
+            init_kernel<T><<<vg, BS, 0, s>>>(n, V.r, rhs, V.r0, V.p, V.v,
+                                             mode == KM_BICGSTAB_SA && sizeof(T) == 8 ? w.y32.p : nullptr, zero ? 1 : 0, tol, w.partials.p, w.counter.p,
                                              S); countLaunch();
         }
         PB_LAUNCH("bicgstab init");
@@ -963,7 +1032,7 @@ KrylovOut runBicgstab(const SellMatrix& A, const T* M, const T* rhs, Vecs<T> V, 
             PB_CUDA(cudaStreamSynchronize(s));
             done = w.host_state->done;
             if (done != 0) break;
-            batch = std::min<long long>(batch * 2, 64);
+            batch = nextBatch(w.host_state->iter);
         }
         out.iterations = w.host_state->iter;
         if (done == 3) {
@@ -1178,7 +1247,7 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
                 done = reliable(1);
                 continue;
             }
-            batch = std::min<long long>(batch * 2, 64);
+            batch = nextBatch(w.host_state->iter);
             continue;
         }
         longest = std::max(longest, seg);
@@ -1190,6 +1259,7 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
                 done = reliable(1);
             } else {
                 done = reliable(0);
+                p_kernel<float><<<vg, BS, 0, s>>>(n, w.p32.p, w.r32.p, w.v32.p, S); countLaunch();
             }
             continue;
         }
@@ -1561,7 +1631,8 @@ void emitBicgstab(const SellMatrix& A, const double* b, double* x, double tol, l
         fcg_init_kernel<<<vg, BS, 0, sub>>>(n, V.r, b, V.p, V.v, precondIn32(mode) ? w.y32.p : nullptr, tol,
                                             w.partials.p, w.counter.p, S); countLaunch();
     } else {
-        init_kernel<double><<<vg, BS, 0, sub>>>(n, V.r, b, V.r0, V.p, V.v, 0, tol, w.partials.p, w.counter.p, S); countLaunch();
+        init_kernel<double><<<vg, BS, 0, sub>>>(n, V.r, b, V.r0, V.p, V.v,
+                                                mode == KM_BICGSTAB_SA ? w.y32.p : nullptr, 0, tol, w.partials.p, w.counter.p, S); countLaunch();
     }
     endConditional(sub);
     beginConditional(body, cudaGraphCondTypeIf, ht, sub);
