@@ -25,6 +25,7 @@
 #include <cstring>
 
 #include "batched.h"
+#include "reduce.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -70,10 +71,6 @@ __device__ __forceinline__ int stateOf(const BState* st, int p) { return __ldcg(
 __device__ __forceinline__ double ld(const double* a, int i) { return __ldcg(a + i); }
 __device__ __forceinline__ float ld(const float* a, int i) { return __ldcg(a + i); }
 
-__device__ __forceinline__ double warpSum(double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
-}
 // block-wide sums of a and b (valid in thread 0); sh holds 2 * MAX_BLOCK / 32 doubles
 __device__ __forceinline__ void blockSum2(double& a, double& b, double* sh) {
     a = warpSum(a);
@@ -927,10 +924,417 @@ std::vector<BatchOut> runBatch(const std::vector<BatchSystem>& sys, BatchPlan& p
     return out;
 }
 
+
+// ---------------------------------------------------------------- flexible CG over the batch
+// Symmetric systems: one flexible CG (krylov.cu) over the block-diagonal matrix, every system
+// with its own scalars, preconditioned by one smoothed-aggregation hierarchy of the whole
+// (aggregates never straddle systems: nothing couples them). It takes 20-30 iterations where
+// Jacobi-BiCGSTAB takes 100-300: 24 systems of 16^3 to 48^3 rows in 4.3 instead of 23.5 ms.
+// Reductions are per slice (one warp), then per system (one block, in a fixed order).
+struct FState {
+    double rr, bb, tol2, dq, dr, alpha, beta, rel;
+    long long iter;
+    int done;  // as KState::done: 0 running, 1 converged, 2 iteration cap, 3 breakdown, 4 b = 0, 5 non-finite
+    int restart, pass, restarts, status;
+};
+constexpr int FLEX_MIN_ROWS = 8192;
+constexpr int FLEX_MAX_ITER = 500;  // iterations (20-30 are usual) after which it has failed
+constexpr int FLEX_UNROLL = 2;      // iterations per pass of the device loop
+
+struct FP {
+    int nprob, nslices;
+    const int *slice_prob, *prob_slice0, *sl_off, *col;
+    const double *A, *b;
+    double *x, *r, *d, *q, *u, *part;  // part: 3 per slice
+    float *r32, *z;
+    FState* st;
+    double tol;
+    long long maxit;
+};
+
+__global__ void flex_begin_kernel(const FP P) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= P.nprob) return;
+    FState z{};
+    z.restart = 1;
+    z.status = PRISM_OK;
+    P.st[p] = z;
+}
+
+// f(slice, system) for every slice, one warp each
+template <typename F>
+__device__ __forceinline__ void forSlices(const FP& P, F f) {
+    const int nw = gridDim.x * (BS / 32);
+    for (int sl = blockIdx.x * (BS / 32) + (threadIdx.x >> 5); sl < P.nslices; sl += nw) f(sl, P.slice_prob[sl]);
+}
+template <typename X>
+__device__ __forceinline__ double sliceDot(const FP& P, int sl, int lane, const X* __restrict__ v) {
+    const int b = P.sl_off[sl], width = (P.sl_off[sl + 1] - b) >> 5;
+    double sum = 0.0;
+    for (int j0 = 0; j0 < width; j0 += 4) {
+        int c[4];
+        double m[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (j0 + j < width) {
+                c[j] = __ldcs(P.col + b + 32 * (j0 + j) + lane);
+                m[j] = __ldcs(P.A + b + 32 * (j0 + j) + lane);
+            }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (j0 + j < width) sum += m[j] * (double)__ldg(v + c[j]);
+    }
+    return sum;
+}
+__device__ __forceinline__ void slicePartials(const FP& P, int sl, int lane, double a, double b, double c) {
+    a = warpSum(a);
+    b = warpSum(b);
+    c = warpSum(c);
+    if (lane == 0) {
+        P.part[3 * (int64_t)sl] = a;
+        P.part[3 * (int64_t)sl + 1] = b;
+        P.part[3 * (int64_t)sl + 2] = c;
+    }
+}
+// the system's sums of the slice partials, valid in thread 0 (one block per system)
+__device__ __forceinline__ void systemSums(const FP& P, int pr, double (&t)[3]) {
+    __shared__ double sh[3][BS / 32];
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int c = P.prob_slice0[pr] + threadIdx.x; c < P.prob_slice0[pr + 1]; c += BS)
+        for (int k = 0; k < 3; ++k) v[k] += P.part[3 * (int64_t)c + k];
+    for (int k = 0; k < 3; ++k) {
+        v[k] = warpSum(v[k]);
+        if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = v[k];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int k = 0; k < 3; ++k) {
+            t[k] = 0.0;
+            for (int w = 0; w < BS / 32; ++w) t[k] += sh[k][w];
+        }
+}
+
+// (re)started systems: r = b - A x, d = q = 0
+__global__ void __launch_bounds__(BS) flex_init_kernel(const FP P) {
+    const int lane = threadIdx.x & 31;
+    forSlices(P, [&](int sl, int pr) {
+        if (!P.st[pr].restart) return;
+        const int i = sl * 32 + lane;
+        const double bi = P.b[i], ri = bi - sliceDot(P, sl, lane, P.x);
+        P.r[i] = ri;
+        P.r32[i] = (float)ri;
+        P.d[i] = 0.0;
+        P.q[i] = 0.0;
+        slicePartials(P, sl, lane, ri * ri, bi * bi, 0.0);
+    });
+}
+__global__ void __launch_bounds__(BS) flex_init_reduce_kernel(const FP P) {
+    FState& S = P.st[blockIdx.x];
+    if (!S.restart) return;
+    double t[3];
+    systemSums(P, blockIdx.x, t);
+    if (threadIdx.x) return;
+    S.rr = t[0];
+    S.bb = t[1];
+    S.tol2 = P.tol * P.tol * t[1];
+    S.dq = 1.0;
+    S.dr = 0.0;
+    S.done = !isfinite(t[0]) || !isfinite(t[1]) ? 5 : t[1] == 0.0 ? 4 : t[0] <= S.tol2 ? 1 : 0;
+}
+// u = A z ; z.q, z.u, z.r
+__global__ void __launch_bounds__(BS) flex_spmv_kernel(const FP P) {
+    pdlEnter();
+    const int lane = threadIdx.x & 31;
+    forSlices(P, [&](int sl, int pr) {
+        if (P.st[pr].done) return;
+        const int i = sl * 32 + lane;
+        const double sum = sliceDot(P, sl, lane, P.z), zi = (double)P.z[i];
+        P.u[i] = sum;
+        slicePartials(P, sl, lane, zi * P.q[i], zi * sum, zi * P.r[i]);
+    });
+}
+__global__ void __launch_bounds__(BS) flex_direction_kernel(const FP P) {
+    pdlEnter();
+    FState& S = P.st[blockIdx.x];
+    if (S.done) return;
+    double t[3];
+    systemSums(P, blockIdx.x, t);
+    if (threadIdx.x) return;
+    const double beta = t[0] / S.dq;
+    const double dq = t[1] - beta * t[0], dr = t[2] - beta * S.dr, alpha = dr / dq;
+    if (!isfinite(t[0]) || !isfinite(t[1]) || !isfinite(t[2])) S.done = 5;
+    else if (!(dq > 0.0) || !isfinite(alpha)) S.done = 3;
+    S.beta = beta;
+    S.alpha = alpha;
+}
+// d = z - beta d ; q = u - beta q ; x += alpha d ; r -= alpha q ; r.r, d.q, d.r
+__global__ void __launch_bounds__(BS) flex_update_kernel(const FP P) {
+    pdlEnter();
+    const int lane = threadIdx.x & 31;
+    forSlices(P, [&](int sl, int pr) {
+        const FState& S = P.st[pr];
+        if (S.done) return;
+        const double alpha = S.alpha, beta = S.beta;
+        const int i = sl * 32 + lane;
+        const double di = (double)P.z[i] - beta * P.d[i];
+        const double qi = P.u[i] - beta * P.q[i];
+        const double ri = P.r[i] - alpha * qi;
+        P.x[i] += alpha * di;
+        P.d[i] = di;
+        P.q[i] = qi;
+        P.r[i] = ri;
+        P.r32[i] = (float)ri;
+        slicePartials(P, sl, lane, ri * ri, di * qi, di * ri);
+    });
+}
+__global__ void __launch_bounds__(BS) flex_convergence_kernel(const FP P) {
+    pdlEnter();
+    FState& S = P.st[blockIdx.x];
+    if (S.done) return;
+    double t[3];
+    systemSums(P, blockIdx.x, t);
+    if (threadIdx.x) return;
+    S.rr = t[0];
+    S.dq = t[1];
+    S.dr = t[2];
+    S.iter += 1;
+    if (!isfinite(t[0]) || !isfinite(t[1])) S.done = 5;
+    else if (t[0] <= S.tol2) S.done = 1;
+    else if (S.iter >= P.maxit) S.done = 2;
+    else if (!(t[1] > 0.0)) S.done = 3;
+}
+// the loop goes on while a system is running
+__global__ void flex_running_kernel(const FP P, cudaGraphConditionalHandle loop) {
+    int any = 0;
+    for (int p = threadIdx.x; p < P.nprob; p += blockDim.x) any |= P.st[p].done == 0;
+    any = __syncthreads_or(any);
+    if (threadIdx.x == 0) cudaGraphSetConditional(loop, any ? 1u : 0u);
+}
+// b - A x of every system started in this pass (x = 0 where b = 0)
+__global__ void __launch_bounds__(BS) flex_residual_kernel(const FP P) {
+    const int lane = threadIdx.x & 31;
+    forSlices(P, [&](int sl, int pr) {
+        if (!P.st[pr].restart) return;
+        const int i = sl * 32 + lane;
+        const double e = P.b[i] - sliceDot(P, sl, lane, P.x);
+        slicePartials(P, sl, lane, e * e, 0.0, 0.0);
+    });
+}
+__global__ void flex_zero_kernel(const FP P) {
+    const int lane = threadIdx.x & 31;
+    forSlices(P, [&](int sl, int pr) {
+        if (P.st[pr].restart && P.st[pr].done == 4) P.x[sl * 32 + lane] = 0.0;
+    });
+}
+// the end of a pass: accept, or start again from x (the recursive residual drifted, or the
+// recurrence broke down), as bicgstab() does
+__global__ void __launch_bounds__(BS) flex_pass_kernel(const FP P) {
+    FState& S = P.st[blockIdx.x];
+    if (!S.restart) return;
+    double t[3];
+    systemSums(P, blockIdx.x, t);
+    if (threadIdx.x) return;
+    S.rel = S.bb > 0.0 ? sqrt(t[0] / S.bb) : 0.0;
+    S.restart = 0;
+    if (S.done == 1) {
+        if (S.rel > 10 * P.tol && ++S.pass < 4) S.restart = 1;
+    } else if (S.done == 3) {
+        if (++S.restarts > 20) S.status = PRISM_BREAKDOWN;
+        else S.restart = 1;
+    } else if (S.done == 2) {
+        S.status = PRISM_NOT_CONVERGED;
+    } else if (S.done == 5 || !isfinite(S.rel)) {
+        S.status = PRISM_NONFINITE;
+    }
+}
+__global__ void flex_again_kernel(const FP P, cudaGraphConditionalHandle loop) {
+    int any = 0;
+    for (int p = threadIdx.x; p < P.nprob; p += blockDim.x) any |= P.st[p].restart;
+    any = __syncthreads_or(any);
+    if (threadIdx.x == 0) cudaGraphSetConditional(loop, any ? 1u : 0u);
+}
+__global__ void flex_open_kernel(cudaGraphConditionalHandle loop) { cudaGraphSetConditional(loop, 1u); }
+
+// the block-diagonal CSR pattern, one system per launch: row starts (padding rows empty), columns
+__global__ void flex_pattern_kernel(int n, int padded, const int* rowptr, const int* col, int nnz, int row0, int entry0,
+                                    int* rp, int* cc) {
+    const int t = blockIdx.x * BS + threadIdx.x;
+    if (t < padded) rp[row0 + t] = entry0 + (t < n ? rowptr[t] : nnz);
+    for (int k = t; k < nnz; k += gridDim.x * BS) cc[entry0 + k] = col[k] + row0;
+}
+
+// Solves the batch in one graph launch; false (and the guesses put back) if a system failed.
+bool runFlex(const std::vector<BatchSystem>& sys, BatchPlan& pl, double tol, long long maxit, bool own_cap,
+             std::vector<BatchOut>& out, cudaStream_t s) {
+    const int nrows = pl.nslices * 32;
+    if (!pl.rowptr) {
+        int64_t nnz = 0;
+        for (const auto& q : sys) nnz += q.nnz_csr;
+        pl.nnz_csr = nnz;
+        pl.rowptr.alloc((size_t)nrows + 1);
+        pl.csr_col.alloc(std::max<int64_t>(nnz, 1));
+        int64_t off = 0;
+        for (size_t i = 0; i < sys.size(); ++i) {
+            const BatchSystem& q = sys[i];
+            flex_pattern_kernel<<<grid(std::max(32 * q.nslices, 1)), BS, 0, s>>>(
+                q.n, 32 * q.nslices, q.rowptr, q.col, (int)q.nnz_csr, 32 * pl.slice0[i], (int)off, pl.rowptr.p, pl.csr_col.p); countLaunch();
+            off += q.nnz_csr;
+        }
+        const int last = (int)nnz;
+        PB_CUDA(cudaMemcpyAsync(pl.rowptr.p + nrows, &last, sizeof(int), cudaMemcpyHostToDevice, s));
+        PB_CUDA(cudaStreamSynchronize(s));
+        for (auto* b : {&pl.fr, &pl.fd, &pl.fq, &pl.fu, &pl.x0}) {
+            b->alloc(nrows);
+            b->zero(s);
+        }
+        for (auto* b : {&pl.fr32, &pl.fz32}) {
+            b->alloc(nrows);
+            b->zero(s);
+        }
+        pl.fstate.alloc(sizeof(FState) * pl.nprob);
+        pl.sa = std::make_unique<SaAmg>();
+        pl.cs = std::make_unique<CaptureStreams>();
+    }
+    SellMatrix A;
+    A.n = nrows;
+    A.nslices = pl.nslices;
+    A.nnz_padded = pl.nnz;
+    A.sl_off = pl.sl_off.p;
+    A.col = pl.col.p;
+    A.diag_pos = pl.diag.p;
+    A.vals = pl.A64.p;
+    A.nnz_csr = pl.nnz_csr;
+    FP P{};
+    P.nprob = pl.nprob;
+    P.nslices = pl.nslices;
+    P.slice_prob = pl.slice_prob.p;
+    P.prob_slice0 = pl.prob_slice0.p;
+    P.sl_off = pl.sl_off.p;
+    P.col = pl.col.p;
+    P.A = pl.A64.p;
+    P.b = pl.b64.p;
+    P.x = pl.x64.p;
+    P.r = pl.fr.p;
+    P.d = pl.fd.p;
+    P.q = pl.fq.p;
+    P.u = pl.fu.p;
+    P.part = pl.cdot.p;
+    P.r32 = pl.fr32.p;
+    P.z = pl.fz32.p;
+    P.st = reinterpret_cast<FState*>(pl.fstate.p);
+    P.tol = tol;
+    P.maxit = std::min<long long>(maxit, FLEX_MAX_ITER);
+
+    std::vector<CopyEntry> tab(sys.size());
+    std::vector<uintptr_t> key = {2, (uintptr_t)P.maxit, 0};
+    uint64_t bits;
+    std::memcpy(&bits, &tol, sizeof bits);
+    key[2] = (uintptr_t)bits;
+    for (size_t i = 0; i < sys.size(); ++i) {
+        const BatchSystem& q = sys[i];
+        tab[i] = {q.vals, q.b, q.x, (long long)q.nnz_padded, (long long)pl.nnz_off[i], 32LL * pl.slice0[i], q.n};
+        for (uintptr_t v : {(uintptr_t)q.vals, (uintptr_t)q.b, (uintptr_t)q.x}) key.push_back(v);
+    }
+    const CopyEntry* dtab = reinterpret_cast<const CopyEntry*>(pl.copy_tab.p);
+    const dim3 copy_grid(64, (unsigned)sys.size());
+    const int sg = std::max(1, std::min(ceil_div(pl.nslices, BS / 32), NUM_SMS * 8));
+    auto gather = [&] {
+        batch_copy_kernel<<<copy_grid, BS, 0, s>>>(dtab, 0, pl.A64.p, pl.b64.p, pl.x64.p); countLaunch();
+        PB_CUDA(cudaMemcpyAsync(pl.x0.p, pl.x64.p, nrows * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    };
+    auto scatter = [&] {
+        batch_copy_kernel<<<copy_grid, BS, 0, s>>>(dtab, 1, pl.A64.p, pl.b64.p, pl.x64.p); countLaunch();
+    };
+    if (!(pl.graph.g && key == pl.graph_key)) {
+        pl.graph.reset();
+        pl.graph_key.clear();
+        const size_t bytes = tab.size() * sizeof(CopyEntry);
+        if (pl.copy_tab.n < bytes) pl.copy_tab.alloc(bytes);
+        pl.copy_tab.upload(reinterpret_cast<const unsigned char*>(tab.data()), bytes, s);
+        dtab = reinterpret_cast<const CopyEntry*>(pl.copy_tab.p);
+        if (!pl.sa->built) {
+            gather();
+            pl.sa->setup(A, pl.rowptr.p, pl.csr_col.p, true, false, s);
+        }
+        PB_CUDA(cudaStreamSynchronize(s));
+        cudaStream_t passes = pl.cs->at(0), loop = pl.cs->at(1);
+        PB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
+        cudaGraph_t g = nullptr;
+        try {
+            gather();
+            pl.sa->setup(A, pl.rowptr.p, pl.csr_col.p, true, false, s);
+            flex_begin_kernel<<<grid(pl.nprob), BS, 0, s>>>(P); countLaunch();
+            cudaGraphConditionalHandle again = createConditional(s, 0);
+            flex_open_kernel<<<1, 1, 0, s>>>(again); countLaunch();
+            beginConditional(s, cudaGraphCondTypeWhile, again, passes);
+            flex_init_kernel<<<sg, BS, 0, passes>>>(P); countLaunch();
+            flex_init_reduce_kernel<<<pl.nprob, BS, 0, passes>>>(P); countLaunch();
+            cudaGraphConditionalHandle running = createConditional(passes, 0);
+            flex_running_kernel<<<1, BS, 0, passes>>>(P, running); countLaunch();
+            beginConditional(passes, cudaGraphCondTypeWhile, running, loop);
+            for (int k = 0; k < FLEX_UNROLL; ++k) {
+                pl.sa->apply(P.r32, P.z, nullptr, loop);
+                launchPdl(flex_spmv_kernel, sg, BS, loop, P);
+                launchPdl(flex_direction_kernel, pl.nprob, BS, loop, P);
+                launchPdl(flex_update_kernel, sg, BS, loop, P);
+                launchPdl(flex_convergence_kernel, pl.nprob, BS, loop, P);
+            }
+            flex_running_kernel<<<1, BS, 0, loop>>>(P, running); countLaunch();
+            endConditional(loop);
+            flex_zero_kernel<<<sg, BS, 0, passes>>>(P); countLaunch();
+            flex_residual_kernel<<<sg, BS, 0, passes>>>(P); countLaunch();
+            flex_pass_kernel<<<pl.nprob, BS, 0, passes>>>(P); countLaunch();
+            flex_again_kernel<<<1, BS, 0, passes>>>(P, again); countLaunch();
+            endConditional(passes);
+            scatter();
+        } catch (...) {
+            cudaStreamEndCapture(s, &g);
+            if (g) cudaGraphDestroy(g);
+            cudaGetLastError();
+            throw;
+        }
+        PB_CUDA(cudaStreamEndCapture(s, &g));
+        const cudaError_t e = cudaGraphInstantiate(&pl.graph.g, g, 0);
+        cudaGraphDestroy(g);
+        if (e != cudaSuccess) pl.graph.g = nullptr;
+        PB_CUDA(e);
+        pl.graph_key = key;
+    }
+    PB_CUDA(cudaGraphLaunch(pl.graph.g, s));
+    graphLaunchCounter().fetch_add(1, std::memory_order_relaxed);
+    std::vector<FState> hs(pl.nprob);
+    PB_CUDA(cudaMemcpyAsync(hs.data(), P.st, pl.nprob * sizeof(FState), cudaMemcpyDeviceToHost, s));
+    PB_CUDA(cudaStreamSynchronize(s));
+    out.assign(pl.nprob, BatchOut{});
+    bool ok = true;
+    for (int i = 0; i < pl.nprob; ++i) {
+        out[i].iterations = hs[i].iter;
+        out[i].passes = hs[i].pass + 1;
+        out[i].rel_residual = hs[i].rel;
+        out[i].status = hs[i].status;
+        const bool capped = own_cap && hs[i].status == PRISM_NOT_CONVERGED && hs[i].iter >= maxit;
+        ok = ok && (hs[i].status == PRISM_OK || capped);
+    }
+    if (verbose()) {
+        long long most = 0;
+        for (const auto& q : out) most = std::max<long long>(most, q.iterations);
+        std::fprintf(stderr, "[prism] batched flexible CG of %d systems (%d rows): at most %lld iterations, %s\n", pl.nprob,
+                     nrows, most, ok ? "ok" : "failed");
+    }
+    if (!ok) {
+        PB_CUDA(cudaMemcpyAsync(pl.x64.p, pl.x0.p, nrows * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        scatter();
+        pl.graph.reset();
+        pl.graph_key.clear();
+    }
+    return ok;
+}
+
 }  // namespace
 
 std::vector<BatchOut> solveBatch(const std::vector<BatchSystem>& sys, BatchPlan& pl, bool mixed, double tol,
-                                 double itol, int max_inner, int max_pass, long long maxit, cudaStream_t s) {
+                                 double itol, int max_inner, int max_pass, long long maxit, bool own_cap,
+                                 cudaStream_t s) {
     if (sys.empty()) return {};
     std::vector<uintptr_t> key;
     for (const auto& q : sys) {
@@ -995,6 +1399,18 @@ std::vector<BatchOut> solveBatch(const std::vector<BatchSystem>& sys, BatchPlan&
         pl.ctl.alloc(4);
         PB_CUDA(cudaStreamSynchronize(s));
         PB_LAUNCH("batched plan");
+    }
+    int64_t rows = 0, entries = 0;
+    bool symmetric = !pl.no_flex;
+    for (const auto& q : sys) {
+        rows += q.n;
+        entries += q.nnz_csr;
+        symmetric = symmetric && q.symmetric;
+    }
+    if (symmetric && rows >= FLEX_MIN_ROWS && entries < ((int64_t)1 << 28) && sys.size() <= 65535) {
+        std::vector<BatchOut> out;
+        if (runFlex(sys, pl, tol, maxit, own_cap, out, s)) return out;
+        pl.no_flex = true;
     }
     if (mixed) return runBatch<float>(sys, pl, tol, itol, max_inner, max_pass, maxit, s);
     return runBatch<double>(sys, pl, tol, itol, max_inner, max_pass, maxit, s);

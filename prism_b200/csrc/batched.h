@@ -1,9 +1,12 @@
 // batched.h -- many independent linear solves in one persistent launch.
 #pragma once
 
+#include <memory>
 #include <vector>
 
 #include "common.h"
+#include "krylov.h"
+#include "samg.h"
 
 namespace pb {
 
@@ -14,13 +17,17 @@ struct BatchSystem {
     const int* sl_off = nullptr;
     const int* sl_col = nullptr;
     const int* diag_pos = nullptr;
+    const int* rowptr = nullptr;  // the CSR view of the pattern, in the order of the SELL slots
+    const int* col = nullptr;
+    int64_t nnz_csr = 0;
+    bool symmetric = false;  // by construction
     const double* vals = nullptr;
     const double* b = nullptr;
     double* x = nullptr;
 };
 
 struct BatchOut {
-    int64_t iterations = 0;  // BiCGSTAB iterations (inner, all passes)
+    int64_t iterations = 0;  // Krylov iterations (all passes)
     int32_t passes = 0;      // refinement passes
     double rel_residual = 0; // FP64 ||b - Ax|| / ||b|| at the end
     int32_t status = PRISM_OK;
@@ -46,6 +53,16 @@ struct BatchPlan {
     DevBuf<unsigned char> state;  // per-problem solver state
     DevBuf<int> ctl;
     BatchTuning tune[2];  // [0] FP64 inner, [1] FP32 inner
+    // flexible CG over the block-diagonal matrix (symmetric systems): its CSR pattern,
+    // multigrid hierarchy, vectors, saved guesses and per-system states
+    int64_t nnz_csr = 0;
+    DevBuf<int> rowptr, csr_col;
+    std::unique_ptr<SaAmg> sa;
+    DevBuf<double> fr, fd, fq, fu, x0;
+    DevBuf<float> fr32, fz32;
+    DevBuf<unsigned char> fstate;
+    std::unique_ptr<CaptureStreams> cs;
+    bool no_flex = false;  // it failed once on these patterns: BiCGSTAB from then on
     // per call: the systems' values, right-hand sides and guesses gathered into the
     // concatenated buffers by one kernel (table of source pointers), and the whole
     // call -- gather, set-up, the persistent solve, scatter of the solutions -- kept
@@ -72,12 +89,15 @@ struct BatchPlan {
     } graph;
 };
 
-// Solves every system to ||b - Ax|| <= tol ||b|| (FP64 residual): BiCGSTAB
+// Solves every system to ||b - Ax|| <= tol ||b|| (FP64 residual). Symmetric systems, from
+// FLEX_MIN_ROWS rows in all: flexible CG with smoothed aggregation over the block-diagonal
+// matrix, each system with its own scalars (BiCGSTAB should one fail). Others: BiCGSTAB
 // inner iterations (FP32 with FP64 dots when mixed, else FP64), Jacobi right
 // preconditioning by column scaling, restarted inner solves reducing the
 // residual by itol, FP64 iterative refinement between them, all inside one
-// cooperative launch. x holds the initial guesses and receives the solutions.
+// cooperative launch. own_cap: maxit is the caller's. x holds the initial guesses and receives the solutions.
 std::vector<BatchOut> solveBatch(const std::vector<BatchSystem>& sys, BatchPlan& plan, bool mixed, double tol,
-                                 double itol, int max_inner, int max_pass, long long maxit, cudaStream_t s);
+                                 double itol, int max_inner, int max_pass, long long maxit, bool own_cap,
+                                 cudaStream_t s);
 
 }  // namespace pb

@@ -1371,16 +1371,21 @@ void explicitUpdate(const SellMatrix& A, const double* b, const double* x, doubl
     PB_LAUNCH("explicit_kernel");
 }
 
-double scaledResidual(const SellMatrix& A, const double* b, const double* x, KrylovWork& w, cudaStream_t s) {
+void scaledResidualParts(const SellMatrix& A, const double* b, const double* x, KrylovWork& w, double* h,
+                         cudaStream_t s) {
     w.ensure(A.nslices * 32, A.nnz_padded, false);
     resid_kernel<<<waveGrid(resid_kernel, ceil_div(A.nslices, WARPS)), BS, 0, s>>>(A.nslices, A.n, A.sl_off, A.col, A.vals, A.diag_pos, b, x,
                                                      w.partials.p, w.counter.p, w.scal.p); countLaunch();
     PB_LAUNCH("resid_kernel");
-    double h[3];
     PB_CUDA(cudaMemcpyAsync(h, w.scal.p, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
+}
+double scaledResidualOf(const double* h) { return h[2] != 0.0 ? NAN : h[0] / (h[1] + EPSILON); }
+
+double scaledResidual(const SellMatrix& A, const double* b, const double* x, KrylovWork& w, cudaStream_t s) {
+    double h[3];
+    scaledResidualParts(A, b, x, w, h, s);
     PB_CUDA(cudaStreamSynchronize(s));
-    if (h[2] != 0.0) return NAN;
-    return h[0] / (h[1] + EPSILON);
+    return scaledResidualOf(h);
 }
 
 double offDiagonalRatio(const SellMatrix& A, KrylovWork& w, cudaStream_t s) {

@@ -108,6 +108,9 @@ bool smoothedFits(const SellMatrix& A);
 void jacobiStep(const SellMatrix& A, const double* b, double* x, KrylovWork& w, cudaStream_t s);
 // max|A x - b| / (max|diag(A) x| + eps)   (numerics/solver.cpp:8-24); returns NaN if non-finite values met
 double scaledResidual(const SellMatrix& A, const double* b, const double* x, KrylovWork& w, cudaStream_t s);
+// the same in two halves: its three parts on their way to h (pinned), and the value once there
+void scaledResidualParts(const SellMatrix& A, const double* b, const double* x, KrylovWork& w, double* h, cudaStream_t s);
+double scaledResidualOf(const double* h);
 // max over rows of sum_{j != i} |a_ij| / |a_ii| (inf for a zero diagonal): below 1, Jacobi
 // converges at least that fast, whatever the coupling
 double offDiagonalRatio(const SellMatrix& A, KrylovWork& w, cudaStream_t s);

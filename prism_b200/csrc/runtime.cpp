@@ -1130,7 +1130,17 @@ FixedPointOut adjointBackward(Transport& eq, const double* dJ, double* gk, doubl
 namespace pb {
 
 // ------------------------------------------------------------------ batched solves
+double* BatchHandle::residuals(size_t n) {
+    if (n > host_n) {
+        if (host) cudaFreeHost(host);
+        host = nullptr;
+        PB_CUDA(cudaMallocHost(&host, 3 * n * sizeof(double)));
+        host_n = n;
+    }
+    return host;
+}
 BatchHandle::~BatchHandle() {
+    if (host) cudaFreeHost(host);
     if (stream) {
         cudaStreamSynchronize(stream);
         cudaStreamDestroy(stream);
@@ -1153,8 +1163,7 @@ std::vector<PrismSolveResult> solveBatch(BatchHandle& h, std::vector<Transport*>
         relax(eq);
         ++eq.phi->event;
         SellMatrix A = m.matrix(eq.A.p);
-        res[i].initial_residual = scaledResidual(A, eq.b.p, eq.phi->v.p, m.kw, m.stream);
-        PB_CUDA(cudaStreamSynchronize(m.stream));
+        scaledResidualParts(A, eq.b.p, eq.phi->v.p, m.kw, h.residuals(eqs.size()) + 3 * i, m.stream);
         BatchSystem& q = sys[i];
         q.n = m.nc;
         q.nslices = m.pat.nslices;
@@ -1162,25 +1171,40 @@ std::vector<PrismSolveResult> solveBatch(BatchHandle& h, std::vector<Transport*>
         q.sl_off = m.pat.sl_off.p;
         q.sl_col = m.pat.sl_col.p;
         q.diag_pos = m.pat.diag_pos.p;
+        q.rowptr = m.pat.rowptr.p;
+        q.col = m.pat.col.p;
+        q.nnz_csr = m.pat.nnz;
+        q.symmetric = symmetricMatrix(eq);
         q.vals = eq.A.p;
         q.b = eq.b.p;
         q.x = eq.phi->v.p;
         maxn = std::max<int64_t>(maxn, m.nc);
     }
+    // every system assembled (each mesh on its own stream): one wait for all of them
+    auto drain = [&] {
+        for (auto* eq : eqs) PB_CUDA(cudaStreamSynchronize(eq->phi->m->stream));
+    };
+    drain();
+    for (size_t i = 0; i < eqs.size(); ++i) res[i].initial_residual = scaledResidualOf(h.residuals(eqs.size()) + 3 * i);
     const bool mixed = o.precision == PRISM_PREC_MIXED;
     const double tol = o.krylov_tol > 0 ? o.krylov_tol : 1e-12;
     const double itol = o.inner_tol > 0 ? o.inner_tol : (mixed ? 1e-4 : std::max(0.5 * tol, 1e-15));
     const long long maxit = o.krylov_max_iter > 0 ? o.krylov_max_iter : 2 * maxn;
     const int max_inner = (int)std::min<long long>(maxit, 1 << 30);
     const auto t1 = std::chrono::steady_clock::now();
-    std::vector<BatchOut> out = pb::solveBatch(sys, h.plan, mixed, tol, itol, max_inner, 64, maxit, h.stream);
+    std::vector<BatchOut> out = pb::solveBatch(sys, h.plan, mixed, tol, itol, max_inner, 64, maxit, o.krylov_max_iter > 0, h.stream);
     const auto t2 = std::chrono::steady_clock::now();
     for (size_t i = 0; i < eqs.size(); ++i) {
         Transport& eq = *eqs[i];
         Mesh& m = *eq.phi->m;
         eq.phi->event += 3;
         SellMatrix A = m.matrix(eq.A.p);
-        const double fin = scaledResidual(A, eq.b.p, eq.phi->v.p, m.kw, m.stream);
+        scaledResidualParts(A, eq.b.p, eq.phi->v.p, m.kw, h.residuals(eqs.size()) + 3 * i, m.stream);
+        if (o.clear_coeffs) zeroOutCoeffs(eq);
+    }
+    drain();
+    for (size_t i = 0; i < eqs.size(); ++i) {
+        const double fin = scaledResidualOf(h.residuals(eqs.size()) + 3 * i);
         PrismSolveResult& r = res[i];
         r.iterations = 1;
         r.final_residual = fin;
@@ -1188,7 +1212,6 @@ std::vector<PrismSolveResult> solveBatch(BatchHandle& h, std::vector<Transport*>
         r.status = std::isnan(fin) ? PRISM_NONFINITE : out[i].status;
         r.krylov_iterations = out[i].iterations;
         r.krylov_rel_residual = out[i].rel_residual;
-        if (o.clear_coeffs) zeroOutCoeffs(eq);
     }
     if (verbose()) {
         for (auto* eq : eqs) PB_CUDA(cudaStreamSynchronize(eq->phi->m->stream));

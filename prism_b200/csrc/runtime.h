@@ -216,6 +216,9 @@ FixedPointOut steadySolve(Transport& eq, const PrismSolveOpts& o, int max_outer,
 // relaxed on its mesh, then all systems are solved together in one persistent
 // launch (batched.h) and each field receives its solution.
 struct BatchHandle {
+    double* host = nullptr;  // pinned: the parts of each system's scaled residual
+    size_t host_n = 0;
+    double* residuals(size_t n);
     BatchPlan plan;
     cudaStream_t stream = nullptr;
     ~BatchHandle();

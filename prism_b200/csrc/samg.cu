@@ -172,9 +172,11 @@ __global__ void mis_decide_kernel(int n, const int* rowptr, const int* strong, u
     const int c = __syncthreads_count(open);
     if (threadIdx.x == 0 && c) atomicAdd(left, c);
 }
-__global__ void mis_root_kernel(int n, const unsigned long long* key, int* root) {
+// in the set (or still undecided after every round); a row without couplings needs no coarse
+// row: the smoother solves it
+__global__ void mis_root_kernel(int n, const unsigned long long* key, const float* wmax, int* root) {
     const int i = blockIdx.x * BS + threadIdx.x;
-    if (i < n) root[i] = key[i] != 0;  // in the set (or still undecided after every round)
+    if (i < n) root[i] = key[i] != 0 && wmax[i] > 0.f;
 }
 __global__ void root_label_kernel(int n, const int* root, const int* id, int* label) {
     const int i = blockIdx.x * BS + threadIdx.x;
@@ -202,13 +204,14 @@ __global__ void join_kernel(int n, const int* rowptr, const int* col, const int*
     out[i] = l;
 }
 
-// keys (row, aggregate) of P's pattern: every entry of A
+// keys (row, aggregate) of P's pattern: every entry of A; rows outside every aggregate give the
+// key past the last row
 __global__ void p_keys_kernel(int n, const int* rowptr, const int* col, const int* agg, long long nc, long long* keys) {
     const int i = blockIdx.x * BS + threadIdx.x;
     if (i >= n) return;
     for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) {
         const int a = agg[col[k]];
-        keys[k] = i * nc + (a >= 0 ? a : agg[i] >= 0 ? agg[i] : 0);
+        keys[k] = a >= 0 ? i * nc + a : agg[i] >= 0 ? i * nc + agg[i] : n * nc;
     }
 }
 // keys of a row product's pattern, one left entry per thread: the output row of entry k
@@ -807,14 +810,20 @@ int64_t patternOf(DevArena& ar, long long* keys, int64_t m, int nrows, long long
     TmpBuf<long long> sorted(std::max<int64_t>(m, 1), s);
     TmpBuf<int> count(1, s);
     int end_bit = 1;
-    while (end_bit < 63 && ((long long)1 << end_bit) < (long long)nrows * ncols) ++end_bit;
+    while (end_bit < 63 && ((long long)1 << end_bit) <= (long long)nrows * ncols) ++end_bit;
     size_t t0 = 0, t1 = 0;
     PB_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, t0, keys, sorted.p, m, 0, end_bit, s));
     PB_CUDA(cub::DeviceSelect::Unique(nullptr, t1, sorted.p, keys, count.p, m, s));
     TmpBuf<unsigned char> tmp(std::max<size_t>(std::max(t0, t1), 1), s);
     PB_CUDA(cub::DeviceRadixSort::SortKeys(tmp.p, t0, keys, sorted.p, m, 0, end_bit, s));
     PB_CUDA(cub::DeviceSelect::Unique(tmp.p, t1, sorted.p, keys, count.p, m, s));
-    const int64_t nnz = readInt(count.p, s);
+    int64_t nnz = readInt(count.p, s);
+    if (nnz > 0) {  // a key past the last row is no entry
+        long long last = 0;
+        PB_CUDA(cudaMemcpyAsync(&last, keys + nnz - 1, sizeof(long long), cudaMemcpyDeviceToHost, s));
+        PB_CUDA(cudaStreamSynchronize(s));
+        if (last == (long long)nrows * ncols) --nnz;
+    }
     rowptr.alloc(ar, (size_t)nrows + 1, s);
     col.alloc(ar, std::max<int64_t>(nnz, 1), s);
     key_cols_kernel<<<grid(nnz), BS, 0, s>>>(nnz, keys, ncols, col.p); countLaunch();
@@ -879,7 +888,7 @@ int aggregate(DevArena& ar, SaLevel& L, cudaStream_t s) {
         if (r % MIS_BATCH == MIS_BATCH - 1 && readInt(left.p + r + 1, s) == 0) break;
     }
     PB_CUDA(cudaMemsetAsync(root.p + n, 0, sizeof(int), s));
-    mis_root_kernel<<<grid(n), BS, 0, s>>>(n, key.p, root.p); countLaunch();
+    mis_root_kernel<<<grid(n), BS, 0, s>>>(n, key.p, wmax.p, root.p); countLaunch();
     size_t tb = 0;
     PB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, root.p, id.p, n + 1, s));
     TmpBuf<unsigned char> tmp(std::max<size_t>(tb, 1), s);
@@ -1032,7 +1041,7 @@ void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, bool s
         levelScaling(L, s);
         if (L.n <= COARSE_MAX || levels.size() >= (size_t)MAX_LEVELS) break;
         const int nc = aggregate(arena, L, s);
-        if (nc > (int)(0.8 * L.n)) break;
+        if (nc == 0 || nc > (int)(0.8 * L.n)) break;
         // P: the aggregates of a row's neighbours
         {
             TmpBuf<long long> keys(std::max<int64_t>(L.nnz, 1), s);
