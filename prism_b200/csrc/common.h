@@ -139,7 +139,7 @@ struct TmpBuf {
 // scratchPool() and returned all at once, for objects made of many buffers
 // (the AMG hierarchy): one pool call per chunk instead of one cudaMalloc per
 // buffer. Chunks grow geometrically (at least MIN_CHUNK, at least the total so
-// far). mark()/rewind() give back everything taken after the mark, for
+// far up to MAX_GROWTH: doubling a hierarchy of a gigabyte reserved twice what it used). mark()/rewind() give back everything taken after the mark, for
 // intermediates of a build; reset() gives back everything. Chunks are
 // allocated in order on the stream of the call, so work on that stream may use
 // them at once; the destructor waits for the device before freeing them.
@@ -172,7 +172,7 @@ public:
                 off_ += bytes;
                 return reinterpret_cast<T*>(p);
             }
-        size_t size = std::max(std::max(bytes, MIN_CHUNK), total_);
+        size_t size = std::max(std::max(bytes, MIN_CHUNK), std::min(total_, MAX_GROWTH));
         if (chunks_.empty()) PB_CUDA(cudaGetDevice(&device_));
         char* p = nullptr;
         PB_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), size, scratchPool(), s));
@@ -203,6 +203,7 @@ private:
     };
     static constexpr size_t ALIGN = 256;
     static constexpr size_t MIN_CHUNK = size_t(2) << 20;
+    static constexpr size_t MAX_GROWTH = size_t(128) << 20;
     std::vector<Chunk> chunks_;
     size_t cur_ = 0, off_ = 0, total_ = 0;
     int device_ = 0;  // device current when the first chunk was taken

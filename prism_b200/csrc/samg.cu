@@ -19,7 +19,7 @@
 //     The two halves of `down` share a launch; A is stored scaled by omega D^-1, so its
 //     pass gathers one vector. Q^T and Q hold fewer entries than A on 2-D meshes.
 //   * The smallest levels (TAIL_ROWS, TAIL_NNZ) run in one launch of a thread-block cluster.
-// The structure is built once per pattern (sorted 64-bit keys); every new matrix refreshes
+// The structure is built once per pattern; every new matrix refreshes
 // the values by gathers in a fixed order. For a symmetric matrix (A P)^T stands for P^T A;
 // otherwise the restriction is smoothed with A^T's values: R^T = (I - omega_p D^-1 A^T) P0
 // takes P^T's place and (S R^T)^T, S with A^T, that of Q^T (Sala and Tuminaro 2008).
@@ -274,6 +274,160 @@ __global__ void sorted_starts_kernel(int nrows, int64_t m, const int* sorted, in
     rowptr[r] = (int)lo;
 }
 
+// Patterns of row products by row: the distinct columns of the right rows that the left row
+// names, collected in shared memory, counted first and then written in increasing order (pass
+// two: out_rowptr given). Against sorting one 64-bit key per product this needs no memory
+// beyond the result: the keys of a 128^3 hex level 0 alone took 1.7 GB, whose mapping made
+// first solves wait for up to a second. A row with more columns than its table holds sets
+// *overflow and the sort takes over.
+struct Union {
+    int rows;
+    const int *l_rowptr, *l_idx;
+    const int *b_rowptr, *b_col;  // b_rowptr null: row j of B is the single column b_col[j] (none if negative)
+    const int* out_rowptr;
+    int *count, *out_col, *overflow;
+};
+
+template <int CAP>
+__global__ void __launch_bounds__(BS) union_thread_kernel(const Union U) {
+    __shared__ int cols[CAP][BS];
+    const int r = blockIdx.x * BS + threadIdx.x, t = threadIdx.x;
+    if (r >= U.rows) return;
+    int len = 0;
+    bool over = false;
+    auto insert = [&](int c) {
+        for (int k = 0; k < len; ++k)
+            if (cols[k][t] == c) return;
+        if (len == CAP) {
+            over = true;
+            return;
+        }
+        int k = len++;
+        for (; k > 0 && cols[k - 1][t] > c; --k) cols[k][t] = cols[k - 1][t];
+        cols[k][t] = c;
+    };
+    for (int q = U.l_rowptr[r]; q < U.l_rowptr[r + 1]; ++q) {
+        const int j = U.l_idx[q];
+        if (!U.b_rowptr) {
+            if (U.b_col[j] >= 0) insert(U.b_col[j]);
+        } else {
+            for (int e = U.b_rowptr[j]; e < U.b_rowptr[j + 1]; ++e) insert(U.b_col[e]);
+        }
+    }
+    if (over) *U.overflow = 1;
+    if (!U.out_rowptr) {
+        U.count[r] = len;
+        return;
+    }
+    const int o = U.out_rowptr[r];
+    for (int k = 0; k < len; ++k) U.out_col[o + k] = cols[k][t];
+}
+
+// T threads per row; groups of GL lanes take one left entry each; H slots (open addressing)
+template <int T, int GL, int H>
+__global__ void __launch_bounds__(BS) union_team_kernel(const Union U) {
+    constexpr int TEAMS = BS / T, G = T / GL, FULL = H / 4 * 3;
+    __shared__ int table[TEAMS][H], list[TEAMS][FULL + T], cnt[TEAMS];
+    const int team = threadIdx.x / T, t = threadIdx.x % T, grp = t / GL, gl = t % GL;
+    const int r = blockIdx.x * TEAMS + team;
+    if (r >= U.rows) return;  // whole teams
+    auto sync = [] {
+        if constexpr (T == 32) __syncwarp();
+        else __syncthreads();
+    };
+    for (int k = t; k < H; k += T) table[team][k] = -1;
+    if (t == 0) cnt[team] = 0;
+    sync();
+    volatile int* count = &cnt[team];
+    for (int q = U.l_rowptr[r] + grp; q < U.l_rowptr[r + 1]; q += G) {
+        const int j = U.l_idx[q];
+        for (int e = U.b_rowptr[j] + gl; e < U.b_rowptr[j + 1]; e += GL) {
+            if (*count >= FULL) break;  // overflow: set below
+            const int c = U.b_col[e];
+            unsigned at = ((unsigned)c * 2654435761u) & (H - 1);
+            for (int probe = 0; probe < H; ++probe, at = (at + 1) & (H - 1)) {
+                const int old = atomicCAS(&table[team][at], -1, c);
+                if (old == c) break;
+                if (old == -1) {
+                    atomicAdd(&cnt[team], 1);
+                    break;
+                }
+            }
+        }
+    }
+    sync();
+    const int len = cnt[team];
+    if (len >= FULL) {
+        if (t == 0) *U.overflow = 1;
+        if (t == 0 && !U.out_rowptr) U.count[r] = 0;
+        return;
+    }
+    if (!U.out_rowptr) {
+        if (t == 0) U.count[r] = len;
+        return;
+    }
+    sync();
+    if (t == 0) cnt[team] = 0;
+    sync();
+    for (int k = t; k < H; k += T)
+        if (table[team][k] >= 0) list[team][atomicAdd(&cnt[team], 1)] = table[team][k];
+    sync();
+    const int o = U.out_rowptr[r];
+    for (int a = t; a < len; a += T) {  // the place of a column: how many are smaller
+        const int c = list[team][a];
+        int rank = 0;
+        for (int b = 0; b < len; ++b) rank += list[team][b] < c;
+        U.out_col[o + rank] = c;
+    }
+}
+
+// Transpose of a CSR pattern: rows spread over the columns by counting, then every column's
+// rows put in increasing order
+__global__ void column_count_kernel(int64_t m, const int* col, int* count) {
+    const int64_t k = blockIdx.x * (int64_t)BS + threadIdx.x;
+    if (k < m) atomicAdd(&count[col[k]], 1);
+}
+__global__ void column_fill_kernel(int n, const int* rowptr, const int* col, const int* t_rowptr, int* cursor, int* t_row) {
+    const int i = blockIdx.x * BS + threadIdx.x;
+    if (i >= n) return;
+    for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) t_row[t_rowptr[col[k]] + atomicAdd(&cursor[col[k]], 1)] = i;
+}
+// src: transposed entry -> entry; place: entry -> transposed entry
+template <int T, int CAP>
+__global__ void __launch_bounds__(BS) column_sort_kernel(int nc, const int* t_rowptr, int* t_row, const int* rowptr,
+                                                         const int* col, int* src, int* place, int* overflow) {
+    constexpr int TEAMS = BS / T;
+    __shared__ int rows[TEAMS][CAP];
+    const int team = threadIdx.x / T, t = threadIdx.x % T;
+    const int c = blockIdx.x * TEAMS + team;
+    if (c >= nc) return;
+    auto sync = [] {
+        if constexpr (T == 32) __syncwarp();
+        else __syncthreads();
+    };
+    const int o = t_rowptr[c], len = t_rowptr[c + 1] - o;
+    if (len > CAP) {
+        if (t == 0) *overflow = 1;
+        return;
+    }
+    for (int k = t; k < len; k += T) rows[team][k] = t_row[o + k];
+    sync();
+    for (int a = t; a < len; a += T) {
+        const int i = rows[team][a];
+        int rank = 0;
+        for (int b = 0; b < len; ++b) rank += rows[team][b] < i;
+        t_row[o + rank] = i;
+        int e = rowptr[i], hi = rowptr[i + 1];  // the entry (i, c), columns sorted
+        while (e < hi) {
+            const int mid = (e + hi) >> 1;
+            if (col[mid] < c) e = mid + 1;
+            else hi = mid;
+        }
+        if (src) src[o + rank] = e;
+        if (place) place[e] = o + rank;
+    }
+}
+
 // ---------------------------------------------------------------- values
 // position of column c in the sorted list col[lo, hi), or -1
 __device__ __forceinline__ int findColumn(const int* __restrict__ col, int lo, int hi, int c) {
@@ -416,7 +570,7 @@ void launchProduct(const Product& P, int64_t nnz_out, int n_b, int64_t nnz_b, cu
     const double out = (double)nnz_out / std::max(P.rows, 1), right = (double)nnz_b / std::max(n_b, 1);
     // one thread per row only where the rows fill the chip: 2,309 rows take 86 us that way, 9 us
     // with a block each
-    if (P.rows > 16384 && out <= 12.0 && right <= 4.0) {
+    if (P.rows > 8192 && out <= 12.0 && right <= 4.0) {
         product_thread_kernel<12><<<grid(P.rows), BS, 0, s>>>(P);
     } else if (P.rows > 16384) {
         const int g = ceil_div(P.rows, BS / 32);
@@ -831,6 +985,48 @@ int64_t patternOf(DevArena& ar, long long* keys, int64_t m, int nrows, long long
     return nnz;
 }
 
+// exclusive offsets of count[0, n) into rowptr[0, n]; returns the total
+int64_t rowOffsets(TmpBuf<int>& count, int n, int* rowptr, cudaStream_t s) {
+    PB_CUDA(cudaMemsetAsync(count.p + n, 0, sizeof(int), s));
+    size_t tb = 0;
+    PB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, count.p, rowptr, n + 1, s));
+    TmpBuf<unsigned char> tmp(std::max<size_t>(tb, 1), s);
+    PB_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, count.p, rowptr, n + 1, s));
+    return readInt(rowptr + n, s);
+}
+
+// U's pattern (U.rows rows; the average numbers of left and right entries choose the kernel);
+// false if a row did not fit
+bool unionPattern(DevArena& ar, Union U, double left, double right, ArenaBuf<int>& rowptr, ArenaBuf<int>& col,
+                  int64_t& nnz, cudaStream_t s) {
+    TmpBuf<int> count((size_t)U.rows + 1, s), overflow(1, s);
+    PB_CUDA(cudaMemsetAsync(overflow.p, 0, sizeof(int), s));
+    U.count = count.p;
+    U.overflow = overflow.p;
+    auto run = [&] {
+        if (!U.b_rowptr || left * right <= 64.0) {
+            union_thread_kernel<32><<<grid(U.rows), BS, 0, s>>>(U);
+        } else if (U.rows > 16384) {
+            if (right <= 12.0) union_team_kernel<32, 8, 256><<<ceil_div(U.rows, BS / 32), BS, 0, s>>>(U);
+            else union_team_kernel<32, 32, 256><<<ceil_div(U.rows, BS / 32), BS, 0, s>>>(U);
+        } else {
+            if (right <= 12.0) union_team_kernel<BS, 8, 4096><<<U.rows, BS, 0, s>>>(U);
+            else union_team_kernel<BS, 32, 4096><<<U.rows, BS, 0, s>>>(U);
+        }
+        countLaunch();
+    };
+    run();
+    rowptr.alloc(ar, (size_t)U.rows + 1, s);
+    nnz = rowOffsets(count, U.rows, rowptr.p, s);
+    if (readInt(overflow.p, s)) return false;
+    col.alloc(ar, std::max<int64_t>(nnz, 1), s);
+    U.out_rowptr = rowptr.p;
+    U.out_col = col.p;
+    run();
+    PB_LAUNCH("smoothed aggregation: pattern");
+    return true;
+}
+
 // Pattern of the row product of m left entries (output row orow[k], right row idx[k]) with B
 int64_t productPattern(DevArena& ar, int64_t m, const int* orow, const int* idx, const int* b_rowptr, const int* b_col,
                        int nrows, long long ncols, ArenaBuf<int>& rowptr, ArenaBuf<int>& col, cudaStream_t s) {
@@ -849,9 +1045,8 @@ int64_t productPattern(DevArena& ar, int64_t m, const int* orow, const int* idx,
     return patternOf(ar, keys.p, total, nrows, ncols, rowptr, col, s);
 }
 
-// Transpose of the pattern (n rows, nc columns): row starts, the row of every entry, and
-// src (entry of the transpose -> entry) or place (entry -> entry of the transpose)
-void transposeOf(DevArena& ar, int n, int nc, int64_t nnz, const int* rowptr, const int* col, ArenaBuf<int>& t_rowptr,
+// the transpose by sorting the entries (columns of more rows than columnTranspose holds)
+void sortedTranspose(DevArena& ar, int n, int nc, int64_t nnz, const int* rowptr, const int* col, ArenaBuf<int>& t_rowptr,
                  ArenaBuf<int>& t_row, ArenaBuf<int>* src, ArenaBuf<int>* place, cudaStream_t s) {
     const size_t m = std::max<int64_t>(nnz, 1);
     TmpBuf<int> erow(m, s), ids(m, s), col_s(m, s), src_t(src ? 0 : m, s);
@@ -870,6 +1065,37 @@ void transposeOf(DevArena& ar, int n, int nc, int64_t nnz, const int* rowptr, co
     if (place) place->alloc(ar, m, s);
     sorted_starts_kernel<<<grid(nc + 1), BS, 0, s>>>(nc, nnz, col_s.p, t_rowptr.p); countLaunch();
     transpose_kernel<<<grid(nnz), BS, 0, s>>>(nnz, order, erow.p, t_row.p, place ? place->p : nullptr); countLaunch();
+}
+
+// Transpose of the pattern (n rows, nc columns): row starts, the row of every entry, and
+// src (entry of the transpose -> entry) or place (entry -> entry of the transpose)
+void transposeOf(DevArena& ar, int n, int nc, int64_t nnz, const int* rowptr, const int* col, ArenaBuf<int>& t_rowptr,
+                 ArenaBuf<int>& t_row, ArenaBuf<int>* src, ArenaBuf<int>* place, cudaStream_t s) {
+    const DevArena::Mark before = ar.mark();
+    const size_t m = std::max<int64_t>(nnz, 1);
+    t_rowptr.alloc(ar, (size_t)nc + 1, s);
+    t_row.alloc(ar, m, s);
+    if (src) src->alloc(ar, m, s);
+    if (place) place->alloc(ar, m, s);
+    TmpBuf<int> count((size_t)nc + 1, s), overflow(1, s);
+    PB_CUDA(cudaMemsetAsync(overflow.p, 0, sizeof(int), s));
+    PB_CUDA(cudaMemsetAsync(count.p, 0, nc * sizeof(int), s));
+    column_count_kernel<<<grid(nnz), BS, 0, s>>>(nnz, col, count.p); countLaunch();
+    rowOffsets(count, nc, t_rowptr.p, s);
+    PB_CUDA(cudaMemsetAsync(count.p, 0, nc * sizeof(int), s));
+    column_fill_kernel<<<grid(n), BS, 0, s>>>(n, rowptr, col, t_rowptr.p, count.p, t_row.p); countLaunch();
+    int* sp = src ? src->p : nullptr;
+    int* pp = place ? place->p : nullptr;
+    if (nc > 16384)
+        column_sort_kernel<32, 512><<<ceil_div(nc, BS / 32), BS, 0, s>>>(nc, t_rowptr.p, t_row.p, rowptr, col, sp, pp, overflow.p);
+    else
+        column_sort_kernel<BS, 8192><<<nc, BS, 0, s>>>(nc, t_rowptr.p, t_row.p, rowptr, col, sp, pp, overflow.p);
+    countLaunch();
+    PB_LAUNCH("smoothed aggregation: transpose");
+    if (readInt(overflow.p, s)) {
+        ar.rewind(before);
+        sortedTranspose(ar, n, nc, nnz, rowptr, col, t_rowptr, t_row, src, place, s);
+    }
 }
 
 // aggregates of level L into L.agg; returns their number
@@ -1043,7 +1269,15 @@ void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, bool s
         const int nc = aggregate(arena, L, s);
         if (nc == 0 || nc > (int)(0.8 * L.n)) break;
         // P: the aggregates of a row's neighbours
-        {
+        Union U{};
+        U.rows = L.n;
+        U.l_rowptr = L.rowptr;
+        U.l_idx = L.col;
+        U.b_col = L.agg.p;
+        const double left = (double)L.nnz / L.n;
+        DevArena::Mark before = arena.mark();
+        if (!unionPattern(arena, U, left, 1.0, L.p_rowptr, L.p_col, L.p_nnz, s)) {
+            arena.rewind(before);
             TmpBuf<long long> keys(std::max<int64_t>(L.nnz, 1), s);
             p_keys_kernel<<<grid(L.n), BS, 0, s>>>(L.n, L.rowptr, L.col, L.agg.p, nc, keys.p); countLaunch();
             L.p_nnz = patternOf(arena, keys.p, L.nnz, L.n, nc, L.p_rowptr, L.p_col, s);
@@ -1052,7 +1286,11 @@ void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, bool s
         if (!sym) L.r_val.alloc(arena, std::max<int64_t>(L.p_nnz, 1), s);
         transposeOf(arena, L.n, nc, L.p_nnz, L.p_rowptr.p, L.p_col.p, L.pt_rowptr, L.pt_row, &L.pt_src, nullptr, s);
         // A P, the pattern of Q
-        {
+        U.b_rowptr = L.p_rowptr.p;
+        U.b_col = L.p_col.p;
+        before = arena.mark();
+        if (!unionPattern(arena, U, left, (double)L.p_nnz / L.n, L.q_rowptr, L.q_col, L.q_nnz, s)) {
+            arena.rewind(before);
             TmpBuf<int> erow(std::max<int64_t>(L.nnz, 1), s);
             entry_rows_kernel<<<grid(L.n), BS, 0, s>>>(L.n, L.rowptr, erow.p); countLaunch();
             L.q_nnz = productPattern(arena, L.nnz, erow.p, L.col, L.p_rowptr.p, L.p_col.p, L.n, nc, L.q_rowptr, L.q_col, s);
@@ -1066,7 +1304,14 @@ void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, bool s
         L.lpr_t = lanesFor(nc, L.q_nnz);
         // P^T A P
         auto C = std::make_unique<SaLevel>();
-        {
+        U.rows = nc;
+        U.l_rowptr = L.pt_rowptr.p;
+        U.l_idx = L.pt_row.p;
+        U.b_rowptr = L.q_rowptr.p;
+        U.b_col = L.q_col.p;
+        before = arena.mark();
+        if (!unionPattern(arena, U, (double)L.p_nnz / nc, (double)L.q_nnz / L.n, C->o_rowptr, C->o_col, C->nnz, s)) {
+            arena.rewind(before);
             TmpBuf<int> erow(std::max<int64_t>(L.p_nnz, 1), s);
             entry_rows_kernel<<<grid(L.n), BS, 0, s>>>(L.n, L.p_rowptr.p, erow.p); countLaunch();
             C->nnz = productPattern(arena, L.p_nnz, L.p_col.p, erow.p, L.q_rowptr.p, L.q_col.p, nc, nc, C->o_rowptr,
