@@ -489,36 +489,7 @@ __device__ __forceinline__ void storeProduct(const Product& P, int r, int e, dou
     }
 }
 
-// One thread per row, for rows of few entries: the sums of up to CH entries at a time live in
-// shared memory, interleaved by thread. (Searching the right matrix for every output entry
-// instead took three times as many loads: 310 us on the 2.1M-row five-point matrix.)
-template <int CH>
-__global__ void __launch_bounds__(BS) product_thread_kernel(const Product P) {
-    __shared__ double acc[CH][BS];
-    __shared__ int cols[CH][BS];
-    const int r = blockIdx.x * BS + threadIdx.x, t = threadIdx.x;
-    if (r >= P.rows) return;
-    const int o1 = P.out_rowptr[r + 1], l0 = P.l_rowptr[r], l1 = P.l_rowptr[r + 1];
-    for (int base = P.out_rowptr[r]; base < o1; base += CH) {
-        const int len = min(CH, o1 - base);
-        for (int k = 0; k < len; ++k) {
-            cols[k][t] = P.out_col[base + k];
-            acc[k][t] = 0.0;
-        }
-        for (int q = l0; q < l1; ++q) {
-            const int j = P.l_idx[q];
-            const double w = valueAt(P.l_val, P.l_src, q);
-            for (int e = P.b_rowptr[j]; e < P.b_rowptr[j + 1]; ++e) {
-                const int c = P.b_col[e];
-                for (int k = 0; k < len; ++k)
-                    if (cols[k][t] == c) acc[k][t] += w * P.b_val[e];
-            }
-        }
-        for (int k = 0; k < len; ++k) storeProduct(P, r, base + k, acc[k][t]);
-    }
-}
-
-// T threads per row (32 or the whole block) in groups of GL lanes: a group takes one left
+// T threads per row (part of a warp, or the whole block) in groups of GL lanes: a group takes one left
 // entry at a time, its lanes the entries of that row of B (distinct columns, so no two lanes
 // of a group meet in one sum), into sums of its own; the groups' sums are added in order.
 template <int T, int GL, int CH>
@@ -530,8 +501,8 @@ __global__ void __launch_bounds__(BS) product_team_kernel(const Product P) {
     const unsigned mask = GL == 32 ? 0xffffffffu : ((1u << GL) - 1u) << (threadIdx.x & 31 & ~(GL - 1));
     const int r = blockIdx.x * TEAMS + team;
     if (r >= P.rows) return;  // whole teams
-    auto sync = [] {
-        if constexpr (T == 32) __syncwarp();
+    auto sync = [&] {
+        if constexpr (T <= 32) __syncwarp(T == 32 ? 0xffffffffu : ((1u << (T & 31)) - 1u) << (threadIdx.x & 31 & ~(T - 1)));
         else __syncthreads();
     };
     const int o1 = P.out_rowptr[r + 1], l0 = P.l_rowptr[r], l1 = P.l_rowptr[r + 1];
@@ -568,10 +539,11 @@ __global__ void __launch_bounds__(BS) product_team_kernel(const Product P) {
 // nnz_out, nnz_b: entries of the product and of B (n_b rows)
 void launchProduct(const Product& P, int64_t nnz_out, int n_b, int64_t nnz_b, cudaStream_t s) {
     const double out = (double)nnz_out / std::max(P.rows, 1), right = (double)nnz_b / std::max(n_b, 1);
-    // one thread per row only where the rows fill the chip: 2,309 rows take 86 us that way, 9 us
-    // with a block each
+    // four lanes per row where rows are short and fill the chip (2.1M seven-point rows: 584 us;
+    // one thread per row 1,078, eight lanes 699), a warp per row for longer ones (218,566 rows of
+    // 37: 607 us, half a warp 610, a quarter 670), the whole block where rows are few
     if (P.rows > 8192 && out <= 12.0 && right <= 4.0) {
-        product_thread_kernel<12><<<grid(P.rows), BS, 0, s>>>(P);
+        product_team_kernel<4, 4, 16><<<ceil_div(P.rows, BS / 4), BS, 0, s>>>(P);
     } else if (P.rows > 16384) {
         const int g = ceil_div(P.rows, BS / 32);
         if (right <= 12.0) product_team_kernel<32, 8, 64><<<g, BS, 0, s>>>(P);
@@ -677,26 +649,29 @@ __global__ void scaled_values_kernel(int64_t m, const int* __restrict__ col, con
 template <int LPR, typename F>
 __device__ __forceinline__ float csrSum(int lo, int hi, int sub, const int* __restrict__ col,
                                         const float* __restrict__ val, F x) {
+    constexpr int W = LPR == 1 ? 8 : 4;  // entries in flight per lane
     float sum = 0.f;
-    int k = lo + sub;
-    for (; k + 3 * LPR < hi; k += 4 * LPR) {  // four entries in flight
-        int c[4];
-        float v[4];
+    for (int k = lo + sub; k < hi; k += W * LPR) {
+        int c[W];
+        float v[W];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            c[u] = col[k + u * LPR];
-            v[u] = val[k + u * LPR];
-        }
+        for (int u = 0; u < W; ++u)
+            if (k + u * LPR < hi) {
+                c[u] = col[k + u * LPR];
+                v[u] = val[k + u * LPR];
+            }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) sum += v[u] * x(c[u]);
+        for (int u = 0; u < W; ++u)
+            if (k + u * LPR < hi) sum += v[u] * x(c[u]);
     }
-    for (; k < hi; k += LPR) sum += val[k] * x(col[k]);
+    if constexpr (LPR > 1)
 #pragma unroll
-    for (int o = LPR / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        for (int o = LPR / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     return sum;
 }
 
-// the SELL-32 row sum of the level-0 matrix, four slots in flight
+// the SELL-32 row sum of the level-0 matrix, four slots in flight (eight: 58 against 53 us in
+// the down-sweep of 2.1M five-point rows)
 __device__ __forceinline__ float sellSum(const int* __restrict__ col, const float* __restrict__ val,
                                          const float* __restrict__ x, int base, int width) {
     float sum = 0.f;
@@ -793,34 +768,6 @@ __global__ void __launch_bounds__(BS) up_kernel(int n, const int* __restrict__ r
     const int lo = valid ? rowptr[row] : 0, hi = valid ? rowptr[row + 1] : 0;
     const float sum = csrSum<LQ>(lo, hi, sub, col, val, [&](int c) { return __ldg(e + c); });
     if (valid && sub == 0) x[row] = y[row] + sum;
-}
-
-// up-sweep of rows of few entries: a warp streams the entries of its 32 rows through shared
-// memory (coalesced whatever the row lengths), then every lane sums its own row's products
-constexpr int CHUNK = 256;
-__global__ void __launch_bounds__(BS) up_stream_kernel(int n, const int* __restrict__ rowptr,
-                                                       const int* __restrict__ col, const float* __restrict__ val,
-                                                       const float* __restrict__ e, const float* __restrict__ y,
-                                                       float* __restrict__ x, const KState* S) {
-    pdlEnter();
-    if (S && S->done) return;
-    __shared__ float prod[WARPS][CHUNK];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r0 = (blockIdx.x * WARPS + warp) * 32;
-    if (r0 >= n) return;
-    const int row = r0 + lane;
-    const int lo = rowptr[min(row, n)], hi = rowptr[min(row + 1, n)];
-    const int first = __shfl_sync(0xffffffffu, lo, 0), last = __shfl_sync(0xffffffffu, hi, 31);
-    float sum = 0.f;
-    for (int base = first; base < last; base += CHUNK) {
-        const int end = min(last, base + CHUNK);
-#pragma unroll 4
-        for (int k = base + lane; k < end; k += 32) prod[warp][k - base] = val[k] * __ldg(e + col[k]);
-        __syncwarp();
-        for (int k = max(lo, base); k < min(hi, end); ++k) sum += prod[warp][k - base];
-        __syncwarp();
-    }
-    if (row < n) x[row] = y[row] + sum;
 }
 
 // coarsest level outside the tail: dense inverse, one warp per row
@@ -1446,9 +1393,11 @@ void SaAmg::apply(const float* r, float* z, const KState* S, cudaStream_t s, boo
                              ? profBegin(PROF_AMG_POST, true, 8.0 * L.q_nnz + 4.0 * (L.n + 1) + 8.0 * L.n +
                                                                   4.0 * levels[l + 1]->n, s)
                              : -1;
+        // one thread per row where rows are short and fill the chip (2.1M rows of 4.3 entries: 26
+        // us, with two lanes 35, with four 61)
         if ((double)L.q_nnz <= 16.0 * L.n && L.n > 32 * NUM_SMS * WARPS) {
-            launchPdl(up_stream_kernel, ceil_div(L.n, 32 * WARPS), BS, s, L.n, (const int*)L.q_rowptr.p,
-                      (const int*)L.q_col.p, (const float*)L.q_val.p, e, (const float*)L.y.p, sol(l), S);
+            launchPdl(up_kernel<1>, grid(L.n), BS, s, L.n, (const int*)L.q_rowptr.p, (const int*)L.q_col.p,
+                      (const float*)L.q_val.p, e, (const float*)L.y.p, sol(l), S);
         } else {
             withLanes(L.lpr_q, [&](auto c) {
                 constexpr int P = decltype(c)::value;
