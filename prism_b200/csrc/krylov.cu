@@ -424,6 +424,14 @@ __global__ void __launch_bounds__(BS) fcg_update_kernel(int n, double* __restric
     }
 }
 
+// a fresh KState for one pass: zeros, the iteration cap
+__device__ void resetState(KState* S, long long maxit) {
+    KState z{};
+    z.maxit = maxit;
+    *S = z;
+}
+__global__ void reset_state_kernel(KState* S, long long maxit) { resetState(S, maxit); }
+
 // column scaling: dinv = 1/diag (1 where diag == 0), As = A dinv[col], xs = diag x
 __global__ void dinv_kernel(int n, const int* diag_pos, const double* vals, double* dinv, const double* x, double* xs) {
     int i = blockIdx.x * BS + threadIdx.x;
@@ -444,23 +452,6 @@ __global__ void to_float_kernel(int64_t nnz, const double* vals, float* out) {
 __global__ void unscale_kernel(int n, const double* dinv, const double* xs, double* x) {
     int i = blockIdx.x * BS + threadIdx.x;
     if (i < n) x[i] = dinv[i] * xs[i];
-}
-// refinement: r = b - A x (FP64) -> r (double) and r32; dots r.r, b.b
-__global__ void __launch_bounds__(BS) refine_residual_kernel(int n, const double* __restrict__ Ax,
-                                                             const double* __restrict__ b, float* __restrict__ r32,
-                                                             double* partials, unsigned int* counter, double* out2) {
-    double d0 = 0.0, d1 = 0.0;
-    for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
-        double ri = b[i] - Ax[i];
-        r32[i] = (float)ri;
-        d0 += ri * ri;
-        d1 += b[i] * b[i];
-    }
-    double v[2] = {d0, d1}, out[2];
-    if (reduceLast<2, false>(v, partials, counter, out) && threadIdx.x == 0) {
-        out2[0] = out[0];
-        out2[1] = out[1];
-    }
 }
 __global__ void fill_zero_f(int n, float* x) {
     int i = blockIdx.x * BS + threadIdx.x;
@@ -596,6 +587,39 @@ __global__ void __launch_bounds__(BS) resid_kernel(int nslices, int n, const int
     }
 }
 
+// the end of a step in one pass over A: the scaled residual's pieces (as resid_kernel) to
+// out[0..2], ||b - A x||^2 and ||b||^2 to out[CHECK_SUMS] and the next
+constexpr int CHECK_SUMS = 4;
+__global__ void __launch_bounds__(BS) check_kernel(int nslices, int n, const int* __restrict__ sl_off,
+                                                   const int* __restrict__ col, const double* __restrict__ val,
+                                                   const int* __restrict__ diag_pos, const double* __restrict__ b,
+                                                   const double* __restrict__ x, double* partials,
+                                                   unsigned int* counter, double* out) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, t[5];
+    for (int sl = blockIdx.x * WARPS + warp; sl < nslices; sl += gridDim.x * WARPS) {
+        const int bo = sl_off[sl], width = (sl_off[sl + 1] - bo) >> 5;
+        const int r = sl * 32 + lane;
+        const double sum = sliceRow<double, 4>(col, val, x, bo, width, lane);
+        if (r >= n) continue;
+        const double br = b[r], e = br - sum, a = fabs(e), d = fabs(val[diag_pos[r]] * x[r]);
+        v[0] += e * e;
+        v[1] += br * br;
+        if (!isfinite(a) || !isfinite(d)) v[4] = 1.0;
+        else {
+            v[2] = fmax(v[2], a);
+            v[3] = fmax(v[3], d);
+        }
+    }
+    if (reduceLast<5, false, BS, 2>(v, partials, counter, t) && threadIdx.x == 0) {
+        out[0] = t[2];
+        out[1] = t[3];
+        out[2] = t[4];
+        out[CHECK_SUMS] = t[0];
+        out[CHECK_SUMS + 1] = t[1];
+    }
+}
+
 // max over rows of sum_{j != i} |a_ij| / |a_ii| (infinite for a zero or non-finite diagonal)
 __global__ void __launch_bounds__(BS) offdiag_ratio_kernel(int nslices, int n, const int* __restrict__ sl_off,
                                                            const int* __restrict__ col, const double* __restrict__ val,
@@ -625,7 +649,7 @@ __global__ void __launch_bounds__(BS) offdiag_ratio_kernel(int nslices, int n, c
 // stream is drained so the zeros land before any kernel of the (non-blocking)
 // solve stream reads them.
 void KrylovWork::ensure(int n_pad, int64_t nnz_padded, bool mixed) {
-    if (!host_state) PB_CUDA(cudaMallocHost(&host_state, sizeof(KState) + 64));
+    if (!host_state) PB_CUDA(cudaMallocHost(&host_state, sizeof(KState) + HOST_SCALARS * sizeof(double)));
     bool fresh = false;
     if (n != n_pad || nnz != nnz_padded) {
         fresh = true;
@@ -997,9 +1021,7 @@ KrylovOut runBicgstab(const SellMatrix& A, const T* M, const T* rhs, Vecs<T> V, 
     const bool flex = flexMode(mode);
     KrylovOut out;
     KState* S = w.state.p;
-    KState init{};
-    init.maxit = maxit;
-    PB_CUDA(cudaMemcpyAsync(S, &init, sizeof(KState), cudaMemcpyHostToDevice, s));
+    reset_state_kernel<<<1, 1, 0, s>>>(S, maxit); countLaunch();
     const int n = A.n, vg = vecGrid(n), sg = sliceGrid(A.nslices);
     int restarts = 0;
     bool zero = from_zero;
@@ -1179,13 +1201,17 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
             out.status = o.status;
             maxit -= o.iterations;
             finish();
-            spmv(A, x, w.tmp.p, s);
-            double rb[2];
-            refine_residual_kernel<<<vecGrid(n), BS, 0, s>>>(n, w.tmp.p, b, reinterpret_cast<float*>(w.s.p),
-                                                             w.partials.p, w.counter.p, w.scal.p); countLaunch();
-            PB_CUDA(cudaMemcpyAsync(rb, w.scal.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
+            const int cg = waveGrid(check_kernel, ceil_div(A.nslices, WARPS));
+            check_kernel<<<cg, BS, 0, s>>>(A.nslices, n, A.sl_off, A.col, A.vals, A.diag_pos, b, x, w.partials.p,
+                                           w.counter.p, w.scal.p); countLaunch();
+            PB_LAUNCH("check_kernel");
+            double* h = w.hostScalars();
+            PB_CUDA(cudaMemcpyAsync(h, w.scal.p, (CHECK_SUMS + 2) * sizeof(double), cudaMemcpyDeviceToHost, s));
             PB_CUDA(cudaStreamSynchronize(s));
+            const double* rb = h + CHECK_SUMS;
             out.rel_residual = rb[1] > 0 ? std::sqrt(rb[0] / rb[1]) : 0.0;
+            out.scaled_residual = scaledResidualOf(h);
+            out.has_scaled = true;
             if (o.status != PRISM_OK || out.rel_residual <= 10 * tol || maxit <= 0 || rb[1] == 0) break;
         }
         if (verbose())
@@ -1427,13 +1453,6 @@ __global__ void ctl_init_res_kernel(SolveCtl* c, const double* scal) {
     c->init_res = scal[2] != 0.0 ? nanValue() : scal[0] / (scal[1] + EPSILON);
 }
 
-// a fresh KState for one pass (runBicgstab's initial state: zeros, the iteration cap)
-__device__ void resetState(KState* S, long long maxit) {
-    KState z{};
-    z.maxit = maxit;
-    *S = z;
-}
-
 // start of one bicgstab() call: its first pass, and the device loop switched on
 __global__ void ctl_krylov_begin_kernel(SolveCtl* c, KState* S, cudaGraphConditionalHandle hk) {
     if (threadIdx.x) return;
@@ -1478,7 +1497,7 @@ __global__ void ctl_krylov_step_kernel(SolveCtl* c, KState* S, const double* sca
             c->phase = PH_CHECK;
         }
     } else if (c->phase == PH_CHECK) {
-        const double rb0 = scal[0], rb1 = scal[1];
+        const double rb0 = scal[CHECK_SUMS], rb1 = scal[CHECK_SUMS + 1];
         c->krylov_rel = rb1 > 0 ? sqrt(rb0 / rb1) : 0.0;
         c->krylov_iterations += S->iter;
         c->maxit_left -= S->iter;
@@ -1648,9 +1667,8 @@ void emitBicgstab(const SellMatrix& A, const double* b, double* x, double tol, l
     if (scaled) {
         unscale_kernel<<<gn, BS, 0, sub>>>(n, w.dinv.p, w.xs.p, x); countLaunch();
     }
-    spmv(A, x, w.tmp.p, sub);
-    refine_residual_kernel<<<vg, BS, 0, sub>>>(n, w.tmp.p, b, reinterpret_cast<float*>(w.s.p), w.partials.p,
-                                               w.counter.p, w.scal.p); countLaunch();
+    check_kernel<<<waveGrid(check_kernel, ceil_div(A.nslices, WARPS)), BS, 0, sub>>>(
+        A.nslices, n, A.sl_off, A.col, A.vals, A.diag_pos, b, x, w.partials.p, w.counter.p, w.scal.p); countLaunch();
     endConditional(sub);
     ctl_krylov_step_kernel<<<1, 32, 0, body>>>(ctl, S, w.scal.p, guard_max, hk); countLaunch();
     endConditional(body);

@@ -64,7 +64,10 @@ struct KrylovWork {
     DevBuf<unsigned char> ctl;        // SolveCtl of a one-launch solve, and its pinned copy
     SolveCtl* host_ctl = nullptr;
     SolveCtl* ctlRecord();            // device record (allocated on first use)
-    KState* host_state = nullptr;  // pinned
+    KState* host_state = nullptr;  // pinned, followed by HOST_SCALARS doubles
+    static constexpr int HOST_SCALARS = 16;  // a check's six, and from INITIAL on the first residual's parts
+    static constexpr int INITIAL = 8;
+    double* hostScalars() { return reinterpret_cast<double*>(host_state + 1); }
     // one BiCGSTAB iteration captured as a CUDA graph, kept per operand set (key:
     // precision, matrix, vectors, preconditioner), least recently used last out
     struct IterGraph {
@@ -81,6 +84,8 @@ struct KrylovOut {
     long long iterations = 0;
     int status = PRISM_OK;
     double rel_residual = 0.0;
+    double scaled_residual = 0.0;  // of the final x (has_scaled)
+    bool has_scaled = false;
 };
 
 enum { SOLVE_PLAIN = 0, SOLVE_FLEXIBLE = 1, SOLVE_SMOOTHED = 2 };

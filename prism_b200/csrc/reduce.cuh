@@ -21,25 +21,25 @@ __device__ __forceinline__ double warpMax(double v) {
     return v;
 }
 
-// Block-reduce NV sums (or maxima), publish the block partial, and let the last
+// Block-reduce NV sums (or maxima; from value MAX_FROM on with that given), publish the block partial, and let the last
 // block to arrive reduce all partials in block order. Returns true in the last
 // block, where out[] holds the grid totals in every thread. partials holds
 // gridDim.x * NV doubles; counter starts at 0 and is left at 0.
-template <int NV, bool MAX, int BLOCK = 256>
+template <int NV, bool MAX, int BLOCK = 256, int MAX_FROM = MAX ? 0 : NV>
 __device__ bool reduceLast(double (&v)[NV], double* partials, unsigned int* counter, double (&out)[NV]) {
     constexpr int NW = BLOCK / 32;
     __shared__ double sh[NV][NW];
     __shared__ int is_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int k = 0; k < NV; ++k) {
-        double x = MAX ? warpMax(v[k]) : warpSum(v[k]);
+        double x = k >= MAX_FROM ? warpMax(v[k]) : warpSum(v[k]);
         if (lane == 0) sh[k][warp] = x;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int k = 0; k < NV; ++k) {
             double s = sh[k][0];
-            for (int w = 1; w < NW; ++w) s = MAX ? fmax(s, sh[k][w]) : s + sh[k][w];
+            for (int w = 1; w < NW; ++w) s = k >= MAX_FROM ? fmax(s, sh[k][w]) : s + sh[k][w];
             partials[blockIdx.x * NV + k] = s;
         }
         __threadfence();
@@ -54,18 +54,18 @@ __device__ bool reduceLast(double (&v)[NV], double* partials, unsigned int* coun
         acc[k] = 0.0;
         for (int b = threadIdx.x; b < (int)gridDim.x; b += BLOCK) {
             double x = __ldcg(&partials[b * NV + k]);
-            acc[k] = MAX ? fmax(acc[k], x) : acc[k] + x;
+            acc[k] = k >= MAX_FROM ? fmax(acc[k], x) : acc[k] + x;
         }
     }
     __syncthreads();
     for (int k = 0; k < NV; ++k) {
-        double x = MAX ? warpMax(acc[k]) : warpSum(acc[k]);
+        double x = k >= MAX_FROM ? warpMax(acc[k]) : warpSum(acc[k]);
         if (lane == 0) sh[k][warp] = x;
     }
     __syncthreads();
     for (int k = 0; k < NV; ++k) {
         double s = sh[k][0];
-        for (int w = 1; w < NW; ++w) s = MAX ? fmax(s, sh[k][w]) : s + sh[k][w];
+        for (int w = 1; w < NW; ++w) s = k >= MAX_FROM ? fmax(s, sh[k][w]) : s + sh[k][w];
         out[k] = s;
     }
     if (threadIdx.x == 0) *counter = 0u;

@@ -655,14 +655,17 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o) {
     PrismSolveResult r{};
     r.status = PRISM_OK;
     double init_res = 0.0, cur = 0.0;
-    bool conv = false;
+    bool conv = false, cur_known = false;
     int64_t iter = 0;
     for (; iter < o.n_iter; ++iter) {
         if (iter == 0) {
             ++phi.event;
-            init_res = scaledResidual(A, eq.b.p, phi.v.p, m.kw, m.stream);
+            m.kw.ensure(A.nslices * 32, A.nnz_padded, false);
+            // read once a later wait has seen it arrive
+            scaledResidualParts(A, eq.b.p, phi.v.p, m.kw, m.kw.hostScalars() + KrylovWork::INITIAL, m.stream);
         }
         phi.event += 2;
+        cur_known = false;
         if (o.method == PRISM_SOLVER_JACOBI) {
             jacobiStep(A, eq.b.p, phi.v.p, m.kw, m.stream);
         } else {
@@ -675,9 +678,12 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o) {
             r.krylov_iterations += k.iterations;
             r.krylov_rel_residual = k.rel_residual;
             if (k.status != PRISM_OK && r.status == PRISM_OK) r.status = k.status;
+            cur_known = k.has_scaled;
+            cur = k.scaled_residual;
         }
         ++phi.event;
-        cur = scaledResidual(A, eq.b.p, phi.v.p, m.kw, m.stream);
+        if (!cur_known) cur = scaledResidual(A, eq.b.p, phi.v.p, m.kw, m.stream);
+        if (iter == 0) init_res = scaledResidualOf(m.kw.hostScalars() + KrylovWork::INITIAL);
         if (std::isnan(cur)) r.status = PRISM_NONFINITE;
         if (cur < o.eps) {
             conv = true;
@@ -1336,7 +1342,6 @@ PrismSolveResult solveCaptured(Transport& eq, const PrismSolveOpts& o) {
         const HoldAmgValues hold(amg, eq.matrix_unchanged);
         emitBicgstab(A, eq.b.p, phi.v.p, ktol, cap, m.kw, body, amg, m.pat.rowptr.p, m.pat.col.p, ctl, m.cs, 1, kind);
         ++phi.event;
-        emitResidual(A, eq.b.p, phi.v.p, m.kw, body);
         emitOuterStep(ctl, m.kw, outer, body);
         endConditional(body);
     }
