@@ -49,13 +49,13 @@ struct ClusterReduce {
             for (int k = 0; k < N; ++k) sh.red[parity][k][warp] = v[k];
         __syncthreads();
         if constexpr (!CL) {
+            // every warp adds the warps' results itself: a barrier less than one warp doing it
 #pragma unroll
-            for (int k = 0; k < N; ++k) {
-                double u[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int k = 0; k < N; ++k) v[k] = sh.red[parity][k][lane % NW];
 #pragma unroll
-                for (int w = 0; w < NW; ++w) u[w & 3] = join(u[w & 3], sh.red[parity][k][w]);
-                v[k] = join(join(u[0], u[1]), join(u[2], u[3]));
-            }
+            for (int o = NW / 2; o > 0; o >>= 1)
+#pragma unroll
+                for (int k = 0; k < N; ++k) v[k] = join(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
         } else {
             if (warp == 0) {
                 double u[N];

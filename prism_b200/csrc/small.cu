@@ -35,8 +35,9 @@ struct SmallParams {
     SolveCtl* out;
 };
 
-// THREADS threads of K rows each per block; CL: more than one block
-template <int THREADS, int K, bool CL>
+// THREADS threads of K rows each per block, the first KEPT entries of a row in registers; CL:
+// more than one block
+template <int THREADS, int K, int KEPT, bool CL>
 __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallParams P) {
     constexpr int ROWS = THREADS * K;  // rows per block
     __shared__ double ph[ROWS], sh[ROWS];  // the gathered vectors: M^-1 p (or x), M^-1 s
@@ -44,7 +45,9 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
     ClusterReduce<THREADS, CL, NV> R(shared);
     const int rank = R.rank;
 
-    int row[K], at[K], width[K];
+    // the first KEPT entries of a row stay in registers
+    int row[K], at[K], width[K], kcol[K][KEPT + 1];
+    double kval[K][KEPT + 1];
     double dinv[K], x[K], r[K], r0[K], p[K], v[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
@@ -57,6 +60,12 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
         dinv[k] = d != 0.0 ? 1.0 / d : 1.0;
         x[k] = in ? P.x[row[k]] : 0.0;
         r[k] = r0[k] = p[k] = v[k] = 0.0;
+#pragma unroll
+        for (int j = 0; j < KEPT; ++j)
+            if (j < width[k]) {
+                kcol[k][j] = __ldg(P.col + at[k] + 32 * j);
+                kval[k][j] = __ldg(P.vals + at[k] + 32 * j);
+            }
     }
     auto rhs = [&](int k) { return row[k] < P.n ? __ldg(P.b + row[k]) : 0.0; };
     auto own = [&](int k) { return k * THREADS + (int)threadIdx.x; };
@@ -67,7 +76,10 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
     // (A y)_row with y spread over the blocks' shared array a; up to 4 entries in flight
     auto rowOf = [&](int k, double* a) {
         double sum = 0.0;
-        for (int j0 = 0; j0 < width[k]; j0 += 4) {
+#pragma unroll
+        for (int j = 0; j < KEPT; ++j)
+            if (j < width[k]) sum += kval[k][j] * gather(a, kcol[k][j]);
+        for (int j0 = KEPT; j0 < width[k]; j0 += 4) {
             int c[4];
             double m[4];
 #pragma unroll
@@ -317,19 +329,20 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
 
 // blocks of the largest cluster the device places (8 is always allowed)
 int maxCtas() {
-    static const int c = clusterPlaced(small_solve_kernel<256, 1, true>, 256) &&
-                                 clusterPlaced(small_solve_kernel<512, 2, true>, 512) &&
-                                 clusterPlaced(small_solve_kernel<512, 4, true>, 512)
+    static const int c = clusterPlaced(small_solve_kernel<256, 1, 7, true>, 256) &&
+                                 clusterPlaced(small_solve_kernel<512, 2, 5, true>, 512) &&
+                                 clusterPlaced(small_solve_kernel<512, 2, 7, true>, 512) &&
+                                 clusterPlaced(small_solve_kernel<512, 4, 0, true>, 512)
                              ? CLUSTER_MAX
                              : 8;
     return c;
 }
 
-template <int T, int K>
+template <int T, int K, int KEPT>
 void launchSmall(const SmallParams& P, cudaStream_t s) {
     const int ctas = ceil_div(P.n, T * K);
-    if (ctas == 1) launchCluster(small_solve_kernel<T, K, false>, 1, T, s, false, P);
-    else launchCluster(small_solve_kernel<T, K, true>, ctas, T, s, false, P);
+    if (ctas == 1) launchCluster(small_solve_kernel<T, K, KEPT, false>, 1, T, s, false, P);
+    else launchCluster(small_solve_kernel<T, K, KEPT, true>, ctas, T, s, false, P);
 }
 
 }  // namespace
@@ -339,16 +352,19 @@ bool smallSolveFits(const SellMatrix& A, long long maxit) {
 }
 
 // Rows per block: one block up to 1,024 rows, whose barriers cost a fraction of a cluster's;
-// then as few rows per block as 16 blocks allow.
+// then as few rows per block as 16 blocks allow. Entries kept in registers (two rows per
+// thread): five for the rows of 2-D meshes (32^2 Poisson 0.31 ms, with seven 0.37, none 0.39),
+// seven for longer ones (22^3 transport 4.46 ms, with five 4.94, none 5.25); four rows per
+// thread leave no room.
 void smallSolve(const SellMatrix& A, const double* b, double* x, long long n_iter, double eps, double tol,
                 long long maxit, bool symmetric, SolveCtl* out, cudaStream_t s) {
     const SmallParams P{A.n, A.sl_off, A.col, A.vals, A.diag_pos, b, x, n_iter, maxit, eps, tol, symmetric ? 1 : 0, out};
     const int max = maxCtas();
-    if (A.n <= 256) launchSmall<256, 1>(P, s);
-    else if (A.n <= 1024) launchSmall<512, 2>(P, s);
-    else if (A.n <= max * 256) launchSmall<256, 1>(P, s);
-    else if (A.n <= max * 1024) launchSmall<512, 2>(P, s);
-    else launchSmall<512, 4>(P, s);
+    const bool two = (A.n > 256 && A.n <= 1024) || (A.n > max * 256 && A.n <= max * 1024);
+    if (two && A.nnz_padded <= 5LL * 32 * A.nslices) launchSmall<512, 2, 5>(P, s);
+    else if (two) launchSmall<512, 2, 7>(P, s);
+    else if (A.n <= max * 256) launchSmall<256, 1, 7>(P, s);
+    else launchSmall<512, 4, 0>(P, s);
 }
 
 }  // namespace pb
