@@ -523,7 +523,8 @@ static bool symmetricMatrix(const Transport& eq) { return eq.has_diff && !eq.has
 // automatic choice on the first solve (a host round trip, never inside a capture)
 static int pcFor(Transport& eq, const PrismSolveOpts& o, const SellMatrix& A) {
     const int c = choosePreconditioner(o.preconditioner, A.n, symmetricMatrix(eq));
-    if (o.preconditioner != PRISM_PC_AUTO || c != PRISM_PC_AMG || eq.spd || autoJacobiRatio() <= 0.0) return c;
+    if (o.preconditioner != PRISM_PC_AUTO || c != PRISM_PC_AMG || eq.spd) return c;
+    if (autoJacobiRatio() <= 0.0) return eq.auto_pc ? eq.auto_pc : c;
     if (eq.auto_pc == 0) {
         Mesh& m = *eq.phi->m;
         if (capturing(m.stream)) fail(PRISM_INTERNAL, "automatic preconditioner not chosen before capture");
@@ -591,10 +592,21 @@ static void checkFcg(const PrismSolveOpts& o) {
     if (o.preconditioner == PRISM_PC_JACOBI) fail(PRISM_BAD_ARG, "flexible CG needs the AMG preconditioner");
 }
 
-// One step by a stand-in (kindFor); should it fail, BiCGSTAB with amg's cycle from the same
-// guess, then and from then on (failed). The guess waits in xs, which AMG solves do not use.
+// A stand-in failed on eq: BiCGSTAB from now on, with Jacobi where the choice is the library's
+// and the size one for the one-launch solve (sizes at which multigrid is chosen for its speed
+// alone), else with amg's cycle. Returns the hierarchy to use (null: Jacobi).
+static Amg* standInGaveUp(Transport& eq, const PrismSolveOpts& o, const SellMatrix& A, Amg* amg) {
+    eq.no_stand_in = true;
+    amg->values_current = false;
+    if (o.preconditioner != PRISM_PC_AUTO || !smallSolveFits(A, 1)) return amg;
+    eq.auto_pc = PRISM_PC_JACOBI;
+    return nullptr;
+}
+
+// One step by a stand-in (kindFor); should it fail, the solve it stands in for from the same
+// guess. The guess waits in xs, which AMG solves do not use.
 static KrylovOut standInSolve(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, int kind,
-                              const PrismSolveOpts& o, Mesh& m, Amg* amg, bool& failed) {
+                              const PrismSolveOpts& o, Mesh& m, Amg* amg, Transport& eq) {
     KrylovWork& w = m.kw;
     w.ensure(A.nslices * 32, A.nnz_padded, false);
     const double itol = o.inner_tol > 0 ? o.inner_tol : 0.1;
@@ -602,10 +614,9 @@ static KrylovOut standInSolve(const SellMatrix& A, const double* b, double* x, d
     KrylovOut k = bicgstab(A, b, x, tol, std::min(maxit, STAND_IN_MAX), kind == SOLVE_FLEXIBLE ? PRISM_PREC_FP64 : o.precision,
                            itol, w, m.stream, amg, m.pat.rowptr.p, m.pat.col.p, kind);
     if (!standInFailed(o, k.status, k.iterations)) return k;
-    failed = true;
+    Amg* plain = standInGaveUp(eq, o, A, amg);
     PB_CUDA(cudaMemcpyAsync(x, w.xs.p, A.n * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
-    amg->values_current = false;
-    KrylovOut f = bicgstab(A, b, x, tol, maxit, o.precision, itol, w, m.stream, amg, m.pat.rowptr.p, m.pat.col.p);
+    KrylovOut f = bicgstab(A, b, x, tol, maxit, o.precision, itol, w, m.stream, plain, m.pat.rowptr.p, m.pat.col.p);
     f.iterations += k.iterations;
     return f;
 }
@@ -670,9 +681,10 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o) {
             jacobiStep(A, eq.b.p, phi.v.p, m.kw, m.stream);
         } else {
             const HoldAmgValues hold(amg, eq.matrix_unchanged || iter > 0);  // A is fixed within one solve
+            if (amg && eq.auto_pc == PRISM_PC_JACOBI && eq.no_stand_in) amg = nullptr;  // gave up in an earlier step
             const int kind = kindFor(eq, o, amg, A);
             KrylovOut k = standsIn(eq, o, kind)
-                              ? standInSolve(A, eq.b.p, phi.v.p, ktol, kmax, kind, o, m, amg, eq.no_stand_in)
+                              ? standInSolve(A, eq.b.p, phi.v.p, ktol, kmax, kind, o, m, amg, eq)
                               : bicgstab(A, eq.b.p, phi.v.p, ktol, kmax, o.precision, itol, m.kw, m.stream, amg,
                                          m.pat.rowptr.p, m.pat.col.p, kind, symmetricMatrix(eq));
             r.krylov_iterations += k.iterations;
@@ -1103,9 +1115,10 @@ FixedPointOut adjointBackward(Transport& eq, const double* dJ, double* gk, doubl
         adjointCorrection(P, lam.p, u.p, d.p, np, s);
         adjointRhs(P, d_dJ.p, lam.p, u.p, d.p, np, rhs.p, s);
         PB_CUDA(cudaMemcpyAsync(lam_prev.p, lam.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        if (amg && eq.no_stand_in && o.preconditioner == PRISM_PC_AUTO && smallSolveFits(AT, 1)) amg = nullptr;
         const HoldAmgValues hold(amg, it > 0);
         KrylovOut k = amg && !eq.no_stand_in && smoothedFits(AT)
-                          ? standInSolve(AT, rhs.p, lam.p, ktol, kmax, SOLVE_FLEXIBLE, fp64, m, amg, eq.no_stand_in)
+                          ? standInSolve(AT, rhs.p, lam.p, ktol, kmax, SOLVE_FLEXIBLE, fp64, m, amg, eq)
                           : bicgstab(AT, rhs.p, lam.p, ktol, kmax, PRISM_PREC_FP64, 0.1, m.kw, s, amg, m.pat.rowptr.p,
                                      m.pat.col.p, SOLVE_PLAIN, true);
         out.krylov += k.iterations;
@@ -1461,8 +1474,7 @@ PrismSolveResult solveAsGraph(Transport& eq, const PrismSolveOpts& o) {
     const bool with_amg = o.method == PRISM_SOLVER_FCG || pcFor(eq, o, A) == PRISM_PC_AMG;
     if (with_amg && standsIn(eq, o, kindFor(eq, o, eq.amg.get(), A))) {
         if (standInFailed(o, out.status, out.krylov_iterations)) {
-            eq.no_stand_in = true;
-            eq.amg->values_current = false;
+            standInGaveUp(eq, o, A, eq.amg.get());
             PB_CUDA(cudaMemcpyAsync(eq.phi->v.p, m.kw.xs.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
             out = solveAssembled(eq, o);
         }

@@ -60,3 +60,70 @@ def test_rows_without_couplings():
     b = np.random.default_rng(3).normal(size=n)
     x = api.FCG(krylov_tol=1e-12).step(prism_b200.lib(), np.arange(n + 1), np.arange(n), d, np.zeros(n), b)
     assert np.allclose(x, b / d, rtol=1e-10, atol=0)
+
+
+@pytest.mark.parametrize("unv", [lambda: meshgen.box_hex(26, 25, 24, jitter=0.2, seed=2), lambda: meshgen.box_hex(150, 99, 1),
+                                 lambda: meshgen.box_tet(13, 12, 14)], ids=["hex3d", "hex2d", "tet"])
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("kappa", [1e-1, 1e-4])
+def test_convection_matches_jacobi(unv, precision, kappa):
+    """BiCGSTAB with the cycle whose restriction is smoothed by A^T, from diffusion- to
+    convection-dominated, against the Jacobi-preconditioned solve of the same system."""
+    lib, out = prism_b200.lib(), []
+    mesh = api.Mesh(unv(), cases.box_case({"T": {"left": ("fixed", 1.0), "right": ("fixed", 0.0)}, "U": {}}), lib=lib)
+    c = mesh.export()["cell_center"]
+    U = api.Vector("U", mesh, np.stack([np.sin(np.pi * c[0]) * np.cos(np.pi * c[1]),
+                                        -np.cos(np.pi * c[0]) * np.sin(np.pi * c[1]), np.zeros(mesh.n_cells)]))
+    T = api.Scalar("T", mesh, 0.0)
+    k = api.Scalar("kappa", mesh, kappa)
+    eqn = api.Transport(api.convection.Upwind(U, T), api.diffusion.NonCorrected(k, T))
+    for solver in (api.BiCGSTAB(krylov_tol=1e-13, preconditioner="amg", precision=precision),
+                   api.BiCGSTAB(krylov_tol=1e-13, preconditioner="jacobi", krylov_max_iter=50000),
+                   api.BiCGSTAB(krylov_tol=1e-13, preconditioner="amg", precision=precision)):
+        T.set_values(np.zeros(mesh.n_cells))
+        r = solver.solve(eqn, 1, 0.0)
+        assert r.status == 0
+        out.append(T.values())
+    assert cases.rel_l2(out[0], out[1]) < 1e-8
+    assert np.array_equal(out[0], out[2])
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_stand_in_that_fails_falls_back(graph):
+    """A few cells of negative diffusivity make the matrix indefinite and multigrid diverge: the
+    solve goes back to the Jacobi-preconditioned BiCGSTAB from the same guess, in graph mode too."""
+    lib, out = prism_b200.lib(), []
+    mesh, T, eqn, (kappa, f) = diffusion(meshgen.box_hex(24, 22, 23), lib)
+    for solver in (api.BiCGSTAB(krylov_tol=1e-12, graph=graph),) * 3 + (api.BiCGSTAB(preconditioner="jacobi"),):
+        # the first solve, an ordinary one, sees a matrix that multigrid solves; then it turns indefinite
+        k = np.ones(mesh.n_cells)
+        if out or not graph:
+            k[::97] = -0.2
+        kappa.set_values(k)
+        T.set_values(np.zeros(mesh.n_cells))
+        r = solver.solve(eqn, 1, 0.0)
+        assert r.status == 0
+        out.append(T.values())
+    for x in out[1:3]:
+        assert cases.rel_l2(x, out[3]) < 1e-8
+
+
+@pytest.mark.parametrize("sizes", [[20, 20], [3, 21, 1, 9, 16, 5]])
+def test_batch_matches_single_solves(sizes):
+    """Batches large enough for flexible CG over the block-diagonal matrix, one of them with
+    systems down to a single row, and one system whose right-hand side is zero."""
+    lib = prism_b200.lib()
+    probs = [cases.diffusion_box(N, lib, seed=70 + i) for i, N in enumerate(sizes)]
+    probs[-1]["f"].set_values(np.zeros(probs[-1]["mesh"].n_cells))
+    bs = api.BatchSolver(api.BiCGSTAB(precision=0, krylov_tol=1e-13), lib=lib)
+    for _ in range(2):
+        for p in probs:
+            p["T"].set_values(np.zeros(p["mesh"].n_cells))
+        assert all(r.status == 0 for r in bs.solve([p["eqn"] for p in probs]))
+    for i, (N, p) in enumerate(zip(sizes, probs)):
+        q = cases.diffusion_box(N, lib, seed=70 + i)
+        if i == len(sizes) - 1:
+            assert np.all(p["T"].values() == 0.0)
+            continue
+        api.BiCGSTAB(krylov_tol=1e-13, preconditioner="jacobi").solve(q["eqn"], 1, 0.0)
+        assert cases.rel_l2(p["T"].values(), q["T"].values()) < 1e-8
