@@ -8,7 +8,7 @@ urf 0.7/0.3 (the 512x512 cavity recipe) on 1448x1448x1 hexes (2,096,704 cells): 
 1e-12 ||b|| like the reference's machine-precision step: the momentum predictors by
 BiCGSTAB with the Jacobi preconditioner that PRISM_PC_AUTO picks for their
 diagonally dominant matrices, the pressure correction by flexible CG preconditioned
-by an FP32 AMG V-cycle), run as one CUDA graph
+by an FP32 smoothed-aggregation V-cycle), run as one CUDA graph
 launch (PrismSolveOpts.graph: the solver loops are device-side conditional nodes
 and the kernels are those of the ordinary path, so the fields are identical).
 Inputs live in HBM; the working set (~1 GB) is larger than L2, so no flush is
@@ -23,12 +23,12 @@ reference's own code (tests/golden/c3_128_solution.npy, made by
 tests/golden/make_c3_solution.py and checked against its committed summary),
 FP64 vs FP32/FP64-reliable-update BiCGSTAB, both AMG-preconditioned, and FP64
 with the Jacobi preconditioner ("s_to_1e8"); the live bandwidth of the dominant
-kernels (the finest-level AMG post-smoothing and restriction SpMVs, the flexible-CG
+kernels (the finest-level multigrid up- and down-sweep, the flexible-CG
 SpMV and the BiCGSTAB SpMV: CUDA events around sampled launches of the ordinary-path
 run);
 the discrete adjoint of steady diffusion on 64^3 x 6 tets ("adjoint": times and
 finite-difference agreement) and 256 independent diffusion solves in one
-persistent launch ("batched").
+graph launch ("batched").
 
 --impl reference times the reference's own code (oracle/_ref/libprism_ref.so,
 compiled from the reference's sources; single-threaded, like the reference) on a
@@ -346,7 +346,7 @@ def adjoint_measure(lib, n=64, directions=2):
 
 def batched_measure(lib, count=256, nmin=16, nmax=96):
     """count independent diffusion problems (N^3 hexes, N log-uniform in [nmin, nmax], seed 4) solved in one
-    persistent launch (mixed precision), against the same systems solved one by one (FP64, Jacobi)."""
+    graph launch (mixed precision), against the same systems solved one by one (FP64, Jacobi)."""
     import numpy as np
     import torch
     from prism_b200 import _abi as A
@@ -380,7 +380,8 @@ def batched_measure(lib, count=256, nmin=16, nmax=96):
         # (values, columns, row offsets, x read, y written) and 23 vector passes
         return 2 * (nnz * (w + 4) + 4 * (n + 1) + 2 * w * n) + 23 * w * n
     shapes = [(p["mesh"].n_cells, p["mesh"].info.nnz) for p in probs]
-    bytes_batched = sum(r.krylov_iterations * iter_bytes(n, z, 4) for r, (n, z) in zip(res, shapes))
+    # one flexible-CG iteration: the FP64 SpMV and the vector update, the multigrid cycle not counted
+    bytes_batched = sum(r.krylov_iterations * (z * 12 + 4 * (n + 1) + 108 * n) for r, (n, z) in zip(res, shapes))
     bytes_seq = sum(k * iter_bytes(n, z, 8) for k, (n, z) in zip(seq_its, shapes))
     return {"workload": f"{count} problems, N^3 hexes with N = round(exp(U(ln {nmin}, ln {nmax}))) (seed 4), "
                         f"{cells} cells; kappa ~ lognormal(0,1), f ~ N(0,1), Fixed 0 walls, Corrected diffusion; "
@@ -393,8 +394,8 @@ def batched_measure(lib, count=256, nmin=16, nmax=96):
             "speedup_vs_sequential": t_seq / times[1],
             "total_iterations": sum(r.krylov_iterations for r in res), "sequential_total_iterations": sum(seq_its),
             "achieved_gbs": bytes_batched / times[1] / 1e9, "sequential_achieved_gbs": bytes_seq / t_seq / 1e9,
-            "achieved_note": "algorithmic bytes of the Krylov iterations (FP32 for the batch, its FP64 refinement "
-                             "steps not counted; FP64 one by one, each call's assembly not counted) / wall time"}
+            "achieved_note": "algorithmic bytes of the Krylov iterations (batch: flexible CG, its multigrid cycles not "
+                             "counted; one by one: FP64 Jacobi-BiCGSTAB; each call's assembly not counted) / wall time"}
 
 
 def run_ours(args, world, rank, local):
@@ -551,10 +552,14 @@ def run_ours(args, world, rank, local):
     fcg = kernel_line("fcg_spmv_kernel<4,6,float> (flexible CG u = A z + three fused dots: the pressure correction)",
                fcg_gbs, fcg_ms, fcg_bytes, prof.fcg_launches, "fcg_spmv_traffic.json")
     if post_gbs:
-        roof = kernel_line(f"post_kernel<{prec},1> (AMG finest level: prolongation + post-smoothing SpMV)",
+        roof = kernel_line("up_kernel<1> (smoothed aggregation, finest level: prolongation and its post-smoothing, "
+                    "x = y + Q e)" if a32 else
+                    f"post_kernel<{prec},1> (AMG finest level: prolongation + post-smoothing SpMV)",
                     post_gbs, post_ms, post_bytes, prof.amg32_post_launches if a32 else prof.amg_post_launches,
                     f"amg{'32' if a32 else ''}_post_traffic.json")
-        roof["down_kernel"] = kernel_line(f"down_kernel<{prec},1> (AMG finest level: smoothed restriction SpMV)",
+        roof["down_kernel"] = kernel_line("down0_kernel (smoothed aggregation, finest level: restriction Q^T b and the "
+                                   "two smoothing steps of b)" if a32 else
+                                   f"down_kernel<{prec},1> (AMG finest level: smoothed restriction SpMV)",
                                    down_gbs, down_ms, down_bytes,
                                    prof.amg32_down_launches if a32 else prof.amg_down_launches,
                                    f"amg{'32' if a32 else ''}_down_traffic.json")
@@ -612,7 +617,7 @@ def run_ours(args, world, rank, local):
                 "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
                 "config": {"workload": f"cavity SIMPLE {N_CAVITY}x{N_CAVITY}x1 ({n} cells), Re=100, Upwind + "
                                        "Corrected, urf 0.7/0.3, solves to 1e-12 (PRISM_PC_AUTO: momentum BiCGSTAB "
-                                       "with Jacobi, pressure correction flexible CG with an FP32 AMG V-cycle), "
+                                       "with Jacobi, pressure correction flexible CG with an FP32 smoothed-aggregation V-cycle), "
                                        "each outer iteration one CUDA graph launch (PrismSolveOpts.graph)",
                            "cells": n, "l2": "inputs larger than L2 (no flush)",
                            "parallelism": f"{world} independent replicas" if world > 1 else "1 GPU",

@@ -508,7 +508,9 @@ int prism_jacobi_step_noalloc(int64_t n, const int32_t* rowptr, const int32_t* c
 /* ---- batched solves --------------------------------------------------------- */
 /* Many independent equations (any meshes on this GPU) solved together: each is
  * assembled and relaxed as in prism_solve, then every system is solved in one
- * persistent launch -- BiCGSTAB with Jacobi preconditioning per system, FP32
+ * launch -- symmetric systems (diffusion without convection) of 8,192 rows and more
+ * in all by flexible CG over the block-diagonal matrix, preconditioned by one
+ * smoothed-aggregation V-cycle, others by BiCGSTAB with Jacobi preconditioning per system, FP32
  * inner iterations with FP64 dot products (precision PRISM_PREC_MIXED) or FP64
  * ones, each inner solve reducing its residual by inner_tol (default 1e-4 mixed)
  * between FP64 refinement steps, until ||b - Ax|| <= krylov_tol ||b|| (default

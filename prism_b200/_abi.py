@@ -32,6 +32,7 @@ PREC_FP64, PREC_MIXED = 0, 1
 TEMPORAL_BACKWARD_EULER, TEMPORAL_ADAM_MOULTON = 0, 1
 PC_AUTO, PC_JACOBI, PC_AMG = 0, 1, 2
 PC_AUTO_MIN_ROWS = 12288
+PC_AUTO_MIN_ROWS_SYM = 8192
 PRECONDITIONERS = {"auto": PC_AUTO, "jacobi": PC_JACOBI, "amg": PC_AMG}
 
 STATUS_NAMES = {

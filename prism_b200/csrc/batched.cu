@@ -1407,7 +1407,7 @@ std::vector<BatchOut> solveBatch(const std::vector<BatchSystem>& sys, BatchPlan&
         entries += q.nnz_csr;
         symmetric = symmetric && q.symmetric;
     }
-    if (symmetric && rows >= FLEX_MIN_ROWS && entries < ((int64_t)1 << 28) && sys.size() <= 65535) {
+    if (symmetric && rows >= FLEX_MIN_ROWS && entries < ((int64_t)1 << 29) && sys.size() <= 65535) {
         std::vector<BatchOut> out;
         if (runFlex(sys, pl, tol, maxit, own_cap, out, s)) return out;
         pl.no_flex = true;

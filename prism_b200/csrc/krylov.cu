@@ -1109,9 +1109,10 @@ void setupCycle(Amg* amg, int mode, const SellMatrix& A, const int* rowptr, cons
 }
 }  // namespace
 
-// Smoothed aggregation up to 2^28 matrix entries (38M rows of a hex mesh): its setup sorts
-// about three 64-bit keys per entry and numbers them with 32-bit ints.
-bool smoothedFits(const SellMatrix& A) { return A.nnz_csr < (int64_t(1) << 28); }
+// Smoothed aggregation up to 2^29 matrix entries (76M rows of a hex mesh): it numbers the entries
+// of Q, about 1.3 times as many, with 32-bit ints, and should rows have to be sorted, the
+// products, three times as many.
+bool smoothedFits(const SellMatrix& A) { return A.nnz_csr < (int64_t(1) << 29); }
 bool fcgSmoothed(const Amg* amg, const SellMatrix& A) { return fcgPre32(amg) && smoothedFits(A); }
 
 bool fcgPre32(const Amg* amg) {

@@ -143,8 +143,9 @@ struct SolveCtl {
 
 // A whole ISolver::solve of a small system with Jacobi-preconditioned FP64 BiCGSTAB in one
 // launch (small.cu): the record lands in *out (device), x is updated in place. It fits up to
-// 32,768 rows; a cap beyond 2^20 iterations keeps to the ordinary path, whose launches stay short.
-bool smallSolveFits(const SellMatrix& A, long long maxit);
+// 32,768 rows; caps beyond 2^20 iterations or 4,096 outer steps keep to the ordinary path, whose
+// launches stay short.
+bool smallSolveFits(const SellMatrix& A, long long maxit, long long n_iter = 1);
 void smallSolve(const SellMatrix& A, const double* b, double* x, long long n_iter, double eps, double tol,
                 long long maxit, bool symmetric, SolveCtl* out, cudaStream_t s);
 

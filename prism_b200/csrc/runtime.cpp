@@ -657,7 +657,7 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o) {
         if (!eq.amg) eq.amg = std::make_shared<Amg>();
         amg = eq.amg.get();
     }
-    if (o.method == PRISM_SOLVER_BICGSTAB && !amg && smallSolveFits(A, kmax)) {
+    if (o.method == PRISM_SOLVER_BICGSTAB && !amg && smallSolveFits(A, kmax, o.n_iter)) {
         const SolveCtl& c = runSmall(A, eq.b.p, phi.v.p, std::max<int64_t>(o.n_iter, 0), o.eps, ktol, kmax,
                                      symmetricMatrix(eq), m.kw, m.stream);
         phi.event += c.outer > 0 ? 1 + 3 * c.outer : 0;
@@ -1334,7 +1334,7 @@ PrismSolveResult solveCaptured(Transport& eq, const PrismSolveOpts& o) {
     const bool stand_in = standsIn(eq, o, kind);
     if (stand_in)
         PB_CUDA(cudaMemcpyAsync(m.kw.xs.p, phi.v.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    if (o.method == PRISM_SOLVER_BICGSTAB && !amg && smallSolveFits(A, kmax)) {
+    if (o.method == PRISM_SOLVER_BICGSTAB && !amg && smallSolveFits(A, kmax, o.n_iter)) {
         smallSolve(A, eq.b.p, phi.v.p, n_iter, o.eps, ktol, kmax, symmetricMatrix(eq), ctl, s);
         if (n_iter > 0) phi.event += 4;
         if (o.clear_coeffs) zeroOutCoeffs(eq);
@@ -1430,7 +1430,7 @@ bool graphReady(const Transport& eq, const PrismSolveOpts& o) {
         if (eq.auto_pc == 0) return false;  // chosen on an ordinary solve first
         pc = eq.auto_pc;
     }
-    if (pc == PRISM_PC_JACOBI && smallSolveFits(m.matrix(eq.A.p), kmax)) return true;
+    if (pc == PRISM_PC_JACOBI && smallSolveFits(m.matrix(eq.A.p), kmax, o.n_iter)) return true;
     if (m.kw.n != m.n_pad) return false;
     if (pc == PRISM_PC_AMG) {
         if (!eq.amg || !m.kw.y) return false;

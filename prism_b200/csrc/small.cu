@@ -347,8 +347,8 @@ void launchSmall(const SmallParams& P, cudaStream_t s) {
 
 }  // namespace
 
-bool smallSolveFits(const SellMatrix& A, long long maxit) {
-    return A.n > 0 && A.n <= maxCtas() * 2048 && maxit <= (1LL << 20);
+bool smallSolveFits(const SellMatrix& A, long long maxit, long long n_iter) {
+    return A.n > 0 && A.n <= maxCtas() * 2048 && maxit <= (1LL << 20) && n_iter <= 4096;
 }
 
 // Rows per block: one block up to 1,024 rows, whose barriers cost a fraction of a cluster's;
