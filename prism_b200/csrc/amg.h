@@ -94,6 +94,7 @@ struct Amg {
     // the smoothed-aggregation hierarchy of flexible CG (fcgMode picks it); this struct's own
     // levels then stay unbuilt
     std::unique_ptr<SaAmg> sa;
+    bool no_sa = false;  // that hierarchy did not fit (memory, 32-bit indices): this struct's own from then on
 
     // Build the hierarchy (first call) or refresh its values (later calls) for
     // the matrix A, whose CSR pattern (device rowptr/col) lists each row's

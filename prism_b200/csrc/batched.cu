@@ -1409,7 +1409,17 @@ std::vector<BatchOut> solveBatch(const std::vector<BatchSystem>& sys, BatchPlan&
     }
     if (symmetric && rows >= FLEX_MIN_ROWS && entries < ((int64_t)1 << 29) && sys.size() <= 65535) {
         std::vector<BatchOut> out;
-        if (runFlex(sys, pl, tol, maxit, own_cap, out, s)) return out;
+        try {
+            if (runFlex(sys, pl, tol, maxit, own_cap, out, s)) return out;
+        } catch (const Error& e) {
+            if (!hierarchyDidNotFit(e)) throw;
+            // the persistent launch needs a fraction of this memory; nothing was written back yet
+            pl.sa.reset();
+            for (auto* b : {&pl.fr, &pl.fd, &pl.fq, &pl.fu, &pl.x0}) b->release();
+            for (auto* b : {&pl.fr32, &pl.fz32}) b->release();
+            for (auto* b : {&pl.rowptr, &pl.csr_col}) b->release();
+            pl.fstate.release();
+        }
         pl.no_flex = true;
     }
     if (mixed) return runBatch<float>(sys, pl, tol, itol, max_inner, max_pass, maxit, s);

@@ -53,8 +53,8 @@ struct DevBuf {
     ~DevBuf() { release(); }
     void alloc(size_t count) {
         release();
-        n = count;
         if (count) PB_CUDA(cudaMalloc(&p, count * sizeof(T)));
+        n = count;
     }
     void release() {
         if (p) cudaFree(p);

@@ -681,7 +681,7 @@ void KrylovWork::ensure(int n_pad, int64_t nnz_padded, bool mixed) {
 }
 void KrylovWork::ensurePrec(bool mixed) {
     bool fresh = false;
-    if (y.n != (size_t)n) {
+    if (y.n != (size_t)n || z.n != (size_t)n) {
         fresh = true;
         y.alloc(n);
         z.alloc(n);
@@ -690,7 +690,7 @@ void KrylovWork::ensurePrec(bool mixed) {
         y32.release();
         z32.release();
     }
-    if (mixed && !y32) {
+    if (mixed && (!y32 || !z32)) {
         fresh = true;
         y32.alloc(n);
         z32.alloc(n);
@@ -1093,8 +1093,8 @@ namespace {
 // recurrences stay FP64) unless the hierarchy has K-cycle levels (FP64 only) or
 // PRISM_FCG_PREC=fp64
 int solveMode(int kind, const Amg* amg, const SellMatrix& A) {
+    if (kind == SOLVE_PLAIN || (kind == SOLVE_SMOOTHED && amg->no_sa)) return KM_BICGSTAB;
     if (kind == SOLVE_SMOOTHED) return KM_BICGSTAB_SA;
-    if (kind == SOLVE_PLAIN) return KM_BICGSTAB;
     return fcgSmoothed(amg, A) ? KM_FCG_SA : fcgPre32(amg) ? KM_FCG_PRE32 : KM_FCG;
 }
 // values of the cycle's hierarchy from the current matrix (built on first use)
@@ -1112,8 +1112,9 @@ void setupCycle(Amg* amg, int mode, const SellMatrix& A, const int* rowptr, cons
 // Smoothed aggregation up to 2^29 matrix entries (76M rows of a hex mesh): it numbers the entries
 // of Q, about 1.3 times as many, with 32-bit ints, and should rows have to be sorted, the
 // products, three times as many.
-bool smoothedFits(const SellMatrix& A) { return A.nnz_csr < (int64_t(1) << 29); }
-bool fcgSmoothed(const Amg* amg, const SellMatrix& A) { return fcgPre32(amg) && smoothedFits(A); }
+bool smoothedFits(const Amg* amg, const SellMatrix& A) { return !amg->no_sa && A.nnz_csr < (int64_t(1) << 29); }
+bool fcgSmoothed(const Amg* amg, const SellMatrix& A) { return fcgPre32(amg) && smoothedFits(amg, A); }
+bool hierarchyDidNotFit(const Error& e) { return e.status == PRISM_OUT_OF_MEMORY || e.status == PRISM_BAD_ARG; }
 
 bool fcgPre32(const Amg* amg) {
     static const bool p64 = [] {
@@ -1150,8 +1151,8 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
     const bool flexible = kind == SOLVE_FLEXIBLE;
     if (flexible && (mixed || !amg)) fail(PRISM_INTERNAL, "flexible CG runs FP64 with AMG only");
     if (kind == SOLVE_SMOOTHED && !amg) fail(PRISM_INTERNAL, "smoothed aggregation without its hierarchy");
-    const int mode = solveMode(kind, amg, A);
-    const bool pre32 = mixed || precondIn32(mode);  // FP32 copy of the hierarchy
+    int mode = solveMode(kind, amg, A);
+    bool pre32 = mixed || precondIn32(mode);  // FP32 copy of the hierarchy
     w.ensure(A.nslices * 32, A.nnz_padded, mixed);
     const int n = A.n;
     const int gn = ceil_div(n, BS);
@@ -1174,9 +1175,20 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
         M32 = w.As32.p;
     } else {
         if (!rowptr || !col) fail(PRISM_INTERNAL, "AMG preconditioner without a CSR pattern");
-        w.ensurePrec(pre32);
         VerboseTimer vt("amg setup", s);
-        setupCycle(amg, mode, A, rowptr, col, pre32, s);
+        w.ensurePrec(pre32);
+        try {
+            setupCycle(amg, mode, A, rowptr, col, pre32, s);
+        } catch (const Error& e) {
+            // smoothed aggregation wants about twice the memory of amg's own hierarchy: go without it
+            if (!smoothedMode(mode) || !hierarchyDidNotFit(e)) throw;
+            amg->sa.reset();
+            amg->no_sa = true;
+            mode = solveMode(kind, amg, A);
+            pre32 = mixed || precondIn32(mode);
+            w.ensurePrec(pre32);
+            setupCycle(amg, mode, A, rowptr, col, pre32, s);
+        }
         M32 = amg->vals32();
         if (mixed && mode == KM_BICGSTAB_SA) {  // the FP32 iteration's matrix
             to_float_kernel<<<std::min<int64_t>((A.nnz_padded + BS - 1) / BS, NUM_SMS * 32), BS, 0, s>>>(A.nnz_padded, A.vals,

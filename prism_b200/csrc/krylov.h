@@ -108,7 +108,9 @@ bool fcgPre32(const Amg* amg);
 // that V-cycle is smoothed aggregation's (samg.h)
 bool fcgSmoothed(const Amg* amg, const SellMatrix& A);
 // smoothed aggregation takes matrices of this size
-bool smoothedFits(const SellMatrix& A);
+bool smoothedFits(const Amg* amg, const SellMatrix& A);
+// e says that the structure of a hierarchy found no memory, or no room in its 32-bit indices
+bool hierarchyDidNotFit(const Error& e);
 // x <- x + D^-1 (b - A x)   (numerics/jacobi.cpp:5-9)
 void jacobiStep(const SellMatrix& A, const double* b, double* x, KrylovWork& w, cudaStream_t s);
 // max|A x - b| / (max|diag(A) x| + eps)   (numerics/solver.cpp:8-24); returns NaN if non-finite values met

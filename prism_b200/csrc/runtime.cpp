@@ -570,7 +570,7 @@ static int kindFor(const Transport& eq, const PrismSolveOpts& o, const Amg* amg,
     if (o.method == PRISM_SOLVER_FCG) return SOLVE_FLEXIBLE;
     if (!on || !amg || o.method != PRISM_SOLVER_BICGSTAB) return SOLVE_PLAIN;
     if (eq.spd) return o.precision == PRISM_PREC_FP64 ? SOLVE_FLEXIBLE : SOLVE_PLAIN;
-    if (eq.no_stand_in || g_in_step || !smoothedFits(A)) return SOLVE_PLAIN;
+    if (eq.no_stand_in || g_in_step || !smoothedFits(amg, A)) return SOLVE_PLAIN;
     return symmetricMatrix(eq) ? SOLVE_FLEXIBLE : SOLVE_SMOOTHED;
 }
 // that kind stands in for the BiCGSTAB with amg's cycle that was asked for
@@ -1117,7 +1117,7 @@ FixedPointOut adjointBackward(Transport& eq, const double* dJ, double* gk, doubl
         PB_CUDA(cudaMemcpyAsync(lam_prev.p, lam.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, s));
         if (amg && eq.no_stand_in && o.preconditioner == PRISM_PC_AUTO && smallSolveFits(AT, 1)) amg = nullptr;
         const HoldAmgValues hold(amg, it > 0);
-        KrylovOut k = amg && !eq.no_stand_in && smoothedFits(AT)
+        KrylovOut k = amg && !eq.no_stand_in && smoothedFits(amg, AT)
                           ? standInSolve(AT, rhs.p, lam.p, ktol, kmax, SOLVE_FLEXIBLE, fp64, m, amg, eq)
                           : bicgstab(AT, rhs.p, lam.p, ktol, kmax, PRISM_PREC_FP64, 0.1, m.kw, s, amg, m.pat.rowptr.p,
                                      m.pat.col.p, SOLVE_PLAIN, true);
