@@ -1126,8 +1126,9 @@ __global__ void flex_zero_kernel(const FP P) {
         if (P.st[pr].restart && P.st[pr].done == 4) P.x[sl * 32 + lane] = 0.0;
     });
 }
-// the end of a pass: accept, or start again from x (the recursive residual drifted, or the
-// recurrence broke down), as bicgstab() does
+// the end of a pass: accept a system whose true residual meets the tolerance, or start again
+// from x (the recursive residual drifted, or the recurrence broke down)
+constexpr int FLEX_MAX_PASS = 4;
 __global__ void __launch_bounds__(BS) flex_pass_kernel(const FP P) {
     FState& S = P.st[blockIdx.x];
     if (!S.restart) return;
@@ -1137,7 +1138,10 @@ __global__ void __launch_bounds__(BS) flex_pass_kernel(const FP P) {
     S.rel = S.bb > 0.0 ? sqrt(t[0] / S.bb) : 0.0;
     S.restart = 0;
     if (S.done == 1) {
-        if (S.rel > 10 * P.tol && ++S.pass < 4) S.restart = 1;
+        if (S.rel > P.tol) {
+            if (++S.pass < FLEX_MAX_PASS) S.restart = 1;
+            else S.status = PRISM_NOT_CONVERGED;
+        }
     } else if (S.done == 3) {
         if (++S.restarts > 20) S.status = PRISM_BREAKDOWN;
         else S.restart = 1;
@@ -1163,8 +1167,11 @@ __global__ void flex_pattern_kernel(int n, int padded, const int* rowptr, const 
     for (int k = t; k < nnz; k += gridDim.x * BS) cc[entry0 + k] = col[k] + row0;
 }
 
-// Solves the batch in one graph launch; false (and the guesses put back) if a system failed.
-bool runFlex(const std::vector<BatchSystem>& sys, BatchPlan& pl, double tol, long long maxit, bool own_cap,
+// Solves the batch in one graph launch. FLEX_SHORT: every system came close, but a residual did
+// not reach the tolerance in FLEX_MAX_PASS passes (x is kept); FLEX_FAILED: a system failed (the
+// guesses are put back).
+enum FlexEnd { FLEX_OK, FLEX_SHORT, FLEX_FAILED };
+FlexEnd runFlex(const std::vector<BatchSystem>& sys, BatchPlan& pl, double tol, long long maxit, bool own_cap,
              std::vector<BatchOut>& out, cudaStream_t s) {
     const int nrows = pl.nslices * 32;
     if (!pl.rowptr) {
@@ -1306,28 +1313,29 @@ bool runFlex(const std::vector<BatchSystem>& sys, BatchPlan& pl, double tol, lon
     PB_CUDA(cudaMemcpyAsync(hs.data(), P.st, pl.nprob * sizeof(FState), cudaMemcpyDeviceToHost, s));
     PB_CUDA(cudaStreamSynchronize(s));
     out.assign(pl.nprob, BatchOut{});
-    bool ok = true;
+    FlexEnd end = FLEX_OK;
     for (int i = 0; i < pl.nprob; ++i) {
         out[i].iterations = hs[i].iter;
         out[i].passes = hs[i].pass + 1;
         out[i].rel_residual = hs[i].rel;
         out[i].status = hs[i].status;
         const bool capped = own_cap && hs[i].status == PRISM_NOT_CONVERGED && hs[i].iter >= maxit;
-        ok = ok && (hs[i].status == PRISM_OK || capped);
+        if (hs[i].status == PRISM_OK || capped) continue;
+        end = std::max(end, hs[i].done == 1 ? FLEX_SHORT : FLEX_FAILED);
     }
     if (verbose()) {
         long long most = 0;
         for (const auto& q : out) most = std::max<long long>(most, q.iterations);
         std::fprintf(stderr, "[prism] batched flexible CG of %d systems (%d rows): at most %lld iterations, %s\n", pl.nprob,
-                     nrows, most, ok ? "ok" : "failed");
+                     nrows, most, end == FLEX_OK ? "ok" : end == FLEX_SHORT ? "residuals above the tolerance" : "failed");
     }
-    if (!ok) {
+    if (end == FLEX_FAILED) {
         PB_CUDA(cudaMemcpyAsync(pl.x64.p, pl.x0.p, nrows * sizeof(double), cudaMemcpyDeviceToDevice, s));
         scatter();
         pl.graph.reset();
         pl.graph_key.clear();
     }
-    return ok;
+    return end;
 }
 
 }  // namespace
@@ -1410,7 +1418,9 @@ std::vector<BatchOut> solveBatch(const std::vector<BatchSystem>& sys, BatchPlan&
     if (symmetric && rows >= FLEX_MIN_ROWS && entries < ((int64_t)1 << 29) && sys.size() <= 65535) {
         std::vector<BatchOut> out;
         try {
-            if (runFlex(sys, pl, tol, maxit, own_cap, out, s)) return out;
+            const FlexEnd end = runFlex(sys, pl, tol, maxit, own_cap, out, s);
+            if (end == FLEX_OK) return out;
+            pl.no_flex = end == FLEX_FAILED;
         } catch (const Error& e) {
             if (!hierarchyDidNotFit(e)) throw;
             // the persistent launch needs a fraction of this memory; nothing was written back yet
@@ -1419,8 +1429,8 @@ std::vector<BatchOut> solveBatch(const std::vector<BatchSystem>& sys, BatchPlan&
             for (auto* b : {&pl.fr32, &pl.fz32}) b->release();
             for (auto* b : {&pl.rowptr, &pl.csr_col}) b->release();
             pl.fstate.release();
+            pl.no_flex = true;
         }
-        pl.no_flex = true;
     }
     if (mixed) return runBatch<float>(sys, pl, tol, itol, max_inner, max_pass, maxit, s);
     return runBatch<double>(sys, pl, tol, itol, max_inner, max_pass, maxit, s);

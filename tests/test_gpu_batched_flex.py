@@ -1,0 +1,32 @@
+"""Batches large enough for flexible CG over the block-diagonal matrix: what a call promises
+(tolerance, iteration cap, independence of the systems from one another)."""
+import numpy as np
+import pytest
+
+from prism_b200 import _abi as A
+from prism_b200 import api
+from tests import cases
+
+pytestmark = pytest.mark.gpu
+
+
+def batch(lib, sizes, **opts):
+    probs = [cases.diffusion_box(N, lib, seed=70 + i) for i, N in enumerate(sizes)]
+    return probs, api.BatchSolver(api.BiCGSTAB(**opts), lib=lib)
+
+
+def solve(bs, probs):
+    for p in probs:
+        p["T"].set_values(np.zeros(p["mesh"].n_cells))
+    return bs.solve([p["eqn"] for p in probs])
+
+
+@pytest.mark.parametrize("precision", [A.PREC_MIXED, A.PREC_FP64])
+@pytest.mark.parametrize("tol", [1e-12, 1e-14, 1e-15])
+@pytest.mark.parametrize("sizes", [[20, 20], [24, 17, 31], [40, 33, 16, 9]])
+def test_residuals_meet_the_tolerance(gpu, sizes, tol, precision):
+    """OK means ||b - A x|| <= krylov_tol ||b||, down to a few units of the last place."""
+    probs, bs = batch(gpu, sizes, precision=precision, krylov_tol=tol)
+    for _ in range(2):
+        res = solve(bs, probs)
+        assert all(r.status == A.OK and r.krylov_rel_residual <= tol for r in res), res
