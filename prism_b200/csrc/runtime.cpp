@@ -592,15 +592,27 @@ static void checkFcg(const PrismSolveOpts& o) {
     if (o.preconditioner == PRISM_PC_JACOBI) fail(PRISM_BAD_ARG, "flexible CG needs the AMG preconditioner");
 }
 
-// A stand-in failed on eq: BiCGSTAB from now on, with Jacobi where the choice is the library's
+// A solve of eq goes without multigrid since a stand-in failed: where the choice is the library's
 // and the size one for the one-launch solve (sizes at which multigrid is chosen for its speed
-// alone), else with amg's cycle. Returns the hierarchy to use (null: Jacobi).
+// alone). A request for AMG or flexible CG stays one.
+static bool gaveUpToJacobi(const Transport& eq, const PrismSolveOpts& o, const SellMatrix& A) {
+    return eq.no_stand_in && o.method == PRISM_SOLVER_BICGSTAB && o.preconditioner == PRISM_PC_AUTO &&
+           smallSolveFits(A, 1);
+}
+// the hierarchy of a solve of eq, as yet unbuilt on the first one (null: none)
+static Amg* hierarchyFor(Transport& eq, const PrismSolveOpts& o, const SellMatrix& A) {
+    if (o.method == PRISM_SOLVER_JACOBI) return nullptr;
+    if (o.method != PRISM_SOLVER_FCG && (pcFor(eq, o, A) != PRISM_PC_AMG || gaveUpToJacobi(eq, o, A))) return nullptr;
+    if (!eq.amg) eq.amg = std::make_shared<Amg>();
+    return eq.amg.get();
+}
+
+// A stand-in failed on eq: BiCGSTAB from now on, with Jacobi (gaveUpToJacobi) or with amg's
+// cycle. Returns the hierarchy to use (null: Jacobi).
 static Amg* standInGaveUp(Transport& eq, const PrismSolveOpts& o, const SellMatrix& A, Amg* amg) {
     eq.no_stand_in = true;
     amg->values_current = false;
-    if (o.preconditioner != PRISM_PC_AUTO || !smallSolveFits(A, 1)) return amg;
-    eq.auto_pc = PRISM_PC_JACOBI;
-    return nullptr;
+    return gaveUpToJacobi(eq, o, A) ? nullptr : amg;
 }
 
 // One step by a stand-in (kindFor); should it fail, the solve it stands in for from the same
@@ -652,11 +664,7 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o) {
     const double ktol = o.krylov_tol > 0 ? o.krylov_tol : 1e-12;
     const long long kmax = o.krylov_max_iter > 0 ? o.krylov_max_iter : 2LL * m.nc;
     const double itol = o.inner_tol > 0 ? o.inner_tol : 0.1;
-    Amg* amg = nullptr;
-    if (o.method == PRISM_SOLVER_FCG || (o.method != PRISM_SOLVER_JACOBI && pcFor(eq, o, A) == PRISM_PC_AMG)) {
-        if (!eq.amg) eq.amg = std::make_shared<Amg>();
-        amg = eq.amg.get();
-    }
+    Amg* amg = hierarchyFor(eq, o, A);
     if (o.method == PRISM_SOLVER_BICGSTAB && !amg && smallSolveFits(A, kmax, o.n_iter)) {
         const SolveCtl& c = runSmall(A, eq.b.p, phi.v.p, std::max<int64_t>(o.n_iter, 0), o.eps, ktol, kmax,
                                      symmetricMatrix(eq), m.kw, m.stream);
@@ -681,7 +689,7 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o) {
             jacobiStep(A, eq.b.p, phi.v.p, m.kw, m.stream);
         } else {
             const HoldAmgValues hold(amg, eq.matrix_unchanged || iter > 0);  // A is fixed within one solve
-            if (amg && eq.auto_pc == PRISM_PC_JACOBI && eq.no_stand_in) amg = nullptr;  // gave up in an earlier step
+            if (gaveUpToJacobi(eq, o, A)) amg = nullptr;  // in an earlier step
             const int kind = kindFor(eq, o, amg, A);
             KrylovOut k = standsIn(eq, o, kind)
                               ? standInSolve(A, eq.b.p, phi.v.p, ktol, kmax, kind, o, m, amg, eq)
@@ -1323,11 +1331,7 @@ PrismSolveResult solveCaptured(Transport& eq, const PrismSolveOpts& o) {
     SellMatrix A = m.matrix(eq.A.p);
     const double ktol = o.krylov_tol > 0 ? o.krylov_tol : 1e-12;
     const long long kmax = o.krylov_max_iter > 0 ? o.krylov_max_iter : 2LL * m.nc;
-    Amg* amg = nullptr;
-    if (o.method == PRISM_SOLVER_FCG || pcFor(eq, o, A) == PRISM_PC_AMG) {
-        if (!eq.amg) eq.amg = std::make_shared<Amg>();
-        amg = eq.amg.get();
-    }
+    Amg* amg = hierarchyFor(eq, o, A);
     const long long n_iter = std::max<long long>(o.n_iter, 0);
     // a stand-in's guess is kept in case it fails (solveAsGraph, which then needs the system too)
     const int kind = kindFor(eq, o, amg, A);
@@ -1430,6 +1434,7 @@ bool graphReady(const Transport& eq, const PrismSolveOpts& o) {
         if (eq.auto_pc == 0) return false;  // chosen on an ordinary solve first
         pc = eq.auto_pc;
     }
+    if (gaveUpToJacobi(eq, o, m.matrix(eq.A.p))) pc = PRISM_PC_JACOBI;
     if (pc == PRISM_PC_JACOBI && smallSolveFits(m.matrix(eq.A.p), kmax, o.n_iter)) return true;
     if (m.kw.n != m.n_pad) return false;
     if (pc == PRISM_PC_AMG) {
@@ -1471,10 +1476,10 @@ PrismSolveResult solveAsGraph(Transport& eq, const PrismSolveOpts& o) {
     if (used != 1) fail(PRISM_INTERNAL, "graph solve recorded no solve");
     out = fromCtl(m.graph_host[0]);
     const SellMatrix A = m.matrix(eq.A.p);
-    const bool with_amg = o.method == PRISM_SOLVER_FCG || pcFor(eq, o, A) == PRISM_PC_AMG;
-    if (with_amg && standsIn(eq, o, kindFor(eq, o, eq.amg.get(), A))) {
+    Amg* amg = hierarchyFor(eq, o, A);
+    if (standsIn(eq, o, kindFor(eq, o, amg, A))) {
         if (standInFailed(o, out.status, out.krylov_iterations)) {
-            standInGaveUp(eq, o, A, eq.amg.get());
+            standInGaveUp(eq, o, A, amg);
             PB_CUDA(cudaMemcpyAsync(eq.phi->v.p, m.kw.xs.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
             out = solveAssembled(eq, o);
         }

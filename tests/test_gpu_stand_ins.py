@@ -1,0 +1,76 @@
+"""Solves by smoothed aggregation that stand in for the method that was asked for: what they
+leave as it was (the caller's choices and caps, the next solve) when one of them fails."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from prism_b200 import _abi as A
+from prism_b200 import api, meshgen
+from tests import cases
+from tests.test_gpu_smoothed import diffusion
+
+pytestmark = pytest.mark.gpu
+
+
+def counted(lib, f):
+    """f() and the kernels it launched."""
+    prof = A.Profile()
+    lib.check(lib.profile_start(0))
+    r = f()
+    lib.check(lib.profile_stop(ctypes.byref(prof)))
+    return r, prof.kernel_launches
+
+
+def solve(solver, eqn, T, n_iter=1, eps=0.0):
+    T.set_values(np.zeros(len(T.values())))
+    return solver.solve(eqn, n_iter, eps)
+
+
+def indefinite(n):
+    """A few negative diffusivities: smoothed aggregation diverges, Jacobi-BiCGSTAB converges."""
+    k = np.ones(n)
+    k[::97] = -0.2
+    return k
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_asked_for_multigrid_is_used(gpu, graph):
+    """12,144 rows, the automatic solve gave up multigrid: AMG and flexible CG that are asked
+    for by name still run (a V-cycle solve launches hundreds of kernels or a loop of them, the
+    one-launch solve a handful) and take the iterations that they take on a fresh equation."""
+    want = {}
+    for given_up in (False, True):
+        mesh, T, eqn, (kappa, f) = diffusion(meshgen.box_hex(24, 22, 23), gpu)
+        good = kappa.values()
+        if given_up:
+            kappa.set_values(indefinite(mesh.n_cells))
+            assert solve(api.BiCGSTAB(), eqn, T).status == A.OK
+            kappa.set_values(good)
+        for solver in (api.FCG(graph=graph), api.BiCGSTAB(preconditioner="amg", graph=graph)):
+            for _ in range(2):  # the second as a graph
+                r, kernels = counted(gpu, lambda: solve(solver, eqn, T))
+                assert r.status == A.OK and kernels > 20 and r.krylov_iterations < 60
+            if given_up and isinstance(solver, api.FCG):
+                assert cases.rel_l2(T.values(), want) < 1e-8
+            want = T.values() if not given_up else want
+
+
+def test_flexible_cg_after_dominance_chose_jacobi(gpu):
+    """39,304 rows whose automatic choice was Jacobi (a small time step), then a failed AMG
+    solve: flexible CG solves the equation as it did before."""
+    mesh = api.Mesh(meshgen.box_hex(34, 34, 34), cases.box_case({"T": {p: ("fixed", 0.0) for p in meshgen.PATCHES}}),
+                    lib=gpu)
+    T = api.Scalar("T", mesh, 0.0)
+    T.set_history_size(1)
+    T.update(np.zeros(mesh.n_cells))
+    kappa = api.Scalar("kappa", mesh, 1.0)
+    f = api.Scalar("f", mesh, np.random.default_rng(1).normal(size=mesh.n_cells))
+    time = api.temporal.BackwardEuler(T, 1e-6)
+    eqn = api.Transport(time, api.diffusion.NonCorrected(kappa, T), api.source.ConstantScalar(f))
+    assert solve(api.BiCGSTAB(), eqn, T).status == A.OK
+    eqn.set_time_step(1e3)
+    kappa.set_values(indefinite(mesh.n_cells))
+    solve(api.BiCGSTAB(preconditioner="amg", krylov_max_iter=1000), eqn, T)
+    kappa.set_values(np.ones(mesh.n_cells))
+    assert solve(api.FCG(), eqn, T).status == A.OK
