@@ -578,10 +578,10 @@ static bool standsIn(const Transport& eq, const PrismSolveOpts& o, int kind) {
     return kind != SOLVE_PLAIN && o.method != PRISM_SOLVER_FCG && !eq.spd;
 }
 constexpr long long STAND_IN_MAX = 500;  // iterations (20-60 are usual) after which it has failed
-// a stand-in's end that has to be mended: anything but success or the caller's own iteration cap
-static bool standInFailed(const PrismSolveOpts& o, int status, long long iterations) {
-    return status != PRISM_OK &&
-           !(status == PRISM_NOT_CONVERGED && o.krylov_max_iter > 0 && iterations >= o.krylov_max_iter);
+// a stand-in's end that has to be mended: anything but success or the caller's own iteration
+// cap, which its iterations count against (used: since the step began)
+static bool standInFailed(const PrismSolveOpts& o, int status, long long used) {
+    return status != PRISM_OK && !(status == PRISM_NOT_CONVERGED && o.krylov_max_iter > 0 && used >= o.krylov_max_iter);
 }
 
 // PRISM_SOLVER_FCG's requirements: FP64, and the AMG preconditioner (its own choice
@@ -616,7 +616,8 @@ static Amg* standInGaveUp(Transport& eq, const PrismSolveOpts& o, const SellMatr
 }
 
 // One step by a stand-in (kindFor); should it fail, the solve it stands in for from the same
-// guess. The guess waits in xs, which AMG solves do not use.
+// guess, with what is left of a cap that the caller set. The guess waits in xs, which AMG solves
+// do not use.
 static KrylovOut standInSolve(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, int kind,
                               const PrismSolveOpts& o, Mesh& m, Amg* amg, Transport& eq) {
     KrylovWork& w = m.kw;
@@ -628,7 +629,12 @@ static KrylovOut standInSolve(const SellMatrix& A, const double* b, double* x, d
     if (!standInFailed(o, k.status, k.iterations)) return k;
     Amg* plain = standInGaveUp(eq, o, A, amg);
     PB_CUDA(cudaMemcpyAsync(x, w.xs.p, A.n * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
-    KrylovOut f = bicgstab(A, b, x, tol, maxit, o.precision, itol, w, m.stream, plain, m.pat.rowptr.p, m.pat.col.p);
+    const long long left = o.krylov_max_iter > 0 ? maxit - k.iterations : maxit;
+    if (left <= 0) {
+        k.has_scaled = false;  // x is the guess again
+        return k;
+    }
+    KrylovOut f = bicgstab(A, b, x, tol, left, o.precision, itol, w, m.stream, plain, m.pat.rowptr.p, m.pat.col.p);
     f.iterations += k.iterations;
     return f;
 }

@@ -74,3 +74,14 @@ def test_flexible_cg_after_dominance_chose_jacobi(gpu):
     solve(api.BiCGSTAB(preconditioner="amg", krylov_max_iter=1000), eqn, T)
     kappa.set_values(np.ones(mesh.n_cells))
     assert solve(api.FCG(), eqn, T).status == A.OK
+
+
+@pytest.mark.parametrize("cap", [3, 40, 600, 1000])
+@pytest.mark.parametrize("preconditioner", ["auto", "amg"])
+def test_iteration_cap_is_kept(gpu, cap, preconditioner):
+    """The stand-in's iterations count against the caller's cap, which bounds them together."""
+    mesh, T, eqn, (kappa, f) = diffusion(meshgen.box_hex(24, 22, 23), gpu)
+    kappa.set_values(indefinite(mesh.n_cells))
+    r = solve(api.BiCGSTAB(preconditioner=preconditioner, krylov_max_iter=cap), eqn, T)
+    assert r.krylov_iterations <= cap
+    assert r.status == A.OK or cap < 600 or preconditioner == "amg"  # plain AMG diverges on it too
