@@ -1447,7 +1447,7 @@ constexpr int GRAPH_UNROLL = 4;  // BiCGSTAB iterations per pass of the device l
 __device__ __forceinline__ double nanValue() { return __longlong_as_double(0x7ff8000000000000LL); }
 
 __global__ void ctl_solve_begin_kernel(SolveCtl* c, long long n_iter, double eps, long long kmax, double tol,
-                                       cudaGraphConditionalHandle ho) {
+                                       int stand_in, cudaGraphConditionalHandle ho) {
     if (threadIdx.x) return;
     cudaGraphSetConditional(ho, 1u);
     SolveCtl z{};
@@ -1455,6 +1455,7 @@ __global__ void ctl_solve_begin_kernel(SolveCtl* c, long long n_iter, double eps
     z.eps = eps;
     z.kmax = kmax;
     z.tol = tol;
+    z.stand_in = stand_in;
     z.status = PRISM_OK;
     z.kstatus = PRISM_OK;
     z.phase = PH_DONE;
@@ -1546,7 +1547,9 @@ __global__ void ctl_outer_step_kernel(SolveCtl* c, const double* scal, cudaGraph
     c->outer += 1;
     const bool conv = cur < c->eps;
     if (conv) c->converged = 1;
-    cudaGraphSetConditional(ho, (!conv && c->outer < c->n_iter) ? 1u : 0u);
+    c->step_iterations = c->kmax - c->maxit_left;
+    c->failed = c->stand_in && c->kstatus != PRISM_OK && !(c->stand_in == 2 && c->kstatus == PRISM_NOT_CONVERGED);
+    cudaGraphSetConditional(ho, (!conv && !c->failed && c->outer < c->n_iter) ? 1u : 0u);
 }
 
 }  // namespace
@@ -1606,9 +1609,9 @@ void endConditional(cudaStream_t body) {
     PB_CUDA(cudaStreamEndCapture(body, &g));
 }
 
-void emitSolveBegin(SolveCtl* ctl, long long n_iter, double eps, long long kmax, double tol,
+void emitSolveBegin(SolveCtl* ctl, long long n_iter, double eps, long long kmax, double tol, int stand_in,
                     cudaGraphConditionalHandle outer, cudaStream_t s) {
-    ctl_solve_begin_kernel<<<1, 32, 0, s>>>(ctl, n_iter, eps, kmax, tol, outer); countLaunch();
+    ctl_solve_begin_kernel<<<1, 32, 0, s>>>(ctl, n_iter, eps, kmax, tol, stand_in, outer); countLaunch();
 }
 
 void emitResidual(const SellMatrix& A, const double* b, const double* x, KrylovWork& w, cudaStream_t s) {

@@ -141,6 +141,10 @@ struct SolveCtl {
     double tol, krylov_rel;
     int phase, pass, restarts, kstatus;
     long long guard;  // controller passes of the current BiCGSTAB solve
+    // a stand-in (runtime.cpp): its first failed step ends the solve (failed; its iterations in
+    // step_iterations). stand_in 2: the iteration cap is the caller's, and reaching it no failure
+    int stand_in, failed;
+    long long step_iterations;
 };
 
 // A whole ISolver::solve of a small system with Jacobi-preconditioned FP64 BiCGSTAB in one
@@ -173,7 +177,7 @@ bool capturing(cudaStream_t s);
 // Device-controlled pieces of solve(), emitted into the capture on s:
 // ctl := ISolver::solve bookkeeping for n_iter steps, eps, kmax, tol
 // (and switches on the outer loop's condition)
-void emitSolveBegin(SolveCtl* ctl, long long n_iter, double eps, long long kmax, double tol,
+void emitSolveBegin(SolveCtl* ctl, long long n_iter, double eps, long long kmax, double tol, int stand_in,
                     cudaGraphConditionalHandle outer, cudaStream_t s);
 // w.scal := max|A x - b|, max|diag(A) x|, non-finite flag (the scaled residual's parts)
 void emitResidual(const SellMatrix& A, const double* b, const double* x, KrylovWork& w, cudaStream_t s);

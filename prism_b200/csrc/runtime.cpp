@@ -662,8 +662,9 @@ PrismSolveResult fromCtl(const SolveCtl& c) {
 }
 }  // namespace
 
-// the steps of ISolver::solve on the assembled, relaxed and pinned system of eq
-static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o) {
+// the steps of ISolver::solve on the assembled, relaxed and pinned system of eq; spent:
+// iterations that count against the first step's cap already
+static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o, long long spent = 0) {
     Scalar& phi = *eq.phi;
     Mesh& m = *phi.m;
     SellMatrix A = m.matrix(eq.A.p);
@@ -671,7 +672,7 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o) {
     const long long kmax = o.krylov_max_iter > 0 ? o.krylov_max_iter : 2LL * m.nc;
     const double itol = o.inner_tol > 0 ? o.inner_tol : 0.1;
     Amg* amg = hierarchyFor(eq, o, A);
-    if (o.method == PRISM_SOLVER_BICGSTAB && !amg && smallSolveFits(A, kmax, o.n_iter)) {
+    if (o.method == PRISM_SOLVER_BICGSTAB && !amg && spent == 0 && smallSolveFits(A, kmax, o.n_iter)) {
         const SolveCtl& c = runSmall(A, eq.b.p, phi.v.p, std::max<int64_t>(o.n_iter, 0), o.eps, ktol, kmax,
                                      symmetricMatrix(eq), m.kw, m.stream);
         phi.event += c.outer > 0 ? 1 + 3 * c.outer : 0;
@@ -697,11 +698,12 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o) {
             const HoldAmgValues hold(amg, eq.matrix_unchanged || iter > 0);  // A is fixed within one solve
             if (gaveUpToJacobi(eq, o, A)) amg = nullptr;  // in an earlier step
             const int kind = kindFor(eq, o, amg, A);
+            const long long cap = iter == 0 && o.krylov_max_iter > 0 ? kmax - spent : kmax;
             KrylovOut k = standsIn(eq, o, kind)
-                              ? standInSolve(A, eq.b.p, phi.v.p, ktol, kmax, kind, o, m, amg, eq)
-                              : bicgstab(A, eq.b.p, phi.v.p, ktol, kmax, o.precision, itol, m.kw, m.stream, amg,
+                              ? standInSolve(A, eq.b.p, phi.v.p, ktol, cap, kind, o, m, amg, eq)
+                              : bicgstab(A, eq.b.p, phi.v.p, ktol, cap, o.precision, itol, m.kw, m.stream, amg,
                                          m.pat.rowptr.p, m.pat.col.p, kind, symmetricMatrix(eq));
-            r.krylov_iterations += k.iterations;
+            r.krylov_iterations += k.iterations + (iter == 0 ? spent : 0);
             r.krylov_rel_residual = k.rel_residual;
             if (k.status != PRISM_OK && r.status == PRISM_OK) r.status = k.status;
             cur_known = k.has_scaled;
@@ -1354,7 +1356,8 @@ PrismSolveResult solveCaptured(Transport& eq, const PrismSolveOpts& o) {
     }
     const long long cap = stand_in ? std::min(kmax, STAND_IN_MAX) : kmax;
     cudaGraphConditionalHandle outer = createConditional(s, 0);
-    emitSolveBegin(ctl, n_iter, o.eps, cap, ktol, outer, s);
+    const int stop = !stand_in ? 0 : o.krylov_max_iter > 0 && o.krylov_max_iter <= STAND_IN_MAX ? 2 : 1;
+    emitSolveBegin(ctl, n_iter, o.eps, cap, ktol, stop, outer, s);
     if (n_iter > 0) {
         ++phi.event;
         emitResidual(A, eq.b.p, phi.v.p, m.kw, s);
@@ -1484,10 +1487,12 @@ PrismSolveResult solveAsGraph(Transport& eq, const PrismSolveOpts& o) {
     const SellMatrix A = m.matrix(eq.A.p);
     Amg* amg = hierarchyFor(eq, o, A);
     if (standsIn(eq, o, kindFor(eq, o, amg, A))) {
-        if (standInFailed(o, out.status, out.krylov_iterations)) {
+        const SolveCtl& c = m.graph_host[0];
+        if (c.failed) {
+            const long long spent = c.step_iterations;
             standInGaveUp(eq, o, A, amg);
             PB_CUDA(cudaMemcpyAsync(eq.phi->v.p, m.kw.xs.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
-            out = solveAssembled(eq, o);
+            if (o.krylov_max_iter <= 0 || spent < o.krylov_max_iter) out = solveAssembled(eq, o, spent);
         }
         if (o.clear_coeffs) zeroOutCoeffs(eq);
     }
