@@ -592,12 +592,14 @@ static void checkFcg(const PrismSolveOpts& o) {
     if (o.preconditioner == PRISM_PC_JACOBI) fail(PRISM_BAD_ARG, "flexible CG needs the AMG preconditioner");
 }
 
-// A solve of eq goes without multigrid since a stand-in failed: where the choice is the library's
-// and the size one for the one-launch solve (sizes at which multigrid is chosen for its speed
-// alone). A request for AMG or flexible CG stays one.
+// What a failed stand-in goes back to: the one-launch Jacobi solve where the choice is the
+// library's and the size one for it (sizes at which multigrid is chosen for its speed alone),
+// else amg's cycle. A request for AMG or flexible CG stays one.
+static bool jacobiInstead(const PrismSolveOpts& o, const SellMatrix& A) {
+    return o.method == PRISM_SOLVER_BICGSTAB && o.preconditioner == PRISM_PC_AUTO && smallSolveFits(A, 1);
+}
 static bool gaveUpToJacobi(const Transport& eq, const PrismSolveOpts& o, const SellMatrix& A) {
-    return eq.no_stand_in && o.method == PRISM_SOLVER_BICGSTAB && o.preconditioner == PRISM_PC_AUTO &&
-           smallSolveFits(A, 1);
+    return eq.no_stand_in && jacobiInstead(o, A);
 }
 // the hierarchy of a solve of eq, as yet unbuilt on the first one (null: none)
 static Amg* hierarchyFor(Transport& eq, const PrismSolveOpts& o, const SellMatrix& A) {
@@ -607,12 +609,12 @@ static Amg* hierarchyFor(Transport& eq, const PrismSolveOpts& o, const SellMatri
     return eq.amg.get();
 }
 
-// A stand-in failed on eq: BiCGSTAB from now on, with Jacobi (gaveUpToJacobi) or with amg's
-// cycle. Returns the hierarchy to use (null: Jacobi).
-static Amg* standInGaveUp(Transport& eq, const PrismSolveOpts& o, const SellMatrix& A, Amg* amg) {
-    eq.no_stand_in = true;
-    amg->values_current = false;
-    return gaveUpToJacobi(eq, o, A) ? nullptr : amg;
+// A stand-in failed on eq, and the solve in its place ended with `status`: that one from now on,
+// unless both met values that are not finite. Those say nothing about the method; a structure
+// that was built from them goes.
+static void standInGaveUp(Transport& eq, Amg* amg, int status) {
+    if (status != PRISM_NONFINITE) eq.no_stand_in = true;
+    else if (amg->sa && amg->sa->fresh) amg->sa->built = false;
 }
 
 // One step by a stand-in (kindFor); should it fail, the solve it stands in for from the same
@@ -627,14 +629,16 @@ static KrylovOut standInSolve(const SellMatrix& A, const double* b, double* x, d
     KrylovOut k = bicgstab(A, b, x, tol, std::min(maxit, STAND_IN_MAX), kind == SOLVE_FLEXIBLE ? PRISM_PREC_FP64 : o.precision,
                            itol, w, m.stream, amg, m.pat.rowptr.p, m.pat.col.p, kind);
     if (!standInFailed(o, k.status, k.iterations)) return k;
-    Amg* plain = standInGaveUp(eq, o, A, amg);
     PB_CUDA(cudaMemcpyAsync(x, w.xs.p, A.n * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
     const long long left = o.krylov_max_iter > 0 ? maxit - k.iterations : maxit;
     if (left <= 0) {
         k.has_scaled = false;  // x is the guess again
         return k;
     }
-    KrylovOut f = bicgstab(A, b, x, tol, left, o.precision, itol, w, m.stream, plain, m.pat.rowptr.p, m.pat.col.p);
+    amg->values_current = false;
+    KrylovOut f = bicgstab(A, b, x, tol, left, o.precision, itol, w, m.stream, jacobiInstead(o, A) ? nullptr : amg,
+                           m.pat.rowptr.p, m.pat.col.p);
+    standInGaveUp(eq, amg, f.status);
     f.iterations += k.iterations;
     return f;
 }
@@ -662,9 +666,9 @@ PrismSolveResult fromCtl(const SolveCtl& c) {
 }
 }  // namespace
 
-// the steps of ISolver::solve on the assembled, relaxed and pinned system of eq; spent:
-// iterations that count against the first step's cap already
-static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o, long long spent = 0) {
+// the steps of ISolver::solve on the assembled, relaxed and pinned system of eq. plain: without
+// stand-ins; spent: iterations that count against the first step's cap already
+static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o, bool plain = false, long long spent = 0) {
     Scalar& phi = *eq.phi;
     Mesh& m = *phi.m;
     SellMatrix A = m.matrix(eq.A.p);
@@ -672,6 +676,7 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o, l
     const long long kmax = o.krylov_max_iter > 0 ? o.krylov_max_iter : 2LL * m.nc;
     const double itol = o.inner_tol > 0 ? o.inner_tol : 0.1;
     Amg* amg = hierarchyFor(eq, o, A);
+    if (plain && jacobiInstead(o, A)) amg = nullptr;
     if (o.method == PRISM_SOLVER_BICGSTAB && !amg && spent == 0 && smallSolveFits(A, kmax, o.n_iter)) {
         const SolveCtl& c = runSmall(A, eq.b.p, phi.v.p, std::max<int64_t>(o.n_iter, 0), o.eps, ktol, kmax,
                                      symmetricMatrix(eq), m.kw, m.stream);
@@ -696,8 +701,9 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o, l
             jacobiStep(A, eq.b.p, phi.v.p, m.kw, m.stream);
         } else {
             const HoldAmgValues hold(amg, eq.matrix_unchanged || iter > 0);  // A is fixed within one solve
-            if (gaveUpToJacobi(eq, o, A)) amg = nullptr;  // in an earlier step
-            const int kind = kindFor(eq, o, amg, A);
+            if ((eq.no_stand_in || (plain && !eq.spd)) && jacobiInstead(o, A)) amg = nullptr;  // since an earlier step
+            int kind = kindFor(eq, o, amg, A);
+            if (plain && standsIn(eq, o, kind)) kind = SOLVE_PLAIN;
             const long long cap = iter == 0 && o.krylov_max_iter > 0 ? kmax - spent : kmax;
             KrylovOut k = standsIn(eq, o, kind)
                               ? standInSolve(A, eq.b.p, phi.v.p, ktol, cap, kind, o, m, amg, eq)
@@ -706,6 +712,7 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o, l
             r.krylov_iterations += k.iterations + (iter == 0 ? spent : 0);
             r.krylov_rel_residual = k.rel_residual;
             if (k.status != PRISM_OK && r.status == PRISM_OK) r.status = k.status;
+            plain = plain || k.status == PRISM_NONFINITE;
             cur_known = k.has_scaled;
             cur = k.scaled_residual;
         }
@@ -1490,9 +1497,11 @@ PrismSolveResult solveAsGraph(Transport& eq, const PrismSolveOpts& o) {
         const SolveCtl& c = m.graph_host[0];
         if (c.failed) {
             const long long spent = c.step_iterations;
-            standInGaveUp(eq, o, A, amg);
             PB_CUDA(cudaMemcpyAsync(eq.phi->v.p, m.kw.xs.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
-            if (o.krylov_max_iter <= 0 || spent < o.krylov_max_iter) out = solveAssembled(eq, o, spent);
+            if (o.krylov_max_iter <= 0 || spent < o.krylov_max_iter) {
+                out = solveAssembled(eq, o, true, spent);
+                standInGaveUp(eq, amg, out.status);
+            }
         }
         if (o.clear_coeffs) zeroOutCoeffs(eq);
     }

@@ -1305,6 +1305,7 @@ void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, bool s
 void SaAmg::setup(const SellMatrix& A, const int* rowptr, const int* col, bool sym, bool keep_values, cudaStream_t s) {
     const bool same = built && symmetric == sym && !levels.empty() && levels[0]->n == A.n && levels[0]->sl_off == A.sl_off;
     if (same && keep_values && levels[0]->vals == A.vals) return;
+    fresh = !same;
     if (!same) {
         build(A, rowptr, col, sym, s);
     } else {

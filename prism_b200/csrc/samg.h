@@ -56,6 +56,7 @@ struct SaAmg {
     DevArena arena;  // declared first: released last
     std::vector<std::unique_ptr<SaLevel>> levels;
     bool built = false, symmetric = true;
+    bool fresh = false;  // the last setup built the structure: it belongs to the matrix of that call
     uint64_t generation = 0;
     int tail = -1;  // first level of the fused coarse tail (-1: none)
     int coarse_n = 0;

@@ -114,3 +114,31 @@ def test_cap_of_every_step(gpu, graph):
     r = solve(solver, eqn, T, 2)
     assert r.status == A.OK and r.iteration == 2 and r.krylov_rel_residual <= 1e-11
     assert r.krylov_iterations <= 2000
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("shape", [(24, 22, 23), (34, 33, 34)])
+@pytest.mark.parametrize("where", ["source", "kappa", "guess"])
+@pytest.mark.parametrize("first", [False, True])
+def test_nan_in_one_call_does_not_change_the_next(gpu, shape, where, first, graph):
+    """A call with a NaN ends as NONFINITE; the calls after it are, bit for bit, those of an
+    equation that never saw one."""
+    out = []
+    for poisoned in (False, True):
+        mesh, T, eqn, (kappa, f) = diffusion(meshgen.box_hex(*shape), gpu)
+        solver = api.BiCGSTAB(graph=graph)
+        for call in range(4):
+            T.set_values(np.zeros(mesh.n_cells))
+            field = {"source": f, "kappa": kappa, "guess": T}[where]
+            good = field.values()
+            if call == (0 if first else 2):
+                if not poisoned:
+                    continue
+                bad = good.copy()
+                bad[37] = np.nan
+                field.set_values(bad)
+            r = solver.solve(eqn, 3, 0.0)
+            field.set_values(good) if where != "guess" else None
+            assert r.status == (A.NONFINITE if call == (0 if first else 2) else A.OK)
+        out.append((T.values(), r.krylov_iterations))
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
