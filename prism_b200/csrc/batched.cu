@@ -1415,11 +1415,11 @@ std::vector<BatchOut> solveBatch(const std::vector<BatchSystem>& sys, BatchPlan&
         entries += q.nnz_csr;
         symmetric = symmetric && q.symmetric;
     }
+    std::vector<BatchOut> flex(sys.size());
     if (symmetric && rows >= FLEX_MIN_ROWS && entries < ((int64_t)1 << 29) && sys.size() <= 65535) {
-        std::vector<BatchOut> out;
         try {
-            const FlexEnd end = runFlex(sys, pl, tol, maxit, own_cap, out, s);
-            if (end == FLEX_OK) return out;
+            const FlexEnd end = runFlex(sys, pl, tol, maxit, own_cap, flex, s);
+            if (end == FLEX_OK) return flex;
             pl.no_flex = end == FLEX_FAILED;
         } catch (const Error& e) {
             if (!hierarchyDidNotFit(e)) throw;
@@ -1432,8 +1432,15 @@ std::vector<BatchOut> solveBatch(const std::vector<BatchSystem>& sys, BatchPlan&
             pl.no_flex = true;
         }
     }
-    if (mixed) return runBatch<float>(sys, pl, tol, itol, max_inner, max_pass, maxit, s);
-    return runBatch<double>(sys, pl, tol, itol, max_inner, max_pass, maxit, s);
+    // flexible CG's iterations count, and against a cap of the caller's
+    long long used = 0;
+    for (const auto& f : flex) used = std::max<long long>(used, f.iterations);
+    const long long left = own_cap ? maxit - used : maxit;
+    if (left <= 0) return flex;
+    std::vector<BatchOut> out = mixed ? runBatch<float>(sys, pl, tol, itol, max_inner, max_pass, left, s)
+                                      : runBatch<double>(sys, pl, tol, itol, max_inner, max_pass, left, s);
+    for (size_t i = 0; i < out.size(); ++i) out[i].iterations += flex[i].iterations;
+    return out;
 }
 
 }  // namespace pb

@@ -30,3 +30,24 @@ def test_residuals_meet_the_tolerance(gpu, sizes, tol, precision):
     for _ in range(2):
         res = solve(bs, probs)
         assert all(r.status == A.OK and r.krylov_rel_residual <= tol for r in res), res
+
+
+def indefinite(p):
+    """A few negative diffusivities: flexible CG fails on this system, BiCGSTAB solves it."""
+    k = np.ones(p["mesh"].n_cells)
+    k[::97] = -0.2
+    p["kappa"].set_values(k)
+
+
+@pytest.mark.parametrize("cap", [0, 40, 320, 600])
+def test_iteration_cap_is_kept(gpu, cap):
+    """Iterations of flexible CG are reported, and count against the caller's cap."""
+    probs, bs = batch(gpu, [20, 21, 9], precision=A.PREC_FP64, krylov_max_iter=cap)
+    indefinite(probs[1])
+    res = solve(bs, probs)
+    assert all(r.krylov_iterations <= cap for r in res) or cap == 0
+    again = solve(bs, probs)  # without flexible CG
+    if cap in (0, 600):
+        assert all(r.status == A.OK for r in res + again)
+    if cap == 0:
+        assert all(a.krylov_iterations < r.krylov_iterations for r, a in zip(res, again))
