@@ -936,6 +936,7 @@ struct FState {
     long long iter;
     int done;  // as KState::done: 0 running, 1 converged, 2 iteration cap, 3 breakdown, 4 b = 0, 5 non-finite
     int restart, pass, restarts, status;
+    int bad;  // the right-hand side, the guess or the matrix is not finite: no system of flexible CG
 };
 constexpr int FLEX_MIN_ROWS = 8192;
 constexpr int FLEX_MAX_ITER = 500;  // iterations (20-30 are usual) after which it has failed
@@ -1014,6 +1015,14 @@ __device__ __forceinline__ void systemSums(const FP& P, int pr, double (&t)[3]) 
         }
 }
 
+// a system that met values that are not finite leaves the cycle, whose coarsest solve couples all
+// systems (0 x NaN); the whole block, after thread 0 set done
+__device__ __forceinline__ void dropNonfinite(const FP& P, int pr) {
+    __syncthreads();
+    if (P.st[pr].done != 5) return;
+    for (int i = 32 * P.prob_slice0[pr] + threadIdx.x; i < 32 * P.prob_slice0[pr + 1]; i += BS) P.r32[i] = 0.f;
+}
+
 // (re)started systems: r = b - A x, d = q = 0
 __global__ void __launch_bounds__(BS) flex_init_kernel(const FP P) {
     const int lane = threadIdx.x & 31;
@@ -1033,13 +1042,16 @@ __global__ void __launch_bounds__(BS) flex_init_reduce_kernel(const FP P) {
     if (!S.restart) return;
     double t[3];
     systemSums(P, blockIdx.x, t);
-    if (threadIdx.x) return;
-    S.rr = t[0];
-    S.bb = t[1];
-    S.tol2 = P.tol * P.tol * t[1];
-    S.dq = 1.0;
-    S.dr = 0.0;
-    S.done = !isfinite(t[0]) || !isfinite(t[1]) ? 5 : t[1] == 0.0 ? 4 : t[0] <= S.tol2 ? 1 : 0;
+    if (threadIdx.x == 0) {
+        S.rr = t[0];
+        S.bb = t[1];
+        S.tol2 = P.tol * P.tol * t[1];
+        S.dq = 1.0;
+        S.dr = 0.0;
+        S.done = !isfinite(t[0]) || !isfinite(t[1]) ? 5 : t[1] == 0.0 ? 4 : t[0] <= S.tol2 ? 1 : 0;
+        if (S.done == 5 && S.pass == 0 && S.restarts == 0) S.bad = 1;
+    }
+    dropNonfinite(P, blockIdx.x);
 }
 // u = A z ; z.q, z.u, z.r
 __global__ void __launch_bounds__(BS) flex_spmv_kernel(const FP P) {
@@ -1093,15 +1105,17 @@ __global__ void __launch_bounds__(BS) flex_convergence_kernel(const FP P) {
     if (S.done) return;
     double t[3];
     systemSums(P, blockIdx.x, t);
-    if (threadIdx.x) return;
-    S.rr = t[0];
-    S.dq = t[1];
-    S.dr = t[2];
-    S.iter += 1;
-    if (!isfinite(t[0]) || !isfinite(t[1])) S.done = 5;
-    else if (t[0] <= S.tol2) S.done = 1;
-    else if (S.iter >= P.maxit) S.done = 2;
-    else if (!(t[1] > 0.0)) S.done = 3;
+    if (threadIdx.x == 0) {
+        S.rr = t[0];
+        S.dq = t[1];
+        S.dr = t[2];
+        S.iter += 1;
+        if (!isfinite(t[0]) || !isfinite(t[1])) S.done = 5;
+        else if (t[0] <= S.tol2) S.done = 1;
+        else if (S.iter >= P.maxit) S.done = 2;
+        else if (!(t[1] > 0.0)) S.done = 3;
+    }
+    dropNonfinite(P, blockIdx.x);
 }
 // the loop goes on while a system is running
 __global__ void flex_running_kernel(const FP P, cudaGraphConditionalHandle loop) {
@@ -1168,8 +1182,9 @@ __global__ void flex_pattern_kernel(int n, int padded, const int* rowptr, const 
 }
 
 // Solves the batch in one graph launch. FLEX_SHORT: every system came close, but a residual did
-// not reach the tolerance in FLEX_MAX_PASS passes (x is kept); FLEX_FAILED: a system failed (the
-// guesses are put back).
+// not reach the tolerance in FLEX_MAX_PASS passes; FLEX_FAILED: a system failed (its guess is put
+// back). The other systems keep their solutions, which BiCGSTAB then finds converged. A system
+// whose input is not finite is no failure.
 enum FlexEnd { FLEX_OK, FLEX_SHORT, FLEX_FAILED };
 FlexEnd runFlex(const std::vector<BatchSystem>& sys, BatchPlan& pl, double tol, long long maxit, bool own_cap,
              std::vector<BatchOut>& out, cudaStream_t s) {
@@ -1202,6 +1217,7 @@ FlexEnd runFlex(const std::vector<BatchSystem>& sys, BatchPlan& pl, double tol, 
         pl.sa = std::make_unique<SaAmg>();
         pl.cs = std::make_unique<CaptureStreams>();
     }
+    const bool fresh = !pl.sa->built;  // the structure is of this call's matrix
     SellMatrix A;
     A.n = nrows;
     A.nslices = pl.nslices;
@@ -1314,14 +1330,20 @@ FlexEnd runFlex(const std::vector<BatchSystem>& sys, BatchPlan& pl, double tol, 
     PB_CUDA(cudaStreamSynchronize(s));
     out.assign(pl.nprob, BatchOut{});
     FlexEnd end = FLEX_OK;
+    bool nonfinite = false;
     for (int i = 0; i < pl.nprob; ++i) {
         out[i].iterations = hs[i].iter;
         out[i].passes = hs[i].pass + 1;
         out[i].rel_residual = hs[i].rel;
         out[i].status = hs[i].status;
         const bool capped = own_cap && hs[i].status == PRISM_NOT_CONVERGED && hs[i].iter >= maxit;
-        if (hs[i].status == PRISM_OK || capped) continue;
+        nonfinite = nonfinite || hs[i].status == PRISM_NONFINITE;
+        if (hs[i].status == PRISM_OK || capped || hs[i].bad) continue;
         end = std::max(end, hs[i].done == 1 ? FLEX_SHORT : FLEX_FAILED);
+        if (hs[i].done == 1) continue;
+        const size_t row = (size_t)32 * pl.slice0[i];
+        PB_CUDA(cudaMemcpyAsync(pl.x64.p + row, pl.x0.p + row, sizeof(double) * 32 * (pl.slice0[i + 1] - pl.slice0[i]),
+                                cudaMemcpyDeviceToDevice, s));
     }
     if (verbose()) {
         long long most = 0;
@@ -1329,9 +1351,9 @@ FlexEnd runFlex(const std::vector<BatchSystem>& sys, BatchPlan& pl, double tol, 
         std::fprintf(stderr, "[prism] batched flexible CG of %d systems (%d rows): at most %lld iterations, %s\n", pl.nprob,
                      nrows, most, end == FLEX_OK ? "ok" : end == FLEX_SHORT ? "residuals above the tolerance" : "failed");
     }
-    if (end == FLEX_FAILED) {
-        PB_CUDA(cudaMemcpyAsync(pl.x64.p, pl.x0.p, nrows * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        scatter();
+    if (end == FLEX_FAILED) scatter();
+    if (nonfinite && fresh) {  // a structure built from such values goes
+        pl.sa->built = false;
         pl.graph.reset();
         pl.graph_key.clear();
     }
@@ -1416,11 +1438,12 @@ std::vector<BatchOut> solveBatch(const std::vector<BatchSystem>& sys, BatchPlan&
         symmetric = symmetric && q.symmetric;
     }
     std::vector<BatchOut> flex(sys.size());
+    bool failed = false;
     if (symmetric && rows >= FLEX_MIN_ROWS && entries < ((int64_t)1 << 29) && sys.size() <= 65535) {
         try {
             const FlexEnd end = runFlex(sys, pl, tol, maxit, own_cap, flex, s);
             if (end == FLEX_OK) return flex;
-            pl.no_flex = end == FLEX_FAILED;
+            failed = end == FLEX_FAILED;
         } catch (const Error& e) {
             if (!hierarchyDidNotFit(e)) throw;
             // the persistent launch needs a fraction of this memory; nothing was written back yet
@@ -1439,7 +1462,13 @@ std::vector<BatchOut> solveBatch(const std::vector<BatchSystem>& sys, BatchPlan&
     if (left <= 0) return flex;
     std::vector<BatchOut> out = mixed ? runBatch<float>(sys, pl, tol, itol, max_inner, max_pass, left, s)
                                       : runBatch<double>(sys, pl, tol, itol, max_inner, max_pass, left, s);
-    for (size_t i = 0; i < out.size(); ++i) out[i].iterations += flex[i].iterations;
+    for (size_t i = 0; i < out.size(); ++i) {
+        out[i].iterations += flex[i].iterations;
+        // values that are not finite in one system's matrix reach all of them, and say nothing
+        // about the method
+        failed = failed && out[i].status != PRISM_NONFINITE;
+    }
+    pl.no_flex = pl.no_flex || failed;
     return out;
 }
 

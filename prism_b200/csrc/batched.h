@@ -62,7 +62,7 @@ struct BatchPlan {
     DevBuf<float> fr32, fz32;
     DevBuf<unsigned char> fstate;
     std::unique_ptr<CaptureStreams> cs;
-    bool no_flex = false;  // it failed once on these patterns: BiCGSTAB from then on
+    bool no_flex = false;  // it failed once on these patterns (or found no memory): BiCGSTAB from then on
     // per call: the systems' values, right-hand sides and guesses gathered into the
     // concatenated buffers by one kernel (table of source pointers), and the whole
     // call -- gather, set-up, the persistent solve, scatter of the solutions -- kept
