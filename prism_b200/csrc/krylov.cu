@@ -1127,9 +1127,12 @@ bool fcgPre32(const Amg* amg) {
 const SolveCtl& runSmall(const SellMatrix& A, const double* b, double* x, long long n_iter, double eps, double tol,
                          long long maxit, bool symmetric, KrylovWork& w, cudaStream_t s) {
     SolveCtl* d = w.ctlRecord();
-    smallSolve(A, b, x, n_iter, eps, tol, maxit, symmetric, d, s);
-    PB_CUDA(cudaMemcpyAsync(w.host_ctl, d, sizeof(SolveCtl), cudaMemcpyDeviceToHost, s));
-    PB_CUDA(cudaStreamSynchronize(s));
+    long long step = 0;
+    do {
+        step = smallSolve(A, b, x, step, n_iter, eps, tol, maxit, symmetric, d, s);
+        PB_CUDA(cudaMemcpyAsync(w.host_ctl, d, sizeof(SolveCtl), cudaMemcpyDeviceToHost, s));
+        PB_CUDA(cudaStreamSynchronize(s));
+    } while (step < n_iter && !w.host_ctl->converged);
     if (verbose())
         std::fprintf(stderr, "[prism] one-launch solve n=%d: %lld iterations, rel residual %.3e, status %d\n", A.n,
                      w.host_ctl->krylov_iterations, w.host_ctl->krylov_rel, w.host_ctl->status);

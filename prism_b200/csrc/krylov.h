@@ -145,15 +145,17 @@ struct SolveCtl {
     // step_iterations). stand_in 2: the iteration cap is the caller's, and reaching it no failure
     int stand_in, failed;
     long long step_iterations;
+    int no_cg;  // one-launch solves: conjugate gradients broke down
 };
 
 // A whole ISolver::solve of a small system with Jacobi-preconditioned FP64 BiCGSTAB in one
 // launch (small.cu): the record lands in *out (device), x is updated in place. It fits up to
-// 32,768 rows; caps beyond 2^20 iterations or 4,096 outer steps keep to the ordinary path, whose
-// launches stay short.
+// 32,768 rows, 2^20 iterations a step and 4,096 outer steps. One launch holds as many steps as
+// keep it within 2^20 iterations (a few seconds; the host cannot stop it); from: the steps that
+// earlier launches did, whose record *out holds. Returns the first step left.
 bool smallSolveFits(const SellMatrix& A, long long maxit, long long n_iter = 1);
-void smallSolve(const SellMatrix& A, const double* b, double* x, long long n_iter, double eps, double tol,
-                long long maxit, bool symmetric, SolveCtl* out, cudaStream_t s);
+long long smallSolve(const SellMatrix& A, const double* b, double* x, long long from, long long n_iter, double eps,
+                     double tol, long long maxit, bool symmetric, SolveCtl* out, cudaStream_t s);
 
 // the same, waited for: the record on the host (valid until the workspace's next solve)
 const SolveCtl& runSmall(const SellMatrix& A, const double* b, double* x, long long n_iter, double eps, double tol,

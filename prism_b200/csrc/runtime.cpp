@@ -1354,7 +1354,9 @@ PrismSolveResult solveCaptured(Transport& eq, const PrismSolveOpts& o) {
     if (stand_in)
         PB_CUDA(cudaMemcpyAsync(m.kw.xs.p, phi.v.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, s));
     if (o.method == PRISM_SOLVER_BICGSTAB && !amg && smallSolveFits(A, kmax, o.n_iter)) {
-        smallSolve(A, eq.b.p, phi.v.p, n_iter, o.eps, ktol, kmax, symmetricMatrix(eq), ctl, s);
+        long long step = 0;
+        do step = smallSolve(A, eq.b.p, phi.v.p, step, n_iter, o.eps, ktol, kmax, symmetricMatrix(eq), ctl, s);
+        while (step < n_iter);
         if (n_iter > 0) phi.event += 4;
         if (o.clear_coeffs) zeroOutCoeffs(eq);
         PrismSolveResult r{};

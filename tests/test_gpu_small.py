@@ -80,3 +80,35 @@ def test_zero_right_hand_side(gpu):
     rowptr, col, val, row = system(n, 3, 3, False)
     x = api.BiCGSTAB(preconditioner="jacobi").step(gpu, rowptr, col, val, np.ones(n), np.zeros(n))
     assert np.all(x == 0.0)
+
+
+@pytest.mark.parametrize("shape", [(10, 10, 10), (15, 14, 13)])
+@pytest.mark.parametrize("symmetric", [False, True])
+def test_outer_steps_are_spread_over_launches(gpu, shape, symmetric):
+    """One launch holds 2^20 iterations at most: with the largest cap a step each, with a third of
+    it three, with a small one all; fields and records are the same, as a graph too."""
+    import ctypes
+    from prism_b200 import meshgen
+    from tests.test_gpu_smoothed import diffusion
+    runs = {}
+    for cap in (0, (1 << 20) // 3, 1 << 20):
+        for graph in (False, True):
+            if symmetric:
+                mesh, T, eqn, keep = diffusion(meshgen.box_hex(*shape), gpu)
+            else:
+                mesh, T, U, eqn = cases.transport_c3(shape[0], gpu, conv="Upwind")
+            solver = api.BiCGSTAB(krylov_max_iter=cap, preconditioner="jacobi", graph=graph)
+            solver.solve(eqn, 1, 0.0)
+            T.set_values(np.zeros(mesh.n_cells))
+            prof = A.Profile()
+            gpu.check(gpu.profile_start(0))
+            r = solver.solve(eqn, 7, 0.0)
+            gpu.check(gpu.profile_stop(ctypes.byref(prof)))
+            runs[cap, graph] = (T.values(), (r.status, r.iteration, r.krylov_iterations, r.initial_residual,
+                                             r.final_residual, r.krylov_rel_residual), prof.kernel_launches)
+    first = runs[0, False]
+    assert first[1][:2] == (A.OK, 7)
+    for x, record, launches in runs.values():
+        assert np.array_equal(x, first[0]) and record == first[1]
+    for graph in (False, True):
+        assert [runs[cap, graph][2] - runs[0, graph][2] for cap in ((1 << 20) // 3, 1 << 20)] == [2, 6]
