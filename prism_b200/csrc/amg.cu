@@ -41,6 +41,7 @@
 #include <type_traits>
 
 #include "amg.h"
+#include "cluster.cuh"
 #include "reduce.cuh"
 
 namespace pb {
@@ -933,26 +934,8 @@ int tailMaxRows() {
 // such a cluster, else the portable 8
 template <typename T>
 int tailCluster() {
-    static const int c = [] {
-        int cl = 8;
-        if (cudaFuncSetAttribute(tail_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
-            cudaLaunchConfig_t cfg{};
-            cfg.gridDim = dim3(16);
-            cfg.blockDim = dim3(TAIL_BS);
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = 16;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, tail_kernel<T>, &cfg) == cudaSuccess && n >= 1) cl = 16;
-        }
-        cudaGetLastError();  // a refused query leaves no sticky error
-        return cl;
-    }();
-    return c;
+    static PerDevice c;
+    return c.get([] { return clusterPlaced(tail_kernel<T>, TAIL_BS) ? CLUSTER_MAX : 8; });
 }
 
 template <typename T>

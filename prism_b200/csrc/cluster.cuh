@@ -83,7 +83,8 @@ struct ClusterReduce {
     }
 };
 
-// Whether the device places a cluster of CLUSTER_MAX blocks of `kernel`
+// Whether the current device places a cluster of CLUSTER_MAX blocks of `kernel` (and allows it to,
+// on this device only)
 template <typename K>
 bool clusterPlaced(K kernel, int threads) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {

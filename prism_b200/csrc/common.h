@@ -36,6 +36,25 @@ inline void cudaCheck(cudaError_t e, const char* what) {
 #define PB_CUDA(call) ::pb::cudaCheck((call), #call)
 #define PB_LAUNCH(what) ::pb::cudaCheck(cudaGetLastError(), what)
 
+// A number that belongs to a device (a launch limit, with the function attribute that it needs),
+// found by f() > 0 on the first use there: a process may run on several.
+class PerDevice {
+public:
+    template <typename F>
+    int get(F f) {
+        int d = 0;
+        PB_CUDA(cudaGetDevice(&d));
+        if (d < 0 || d >= MAX) return f();
+        int v = v_[d].load(std::memory_order_acquire);
+        if (!v) v_[d].store(v = f(), std::memory_order_release);
+        return v;
+    }
+
+private:
+    static constexpr int MAX = 64;
+    std::atomic<int> v_[MAX] = {};
+};
+
 // Owning device allocation (cudaMalloc / cudaFree).
 template <typename T>
 struct DevBuf {

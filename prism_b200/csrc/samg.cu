@@ -892,8 +892,8 @@ __global__ void __launch_bounds__(TAIL_BS) tail_kernel(const __grid_constant__ T
 
 // CTAs of the tail's cluster: 16 where the device can place it, else 8
 int tailCluster() {
-    static const int c = clusterPlaced(tail_kernel, TAIL_BS) ? CLUSTER_MAX : 8;
-    return c;
+    static PerDevice c;
+    return c.get([] { return clusterPlaced(tail_kernel, TAIL_BS) ? CLUSTER_MAX : 8; });
 }
 
 // ---------------------------------------------------------------- host side of the structure

@@ -338,13 +338,15 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
 
 // blocks of the largest cluster the device places (8 is always allowed)
 int maxCtas() {
-    static const int c = clusterPlaced(small_solve_kernel<256, 1, 7, true>, 256) &&
-                                 clusterPlaced(small_solve_kernel<512, 2, 5, true>, 512) &&
-                                 clusterPlaced(small_solve_kernel<512, 2, 7, true>, 512) &&
-                                 clusterPlaced(small_solve_kernel<512, 4, 0, true>, 512)
-                             ? CLUSTER_MAX
-                             : 8;
-    return c;
+    static PerDevice c;
+    return c.get([] {
+        return clusterPlaced(small_solve_kernel<256, 1, 7, true>, 256) &&
+                       clusterPlaced(small_solve_kernel<512, 2, 5, true>, 512) &&
+                       clusterPlaced(small_solve_kernel<512, 2, 7, true>, 512) &&
+                       clusterPlaced(small_solve_kernel<512, 4, 0, true>, 512)
+                   ? CLUSTER_MAX
+                   : 8;
+    });
 }
 
 template <int T, int K, int KEPT>
