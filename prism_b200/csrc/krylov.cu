@@ -1095,7 +1095,7 @@ namespace {
 int solveMode(int kind, const Amg* amg, const SellMatrix& A) {
     if (kind == SOLVE_PLAIN || (kind == SOLVE_SMOOTHED && amg->no_sa)) return KM_BICGSTAB;
     if (kind == SOLVE_SMOOTHED) return KM_BICGSTAB_SA;
-    return fcgSmoothed(amg, A) ? KM_FCG_SA : fcgPre32(amg) ? KM_FCG_PRE32 : KM_FCG;
+    return kind == SOLVE_FLEXIBLE && fcgSmoothed(amg, A) ? KM_FCG_SA : fcgPre32(amg) ? KM_FCG_PRE32 : KM_FCG;
 }
 // values of the cycle's hierarchy from the current matrix (built on first use)
 void setupCycle(Amg* amg, int mode, const SellMatrix& A, const int* rowptr, const int* col, bool pre32,
@@ -1151,7 +1151,7 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
         return out;
     }
     const bool mixed = precision == PRISM_PREC_MIXED;
-    const bool flexible = kind == SOLVE_FLEXIBLE;
+    const bool flexible = kind == SOLVE_FLEXIBLE || kind == SOLVE_FLEXIBLE_OWN;
     if (flexible && (mixed || !amg)) fail(PRISM_INTERNAL, "flexible CG runs FP64 with AMG only");
     if (kind == SOLVE_SMOOTHED && !amg) fail(PRISM_INTERNAL, "smoothed aggregation without its hierarchy");
     int mode = solveMode(kind, amg, A);
@@ -1334,6 +1334,29 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
                      "%d stalled segments restarted, rel residual %.3e, status %d\n", n, out.iterations, n_reliable,
                      restarts, stalls, out.rel_residual, out.status);
     return out;
+}
+
+KrylovOut standInSolve(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, long long cap,
+                       double inner_tol, KrylovWork& w, cudaStream_t s, Amg* amg, const int* rowptr, const int* col,
+                       int kind, int precision, const Instead& instead, int* instead_status) {
+    *instead_status = -1;
+    w.ensure(A.nslices * 32, A.nnz_padded, false);
+    PB_CUDA(cudaMemcpyAsync(w.xs.p, x, A.n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    KrylovOut k = bicgstab(A, b, x, tol, std::min(maxit, STAND_IN_MAX), kind == SOLVE_FLEXIBLE ? PRISM_PREC_FP64 : precision,
+                           inner_tol, w, s, amg, rowptr, col, kind);
+    const long long left = cap > 0 ? maxit - k.iterations : maxit;
+    if (k.status == PRISM_OK || (k.status == PRISM_NOT_CONVERGED && left <= 0)) return k;
+    PB_CUDA(cudaMemcpyAsync(x, w.xs.p, A.n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    if (left <= 0) {
+        k.has_scaled = false;  // x is the guess again
+        return k;
+    }
+    amg->values_current = false;
+    KrylovOut f = bicgstab(A, b, x, tol, left, instead.precision, inner_tol, w, s, instead.amg, rowptr, col, instead.kind,
+                           instead.symmetric);
+    *instead_status = f.status;
+    f.iterations += k.iterations;
+    return f;
 }
 
 int profBegin(int kind, bool fp32, double bytes, cudaStream_t s) {
@@ -1637,7 +1660,7 @@ void emitOuterStep(SolveCtl* ctl, KrylovWork& w, cudaGraphConditionalHandle oute
 void emitBicgstab(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, KrylovWork& w,
                   cudaStream_t s, Amg* amg, const int* rowptr, const int* col, SolveCtl* ctl, CaptureStreams& cs,
                   int depth, int kind) {
-    const bool flexible = kind == SOLVE_FLEXIBLE;
+    const bool flexible = kind == SOLVE_FLEXIBLE || kind == SOLVE_FLEXIBLE_OWN;
     if (kind != SOLVE_PLAIN && !amg) fail(PRISM_INTERNAL, "a multigrid solve without its hierarchy");
     const int mode = solveMode(kind, amg, A);
     w.ensure(A.nslices * 32, A.nnz_padded, false);

@@ -88,7 +88,7 @@ struct KrylovOut {
     bool has_scaled = false;
 };
 
-enum { SOLVE_PLAIN = 0, SOLVE_FLEXIBLE = 1, SOLVE_SMOOTHED = 2 };
+enum { SOLVE_PLAIN = 0, SOLVE_FLEXIBLE = 1, SOLVE_SMOOTHED = 2, SOLVE_FLEXIBLE_OWN = 3 };
 // x <- BiCGSTAB solve of A x = b from the guess x, stopping at ||b - A x|| <= tol ||b||.
 // precision: PRISM_PREC_FP64 or PRISM_PREC_MIXED. Right preconditioning: Jacobi
 // (column scaling) when amg is null, else one V-cycle of amg, whose hierarchy is
@@ -98,11 +98,26 @@ enum { SOLVE_PLAIN = 0, SOLVE_FLEXIBLE = 1, SOLVE_SMOOTHED = 2 };
 // the FP32 cycle of smoothed aggregation), or SOLVE_FLEXIBLE: FP64 only -- flexible conjugate gradients (Notay 2000, one
 // previous direction kept) preconditioned by amg->applyK(), for symmetric
 // positive (semi-)definite A (the pressure-correction equation), in place of
-// BiCGSTAB; same stopping rule, passes and statuses. symmetric: A is symmetric by construction
+// BiCGSTAB; same stopping rule, passes and statuses. SOLVE_FLEXIBLE_OWN: the same with amg's own
+// cycle, where SOLVE_FLEXIBLE takes smoothed aggregation's (fcgSmoothed). symmetric: A is symmetric by construction
 // (the one-launch solve of a small system may then run conjugate gradients).
 KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, int precision,
                    double inner_tol, KrylovWork& w, cudaStream_t s, Amg* amg = nullptr, const int* rowptr = nullptr,
                    const int* col = nullptr, int kind = SOLVE_PLAIN, bool symmetric = false);
+// The solve `kind` with smoothed aggregation; should it fail (within STAND_IN_MAX iterations), the
+// one that `instead` names, from the same guess and with what is left of cap, the caller's
+// limit (0: none). The guess waits in w.xs, which multigrid solves do not use.
+// *instead_status: how the latter ended (-1: it did not run).
+constexpr long long STAND_IN_MAX = 500;  // iterations (20-60 are usual) after which it has failed
+struct Instead {
+    int kind;
+    Amg* amg;
+    int precision;
+    bool symmetric;
+};
+KrylovOut standInSolve(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, long long cap,
+                       double inner_tol, KrylovWork& w, cudaStream_t s, Amg* amg, const int* rowptr, const int* col,
+                       int kind, int precision, const Instead& instead, int* instead_status);
 // flexible CG with amg preconditions with an FP32 V-cycle (else with the FP64 cycle)
 bool fcgPre32(const Amg* amg);
 // that V-cycle is smoothed aggregation's (samg.h)

@@ -558,30 +558,31 @@ struct InStep {
 
 // How an AMG solve of eq runs. The spd pressure correction: flexible CG (FP64 recurrences).
 // A user's equation: flexible CG where its matrix is symmetric, else BiCGSTAB with the cycle of
-// smoothed aggregation, which takes a third of the iterations of amg's own hierarchy; both go
-// back to the latter should they fail (standInSolve). Inside a step the momentum predictors
-// keep amg's cycle: nothing could step in for a solve that failed in a captured step.
+// smoothed aggregation, which takes a third of the iterations of amg's own hierarchy. All of
+// these go back to the latter should they fail (standInSolve). Inside a step the momentum
+// predictors keep amg's cycle: nothing could step in for a solve that failed in a captured step.
 // PRISM_PRESSURE_SOLVER=bicgstab keeps BiCGSTAB with amg's cycle everywhere.
 static int kindFor(const Transport& eq, const PrismSolveOpts& o, const Amg* amg, const SellMatrix& A) {
     static const bool on = [] {
         const char* e = std::getenv("PRISM_PRESSURE_SOLVER");
         return !(e && std::strcmp(e, "bicgstab") == 0);
     }();
-    if (o.method == PRISM_SOLVER_FCG) return SOLVE_FLEXIBLE;
+    const int flexible = eq.no_stand_in ? SOLVE_FLEXIBLE_OWN : SOLVE_FLEXIBLE;
+    if (o.method == PRISM_SOLVER_FCG) return flexible;
     if (!on || !amg || o.method != PRISM_SOLVER_BICGSTAB) return SOLVE_PLAIN;
-    if (eq.spd) return o.precision == PRISM_PREC_FP64 ? SOLVE_FLEXIBLE : SOLVE_PLAIN;
+    if (eq.spd) return o.precision == PRISM_PREC_FP64 ? flexible : SOLVE_PLAIN;
     if (eq.no_stand_in || g_in_step || !smoothedFits(amg, A)) return SOLVE_PLAIN;
     return symmetricMatrix(eq) ? SOLVE_FLEXIBLE : SOLVE_SMOOTHED;
 }
-// that kind stands in for the BiCGSTAB with amg's cycle that was asked for
-static bool standsIn(const Transport& eq, const PrismSolveOpts& o, int kind) {
-    return kind != SOLVE_PLAIN && o.method != PRISM_SOLVER_FCG && !eq.spd;
+// that kind is asked for by nobody (BiCGSTAB with amg's cycle was) or runs with smoothed
+// aggregation where flexible CG with amg's own cycle would do
+static bool standsIn(const Transport& eq, const PrismSolveOpts& o, int kind, const Amg* amg, const SellMatrix& A) {
+    if (kind == SOLVE_PLAIN || kind == SOLVE_FLEXIBLE_OWN) return false;
+    return (o.method != PRISM_SOLVER_FCG && !eq.spd) || fcgSmoothed(amg, A);
 }
-constexpr long long STAND_IN_MAX = 500;  // iterations (20-60 are usual) after which it has failed
-// a stand-in's end that has to be mended: anything but success or the caller's own iteration
-// cap, which its iterations count against (used: since the step began)
-static bool standInFailed(const PrismSolveOpts& o, int status, long long used) {
-    return status != PRISM_OK && !(status == PRISM_NOT_CONVERGED && o.krylov_max_iter > 0 && used >= o.krylov_max_iter);
+// what it stands in for
+static int standsInFor(const Transport& eq, const PrismSolveOpts& o) {
+    return o.method == PRISM_SOLVER_FCG || eq.spd ? SOLVE_FLEXIBLE_OWN : SOLVE_PLAIN;
 }
 
 // PRISM_SOLVER_FCG's requirements: FP64, and the AMG preconditioner (its own choice
@@ -617,35 +618,28 @@ static void standInGaveUp(Transport& eq, Amg* amg, int status) {
     else if (amg->sa && amg->sa->fresh) amg->sa->built = false;
 }
 
-// One step by a stand-in (kindFor); should it fail, the solve it stands in for from the same
-// guess, with what is left of a cap that the caller set. The guess waits in xs, which AMG solves
-// do not use.
-static KrylovOut standInSolve(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, int kind,
-                              const PrismSolveOpts& o, Mesh& m, Amg* amg, Transport& eq) {
-    KrylovWork& w = m.kw;
-    w.ensure(A.nslices * 32, A.nnz_padded, false);
-    const double itol = o.inner_tol > 0 ? o.inner_tol : 0.1;
-    PB_CUDA(cudaMemcpyAsync(w.xs.p, x, A.n * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
-    KrylovOut k = bicgstab(A, b, x, tol, std::min(maxit, STAND_IN_MAX), kind == SOLVE_FLEXIBLE ? PRISM_PREC_FP64 : o.precision,
-                           itol, w, m.stream, amg, m.pat.rowptr.p, m.pat.col.p, kind);
-    if (!standInFailed(o, k.status, k.iterations)) return k;
-    PB_CUDA(cudaMemcpyAsync(x, w.xs.p, A.n * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
-    const long long left = o.krylov_max_iter > 0 ? maxit - k.iterations : maxit;
-    if (left <= 0) {
-        k.has_scaled = false;  // x is the guess again
-        return k;
-    }
-    amg->values_current = false;
-    KrylovOut f = bicgstab(A, b, x, tol, left, o.precision, itol, w, m.stream, jacobiInstead(o, A) ? nullptr : amg,
-                           m.pat.rowptr.p, m.pat.col.p);
-    standInGaveUp(eq, amg, f.status);
-    f.iterations += k.iterations;
-    return f;
+// One step by a stand-in (kindFor), and what eq learns from it
+static KrylovOut standInStep(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, int kind,
+                             const PrismSolveOpts& o, Mesh& m, Amg* amg, Transport& eq) {
+    const bool jacobi = jacobiInstead(o, A);
+    const Instead instead{jacobi ? SOLVE_PLAIN : standsInFor(eq, o), jacobi ? nullptr : amg, o.precision, symmetricMatrix(eq)};
+    int ended = -1;
+    KrylovOut k = standInSolve(A, b, x, tol, maxit, o.krylov_max_iter, o.inner_tol > 0 ? o.inner_tol : 0.1, m.kw, m.stream,
+                               amg, m.pat.rowptr.p, m.pat.col.p, kind, o.precision, instead, &ended);
+    if (ended >= 0) standInGaveUp(eq, amg, ended);
+    return k;
 }
 
 namespace {
 // set while a solve or step is being captured into a graph (graph_capture below)
 struct GraphCapture {
+    // captured steps: pressure solves with smoothed aggregation, and whether their cap is the caller's
+    struct Pressure {
+        int slot;
+        Transport* eq;
+        bool own_cap;
+    };
+    std::vector<Pressure> pressure;
     Mesh* m = nullptr;
     int used = 0;
 };
@@ -701,12 +695,12 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o, b
             jacobiStep(A, eq.b.p, phi.v.p, m.kw, m.stream);
         } else {
             const HoldAmgValues hold(amg, eq.matrix_unchanged || iter > 0);  // A is fixed within one solve
-            if ((eq.no_stand_in || (plain && !eq.spd)) && jacobiInstead(o, A)) amg = nullptr;  // since an earlier step
+            if ((eq.no_stand_in || plain) && jacobiInstead(o, A)) amg = nullptr;  // since an earlier step
             int kind = kindFor(eq, o, amg, A);
-            if (plain && standsIn(eq, o, kind)) kind = SOLVE_PLAIN;
+            if (plain && standsIn(eq, o, kind, amg, A)) kind = standsInFor(eq, o);
             const long long cap = iter == 0 && o.krylov_max_iter > 0 ? kmax - spent : kmax;
-            KrylovOut k = standsIn(eq, o, kind)
-                              ? standInSolve(A, eq.b.p, phi.v.p, ktol, cap, kind, o, m, amg, eq)
+            KrylovOut k = standsIn(eq, o, kind, amg, A)
+                              ? standInStep(A, eq.b.p, phi.v.p, ktol, cap, kind, o, m, amg, eq)
                               : bicgstab(A, eq.b.p, phi.v.p, ktol, cap, o.precision, itol, m.kw, m.stream, amg,
                                          m.pat.rowptr.p, m.pat.col.p, kind, symmetricMatrix(eq));
             r.krylov_iterations += k.iterations + (iter == 0 ? spent : 0);
@@ -1131,6 +1125,7 @@ FixedPointOut adjointBackward(Transport& eq, const double* dJ, double* gk, doubl
     const double ktol = o.krylov_tol > 0 ? o.krylov_tol : 1e-12;
     const long long kmax = o.krylov_max_iter > 0 ? o.krylov_max_iter : 2LL * m.nc;
     PrismSolveOpts fp64 = o;
+    fp64.method = PRISM_SOLVER_BICGSTAB;
     fp64.precision = PRISM_PREC_FP64;
     fp64.inner_tol = 0.0;
     double h[2];
@@ -1141,7 +1136,7 @@ FixedPointOut adjointBackward(Transport& eq, const double* dJ, double* gk, doubl
         if (amg && eq.no_stand_in && o.preconditioner == PRISM_PC_AUTO && smallSolveFits(AT, 1)) amg = nullptr;
         const HoldAmgValues hold(amg, it > 0);
         KrylovOut k = amg && !eq.no_stand_in && smoothedFits(amg, AT)
-                          ? standInSolve(AT, rhs.p, lam.p, ktol, kmax, SOLVE_FLEXIBLE, fp64, m, amg, eq)
+                          ? standInStep(AT, rhs.p, lam.p, ktol, kmax, SOLVE_FLEXIBLE, fp64, m, amg, eq)
                           : bicgstab(AT, rhs.p, lam.p, ktol, kmax, PRISM_PREC_FP64, 0.1, m.kw, s, amg, m.pat.rowptr.p,
                                      m.pat.col.p, SOLVE_PLAIN, true);
         out.krylov += k.iterations;
@@ -1350,7 +1345,8 @@ PrismSolveResult solveCaptured(Transport& eq, const PrismSolveOpts& o) {
     const long long n_iter = std::max<long long>(o.n_iter, 0);
     // a stand-in's guess is kept in case it fails (solveAsGraph, which then needs the system too)
     const int kind = kindFor(eq, o, amg, A);
-    const bool stand_in = standsIn(eq, o, kind);
+    const bool stand_in = !g_in_step && standsIn(eq, o, kind, amg, A);
+    if (!stand_in && standsIn(eq, o, kind, amg, A)) g_capture->pressure.push_back({slot, &eq, o.krylov_max_iter > 0});
     if (stand_in)
         PB_CUDA(cudaMemcpyAsync(m.kw.xs.p, phi.v.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, s));
     if (o.method == PRISM_SOLVER_BICGSTAB && !amg && smallSolveFits(A, kmax, o.n_iter)) {
@@ -1435,6 +1431,11 @@ int runAsGraph(Mesh& m, const std::function<void()>& f) {
         PB_CUDA(cudaMemcpyAsync(m.graph_host, m.graph_ctl.p, ctx.used * sizeof(SolveCtl), cudaMemcpyDeviceToHost,
                                 m.stream));
     PB_CUDA(cudaStreamSynchronize(m.stream));
+    // nothing steps in for a solve inside a captured step; the steps after it go without
+    for (const auto& q : ctx.pressure) {
+        const int status = m.graph_host[q.slot].status;
+        if (status == PRISM_BREAKDOWN || (status == PRISM_NOT_CONVERGED && !q.own_cap)) q.eq->no_stand_in = true;
+    }
     return ctx.used;
 }
 
@@ -1465,7 +1466,7 @@ bool graphReady(const Transport& eq, const PrismSolveOpts& o) {
         for (auto& L : eq.amg->levels)
             if (!L->b || !L->dinv) return false;
         if (eq.amg->k_levels > 0 && !eq.amg->kscal) return false;
-        if (kind == SOLVE_FLEXIBLE && fcgPre32(eq.amg.get())) {
+        if (kind != SOLVE_PLAIN && fcgPre32(eq.amg.get())) {
             if (!m.kw.y32 || (!eq.amg->coarse_inv32 && eq.amg->coarse_inv)) return false;
             for (auto& L : eq.amg->levels)
                 if (!L->b32 || !L->vals32) return false;
@@ -1495,7 +1496,7 @@ PrismSolveResult solveAsGraph(Transport& eq, const PrismSolveOpts& o) {
     out = fromCtl(m.graph_host[0]);
     const SellMatrix A = m.matrix(eq.A.p);
     Amg* amg = hierarchyFor(eq, o, A);
-    if (standsIn(eq, o, kindFor(eq, o, amg, A))) {
+    if (standsIn(eq, o, kindFor(eq, o, amg, A), amg, A)) {
         const SolveCtl& c = m.graph_host[0];
         if (c.failed) {
             const long long spent = c.step_iterations;

@@ -142,3 +142,50 @@ def test_nan_in_one_call_does_not_change_the_next(gpu, shape, where, first, grap
             assert r.status == (A.NONFINITE if call == (0 if first else 2) else A.OK)
         out.append((T.values(), r.krylov_iterations))
     assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
+
+
+def band(n, k, c):
+    """Unit diagonal and k neighbours of weight c on either side: positive definite for the k and c
+    used here (symbol >= 0.05), but D^-1 A reaches 1 + 2 k c, beyond what damped Jacobi smooths."""
+    i = np.repeat(np.arange(n), 2 * k + 1)
+    j = i + np.tile(np.arange(-k, k + 1), n)
+    keep = (j >= 0) & (j < n)
+    i, j = i[keep], j[keep]
+    rowptr = np.zeros(n + 1, np.int64)
+    np.add.at(rowptr, i + 1, 1)
+    return np.cumsum(rowptr), j.astype(np.int64), np.where(i == j, 1.0, c), i
+
+
+def solve_csr(lib, solver, rowptr, col, val, b):
+    o, r, x = solver.opts(lib), A.SolveResult(), np.zeros(len(b))
+    lib.check(lib.solve_csr(len(b), rowptr.ctypes.data_as(A.pi64), col.ctypes.data_as(A.pi64), api._f64p(val),
+                            api._f64p(b), api._f64p(x), ctypes.byref(o), ctypes.byref(r)))
+    return x, r
+
+
+# condition numbers below 80: ||x - x*|| <= 80 ||r|| / ||A|| with ||r|| <= 1e-11 ||b|| (ten times the
+# tolerance is accepted) is below 1e-8 ||x*||
+@pytest.mark.parametrize("n, k, c", [(3000, 3, 0.2), (40000, 3, 0.3), (40000, 5, 0.2), (40000, 12, 0.1), (40000, 8, 0.2)])
+def test_flexible_cg_beyond_dominance(gpu, n, k, c):
+    rowptr, col, val, row = band(n, k, c)
+    x = np.random.default_rng(0).normal(size=n)
+    b = np.zeros(n)
+    np.add.at(b, row, val * x[col])
+    y, r = solve_csr(gpu, api.FCG(krylov_tol=1e-12), rowptr, col, val, b)
+    assert r.status == A.OK and cases.rel_l2(y, x) < 1e-8
+    assert r.krylov_iterations < 700 or c == 0.2 and k == 8
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_flexible_cg_goes_back_to_amgs_own_cycle(gpu, graph):
+    """A first matrix without couplings leaves smoothed aggregation nothing to coarsen; the next
+    one's solve fails with it, and goes on with the plain cycle from the same guess."""
+    mesh, T, eqn, (k, f) = heat(gpu, (700, 500, 1), 0.0, 1e-6)
+    solver = api.FCG(graph=graph)
+    assert solve(solver, eqn, T).status == A.OK
+    k.set_values(np.random.default_rng(2).lognormal(0.0, 1.0, mesh.n_cells))
+    eqn.set_time_step(1e6)
+    for call in range(2):
+        r = solve(solver, eqn, T)
+        assert r.status == A.OK and r.krylov_rel_residual <= 1e-11
+        assert r.krylov_iterations < (900 if call == 0 else 400)
