@@ -91,9 +91,11 @@ struct Amg {
     // extra coarse-level launches cost more than that saved)
     void forPressure();
     bool kLevel(size_t l) const;
-    // the smoothed-aggregation hierarchy of flexible CG (fcgMode picks it); this struct's own
+    // the smoothed-aggregation hierarchy (solveMode in krylov.cu picks it); this struct's own
     // levels then stay unbuilt
     std::unique_ptr<SaAmg> sa;
+    // its symmetric form is for weakly diagonally dominant matrices (lookAtDominance)
+    bool not_dominant = false;
     bool no_sa = false;  // that hierarchy did not fit (memory, 32-bit indices): this struct's own from then on
 
     // Build the hierarchy (first call) or refresh its values (later calls) for

@@ -855,13 +855,14 @@ API int prism_solve_csr(int64_t n, const int64_t* rowptr, const int64_t* col, co
             const double tol = o->krylov_tol > 0 ? o->krylov_tol : 1e-12, itol = o->inner_tol > 0 ? o->inner_tol : 0.1;
             const long long maxit = o->krylov_max_iter > 0 ? o->krylov_max_iter : 2 * n;
             int instead = -1;
-            if (fcg)
+            if (fcg) lookAtDominance(&amg, A, kw, s);
+            if (fcg && fcgSmoothed(&amg, A))
                 k = standInSolve(A, d_b.p, d_x.p, tol, maxit, o->krylov_max_iter, itol, kw, s, &amg, d_rp.p, d_col.p,
                                  SOLVE_FLEXIBLE, PRISM_PREC_FP64,
                                  Instead{SOLVE_FLEXIBLE_OWN, &amg, PRISM_PREC_FP64, false}, &instead);
             else
                 k = bicgstab(A, d_b.p, d_x.p, tol, maxit, o->precision, itol, kw, s, use_amg ? &amg : nullptr, d_rp.p,
-                             d_col.p);
+                             d_col.p, fcg ? SOLVE_FLEXIBLE_OWN : SOLVE_PLAIN);
         }
         double res = scaledResidual(A, d_b.p, d_x.p, kw, s);
         d_x.download(x, n, s);

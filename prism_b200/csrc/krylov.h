@@ -122,6 +122,10 @@ KrylovOut standInSolve(const SellMatrix& A, const double* b, double* x, double t
 bool fcgPre32(const Amg* amg);
 // that V-cycle is smoothed aggregation's (samg.h)
 bool fcgSmoothed(const Amg* amg, const SellMatrix& A);
+// Looks whether symmetric A is weakly diagonally dominant, for the smoothed aggregation of
+// flexible CG (Amg::not_dominant): before its hierarchy is built and, where the answer was no,
+// before every solve (a host wait each, so never inside a capture).
+void lookAtDominance(Amg* amg, const SellMatrix& A, KrylovWork& w, cudaStream_t s);
 // smoothed aggregation takes matrices of this size
 bool smoothedFits(const Amg* amg, const SellMatrix& A);
 // e says that the structure of a hierarchy found no memory, or no room in its 32-bit indices

@@ -572,7 +572,12 @@ static int kindFor(const Transport& eq, const PrismSolveOpts& o, const Amg* amg,
     if (!on || !amg || o.method != PRISM_SOLVER_BICGSTAB) return SOLVE_PLAIN;
     if (eq.spd) return o.precision == PRISM_PREC_FP64 ? flexible : SOLVE_PLAIN;
     if (eq.no_stand_in || g_in_step || !smoothedFits(amg, A)) return SOLVE_PLAIN;
-    return symmetricMatrix(eq) ? SOLVE_FLEXIBLE : SOLVE_SMOOTHED;
+    if (symmetricMatrix(eq)) return amg->not_dominant ? SOLVE_PLAIN : SOLVE_FLEXIBLE;
+    return SOLVE_SMOOTHED;
+}
+// flexible CG is what an AMG solve of eq would be
+static bool flexibleFor(const Transport& eq, const PrismSolveOpts& o) {
+    return o.method == PRISM_SOLVER_FCG || eq.spd || symmetricMatrix(eq);
 }
 // that kind is asked for by nobody (BiCGSTAB with amg's cycle was) or runs with smoothed
 // aggregation where flexible CG with amg's own cycle would do
@@ -611,11 +616,20 @@ static Amg* hierarchyFor(Transport& eq, const PrismSolveOpts& o, const SellMatri
 }
 
 // A stand-in failed on eq, and the solve in its place ended with `status`: that one from now on,
-// unless both met values that are not finite. Those say nothing about the method; a structure
-// that was built from them goes.
-static void standInGaveUp(Transport& eq, Amg* amg, int status) {
-    if (status != PRISM_NONFINITE) eq.no_stand_in = true;
-    else if (amg->sa && amg->sa->fresh) amg->sa->built = false;
+// unless the matrix or a vector was none for it. Values that are not finite say nothing about
+// the method (a structure that was built from them goes), and a symmetric matrix that is no
+// longer dominant goes without for as long as it is not.
+static void standInGaveUp(Transport& eq, Amg* amg, int status, int kind, const SellMatrix& A, Mesh& m) {
+    if (status == PRISM_NONFINITE) {
+        if (amg->sa && amg->sa->fresh) amg->sa->built = false;
+        return;
+    }
+    if (kind == SOLVE_FLEXIBLE && fcgSmoothed(amg, A)) {
+        amg->not_dominant = true;
+        lookAtDominance(amg, A, m.kw, m.stream);
+        if (amg->not_dominant) return;
+    }
+    eq.no_stand_in = true;
 }
 
 // One step by a stand-in (kindFor), and what eq learns from it
@@ -626,7 +640,7 @@ static KrylovOut standInStep(const SellMatrix& A, const double* b, double* x, do
     int ended = -1;
     KrylovOut k = standInSolve(A, b, x, tol, maxit, o.krylov_max_iter, o.inner_tol > 0 ? o.inner_tol : 0.1, m.kw, m.stream,
                                amg, m.pat.rowptr.p, m.pat.col.p, kind, o.precision, instead, &ended);
-    if (ended >= 0) standInGaveUp(eq, amg, ended);
+    if (ended >= 0) standInGaveUp(eq, amg, ended, kind, A, m);
     return k;
 }
 
@@ -670,7 +684,9 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o, b
     const long long kmax = o.krylov_max_iter > 0 ? o.krylov_max_iter : 2LL * m.nc;
     const double itol = o.inner_tol > 0 ? o.inner_tol : 0.1;
     Amg* amg = hierarchyFor(eq, o, A);
-    if (plain && jacobiInstead(o, A)) amg = nullptr;
+    if (amg && flexibleFor(eq, o) && (amg->not_dominant || kindFor(eq, o, amg, A) == SOLVE_FLEXIBLE))
+        lookAtDominance(amg, A, m.kw, m.stream);
+    if (amg && (plain || (flexibleFor(eq, o) && amg->not_dominant)) && jacobiInstead(o, A)) amg = nullptr;
     if (o.method == PRISM_SOLVER_BICGSTAB && !amg && spent == 0 && smallSolveFits(A, kmax, o.n_iter)) {
         const SolveCtl& c = runSmall(A, eq.b.p, phi.v.p, std::max<int64_t>(o.n_iter, 0), o.eps, ktol, kmax,
                                      symmetricMatrix(eq), m.kw, m.stream);
@@ -1121,6 +1137,8 @@ FixedPointOut adjointBackward(Transport& eq, const double* dJ, double* gk, doubl
     if (choosePreconditioner(o.preconditioner, m.nc, true) == PRISM_PC_AMG) {  // diffusion only: A^T = A
         if (!eq.amg_adj) eq.amg_adj = std::make_shared<Amg>();
         amg = eq.amg_adj.get();
+        lookAtDominance(amg, AT, m.kw, s);
+        if (amg->not_dominant && o.preconditioner == PRISM_PC_AUTO && smallSolveFits(AT, 1)) amg = nullptr;
     }
     const double ktol = o.krylov_tol > 0 ? o.krylov_tol : 1e-12;
     const long long kmax = o.krylov_max_iter > 0 ? o.krylov_max_iter : 2LL * m.nc;
@@ -1135,7 +1153,7 @@ FixedPointOut adjointBackward(Transport& eq, const double* dJ, double* gk, doubl
         PB_CUDA(cudaMemcpyAsync(lam_prev.p, lam.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, s));
         if (amg && eq.no_stand_in && o.preconditioner == PRISM_PC_AUTO && smallSolveFits(AT, 1)) amg = nullptr;
         const HoldAmgValues hold(amg, it > 0);
-        KrylovOut k = amg && !eq.no_stand_in && smoothedFits(amg, AT)
+        KrylovOut k = amg && !eq.no_stand_in && smoothedFits(amg, AT) && !amg->not_dominant
                           ? standInStep(AT, rhs.p, lam.p, ktol, kmax, SOLVE_FLEXIBLE, fp64, m, amg, eq)
                           : bicgstab(AT, rhs.p, lam.p, ktol, kmax, PRISM_PREC_FP64, 0.1, m.kw, s, amg, m.pat.rowptr.p,
                                      m.pat.col.p, SOLVE_PLAIN, true);
@@ -1453,6 +1471,7 @@ bool graphReady(const Transport& eq, const PrismSolveOpts& o) {
         if (eq.auto_pc == 0) return false;  // chosen on an ordinary solve first
         pc = eq.auto_pc;
     }
+    if (pc == PRISM_PC_AMG && eq.amg && eq.amg->not_dominant && flexibleFor(eq, o)) return false;  // looked at again
     if (gaveUpToJacobi(eq, o, m.matrix(eq.A.p))) pc = PRISM_PC_JACOBI;
     if (pc == PRISM_PC_JACOBI && smallSolveFits(m.matrix(eq.A.p), kmax, o.n_iter)) return true;
     if (m.kw.n != m.n_pad) return false;
@@ -1496,14 +1515,15 @@ PrismSolveResult solveAsGraph(Transport& eq, const PrismSolveOpts& o) {
     out = fromCtl(m.graph_host[0]);
     const SellMatrix A = m.matrix(eq.A.p);
     Amg* amg = hierarchyFor(eq, o, A);
-    if (standsIn(eq, o, kindFor(eq, o, amg, A), amg, A)) {
+    const int kind = kindFor(eq, o, amg, A);
+    if (standsIn(eq, o, kind, amg, A)) {
         const SolveCtl& c = m.graph_host[0];
         if (c.failed) {
             const long long spent = c.step_iterations;
             PB_CUDA(cudaMemcpyAsync(eq.phi->v.p, m.kw.xs.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
             if (o.krylov_max_iter <= 0 || spent < o.krylov_max_iter) {
                 out = solveAssembled(eq, o, true, spent);
-                standInGaveUp(eq, amg, out.status);
+                standInGaveUp(eq, amg, out.status, kind, A, m);
             }
         }
         if (o.clear_coeffs) zeroOutCoeffs(eq);

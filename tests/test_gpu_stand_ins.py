@@ -189,3 +189,39 @@ def test_flexible_cg_goes_back_to_amgs_own_cycle(gpu, graph):
         r = solve(solver, eqn, T)
         assert r.status == A.OK and r.krylov_rel_residual <= 1e-11
         assert r.krylov_iterations < (900 if call == 0 else 400)
+
+
+def test_flexible_cg_beyond_dominance_takes_amgs_own_cycle(gpu):
+    """No attempt with smoothed aggregation first, whose smoother does not reach that spectrum."""
+    for n, k, c in ((3000, 3, 0.3), (40000, 5, 0.2)):
+        rowptr, col, val, row = band(n, k, c)
+        b = np.random.default_rng(0).normal(size=n)
+        x, r = solve_csr(gpu, api.FCG(krylov_tol=1e-12), rowptr, col, val, b)
+        assert r.status == A.OK and r.krylov_iterations < 100
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("preconditioner", ["auto", "amg"])
+@pytest.mark.parametrize("first", [False, True])
+def test_dominance_is_looked_at_again(gpu, preconditioner, graph, first):
+    """An equation with negative diffusivities for two solves (its first, or later ones) gets its
+    smoothed-aggregation solve back once they are gone, bit for bit that of an equation that never
+    had them."""
+    out = []
+    for had in (False, True):
+        mesh, T, eqn, (kappa, f) = diffusion(meshgen.box_hex(24, 22, 23), gpu)
+        solver = api.BiCGSTAB(preconditioner=preconditioner, graph=graph)
+        good = kappa.values()
+        if not first:
+            assert solve(solver, eqn, T).status == A.OK
+        if had:
+            kappa.set_values(indefinite(mesh.n_cells))
+            for _ in range(2):
+                r = solve(solver, eqn, T)
+                assert r.status == A.OK or preconditioner == "amg"  # plain AMG diverges
+            kappa.set_values(good)
+        for _ in range(2):
+            r = solve(solver, eqn, T)
+            assert r.status == A.OK
+        out.append((T.values(), r.krylov_iterations))
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
