@@ -1442,7 +1442,10 @@ std::vector<BatchOut> solveBatch(const std::vector<BatchSystem>& sys, BatchPlan&
     if (symmetric && rows >= FLEX_MIN_ROWS && entries < ((int64_t)1 << 29) && sys.size() <= 65535) {
         try {
             const FlexEnd end = runFlex(sys, pl, tol, maxit, own_cap, flex, s);
-            if (end == FLEX_OK) return flex;
+            if (end == FLEX_OK) {
+                pl.look_at_dominance = false;
+                return flex;
+            }
             failed = end == FLEX_FAILED;
         } catch (const Error& e) {
             if (!hierarchyDidNotFit(e)) throw;
@@ -1468,7 +1471,7 @@ std::vector<BatchOut> solveBatch(const std::vector<BatchSystem>& sys, BatchPlan&
         // about the method
         failed = failed && out[i].status != PRISM_NONFINITE;
     }
-    pl.no_flex = pl.no_flex || failed;
+    if (failed) (pl.look_at_dominance ? pl.no_flex : pl.look_at_dominance) = true;
     return out;
 }
 

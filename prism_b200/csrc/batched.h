@@ -20,7 +20,7 @@ struct BatchSystem {
     const int* rowptr = nullptr;  // the CSR view of the pattern, in the order of the SELL slots
     const int* col = nullptr;
     int64_t nnz_csr = 0;
-    bool symmetric = false;  // by construction
+    bool symmetric = false;  // by construction, and fit for flexible CG (BatchPlan::look_at_dominance)
     const double* vals = nullptr;
     const double* b = nullptr;
     double* x = nullptr;
@@ -62,7 +62,9 @@ struct BatchPlan {
     DevBuf<float> fr32, fz32;
     DevBuf<unsigned char> fstate;
     std::unique_ptr<CaptureStreams> cs;
-    bool no_flex = false;  // it failed once on these patterns (or found no memory): BiCGSTAB from then on
+    // it failed: its next systems are looked at first (weaklyDominant); it failed on dominant ones,
+    // or found no memory: BiCGSTAB from then on
+    bool look_at_dominance = false, no_flex = false;
     // per call: the systems' values, right-hand sides and guesses gathered into the
     // concatenated buffers by one kernel (table of source pointers), and the whole
     // call -- gather, set-up, the persistent solve, scatter of the solutions -- kept

@@ -1119,9 +1119,12 @@ bool fcgSmoothed(const Amg* amg, const SellMatrix& A) {
 // The smoother weights of the symmetric cycle (up to 1.1) are for a spectrum of D^-1 A that ends
 // at 2, which weak dominance guarantees on the finest level. Beyond it the cycle amplifies what
 // it should smooth: 40,000 rows with D^-1 A up to 3 took 69,735 iterations, amg's own cycle 51.
+bool weaklyDominant(const SellMatrix& A, KrylovWork& w, cudaStream_t s) {
+    return offDiagonalRatio(A, w, s) <= 1.0 + 1e-10;  // rows that sum to zero, to rounding
+}
 void lookAtDominance(Amg* amg, const SellMatrix& A, KrylovWork& w, cudaStream_t s) {
     if (!smoothedFits(amg, A) || !fcgPre32(amg) || (amg->sa && amg->sa->built && !amg->not_dominant)) return;
-    amg->not_dominant = !(offDiagonalRatio(A, w, s) <= 1.0 + 1e-10);  // rows that sum to zero, to rounding
+    amg->not_dominant = !weaklyDominant(A, w, s);
 }
 bool hierarchyDidNotFit(const Error& e) { return e.status == PRISM_OUT_OF_MEMORY || e.status == PRISM_BAD_ARG; }
 

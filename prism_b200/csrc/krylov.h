@@ -125,6 +125,7 @@ bool fcgSmoothed(const Amg* amg, const SellMatrix& A);
 // Looks whether symmetric A is weakly diagonally dominant, for the smoothed aggregation of
 // flexible CG (Amg::not_dominant): before its hierarchy is built and, where the answer was no,
 // before every solve (a host wait each, so never inside a capture).
+bool weaklyDominant(const SellMatrix& A, KrylovWork& w, cudaStream_t s);
 void lookAtDominance(Amg* amg, const SellMatrix& A, KrylovWork& w, cudaStream_t s);
 // smoothed aggregation takes matrices of this size
 bool smoothedFits(const Amg* amg, const SellMatrix& A);

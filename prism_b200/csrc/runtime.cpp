@@ -1229,7 +1229,7 @@ std::vector<PrismSolveResult> solveBatch(BatchHandle& h, std::vector<Transport*>
         q.rowptr = m.pat.rowptr.p;
         q.col = m.pat.col.p;
         q.nnz_csr = m.pat.nnz;
-        q.symmetric = symmetricMatrix(eq);
+        q.symmetric = symmetricMatrix(eq) && (!h.plan.look_at_dominance || weaklyDominant(A, m.kw, m.stream));
         q.vals = eq.A.p;
         q.b = eq.b.p;
         q.x = eq.phi->v.p;

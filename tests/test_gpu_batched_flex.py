@@ -84,3 +84,22 @@ def test_nan_in_one_system(gpu, where, when):
                 assert cases.rel_l2(y[i], x[i]) < 1e-8
             else:
                 assert np.array_equal(x[i], y[i]) and its[i] == its_y[i]
+
+
+def test_failed_system_does_not_change_later_calls(gpu):
+    """Once its negative diffusivities are gone, a batch is again solved as one that never had them."""
+    out = []
+    for had in (False, True):
+        probs, bs = batch(gpu, [20, 21, 9], precision=A.PREC_FP64)
+        assert all(r.status == A.OK for r in solve(bs, probs))
+        if had:
+            good = probs[1]["kappa"].values()
+            indefinite(probs[1])
+            for _ in range(3):
+                assert all(r.status == A.OK for r in solve(bs, probs))
+            probs[1]["kappa"].set_values(good)
+        for _ in range(2):
+            res = solve(bs, probs)
+            out.append(([p["T"].values() for p in probs], [r.krylov_iterations for r in res]))
+    for x, its in out[1:]:
+        assert its == out[0][1] and all(np.array_equal(a, b) for a, b in zip(x, out[0][0]))
