@@ -1352,7 +1352,8 @@ FlexEnd runFlex(const std::vector<BatchSystem>& sys, BatchPlan& pl, double tol, 
                      nrows, most, end == FLEX_OK ? "ok" : end == FLEX_SHORT ? "residuals above the tolerance" : "failed");
     }
     if (end == FLEX_FAILED) scatter();
-    if (nonfinite && fresh) {  // a structure built from such values goes
+    // a structure built from such values goes, and one that failed on the matrices of another call
+    if (nonfinite ? fresh : end == FLEX_FAILED && !fresh) {
         pl.sa->built = false;
         pl.graph.reset();
         pl.graph_key.clear();

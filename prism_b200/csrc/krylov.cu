@@ -1348,26 +1348,39 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
     return out;
 }
 
+bool staleStructure(const Amg* amg, int status, int kind, const SellMatrix& A, KrylovWork& w, cudaStream_t s) {
+    return status != PRISM_NONFINITE && amg->sa && amg->sa->built && !amg->sa->fresh &&
+           (kind != SOLVE_FLEXIBLE || weaklyDominant(A, w, s));
+}
+
 KrylovOut standInSolve(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, long long cap,
                        double inner_tol, KrylovWork& w, cudaStream_t s, Amg* amg, const int* rowptr, const int* col,
                        int kind, int precision, const Instead& instead, int* instead_status) {
     *instead_status = -1;
     w.ensure(A.nslices * 32, A.nnz_padded, false);
     PB_CUDA(cudaMemcpyAsync(w.xs.p, x, A.n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    KrylovOut k = bicgstab(A, b, x, tol, std::min(maxit, STAND_IN_MAX), kind == SOLVE_FLEXIBLE ? PRISM_PREC_FP64 : precision,
-                           inner_tol, w, s, amg, rowptr, col, kind);
-    const long long left = cap > 0 ? maxit - k.iterations : maxit;
-    if (k.status == PRISM_OK || (k.status == PRISM_NOT_CONVERGED && left <= 0)) return k;
-    PB_CUDA(cudaMemcpyAsync(x, w.xs.p, A.n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    if (left <= 0) {
-        k.has_scaled = false;  // x is the guess again
-        return k;
+    long long left = maxit, used = 0;
+    while (true) {
+        KrylovOut k = bicgstab(A, b, x, tol, std::min(left, STAND_IN_MAX),
+                               kind == SOLVE_FLEXIBLE ? PRISM_PREC_FP64 : precision, inner_tol, w, s, amg, rowptr, col, kind);
+        used += k.iterations;
+        if (cap > 0) left -= k.iterations;
+        k.iterations = used;
+        if (k.status == PRISM_OK || (k.status == PRISM_NOT_CONVERGED && left <= 0)) return k;
+        PB_CUDA(cudaMemcpyAsync(x, w.xs.p, A.n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        if (left <= 0) {
+            k.has_scaled = false;  // x is the guess again
+            return k;
+        }
+        if (!staleStructure(amg, k.status, kind, A, w, s)) break;
+        amg->sa->built = false;
+        amg->values_current = false;
     }
     amg->values_current = false;
     KrylovOut f = bicgstab(A, b, x, tol, left, instead.precision, inner_tol, w, s, instead.amg, rowptr, col, instead.kind,
                            instead.symmetric);
     *instead_status = f.status;
-    f.iterations += k.iterations;
+    f.iterations += used;
     return f;
 }
 

@@ -104,9 +104,10 @@ enum { SOLVE_PLAIN = 0, SOLVE_FLEXIBLE = 1, SOLVE_SMOOTHED = 2, SOLVE_FLEXIBLE_O
 KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, int precision,
                    double inner_tol, KrylovWork& w, cudaStream_t s, Amg* amg = nullptr, const int* rowptr = nullptr,
                    const int* col = nullptr, int kind = SOLVE_PLAIN, bool symmetric = false);
-// The solve `kind` with smoothed aggregation; should it fail (within STAND_IN_MAX iterations), the
-// one that `instead` names, from the same guess and with what is left of cap, the caller's
-// limit (0: none). The guess waits in w.xs, which multigrid solves do not use.
+// The solve `kind` with smoothed aggregation; should it fail (within STAND_IN_MAX iterations),
+// once more with the structure built for this matrix where that of an earlier one was refreshed
+// (staleStructure), then the solve that `instead` names; each from the same guess and with what
+// is left of cap, the caller's limit (0: none). The guess waits in w.xs, which multigrid solves do not use.
 // *instead_status: how the latter ended (-1: it did not run).
 constexpr long long STAND_IN_MAX = 500;  // iterations (20-60 are usual) after which it has failed
 struct Instead {
@@ -115,6 +116,7 @@ struct Instead {
     int precision;
     bool symmetric;
 };
+bool staleStructure(const Amg* amg, int status, int kind, const SellMatrix& A, KrylovWork& w, cudaStream_t s);
 KrylovOut standInSolve(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, long long cap,
                        double inner_tol, KrylovWork& w, cudaStream_t s, Amg* amg, const int* rowptr, const int* col,
                        int kind, int precision, const Instead& instead, int* instead_status);

@@ -1449,10 +1449,11 @@ int runAsGraph(Mesh& m, const std::function<void()>& f) {
         PB_CUDA(cudaMemcpyAsync(m.graph_host, m.graph_ctl.p, ctx.used * sizeof(SolveCtl), cudaMemcpyDeviceToHost,
                                 m.stream));
     PB_CUDA(cudaStreamSynchronize(m.stream));
-    // nothing steps in for a solve inside a captured step; the steps after it go without
+    // nothing steps in for a solve inside a captured step: the next step, an ordinary one, builds
+    // the structure anew and may give up
     for (const auto& q : ctx.pressure) {
         const int status = m.graph_host[q.slot].status;
-        if (status == PRISM_BREAKDOWN || (status == PRISM_NOT_CONVERGED && !q.own_cap)) q.eq->no_stand_in = true;
+        if (status == PRISM_BREAKDOWN || (status == PRISM_NOT_CONVERGED && !q.own_cap)) q.eq->amg->sa->built = false;
     }
     return ctx.used;
 }
@@ -1522,8 +1523,10 @@ PrismSolveResult solveAsGraph(Transport& eq, const PrismSolveOpts& o) {
             const long long spent = c.step_iterations;
             PB_CUDA(cudaMemcpyAsync(eq.phi->v.p, m.kw.xs.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
             if (o.krylov_max_iter <= 0 || spent < o.krylov_max_iter) {
-                out = solveAssembled(eq, o, true, spent);
-                standInGaveUp(eq, amg, out.status, kind, A, m);
+                const bool again = staleStructure(amg, out.status, kind, A, m.kw, m.stream);
+                if (again) amg->sa->built = false;
+                out = solveAssembled(eq, o, !again, spent);
+                if (!again) standInGaveUp(eq, amg, out.status, kind, A, m);
             }
         }
         if (o.clear_coeffs) zeroOutCoeffs(eq);

@@ -103,3 +103,19 @@ def test_failed_system_does_not_change_later_calls(gpu):
             out.append(([p["T"].values() for p in probs], [r.krylov_iterations for r in res]))
     for x, its in out[1:]:
         assert its == out[0][1] and all(np.array_equal(a, b) for a, b in zip(x, out[0][0]))
+
+
+def test_structure_of_other_matrices_is_built_anew(gpu):
+    """Matrices without couplings in the first call left flexible CG nothing to coarsen: it fails
+    in the second, and the third has a structure of its own."""
+    from tests.test_gpu_stand_ins import heat
+    probs = [heat(gpu, shape, 0.0, 1e-6) for shape in ((700, 500, 1), (20, 20, 20))]
+    bs = api.BatchSolver(api.BiCGSTAB(precision=A.PREC_FP64), lib=gpu)
+    for call in range(3):
+        for mesh, T, eqn, (k, f) in probs:
+            T.set_values(np.zeros(mesh.n_cells))
+            if call == 1:
+                k.set_values(np.random.default_rng(2).lognormal(0.0, 1.0, mesh.n_cells))
+                eqn.set_time_step(1e6)
+        res = bs.solve([p[2] for p in probs])
+        assert all(r.status == A.OK and (call == 1 or r.krylov_iterations < 60) for r in res)
