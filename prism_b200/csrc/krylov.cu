@@ -228,18 +228,18 @@ __global__ void __launch_bounds__(BS) p_kernel(int n, T* __restrict__ p, const T
         p[i] = (T)((double)r[i] + beta * ((double)p[i] - w * (double)v[i]));
 }
 
-// s = r - alpha v, ahead of a preconditioner; c32 (optional): the FP32 copy that an FP32
+// s = r - alpha v, ahead of a preconditioner; c32 (optional): the FP32 copy, scaled, that an FP32
 // preconditioner of an FP64 iteration reads
 template <typename T>
 __global__ void __launch_bounds__(BS) s_kernel(int n, T* __restrict__ s, const T* __restrict__ r,
                                                const T* __restrict__ v, float* __restrict__ c32, const KState* S) {
     pdlEnter();
     if (S->done) return;
-    const double alpha = S->alpha;
+    const double alpha = S->alpha, scale = S->scale;
     for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
         const T si = (T)((double)r[i] - alpha * (double)v[i]);
         s[i] = si;
-        if (c32) c32[i] = (float)si;
+        if (c32) c32[i] = (float)(si * scale);
     }
 }
 
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(BS) xrp_kernel(int n, T* __restrict__ x, T* __
     pdlEnter();
     const bool done = S->done != 0;
     if (done && !S->pending) return;
-    const double alpha = S->alpha, w = S->w, beta = S->beta;
+    const double alpha = S->alpha, w = S->w, beta = S->beta, scale = S->scale;
     for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
         const double pi = (double)p[i];
         const T ri = (T)((double)s[i] - w * (double)t[i]);
@@ -263,12 +263,21 @@ __global__ void __launch_bounds__(BS) xrp_kernel(int n, T* __restrict__ x, T* __
         if (!done) {
             const T pn = (T)((double)ri + beta * (pi - w * (double)v[i]));
             p[i] = pn;
-            if (c32) c32[i] = (float)pn;
+            if (c32) c32[i] = (float)(pn * scale);
         }
     }
 }
 
 // r = b - r (r holds A x) or r = b (x = 0); r0 = p = r (c32: p's FP32 copy); v = 0; set up the state.
+// FP32 copies written in passing are right where the scale turns out as 1; elsewhere the last block
+// writes them again
+template <typename T>
+__device__ void rescaleCopies(int n, const T* r, float* c32, double rr) {
+    const double scale = cycleScale(rr);
+    if (scale == 1.0) return;
+    for (int i = threadIdx.x; i < n; i += BS) c32[i] = (float)((double)__ldcg(r + i) * scale);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(BS) init_kernel(int n, T* __restrict__ r, const T* __restrict__ b,
                                                   T* __restrict__ r0, T* __restrict__ p, T* __restrict__ v,
@@ -287,11 +296,14 @@ __global__ void __launch_bounds__(BS) init_kernel(int n, T* __restrict__ r, cons
         d1 += bi * bi;
     }
     double vv[2] = {d0, d1}, out[2];
-    if (reduceLast<2, false>(vv, partials, counter, out) && threadIdx.x == 0) {
+    if (!reduceLast<2, false>(vv, partials, counter, out)) return;
+    if (c32) rescaleCopies(n, r, c32, out[0]);
+    if (threadIdx.x == 0) {
         S->rr = out[0];
         S->bb = out[1];
         S->r0sq = out[0];
         S->tol2 = tol * tol * out[1];
+        S->scale = cycleScale(out[0]);
         S->rho = out[0];
         S->beta = out[0];
         S->alpha = 1.0;
@@ -330,11 +342,14 @@ __global__ void __launch_bounds__(BS) fcg_init_kernel(int n, double* __restrict_
         d1 += bi * bi;
     }
     double vv[2] = {d0, d1}, out[2];
-    if (reduceLast<2, false>(vv, partials, counter, out) && threadIdx.x == 0) {
+    if (!reduceLast<2, false>(vv, partials, counter, out)) return;
+    if (r32) rescaleCopies(n, r, r32, out[0]);
+    if (threadIdx.x == 0) {
         S->rr = out[0];
         S->bb = out[1];
         S->r0sq = out[0];
         S->tol2 = tol * tol * out[1];
+        S->scale = cycleScale(out[0]);
         S->dq = 1.0;
         S->dr = 0.0;
         S->alpha = 0.0;
@@ -387,7 +402,7 @@ __global__ void __launch_bounds__(BS, MINB) fcg_spmv_kernel(int nslices, int n, 
 }
 
 // d = z - beta d ; q = u - beta q ; x += alpha d ; r -= alpha q ; r.r, d.q, d.r -> convergence
-// (r32: the FP32 copy of r that an FP32 preconditioner reads)
+// (r32: the FP32 copy of r, scaled, that an FP32 preconditioner reads)
 template <typename TZ>
 __global__ void __launch_bounds__(BS) fcg_update_kernel(int n, double* __restrict__ x, double* __restrict__ r,
                                                         double* __restrict__ d, double* __restrict__ q,
@@ -396,7 +411,7 @@ __global__ void __launch_bounds__(BS) fcg_update_kernel(int n, double* __restric
                                                         unsigned int* counter, KState* S) {
     pdlEnter();
     if (S->done) return;
-    const double alpha = S->alpha, beta = S->beta;
+    const double alpha = S->alpha, beta = S->beta, scale = S->scale;
     double d0 = 0.0, d1 = 0.0, d2 = 0.0;
     for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
         const double di = (double)z[i] - beta * d[i];
@@ -406,7 +421,7 @@ __global__ void __launch_bounds__(BS) fcg_update_kernel(int n, double* __restric
         d[i] = di;
         q[i] = qi;
         r[i] = ri;
-        if (r32) r32[i] = (float)ri;
+        if (r32) r32[i] = (float)(ri * scale);
         d0 += ri * ri;
         d1 += di * qi;
         d2 += di * ri;
