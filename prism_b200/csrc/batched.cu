@@ -1437,7 +1437,7 @@ std::vector<BatchOut> solveBatch(const std::vector<BatchSystem>& sys, BatchPlan&
         PB_LAUNCH("batched plan");
     }
     int64_t rows = 0, entries = 0;
-    bool symmetric = !pl.no_flex;
+    bool symmetric = !pl.no_flex && !fp64Cycles();
     for (const auto& q : sys) {
         rows += q.n;
         entries += q.nnz_csr;

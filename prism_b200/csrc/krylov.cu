@@ -1124,10 +1124,19 @@ void setupCycle(Amg* amg, int mode, const SellMatrix& A, const int* rowptr, cons
 }
 }  // namespace
 
+bool fp64Cycles() {
+    static const bool on = [] {
+        const char* e = std::getenv("PRISM_FCG_PREC");
+        return e && std::strcmp(e, "fp64") == 0;
+    }();
+    return on;
+}
 // Smoothed aggregation up to 2^29 matrix entries (76M rows of a hex mesh): it numbers the entries
 // of Q, about 1.3 times as many, with 32-bit ints, and should rows have to be sorted, the
 // products, three times as many.
-bool smoothedFits(const Amg* amg, const SellMatrix& A) { return !amg->no_sa && A.nnz_csr < (int64_t(1) << 29); }
+bool smoothedFits(const Amg* amg, const SellMatrix& A) {
+    return !fp64Cycles() && !amg->no_sa && A.nnz_csr < (int64_t(1) << 29);
+}
 bool fcgSmoothed(const Amg* amg, const SellMatrix& A) {
     return fcgPre32(amg) && smoothedFits(amg, A) && !amg->not_dominant;
 }
@@ -1143,13 +1152,7 @@ void lookAtDominance(Amg* amg, const SellMatrix& A, KrylovWork& w, cudaStream_t 
 }
 bool hierarchyDidNotFit(const Error& e) { return e.status == PRISM_OUT_OF_MEMORY || e.status == PRISM_BAD_ARG; }
 
-bool fcgPre32(const Amg* amg) {
-    static const bool p64 = [] {
-        const char* e = std::getenv("PRISM_FCG_PREC");
-        return e && std::strcmp(e, "fp64") == 0;
-    }();
-    return !p64 && amg->k_levels == 0;
-}
+bool fcgPre32(const Amg* amg) { return !fp64Cycles() && amg->k_levels == 0; }
 
 const SolveCtl& runSmall(const SellMatrix& A, const double* b, double* x, long long n_iter, double eps, double tol,
                          long long maxit, bool symmetric, KrylovWork& w, cudaStream_t s) {

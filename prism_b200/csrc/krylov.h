@@ -121,6 +121,9 @@ bool staleStructure(const Amg* amg, int status, int kind, const SellMatrix& A, K
 KrylovOut standInSolve(const SellMatrix& A, const double* b, double* x, double tol, long long maxit, long long cap,
                        double inner_tol, KrylovWork& w, cudaStream_t s, Amg* amg, const int* rowptr, const int* col,
                        int kind, int precision, const Instead& instead, int* instead_status);
+// PRISM_FCG_PREC=fp64: FP64 iterations are preconditioned by FP64 cycles only (amg's own; batches
+// by Jacobi)
+bool fp64Cycles();
 // flexible CG with amg preconditions with an FP32 V-cycle (else with the FP64 cycle)
 bool fcgPre32(const Amg* amg);
 // that V-cycle is smoothed aggregation's (samg.h)

@@ -63,3 +63,44 @@ def test_batch(gpu):
         want = got if want is None else want
         for (x, its), (y, its_y) in zip(got, want):
             assert np.array_equal(x, y) and its == its_y
+
+
+SCRIPT = """
+import sys
+sys.path.insert(0, {root!r})
+import numpy as np
+import prism_b200
+from prism_b200 import api, meshgen
+from tests import cases
+from tests.test_gpu_smoothed import diffusion
+lib = prism_b200.lib()
+mesh, T, eqn, keep = diffusion(meshgen.box_hex(34, 33, 32), lib)
+a = api.BiCGSTAB().solve(eqn, 1, 0.0)
+mesh2, T2, U, eqn2 = cases.transport_c3(32, lib, conv="Upwind")
+b = api.BiCGSTAB(preconditioner="amg").solve(eqn2, 1, 0.0)
+probs = [cases.diffusion_box(N, lib, seed=N) for N in (20, 21)]
+c = api.BatchSolver(api.BiCGSTAB(precision=0), lib=lib).solve([p["eqn"] for p in probs])
+its = [r.krylov_iterations for r in [a, b] + c]
+np.savez({path!r}, its=its, T=T.values(), T2=T2.values(), b0=probs[0]["T"].values())
+"""
+
+
+def test_fp64_cycles_on_request(tmp_path):
+    """PRISM_FCG_PREC=fp64 (read once per process): no FP32 cycle inside an FP64 solve. Users'
+    equations then run as with PRISM_PRESSURE_SOLVER=bicgstab, by BiCGSTAB with amg's FP64 cycle,
+    and batches by BiCGSTAB."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = {}
+    for name, env in (("default", {}), ("fp64", {"PRISM_FCG_PREC": "fp64"}), ("plain", {"PRISM_PRESSURE_SOLVER": "bicgstab"})):
+        path = str(tmp_path / (name + ".npz"))
+        subprocess.run([sys.executable, "-c", SCRIPT.format(root=root, path=path)], env=dict(os.environ, **env),
+                       check=True, timeout=300)
+        out[name] = np.load(path)
+    for field in ("T", "T2"):
+        assert np.array_equal(out["fp64"][field], out["plain"][field])
+    for field in ("T", "T2", "b0"):
+        assert cases.rel_l2(out["fp64"][field], out["default"][field]) < 1e-8
+    assert np.all(out["fp64"]["its"][2:] > 2 * out["default"]["its"][2:])
