@@ -1057,10 +1057,14 @@ FixedPointOut steadySolve(Transport& eq, const PrismSolveOpts& o, int max_outer,
     FixedPointOut out;
     DevBuf<double> prev(m.n_pad), scratch(2 * NUM_SMS * 8 + 2);
     double h[2];
+    bool clean_before = false;
     for (int it = 0; it < max_outer; ++it) {
         PB_CUDA(cudaMemcpyAsync(prev.p, phi.v.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, m.stream));
-        // without convection and time terms the matrix does not depend on phi
-        const MatrixUnchanged unchanged(eq, it > 0 && symmetricMatrix(eq) && !eq.has_temporal);
+        // without convection and time terms the matrix does not depend on phi: two solves have the
+        // same one if both began with cleared coefficients
+        const bool clean = eq.clean;
+        const MatrixUnchanged unchanged(eq, clean && clean_before && symmetricMatrix(eq) && !eq.has_temporal);
+        clean_before = clean;
         PrismSolveResult r = solve(eq, o);
         out.krylov += r.krylov_iterations;
         ++out.outer;

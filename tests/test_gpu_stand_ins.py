@@ -246,3 +246,21 @@ def test_structure_of_another_matrix_is_built_anew(gpu, solver, graph):
             assert r.status == A.OK and (r.krylov_iterations < 60 or began and call == 0)
         out.append((T.values(), r.krylov_iterations))
     assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
+
+
+@pytest.mark.parametrize("clear", [True, False])
+def test_fixed_point_with_coefficients_left_over(gpu, clear):
+    """The first solve of a fixed point assembles onto what update_coeffs() left (here of a uniform
+    coefficient, a million times larger), the next ones, with cleared coefficients, another matrix:
+    their multigrid values are their own (sigma 2: a uniform coefficient's hierarchy would take
+    some hundred iterations where its own takes a few tens). Without clearing, every solve has
+    another matrix."""
+    mesh, T, eqn, (kappa, f) = diffusion(meshgen.box_hex(34, 33, 32), gpu)
+    kappa.set_values(np.full(mesh.n_cells, 1e6))
+    eqn.update_coeffs()
+    kappa.set_values(np.random.default_rng(5).lognormal(0.0, 2.0, mesh.n_cells))
+    o = api.BiCGSTAB(preconditioner="amg").opts(gpu, n_iter=1, eps=0.0, clear_coeffs=clear)
+    r = A.FixedPointResult()
+    gpu.check(gpu.adjoint_forward(eqn.h, ctypes.byref(o), 3, 0.0, ctypes.byref(r)))
+    print(f"{r.krylov_iterations} iterations in {r.outer_iterations} solves")
+    assert r.status == A.OK and r.krylov_iterations < 120
