@@ -45,6 +45,10 @@ constexpr int MAX_LEVELS = 12;
 constexpr int MIS_ROUNDS = 24;   // 6-9 rounds leave nothing undecided on the meshes seen
 constexpr int MIS_BATCH = 8;     // rounds between two looks at the number left
 constexpr double STRONG = 0.25;
+// Products per left entry beyond which a row that does not fit its table makes the hierarchy give
+// way to one with a piecewise-constant prolongation: a row coupled to all others fills A P. Meshes
+// have 2 to 20; one such row among 26,000 has 740, whose structure and values took 26 s against 1 s.
+constexpr long long MAX_PRODUCTS = 32;
 
 inline int grid(int64_t n) { return std::max(1, ceil_div(n, BS)); }
 
@@ -987,6 +991,7 @@ int64_t productPattern(DevArena& ar, int64_t m, const int* orow, const int* idx,
     long long total = 0;
     PB_CUDA(cudaMemcpyAsync(&total, off.p + m, sizeof(long long), cudaMemcpyDeviceToHost, s));
     PB_CUDA(cudaStreamSynchronize(s));
+    if (total > MAX_PRODUCTS * m) fail(PRISM_BAD_ARG, "multigrid structure too dense for smoothed aggregation");
     TmpBuf<long long> keys(std::max<long long>(total, 1), s);
     product_keys_kernel<<<grid(m), BS, 0, s>>>(m, orow, idx, b_rowptr, b_col, off.p, ncols, keys.p); countLaunch();
     return patternOf(ar, keys.p, total, nrows, ncols, rowptr, col, s);

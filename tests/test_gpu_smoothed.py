@@ -159,3 +159,46 @@ def test_little_device_memory(what):
     for x in out[1:]:
         assert cases.rel_l2(x, out[0]) < 1e-7
     assert np.array_equal(out[-1], out[0])
+
+
+def hub(n, reach):
+    """A chain of n - 1 rows and a hub (row 0) coupled to `reach` of them: an M-matrix with 0.05 to
+    spare on the diagonal, x, and b = A x."""
+    i, h = np.arange(1, n), 1 + np.arange(reach) * ((n - 1) // reach)
+    rows = np.concatenate([h, 0 * h, i[1:], i[:-1]])
+    cols = np.concatenate([0 * h, h, i[:-1], i[1:]])
+    off = np.where((rows == 0) | (cols == 0), -0.05, -1.0)
+    diag = np.zeros(n)
+    np.add.at(diag, rows, -off)
+    rows, cols, val = np.concatenate([rows, np.arange(n)]), np.concatenate([cols, np.arange(n)]), np.concatenate([off, diag + 0.05])
+    order = np.lexsort((cols, rows))
+    rows, cols, val = rows[order], cols[order], val[order]
+    rowptr = np.zeros(n + 1, np.int64)
+    np.add.at(rowptr, rows + 1, 1)
+    x = np.random.default_rng(n).normal(size=n)
+    b = np.zeros(n)
+    np.add.at(b, rows, val * x[cols])
+    return np.cumsum(rowptr), cols, val, x, b
+
+
+# ||r|| <= 1e-12 ||b|| (ten times the tolerance is accepted), ||b|| below 1e5 and ||A^-1|| below 20 bound
+# the error by 2e-6, against ||x|| above 38: 1e-7
+def test_rows_that_do_not_fit_their_tables():
+    """The hub's 286 aggregates do not fit the prolongation's tables of 32, nor the rows of A P next
+    to it; the columns of 2,000 rows not the transposes' of 512, and the Galerkin rows not theirs of
+    192: the sorted structures take over."""
+    rowptr, cols, val, x, b = hub(130000, 2000)
+    y = api.FCG(krylov_tol=1e-13).step(prism_b200.lib(), rowptr, cols, val, np.zeros(len(b)), b)
+    assert cases.rel_l2(y, x) < 1e-7
+
+
+@pytest.mark.parametrize("n", [1500, 26000])
+def test_row_coupled_to_all_others(n):
+    """It would fill A P: the solve takes amg's own cycle, in about a second at 26,000 rows, where
+    the dense structure took 26."""
+    import time
+    rowptr, cols, val, x, b = hub(n, n - 1)
+    t = time.time()
+    y = api.FCG(krylov_tol=1e-13).step(prism_b200.lib(), rowptr, cols, val, np.zeros(n), b)
+    assert time.time() - t < 10.0
+    assert cases.rel_l2(y, x) < 1e-7
