@@ -119,3 +119,17 @@ def test_structure_of_other_matrices_is_built_anew(gpu):
                 eqn.set_time_step(1e6)
         res = bs.solve([p[2] for p in probs])
         assert all(r.status == A.OK and (call == 1 or r.krylov_iterations < 60) for r in res)
+
+
+def test_more_systems_than_the_coarsest_solve_holds(gpu):
+    """130 systems leave 130 rows without couplings on the coarsest level, more than the dense
+    inverse takes: damped Jacobi sweeps solve it, and the fused tail is off."""
+    sizes = [3 + i % 4 for i in range(126)] + [9, 1, 2, 11]
+    probs, bs = batch(gpu, sizes, precision=A.PREC_FP64, krylov_tol=1e-13)
+    assert sum(N ** 3 for N in sizes) >= 8192
+    res = solve(bs, probs)
+    assert all(r.status == A.OK and r.krylov_rel_residual <= 1e-13 and r.krylov_iterations < 40 for r in res)
+    for i in (0, 1, 2, 3, 126, 127, 128, 129):
+        q = cases.diffusion_box(sizes[i], gpu, seed=70 + i)
+        api.BiCGSTAB(krylov_tol=1e-13, preconditioner="jacobi").solve(q["eqn"], 1, 0.0)
+        assert cases.rel_l2(probs[i]["T"].values(), q["T"].values()) < 1e-8
