@@ -45,9 +45,10 @@ constexpr int MAX_LEVELS = 12;
 constexpr int MIS_ROUNDS = 24;   // 6-9 rounds leave nothing undecided on the meshes seen
 constexpr int MIS_BATCH = 8;     // rounds between two looks at the number left
 constexpr double STRONG = 0.25;
-// Products per left entry beyond which a row that does not fit its table makes the hierarchy give
-// way to one with a piecewise-constant prolongation: a row coupled to all others fills A P. Meshes
-// have 2 to 20; one such row among 26,000 has 740, whose structure and values took 26 s against 1 s.
+// Products per entry (A P: of A; P^T A P: of P and A P) beyond which a row that does not fit its
+// table makes the hierarchy give way to one with a piecewise-constant prolongation: a row coupled to
+// all others fills A P. Meshes have 2 to 10; one such row among 26,000 has 740, whose structure and
+// values took 26 s against 1 s.
 constexpr long long MAX_PRODUCTS = 32;
 
 inline int grid(int64_t n) { return std::max(1, ceil_div(n, BS)); }
@@ -978,8 +979,9 @@ bool unionPattern(DevArena& ar, Union U, double left, double right, ArenaBuf<int
     return true;
 }
 
-// Pattern of the row product of m left entries (output row orow[k], right row idx[k]) with B
-int64_t productPattern(DevArena& ar, int64_t m, const int* orow, const int* idx, const int* b_rowptr, const int* b_col,
+// Pattern of the row product of m left entries (output row orow[k], right row idx[k]) with B;
+// entries: of the matrices that it is made from
+int64_t productPattern(DevArena& ar, int64_t entries, int64_t m, const int* orow, const int* idx, const int* b_rowptr, const int* b_col,
                        int nrows, long long ncols, ArenaBuf<int>& rowptr, ArenaBuf<int>& col, cudaStream_t s) {
     TmpBuf<long long> count(m + 1, s), off(m + 1, s);
     product_count_kernel<<<grid(m), BS, 0, s>>>(m, idx, b_rowptr, count.p); countLaunch();
@@ -991,7 +993,7 @@ int64_t productPattern(DevArena& ar, int64_t m, const int* orow, const int* idx,
     long long total = 0;
     PB_CUDA(cudaMemcpyAsync(&total, off.p + m, sizeof(long long), cudaMemcpyDeviceToHost, s));
     PB_CUDA(cudaStreamSynchronize(s));
-    if (total > MAX_PRODUCTS * m) fail(PRISM_BAD_ARG, "multigrid structure too dense for smoothed aggregation");
+    if (total > MAX_PRODUCTS * entries) fail(PRISM_BAD_ARG, "multigrid structure too dense for smoothed aggregation");
     TmpBuf<long long> keys(std::max<long long>(total, 1), s);
     product_keys_kernel<<<grid(m), BS, 0, s>>>(m, orow, idx, b_rowptr, b_col, off.p, ncols, keys.p); countLaunch();
     return patternOf(ar, keys.p, total, nrows, ncols, rowptr, col, s);
@@ -1245,7 +1247,7 @@ void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, bool s
             arena.rewind(before);
             TmpBuf<int> erow(std::max<int64_t>(L.nnz, 1), s);
             entry_rows_kernel<<<grid(L.n), BS, 0, s>>>(L.n, L.rowptr, erow.p); countLaunch();
-            L.q_nnz = productPattern(arena, L.nnz, erow.p, L.col, L.p_rowptr.p, L.p_col.p, L.n, nc, L.q_rowptr, L.q_col, s);
+            L.q_nnz = productPattern(arena, L.nnz, L.nnz, erow.p, L.col, L.p_rowptr.p, L.p_col.p, L.n, nc, L.q_rowptr, L.q_col, s);
         }
         L.ap_val.alloc(arena, std::max<int64_t>(L.q_nnz, 1), s);
         L.q_val.alloc(arena, std::max<int64_t>(L.q_nnz, 1), s);
@@ -1266,8 +1268,8 @@ void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, bool s
             arena.rewind(before);
             TmpBuf<int> erow(std::max<int64_t>(L.p_nnz, 1), s);
             entry_rows_kernel<<<grid(L.n), BS, 0, s>>>(L.n, L.p_rowptr.p, erow.p); countLaunch();
-            C->nnz = productPattern(arena, L.p_nnz, L.p_col.p, erow.p, L.q_rowptr.p, L.q_col.p, nc, nc, C->o_rowptr,
-                                    C->o_col, s);
+            C->nnz = productPattern(arena, L.p_nnz + L.q_nnz, L.p_nnz, L.p_col.p, erow.p, L.q_rowptr.p, L.q_col.p, nc, nc,
+                                    C->o_rowptr, C->o_col, s);
         }
         C->n = nc;
         C->rowptr = C->o_rowptr.p;

@@ -1,11 +1,14 @@
 """Flexible CG with the smoothed-aggregation cycle, at the sizes where its levels, tail and
 coarsest solve change: one dense level, levels inside the fused tail only, levels above it,
 thin and ragged boxes, tetrahedra, strongly varying coefficients and rows without couplings."""
+import ctypes
+
 import numpy as np
 import pytest
 
 import oracle
 import prism_b200
+from prism_b200 import _abi as A
 from prism_b200 import api, meshgen
 from tests import cases
 
@@ -162,9 +165,9 @@ def test_little_device_memory(what):
 
 
 def hub(n, reach):
-    """A chain of n - 1 rows and a hub (row 0) coupled to `reach` of them: an M-matrix with 0.05 to
+    """A chain of n - 1 rows and a hub (row 0) coupled to the first `reach` of them: an M-matrix with 0.05 to
     spare on the diagonal, x, and b = A x."""
-    i, h = np.arange(1, n), 1 + np.arange(reach) * ((n - 1) // reach)
+    i, h = np.arange(1, n), np.arange(1, 1 + reach)
     rows = np.concatenate([h, 0 * h, i[1:], i[:-1]])
     cols = np.concatenate([0 * h, h, i[:-1], i[1:]])
     off = np.where((rows == 0) | (cols == 0), -0.05, -1.0)
@@ -184,11 +187,16 @@ def hub(n, reach):
 # ||r|| <= 1e-12 ||b|| (ten times the tolerance is accepted), ||b|| below 1e5 and ||A^-1|| below 20 bound
 # the error by 2e-6, against ||x|| above 38: 1e-7
 def test_rows_that_do_not_fit_their_tables():
-    """The hub's 286 aggregates do not fit the prolongation's tables of 32, nor the rows of A P next
-    to it; the columns of 2,000 rows not the transposes' of 512, and the Galerkin rows not theirs of
-    192: the sorted structures take over."""
-    rowptr, cols, val, x, b = hub(130000, 2000)
-    y = api.FCG(krylov_tol=1e-13).step(prism_b200.lib(), rowptr, cols, val, np.zeros(len(b)), b)
+    """The hub's 200 aggregates do not fit the prolongation's tables of 32, nor those of the rows of
+    A P and of the Galerkin matrix next to it; its column of 600 rows not the transpose's of 512: the
+    sorted structures take over. With smoothed aggregation the solve takes a quarter of the
+    iterations of amg's own hierarchy (70 to 80)."""
+    rowptr, cols, val, x, b = hub(130000, 600)
+    o, r, y = api.FCG(krylov_tol=1e-13).opts(prism_b200.lib()), A.SolveResult(), np.zeros(len(b))
+    prism_b200.lib().check(prism_b200.lib().solve_csr(
+        len(b), rowptr.ctypes.data_as(A.pi64), np.ascontiguousarray(cols, np.int64).ctypes.data_as(A.pi64),
+        api._f64p(val), api._f64p(b), api._f64p(y), ctypes.byref(o), ctypes.byref(r)))
+    assert r.status == A.OK and r.krylov_iterations < 50
     assert cases.rel_l2(y, x) < 1e-7
 
 
