@@ -1356,7 +1356,10 @@ FlexEnd runFlex(const std::vector<BatchSystem>& sys, BatchPlan& pl, double tol, 
         std::fprintf(stderr, "[prism] batched flexible CG of %d systems (%d rows): at most %lld iterations, %s\n", pl.nprob,
                      nrows, most, end == FLEX_OK ? "ok" : end == FLEX_SHORT ? "residuals above the tolerance" : "failed");
     }
-    if (end == FLEX_FAILED) scatter();
+    if (end == FLEX_FAILED) {
+        scatter();
+        PB_CUDA(cudaStreamSynchronize(s));  // the systems' own streams go on with the guesses
+    }
     // a structure built from such values goes, and one that failed on the matrices of another call
     if (nonfinite ? fresh : end == FLEX_FAILED && !fresh) {
         pl.sa->built = false;

@@ -133,3 +133,17 @@ def test_more_systems_than_the_coarsest_solve_holds(gpu):
         q = cases.diffusion_box(sizes[i], gpu, seed=70 + i)
         api.BiCGSTAB(krylov_tol=1e-13, preconditioner="jacobi").solve(q["eqn"], 1, 0.0)
         assert cases.rel_l2(probs[i]["T"].values(), q["T"].values()) < 1e-8
+
+
+def test_guess_is_back_where_the_cap_ends_a_failed_system(gpu):
+    """A breakdown at the caller's cap leaves no iterations for BiCGSTAB: the field is the guess when
+    the call's own residuals are taken from it, and when it returns."""
+    probs, bs = batch(gpu, [20, 21, 9], precision=A.PREC_FP64, krylov_max_iter=5)
+    indefinite(probs[1])
+    for p in probs:
+        p["T"].set_values(np.full(p["mesh"].n_cells, 0.25))
+    res = bs.solve([p["eqn"] for p in probs])
+    assert all(r.krylov_iterations <= 5 for r in res)
+    if res[1].status == A.BREAKDOWN:
+        assert np.all(probs[1]["T"].values() == 0.25)
+        assert res[1].final_residual == res[1].initial_residual
