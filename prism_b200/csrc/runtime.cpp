@@ -1193,6 +1193,7 @@ double* BatchHandle::residuals(size_t n) {
     if (n > host_n) {
         if (host) cudaFreeHost(host);
         host = nullptr;
+        host_n = 0;
         PB_CUDA(cudaMallocHost(&host, 3 * n * sizeof(double)));
         host_n = n;
     }
@@ -1214,6 +1215,14 @@ std::vector<PrismSolveResult> solveBatch(BatchHandle& h, std::vector<Transport*>
     std::vector<PrismSolveResult> res(eqs.size());
     std::vector<BatchSystem> sys(eqs.size());
     int64_t maxn = 0;
+    // residuals are on their way to h's pinned memory until their streams are waited for, also where
+    // an equation of the batch is refused
+    struct Drain {
+        const std::vector<Transport*>& eqs;
+        ~Drain() {
+            for (auto* eq : eqs) cudaStreamSynchronize(eq->phi->m->stream);
+        }
+    } drain_on_error{eqs};
     const auto t0 = std::chrono::steady_clock::now();
     for (size_t i = 0; i < eqs.size(); ++i) {
         Transport& eq = *eqs[i];

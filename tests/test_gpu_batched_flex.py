@@ -147,3 +147,22 @@ def test_guess_is_back_where_the_cap_ends_a_failed_system(gpu):
     if res[1].status == A.BREAKDOWN:
         assert np.all(probs[1]["T"].values() == 0.25)
         assert res[1].final_residual == res[1].initial_residual
+
+
+def test_refused_equation_leaves_the_batch_usable(gpu):
+    """An equation without a boundary handler ends the call while the others' residuals are on
+    their way to the batch's pinned memory, which the next, larger call allocates anew."""
+    from prism_b200 import PrismError
+    from tests.test_failures import no_handler_case
+    refused = no_handler_case(gpu)[-1]
+    probs, bs = batch(gpu, [20, 21, 9], precision=A.PREC_FP64)
+    for _ in range(3):
+        with pytest.raises(PrismError) as e:
+            bs.solve([probs[0]["eqn"], refused])
+        assert e.value.status == A.NO_BC_HANDLER
+    probs[0]["eqn"].zero_out_coeffs()  # it was assembled before the refusal
+    got = solve(bs, probs), [p["T"].values() for p in probs]
+    probs, bs = batch(gpu, [20, 21, 9], precision=A.PREC_FP64)
+    want = solve(bs, probs), [p["T"].values() for p in probs]
+    assert all(np.array_equal(a, b) for a, b in zip(got[1], want[1]))
+    assert [r.initial_residual for r in got[0]] == [r.initial_residual for r in want[0]]
