@@ -7,14 +7,16 @@
 // textbook recurrences Eigen uses) with Jacobi right preconditioning, applied
 // by scaling the columns once per step: A' = A D^-1, x' = D x, so every
 // iteration is three streaming kernels and no preconditioner pass:
-//   v = A' p ; r0.v -> alpha                    SpMV + fused dot
-//   s = r - alpha v (formed where it is read, and kept) ; t = A' s ;
-//   t.s, t.t, r0.s, r0.t, s.s -> w, r0.r, r.r, beta, convergence    SpMV + fused dots
-//   x += alpha p + w s ; r = s - w t ; p = r + beta (p - w v)       vector kernel
-// (r0.r = r0.s - w r0.t and r.r = s.s - w t.s, so the update needs no reduction and can
-// carry the next direction. Five kernels, with s, the update and p each on its own, took 16.9
-// against 13.7 us an iteration on 66,748 seven-point rows, 25.5 against 21.8 us on 262,144
-// five-point rows and the same 104 us on 2.1M, where the bytes decide.)
+//   p = r + beta q (formed where it is read, and kept) ; v = A' p ; r0.v -> alpha   SpMV + fused dot
+//   s = r - alpha v (the same) ; t = A' s ; t.s, t.t -> w                           SpMV + fused dots
+//   x += alpha p + w s ; r = s - w t ; q = p - w v (in t's place) ; r0.r, r.r -> beta, convergence
+// (With p, s and the update each on its own, five kernels: 23.9 against 20.0 us an iteration on
+// 64,000 seven-point rows, 36.5 against 30.1 on 262,144 and 133 against 127 on 2.1M; with p alone on
+// its own 20.6, 31.8 and 126.
+// r0.r is taken from the updated r: as r0.s - w r0.t, which would let the last kernel go without
+// a reduction and write p itself, it loses its relative accuracy where r vanishes on r0's support,
+// and with it beta and the breakdown test: upwind momentum matrices of 10,000 rows took 20,000
+// iterations and more, against 2,000 to 4,000.)
 // Scalars live in device memory (KState); every reduction is a fixed-order
 // two-stage tree (block partials, then the last block to finish reduces them),
 // so results are bitwise reproducible run to run. The host launches batches of
@@ -90,9 +92,9 @@ int waveGrid(K kernel, int needed) {
 // STAGE 0: plain; 1: alpha = rho / (u.y)
 // The columns and values of up to 8 slots are loaded before their gathers, so
 // a row's loads are all in flight at once; the sum runs over the slots in order.
-template <typename T, int W = 8, typename TX = T>
-__device__ __forceinline__ T sliceRow(const int* __restrict__ col, const T* __restrict__ val,
-                                      const TX* __restrict__ x, int b, int width, int lane) {
+template <typename T, int W, typename X>
+__device__ __forceinline__ T sliceSum(const int* __restrict__ col, const T* __restrict__ val, int b, int width, int lane,
+                                      X x) {
     T sum = 0;
     for (int j0 = 0; j0 < width; j0 += W) {
         int c[W];
@@ -105,9 +107,22 @@ __device__ __forceinline__ T sliceRow(const int* __restrict__ col, const T* __re
             }
 #pragma unroll
         for (int k = 0; k < W; ++k)
-            if (j0 + k < width) sum += v[k] * (T)__ldg(x + c[k]);
+            if (j0 + k < width) sum += v[k] * x(c[k]);
     }
     return sum;
+}
+template <typename T, int W = 8, typename TX = T>
+__device__ __forceinline__ T sliceRow(const int* __restrict__ col, const T* __restrict__ val,
+                                      const TX* __restrict__ x, int b, int width, int lane) {
+    return sliceSum<T, W>(col, val, b, width, lane, [&](int c) { return (T)__ldg(x + c); });
+}
+
+// r0.v -> alpha; r0.v = 0 (or a non-finite alpha) breaks the recurrence down: the host restarts
+// from the current x (every later kernel of this iteration returns at once)
+__device__ __forceinline__ void setAlpha(KState* S, double r0v) {
+    const double alpha = S->rho / r0v;
+    if (r0v == 0.0 || !isfinite(alpha)) S->done = isfinite(r0v) ? 3 : 5;
+    else S->alpha = alpha;
 }
 
 template <typename T, int STAGE, int W = 8, int MINB = 5, typename TX = T>
@@ -117,10 +132,7 @@ __global__ void __launch_bounds__(BS, MINB) spmv_kernel(int nslices, int n, cons
                                                   const T* __restrict__ u, double* partials,
                                                   unsigned int* counter, KState* S) {
     pdlEnter();
-    if (STAGE != 0 && S->done) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) S->pending = 0;  // the last update has run
-        return;
-    }
+    if (STAGE != 0 && S->done) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double d0 = 0.0;
     for (int sl = blockIdx.x * WARPS + warp; sl < nslices; sl += gridDim.x * WARPS) {
@@ -133,30 +145,48 @@ __global__ void __launch_bounds__(BS, MINB) spmv_kernel(int nslices, int n, cons
     }
     if (STAGE == 0) return;
     double v[1] = {d0}, out[1];
-    if (reduceLast<1, false>(v, partials, counter, out) && threadIdx.x == 0) {
-        // r0.v = 0 (or a non-finite alpha) breaks the recurrence down: the host restarts
-        // from the current x (every later kernel of this iteration returns at once)
-        const double alpha = S->rho / out[0];
-        if (out[0] == 0.0 || !isfinite(alpha)) S->done = isfinite(out[0]) ? 3 : 5;
-        else S->alpha = alpha;
-    }
+    if (reduceLast<1, false>(v, partials, counter, out) && threadIdx.x == 0) setAlpha(S, out[0]);
 }
 
-// t = A q with the dots t.s, t.t, r0.s, r0.t, s.s -> w, r0.r, r.r of r = s - w t, beta and the
-// convergence test. FORM: q = s = r - alpha v, formed from r and v where it is gathered and
+// v = A p with r0.v -> alpha, for p = r + beta q, formed where it is gathered and written for this row
+template <int W, int MINB>
+__global__ void __launch_bounds__(BS, MINB) spmv1_form_kernel(int nslices, int n, const int* __restrict__ sl_off,
+                                                              const int* __restrict__ col,
+                                                              const double* __restrict__ val,
+                                                              const double* __restrict__ r,
+                                                              const double* __restrict__ q, double* __restrict__ p,
+                                                              double* __restrict__ v, const double* __restrict__ r0,
+                                                              double* partials, unsigned int* counter, KState* S) {
+    pdlEnter();
+    if (S->done) return;
+    const double beta = S->beta;
+    auto form = [&](int c) { return __ldg(r + c) + beta * __ldg(q + c); };
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double d = 0.0;
+    for (int sl = blockIdx.x * WARPS + warp; sl < nslices; sl += gridDim.x * WARPS) {
+        const int b = sl_off[sl], width = (sl_off[sl + 1] - b) >> 5, i = sl * 32 + lane;
+        const double sum = sliceSum<double, W>(col, val, b, width, lane, form);
+        p[i] = i < n ? form(i) : 0.0;
+        v[i] = sum;
+        if (i < n) d += sum * r0[i];
+    }
+    double dots[1] = {d}, out[1];
+    if (reduceLast<1, false>(dots, partials, counter, out) && threadIdx.x == 0) setAlpha(S, out[0]);
+}
+
+// t = A q with the dots t.s, t.t -> w. FORM: q = s = r - alpha v, formed where it is gathered and
 // written for this row; else q is given (M^-1 s of a preconditioner) and s read.
 template <typename T, bool FORM, int W, int MINB, typename TX = T>
 __global__ void __launch_bounds__(BS, MINB) spmv2_kernel(int nslices, int n, const int* __restrict__ sl_off,
                                                    const int* __restrict__ col, const T* __restrict__ val,
                                                    const TX* __restrict__ q, T* __restrict__ t, T* __restrict__ s,
                                                    const T* __restrict__ r, const T* __restrict__ v,
-                                                   const T* __restrict__ r0, double* partials, unsigned int* counter,
-                                                   KState* S) {
+                                                   double* partials, unsigned int* counter, KState* S) {
     pdlEnter();
     if (S->done) return;
     const double alpha = S->alpha;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double d[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    double d[2] = {0.0, 0.0};
     for (int sl = blockIdx.x * WARPS + warp; sl < nslices; sl += gridDim.x * WARPS) {
         const int b = sl_off[sl];
         const int width = (sl_off[sl + 1] - b) >> 5;
@@ -164,20 +194,7 @@ __global__ void __launch_bounds__(BS, MINB) spmv2_kernel(int nslices, int n, con
         T sum, si;
         if constexpr (FORM) {
             auto form = [&](int c) { return (T)((double)__ldg(r + c) - alpha * (double)__ldg(v + c)); };
-            sum = 0;
-            for (int j0 = 0; j0 < width; j0 += W) {
-                int c[W];
-                T m[W];
-#pragma unroll
-                for (int k = 0; k < W; ++k)
-                    if (j0 + k < width) {
-                        c[k] = __ldcs(col + b + 32 * (j0 + k) + lane);
-                        m[k] = __ldcs(val + b + 32 * (j0 + k) + lane);
-                    }
-#pragma unroll
-                for (int k = 0; k < W; ++k)
-                    if (j0 + k < width) sum += m[k] * form(c[k]);
-            }
+            sum = sliceSum<T, W>(col, val, b, width, lane, form);
             si = i < n ? form(i) : (T)0;
             s[i] = si;
         } else {
@@ -186,46 +203,31 @@ __global__ void __launch_bounds__(BS, MINB) spmv2_kernel(int nslices, int n, con
         }
         t[i] = sum;
         if (i < n) {
-            const double sd = (double)si, td = (double)sum, r0i = (double)r0[i];
-            d[0] += td * sd;
-            d[1] += td * td;
-            d[2] += r0i * sd;
-            d[3] += r0i * td;
-            d[4] += sd * sd;
+            d[0] += (double)sum * (double)si;
+            d[1] += (double)sum * (double)sum;
         }
     }
-    double out[5];
-    if (reduceLast<5, false>(d, partials, counter, out) && threadIdx.x == 0) {
-        const double w = out[1] > 0.0 ? out[0] / out[1] : 0.0;
-        const double rho_new = out[2] - w * out[3], rr = out[4] - w * out[0];
-        S->w = w;
+    double out[2];
+    if (reduceLast<2, false>(d, partials, counter, out) && threadIdx.x == 0) {
         S->ts = out[0];
         S->tt = out[1];
-        S->rr = rr;
-        S->iter += 1;
-        int done = 0;
-        if (!isfinite(rho_new) || !isfinite(rr)) done = 5;
-        else if (S->reliable && (rr <= S->tol2 || rr < S->delta2 * S->rr_update)) done = 6;
-        else if (rr <= S->tol2) done = 1;
-        else if (S->iter >= S->maxit) done = 2;
-        else if (w == 0.0 || fabs(rho_new) < EPSILON * EPSILON * S->r0sq) done = 3;
-        else {
-            S->beta = (rho_new / S->rho) * (S->alpha / w);
-            S->rho = rho_new;
-        }
-        S->pending = done != 0;
-        S->done = done;
+        S->w = out[1] > 0.0 ? out[0] / out[1] : 0.0;
     }
 }
 
-// p = r + beta (p - w v): after a reliable update that continues the recurrence
+// p = r + beta (p - w v), ahead of a preconditioner (c32 as in s_kernel) or in FP32, where q in its
+// place would be rounded once more
 template <typename T>
 __global__ void __launch_bounds__(BS) p_kernel(int n, T* __restrict__ p, const T* __restrict__ r,
-                                               const T* __restrict__ v, const KState* S) {
+                                               const T* __restrict__ v, float* __restrict__ c32, const KState* S) {
+    pdlEnter();
     if (S->done) return;
-    const double beta = S->beta, w = S->w;
-    for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS)
-        p[i] = (T)((double)r[i] + beta * ((double)p[i] - w * (double)v[i]));
+    const double beta = S->beta, w = S->w, scale = S->scale;
+    for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
+        const T pi = (T)((double)r[i] + beta * ((double)p[i] - w * (double)v[i]));
+        p[i] = pi;
+        if (c32) c32[i] = (float)(pi * scale);
+    }
 }
 
 // s = r - alpha v, ahead of a preconditioner; c32 (optional): the FP32 copy, scaled, that an FP32
@@ -243,62 +245,61 @@ __global__ void __launch_bounds__(BS) s_kernel(int n, T* __restrict__ s, const T
     }
 }
 
-// x += alpha y + w q ; r = s - w t ; p = r + beta (p - w v), with y = p and q = s, or M^-1 of
-// them (y null: y = p); c32 as in s_kernel, of p. The last direction of a solve that stops is
-// left as it was.
-template <typename T, typename TQ = T>
-__global__ void __launch_bounds__(BS) xrp_kernel(int n, T* __restrict__ x, T* __restrict__ r, T* __restrict__ p,
-                                                 const TQ* __restrict__ y, const TQ* __restrict__ q,
-                                                 const T* __restrict__ s, const T* __restrict__ t,
-                                                 const T* __restrict__ v, float* __restrict__ c32, const KState* S) {
+// x += alpha y + w z ; r = s - w t ; r0.r, r.r -> beta, convergence, with y = p and z = s, or M^-1 of
+// them. NEXT: t = p - w v, what the next direction needs besides r
+template <typename T, bool NEXT, typename TQ = T>
+__global__ void __launch_bounds__(BS) xr_kernel(int n, T* __restrict__ x, T* __restrict__ r, const TQ* __restrict__ y,
+                                                const TQ* __restrict__ z, const T* __restrict__ s, T* __restrict__ t,
+                                                const T* __restrict__ v, const T* __restrict__ r0, double* partials,
+                                                unsigned int* counter, KState* S) {
     pdlEnter();
-    const bool done = S->done != 0;
-    if (done && !S->pending) return;
-    const double alpha = S->alpha, w = S->w, beta = S->beta, scale = S->scale;
+    if (S->done) return;
+    const double alpha = S->alpha, w = S->w;
+    double d0 = 0.0, d1 = 0.0;
     for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
-        const double pi = (double)p[i];
+        const double yi = (double)y[i];
         const T ri = (T)((double)s[i] - w * (double)t[i]);
-        x[i] = (T)((double)x[i] + alpha * (y ? (double)y[i] : pi) + w * (double)q[i]);
+        x[i] = (T)((double)x[i] + alpha * yi + w * (double)z[i]);
         r[i] = ri;
-        if (!done) {
-            const T pn = (T)((double)ri + beta * (pi - w * (double)v[i]));
-            p[i] = pn;
-            if (c32) c32[i] = (float)(pn * scale);
+        if (NEXT) t[i] = (T)(yi - w * (double)v[i]);
+        d0 += (double)r0[i] * (double)ri;
+        d1 += (double)ri * (double)ri;
+    }
+    double dots[2] = {d0, d1}, out[2];
+    if (reduceLast<2, false>(dots, partials, counter, out) && threadIdx.x == 0) {
+        const double rho_new = out[0], rr = out[1];
+        S->rr = rr;
+        S->iter += 1;
+        if (!isfinite(rho_new) || !isfinite(rr)) S->done = 5;
+        else if (S->reliable && (rr <= S->tol2 || rr < S->delta2 * S->rr_update)) S->done = 6;
+        else if (rr <= S->tol2) S->done = 1;
+        else if (S->iter >= S->maxit) S->done = 2;
+        else if (w == 0.0 || fabs(rho_new) < EPSILON * EPSILON * S->r0sq) S->done = 3;
+        else {
+            S->beta = (rho_new / S->rho) * (alpha / w);
+            S->rho = rho_new;
         }
     }
 }
 
-// r = b - r (r holds A x) or r = b (x = 0); r0 = p = r (c32: p's FP32 copy); v = 0; set up the state.
-// FP32 copies written in passing are right where the scale turns out as 1; elsewhere the last block
-// writes them again
+// r = b - r (r holds A x) or r = b (x = 0); r0 = r; p = v = 0 (or q twice: the first direction is r
+// whatever beta is); set up the state.
 template <typename T>
-__device__ void rescaleCopies(int n, const T* r, float* c32, double rr) {
-    const double scale = cycleScale(rr);
-    if (scale == 1.0) return;
-    for (int i = threadIdx.x; i < n; i += BS) c32[i] = (float)((double)__ldcg(r + i) * scale);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(BS) init_kernel(int n, T* __restrict__ r, const T* __restrict__ b,
-                                                  T* __restrict__ r0, T* __restrict__ p, T* __restrict__ v,
-                                                  float* __restrict__ c32, int from_zero, double tol, double* partials,
-                                                  unsigned int* counter, KState* S) {
+__global__ void __launch_bounds__(BS) init_kernel(int n, T* r, const T* b, T* r0, T* p, T* v, int from_zero, double tol,
+                                                  double* partials, unsigned int* counter, KState* S) {
     double d0 = 0.0, d1 = 0.0;
     for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
         double bi = (double)b[i];
         T ri = from_zero ? b[i] : (T)(bi - (double)r[i]);
         r[i] = ri;
         r0[i] = ri;
-        p[i] = ri;
-        if (c32) c32[i] = (float)ri;
+        p[i] = 0;
         v[i] = 0;
         d0 += (double)ri * (double)ri;
         d1 += bi * bi;
     }
     double vv[2] = {d0, d1}, out[2];
-    if (!reduceLast<2, false>(vv, partials, counter, out)) return;
-    if (c32) rescaleCopies(n, r, c32, out[0]);
-    if (threadIdx.x == 0) {
+    if (reduceLast<2, false>(vv, partials, counter, out) && threadIdx.x == 0) {
         S->rr = out[0];
         S->bb = out[1];
         S->r0sq = out[0];
@@ -308,7 +309,6 @@ __global__ void __launch_bounds__(BS) init_kernel(int n, T* __restrict__ r, cons
         S->beta = out[0];
         S->alpha = 1.0;
         S->w = 1.0;
-        S->pending = 0;
         if (!isfinite(out[0]) || !isfinite(out[1])) S->done = 5;
         else if (out[1] == 0.0) S->done = 4;
         else if (out[0] <= S->tol2) S->done = 1;
@@ -325,6 +325,14 @@ __global__ void __launch_bounds__(BS) init_kernel(int n, T* __restrict__ r, cons
 // (q = A d is carried, not recomputed: A d = A z - beta A d_prev). dq and dr
 // are the previous direction's d.q and d.r, taken exactly in the update pass;
 // dq' expands d.q for symmetric A.
+
+// FP32 copies written in passing are right where the scale turns out as 1; elsewhere the last block
+// writes them again
+__device__ void rescaleCopies(int n, const double* r, float* c32, double rr) {
+    const double scale = cycleScale(rr);
+    if (scale == 1.0) return;
+    for (int i = threadIdx.x; i < n; i += BS) c32[i] = (float)(__ldcg(r + i) * scale);
+}
 
 // r = b - r (r holds A x); d = q = 0; state as init_kernel
 __global__ void __launch_bounds__(BS) fcg_init_kernel(int n, double* __restrict__ r, const double* __restrict__ b,
@@ -483,7 +491,7 @@ __global__ void flush_kernel(int n, double* __restrict__ xs, float* __restrict__
 }
 // Reliable update, part 2 (Ax = A' xs already in `ax`): r64 = b - ax, r32 = (float) r64,
 // rr = r64.r64, rho = r0.r32; continue the recurrence or declare convergence.
-// first != 0: (re)start -- r0 = p = r32, v = 0, fresh recurrence scalars.
+// first != 0: (re)start -- r0 = r32, p = v = 0, fresh recurrence scalars.
 __global__ void __launch_bounds__(BS) reliable_kernel(int n, const double* __restrict__ ax, const double* __restrict__ b,
                                                       double* __restrict__ r64, float* __restrict__ r32,
                                                       float* __restrict__ r032, float* __restrict__ p32,
@@ -497,7 +505,7 @@ __global__ void __launch_bounds__(BS) reliable_kernel(int n, const double* __res
         r32[i] = rf;
         if (first) {
             r032[i] = rf;
-            p32[i] = rf;
+            p32[i] = 0.0f;
             v32[i] = 0.0f;
         }
         d0 += ri * ri;
@@ -508,7 +516,6 @@ __global__ void __launch_bounds__(BS) reliable_kernel(int n, const double* __res
     if (reduceLast<3, false>(v, partials, counter, out) && threadIdx.x == 0) {
         S->rr = out[0];
         S->rr_update = out[0];
-        S->pending = 0;
         if (first) {
             S->bb = out[2];
             S->tol2 = tol * tol * out[2];
@@ -812,8 +819,9 @@ inline void precApply(Amg* amg, const float* r, float* z, const KState* S, cudaS
 // blocks per SM. Measured on the 128^3 transport matrix (ncu, FP64): 4x6 (40 registers,
 // 71% warps active) 45 / 43 us for the two stages against 47 / 53 us for 8x5 (48
 // registers, 60%) and 52 / 50 us for 4x8 (32 registers, 97%). PRISM_SPMV_SHAPE = "WxMINB"
-// (4x6, 8x5, 4x8) overrides it. The second stage sums five dots and takes 4 blocks per SM (64
-// registers; at 6 it spills).
+// (4x6, 8x5, 4x8) overrides it. The stages that form their vector take 5 blocks per SM (48 registers;
+// 4: 132 against 127 us an iteration on 2.1M seven-point rows, 20.0 as well on 64,000; 6 spill: 145, 23).
+constexpr int FORM_MINB = 5;
 int spmvShape() {
     static const int v = [] {
         const char* e = std::getenv("PRISM_SPMV_SHAPE");
@@ -823,14 +831,19 @@ int spmvShape() {
     }();
     return v;
 }
-// f(first SpMV, second SpMV forming s, second SpMV given M^-1 s)
+// f(first SpMV forming p, given p or M^-1 p, second SpMV forming s, given M^-1 s)
 template <typename T, typename F>
 void withSpmvShape(F&& f) {
     switch (spmvShape()) {
-        case 0: f(spmv_kernel<T, 1, 8, 5>, spmv2_kernel<T, true, 8, 5>, spmv2_kernel<T, false, 8, 5>); break;
-        case 1: f(spmv_kernel<T, 1, 4, 8>, spmv2_kernel<T, true, 4, 8>, spmv2_kernel<T, false, 4, 8>); break;
-        default: f(spmv_kernel<T, 1, 4, 6>, spmv2_kernel<T, true, 4, 4>, spmv2_kernel<T, false, 4, 4>); break;
+        case 0: f(spmv1_form_kernel<8, 5>, spmv_kernel<T, 1, 8, 5>, spmv2_kernel<T, true, 8, 5>, spmv2_kernel<T, false, 8, 5>); break;
+        case 1: f(spmv1_form_kernel<4, 8>, spmv_kernel<T, 1, 4, 8>, spmv2_kernel<T, true, 4, 8>, spmv2_kernel<T, false, 4, 8>); break;
+        default: f(spmv1_form_kernel<4, FORM_MINB>, spmv_kernel<T, 1, 4, 6>, spmv2_kernel<T, true, 4, FORM_MINB>, spmv2_kernel<T, false, 4, 6>); break;
     }
+}
+// the iteration forms p in its first SpMV, from r and q (kept in t)
+template <typename T>
+bool formsDirection(const Amg* amg) {
+    return sizeof(T) == 8 && !amg;
 }
 
 // Krylov method of a solve: BiCGSTAB (Jacobi or amg's V-cycle), flexible CG preconditioned
@@ -851,33 +864,41 @@ void iterateEager(const SellMatrix& A, const T* M, Vecs<T> V, Amg* amg, T* y, T*
         precApply(amg, r, out, S, s, sample);
     };
     const int n = A.n, vg = vecGrid(n);
-    decltype(&spmv_kernel<T, 1>) k1 = nullptr;
-    withSpmvShape<T>([&](auto k, auto, auto) { k1 = k; });
-    decltype(&spmv2_kernel<T, true, 4, 6>) k2 = nullptr;
-    withSpmvShape<T>([&](auto, auto form, auto plain) { k2 = amg ? plain : form; });
-    const int sg1 = waveGrid(k1, ceil_div(A.nslices, WARPS));
-    const int sg2 = waveGrid(k2, ceil_div(A.nslices, WARPS));
-    for (long long it = 0; it < count; ++it) {
-        const T* dp = V.p;
-        if (amg) {
-            cycle(V.p, y);
-            dp = y;
+    withSpmvShape<T>([&](auto k1_form, auto k1, auto k2_form, auto k2_given) {
+        const auto k2 = amg ? k2_given : k2_form;
+        const int needed = ceil_div(A.nslices, WARPS);
+        const int sgf = waveGrid(k1_form, needed), sg1 = waveGrid(k1, needed), sg2 = waveGrid(k2, needed);
+        for (long long it = 0; it < count; ++it) {
+            const T *dp = V.p, *ds = V.s;
+            if (!formsDirection<T>(amg)) launchPdl(p_kernel<T>, vg, BS, s, n, V.p, V.r, V.v, (float*)nullptr, S);
+            if (amg) {
+                cycle(V.p, y);
+                dp = y;
+            }
+            const int slot = sample ? profBegin(PROF_SPMV, sizeof(T) == 4, spmvBytes<T>(A), s) : -1;
+            if constexpr (sizeof(T) == 8) {
+                if (formsDirection<T>(amg))
+                    launchPdl(k1_form, sgf, BS, s, A.nslices, n, A.sl_off, A.col, M, V.r, V.t, V.p, V.v, V.r0,
+                              w.partials.p, w.counter.p, S);
+            }
+            if (!formsDirection<T>(amg))
+                launchPdl(k1, sg1, BS, s, A.nslices, n, A.sl_off, A.col, M, dp, V.v, V.r0, w.partials.p, w.counter.p, S);
+            profEnd(slot, s);
+            if (amg) {
+                launchPdl(s_kernel<T>, vg, BS, s, n, V.s, V.r, V.v, (float*)nullptr, S);
+                cycle(V.s, z);
+                ds = z;
+            }
+            launchPdl(k2, sg2, BS, s, A.nslices, n, A.sl_off, A.col, M, ds, V.t, V.s, V.r, V.v, w.partials.p,
+                      w.counter.p, S);
+            if (formsDirection<T>(amg))
+                launchPdl(xr_kernel<T, true>, vg, BS, s, n, V.x, V.r, dp, ds, V.s, V.t, V.v, V.r0, w.partials.p,
+                          w.counter.p, S);
+            else
+                launchPdl(xr_kernel<T, false>, vg, BS, s, n, V.x, V.r, dp, ds, V.s, V.t, V.v, V.r0, w.partials.p,
+                          w.counter.p, S);
         }
-        const int slot = sample ? profBegin(PROF_SPMV, sizeof(T) == 4, spmvBytes<T>(A), s) : -1;
-        launchPdl(k1, sg1, BS, s, A.nslices, n, A.sl_off, A.col, M, dp, V.v, V.r0, w.partials.p,
-                  w.counter.p, S);
-        profEnd(slot, s);
-        const T* ds = V.s;
-        if (amg) {
-            launchPdl(s_kernel<T>, vg, BS, s, n, V.s, V.r, V.v, (float*)nullptr, S);
-            cycle(V.s, z);
-            ds = z;
-        }
-        launchPdl(k2, sg2, BS, s, A.nslices, n, A.sl_off, A.col, M, ds, V.t, V.s, V.r, V.v, V.r0, w.partials.p,
-                  w.counter.p, S);
-        launchPdl(xrp_kernel<T, T>, vg, BS, s, n, V.x, V.r, V.p, amg ? dp : (const T*)nullptr, ds, V.s, V.t, V.v,
-                  (float*)nullptr, S);
-    }
+    });
 }
 
 // `count` FP64 BiCGSTAB iterations with the FP32 cycle of smoothed aggregation: p and s go to
@@ -887,12 +908,13 @@ void iterateSmoothed(const SellMatrix& A, const double* M, Vecs<double> V, Amg* 
     KState* S = w.state.p;
     const int n = A.n, vg = vecGrid(n);
     auto k1 = spmv_kernel<double, 1, 4, 6, float>;
-    auto k2 = spmv2_kernel<double, false, 4, 4, float>;
+    auto k2 = spmv2_kernel<double, false, 4, 6, float>;
     const int sg1 = waveGrid(k1, ceil_div(A.nslices, WARPS)), sg2 = waveGrid(k2, ceil_div(A.nslices, WARPS));
     float* in = w.y32.p;
     float* ph = w.z32.p;
     float* sh = reinterpret_cast<float*>(w.z.p);
     for (long long it = 0; it < count; ++it) {
+        launchPdl(p_kernel<double>, vg, BS, s, n, V.p, V.r, V.v, in, S);
         amg->sa->apply(in, ph, S, s, sample);
         const int slot = sample ? profBegin(PROF_SPMV, false, spmvBytes<double>(A) - 4.0 * A.n, s) : -1;
         launchPdl(k1, sg1, BS, s, A.nslices, n, A.sl_off, A.col, M, (const float*)ph, V.v, V.r0, w.partials.p,
@@ -900,10 +922,10 @@ void iterateSmoothed(const SellMatrix& A, const double* M, Vecs<double> V, Amg* 
         profEnd(slot, s);
         launchPdl(s_kernel<double>, vg, BS, s, n, V.s, V.r, V.v, in, S);
         amg->sa->apply(in, sh, S, s);
-        launchPdl(k2, sg2, BS, s, A.nslices, n, A.sl_off, A.col, M, (const float*)sh, V.t, V.s, V.r, V.v, V.r0,
-                  w.partials.p, w.counter.p, S);
-        launchPdl(xrp_kernel<double, float>, vg, BS, s, n, V.x, V.r, V.p, (const float*)ph, (const float*)sh, V.s, V.t,
-                  V.v, in, S);
+        launchPdl(k2, sg2, BS, s, A.nslices, n, A.sl_off, A.col, M, (const float*)sh, V.t, V.s, V.r, V.v, w.partials.p,
+                  w.counter.p, S);
+        launchPdl(xr_kernel<double, false, float>, vg, BS, s, n, V.x, V.r, (const float*)ph, (const float*)sh, V.s, V.t,
+                  V.v, V.r0, w.partials.p, w.counter.p, S);
     }
 }
 
@@ -1053,9 +1075,9 @@ KrylovOut runBicgstab(const SellMatrix& A, const T* M, const T* rhs, Vecs<T> V, 
             }
         }
         if (!flex) {
-            init_kernel<T><<<vg, BS, 0, s>>>(n, V.r, rhs, V.r0, V.p, V.v,
-                                             mode == KM_BICGSTAB_SA && sizeof(T) == 8 ? w.y32.p : nullptr, zero ? 1 : 0, tol, w.partials.p, w.counter.p,
-                                             S); countLaunch();
+            const bool form = formsDirection<T>(amg);
+            init_kernel<T><<<vg, BS, 0, s>>>(n, V.r, rhs, V.r0, form ? V.t : V.p, form ? V.t : V.v, zero ? 1 : 0, tol,
+                                             w.partials.p, w.counter.p, S); countLaunch();
         }
         PB_LAUNCH("bicgstab init");
         zero = false;
@@ -1331,7 +1353,6 @@ KrylovOut bicgstab(const SellMatrix& A, const double* b, double* x, double tol, 
                 done = reliable(1);
             } else {
                 done = reliable(0);
-                p_kernel<float><<<vg, BS, 0, s>>>(n, w.p32.p, w.r32.p, w.v32.p, S); countLaunch();
             }
             continue;
         }
@@ -1740,8 +1761,9 @@ void emitBicgstab(const SellMatrix& A, const double* b, double* x, double tol, l
         fcg_init_kernel<<<vg, BS, 0, sub>>>(n, V.r, b, V.p, V.v, precondIn32(mode) ? w.y32.p : nullptr, tol,
                                             w.partials.p, w.counter.p, S); countLaunch();
     } else {
-        init_kernel<double><<<vg, BS, 0, sub>>>(n, V.r, b, V.r0, V.p, V.v,
-                                                mode == KM_BICGSTAB_SA ? w.y32.p : nullptr, 0, tol, w.partials.p, w.counter.p, S); countLaunch();
+        const bool form = formsDirection<double>(amg);
+        init_kernel<double><<<vg, BS, 0, sub>>>(n, V.r, b, V.r0, form ? V.t : V.p, form ? V.t : V.v, 0, tol, w.partials.p,
+                                                w.counter.p, S); countLaunch();
     }
     endConditional(sub);
     beginConditional(body, cudaGraphCondTypeIf, ht, sub);

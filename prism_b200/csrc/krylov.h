@@ -45,7 +45,6 @@ struct KState {
     int done;  // 0 running, 1 converged, 2 max iterations, 3 restart needed, 4 zero rhs, 5 non-finite,
                // 6 reliable update due (mixed precision)
     int reliable;
-    int pending;  // BiCGSTAB: done was set with this iteration's update of x, r and p still to come
 };
 
 // Workspace owned by a mesh, sized on first use.

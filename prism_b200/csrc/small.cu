@@ -20,7 +20,7 @@ namespace pb {
 
 namespace {
 
-constexpr int NV = 5;  // values of one reduction, at most
+constexpr int NV = 3;  // values of one reduction, at most
 
 struct SmallParams {
     int n;
@@ -248,28 +248,29 @@ __global__ void __launch_bounds__(THREADS, 1) small_solve_kernel(const SmallPara
                         sh[own(k)] = dinv[k] * r[k];
                     }
                     R.barrier();
-                    // t = A M^-1 s; the dots of r = s - w t follow from those of s and t, so the
-                    // update needs no reduction of its own
-                    double t[K];
-                    d[0] = d[1] = d[2] = d[3] = d[4] = 0.0;
+                    double t[K];  // A M^-1 s
+                    d[0] = d[1] = 0.0;
 #pragma unroll
                     for (int k = 0; k < K; ++k) {
                         t[k] = rowOf(k, sh);
                         d[0] += t[k] * r[k];
                         d[1] += t[k] * t[k];
-                        d[2] += r0[k] * r[k];
-                        d[3] += r0[k] * t[k];
-                        d[4] += r[k] * r[k];
                     }
-                    R.template all<5>(d);
+                    R.template all<2>(d);
                     w = d[1] > 0.0 ? d[0] / d[1] : 0.0;
+                    // r0.r of the updated r (as r0.s - w r0.t it loses its accuracy where r
+                    // vanishes on r0's support: krylov.cu)
+                    d[0] = d[1] = 0.0;
 #pragma unroll
                     for (int k = 0; k < K; ++k) {
                         x[k] += alpha * (dinv[k] * p[k]) + w * (dinv[k] * r[k]);
                         r[k] -= w * t[k];
+                        d[0] += r0[k] * r[k];
+                        d[1] += r[k] * r[k];
                     }
+                    R.template all<2>(d);
                     ++iter;
-                    const double rho_new = d[2] - w * d[3], rr = d[4] - w * d[0];
+                    const double rho_new = d[0], rr = d[1];
                     if (!isfinite(rho_new) || !isfinite(rr)) done = 5;
                     else if (rr <= tol2) done = 1;
                     else if (iter >= left) done = 2;
