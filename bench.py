@@ -547,8 +547,9 @@ def run_ours(args, world, rank, local):
                 "unit": "GB/s", "frac": gbs / hbm if gbs else None, "traffic": traffic_for(traffic_file, nbytes),
                 "algorithmic_bytes_per_launch": nbytes, "avg_launch_ms": ms, "sampled_launches": launches}
 
-    spmv = kernel_line("spmv_kernel<double,1> (SELL-32 SpMV + fused dot, BiCGSTAB v = A y: the momentum predictors)",
-                spmv_gbs, spmv_ms, spmv_bytes, prof.fp64_launches, "spmv_fp64_traffic.json")
+    spmv = kernel_line("spmv1_form_kernel<4,5> (SELL-32 SpMV + fused dot, BiCGSTAB v = A p with p = r + beta q formed "
+                "where it is read: the momentum predictors)",
+                spmv_gbs, spmv_ms, spmv_bytes, prof.fp64_launches, "spmv_form_traffic.json")
     fcg = kernel_line("fcg_spmv_kernel<4,6,float> (flexible CG u = A z + three fused dots: the pressure correction)",
                fcg_gbs, fcg_ms, fcg_bytes, prof.fcg_launches, "fcg_spmv_traffic.json")
     if post_gbs:

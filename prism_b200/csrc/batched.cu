@@ -933,10 +933,10 @@ std::vector<BatchOut> runBatch(const std::vector<BatchSystem>& sys, BatchPlan& p
 // Reductions are per slice (one warp), then per system (one block, in a fixed order).
 struct FState {
     double rr, bb, tol2, dq, dr, alpha, beta, rel;
-    double scale;  // of r32 (cycleScale)
     long long iter;
     int done;  // as KState::done: 0 running, 1 converged, 2 iteration cap, 3 breakdown, 4 b = 0, 5 non-finite
     int restart, pass, restarts, status;
+    int shift;  // scale of r32 (cycleShift)
     int bad;  // the right-hand side, the guess or the matrix is not finite: no system of flexible CG
 };
 constexpr int FLEX_MIN_ROWS = 8192;
@@ -1051,12 +1051,12 @@ __global__ void __launch_bounds__(BS) flex_init_reduce_kernel(const FP P) {
         S.dr = 0.0;
         S.done = !isfinite(t[0]) || !isfinite(t[1]) ? 5 : t[1] == 0.0 ? 4 : t[0] <= S.tol2 ? 1 : 0;
         if (S.done == 5 && S.pass == 0 && S.restarts == 0) S.bad = 1;
-        S.scale = cycleScale(t[0]);
+        S.shift = cycleShift(t[0]);
     }
     dropNonfinite(P, blockIdx.x);
-    if (S.done == 5 || S.scale == 1.0) return;
+    if (S.done == 5 || S.shift == 0) return;
     for (int i = 32 * P.prob_slice0[blockIdx.x] + threadIdx.x; i < 32 * P.prob_slice0[blockIdx.x + 1]; i += BS)
-        P.r32[i] = (float)(P.r[i] * S.scale);
+        P.r32[i] = cycleCopy(P.r[i], S.shift);
 }
 // u = A z ; z.q, z.u, z.r
 __global__ void __launch_bounds__(BS) flex_spmv_kernel(const FP P) {
@@ -1100,7 +1100,7 @@ __global__ void __launch_bounds__(BS) flex_update_kernel(const FP P) {
         P.d[i] = di;
         P.q[i] = qi;
         P.r[i] = ri;
-        P.r32[i] = (float)(ri * S.scale);
+        P.r32[i] = cycleCopy(ri, S.shift);
         slicePartials(P, sl, lane, ri * ri, di * qi, di * ri);
     });
 }

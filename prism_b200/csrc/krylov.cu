@@ -222,11 +222,12 @@ __global__ void __launch_bounds__(BS) p_kernel(int n, T* __restrict__ p, const T
                                                const T* __restrict__ v, float* __restrict__ c32, const KState* S) {
     pdlEnter();
     if (S->done) return;
-    const double beta = S->beta, w = S->w, scale = S->scale;
+    const double beta = S->beta, w = S->w;
+    const int shift = S->shift;
     for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
         const T pi = (T)((double)r[i] + beta * ((double)p[i] - w * (double)v[i]));
         p[i] = pi;
-        if (c32) c32[i] = (float)(pi * scale);
+        if (c32) c32[i] = cycleCopy((double)pi, shift);
     }
 }
 
@@ -237,11 +238,12 @@ __global__ void __launch_bounds__(BS) s_kernel(int n, T* __restrict__ s, const T
                                                const T* __restrict__ v, float* __restrict__ c32, const KState* S) {
     pdlEnter();
     if (S->done) return;
-    const double alpha = S->alpha, scale = S->scale;
+    const double alpha = S->alpha;
+    const int shift = S->shift;
     for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
         const T si = (T)((double)r[i] - alpha * (double)v[i]);
         s[i] = si;
-        if (c32) c32[i] = (float)(si * scale);
+        if (c32) c32[i] = cycleCopy((double)si, shift);
     }
 }
 
@@ -304,7 +306,7 @@ __global__ void __launch_bounds__(BS) init_kernel(int n, T* r, const T* b, T* r0
         S->bb = out[1];
         S->r0sq = out[0];
         S->tol2 = tol * tol * out[1];
-        S->scale = cycleScale(out[0]);
+        S->shift = cycleShift(out[0]);
         S->rho = out[0];
         S->beta = out[0];
         S->alpha = 1.0;
@@ -329,9 +331,9 @@ __global__ void __launch_bounds__(BS) init_kernel(int n, T* r, const T* b, T* r0
 // FP32 copies written in passing are right where the scale turns out as 1; elsewhere the last block
 // writes them again
 __device__ void rescaleCopies(int n, const double* r, float* c32, double rr) {
-    const double scale = cycleScale(rr);
-    if (scale == 1.0) return;
-    for (int i = threadIdx.x; i < n; i += BS) c32[i] = (float)(__ldcg(r + i) * scale);
+    const int shift = cycleShift(rr);
+    if (shift == 0) return;
+    for (int i = threadIdx.x; i < n; i += BS) c32[i] = cycleCopy(__ldcg(r + i), shift);
 }
 
 // r = b - r (r holds A x); d = q = 0; state as init_kernel
@@ -357,7 +359,7 @@ __global__ void __launch_bounds__(BS) fcg_init_kernel(int n, double* __restrict_
         S->bb = out[1];
         S->r0sq = out[0];
         S->tol2 = tol * tol * out[1];
-        S->scale = cycleScale(out[0]);
+        S->shift = cycleShift(out[0]);
         S->dq = 1.0;
         S->dr = 0.0;
         S->alpha = 0.0;
@@ -410,9 +412,8 @@ __global__ void __launch_bounds__(BS, MINB) fcg_spmv_kernel(int nslices, int n, 
 }
 
 // d = z - beta d ; q = u - beta q ; x += alpha d ; r -= alpha q ; r.r, d.q, d.r -> convergence
-// (r32: the FP32 copy of r, scaled, that an FP32 preconditioner reads). Eight blocks per SM, the scale
-// read where it is used: HBM-bound, and at the 40 registers it takes by itself a quarter of the
-// warps are missing (a solve of 2.1M five-point rows 8.70 against 8.77 ms).
+// (r32, with an FP32 preconditioner: the scaled copy of r that it reads). Eight blocks per SM:
+// HBM-bound, and at the 40 registers it takes by itself a quarter of the warps are missing.
 template <typename TZ>
 __global__ void __launch_bounds__(BS, 8) fcg_update_kernel(int n, double* __restrict__ x, double* __restrict__ r,
                                                         double* __restrict__ d, double* __restrict__ q,
@@ -422,6 +423,7 @@ __global__ void __launch_bounds__(BS, 8) fcg_update_kernel(int n, double* __rest
     pdlEnter();
     if (S->done) return;
     const double alpha = S->alpha, beta = S->beta;
+    const int shift = S->shift;
     double d0 = 0.0, d1 = 0.0, d2 = 0.0;
     for (int i = blockIdx.x * BS + threadIdx.x; i < n; i += gridDim.x * BS) {
         const double di = (double)z[i] - beta * d[i];
@@ -431,7 +433,7 @@ __global__ void __launch_bounds__(BS, 8) fcg_update_kernel(int n, double* __rest
         d[i] = di;
         q[i] = qi;
         r[i] = ri;
-        if (r32) r32[i] = (float)(ri * __ldg(&S->scale));
+        if constexpr (sizeof(TZ) == 4) r32[i] = cycleCopy(ri, shift);
         d0 += ri * ri;
         d1 += di * qi;
         d2 += di * ri;
@@ -774,6 +776,8 @@ template <typename T>
 double spmvBytes(const SellMatrix& A) {
     return (double)A.nnz_csr * (sizeof(T) + 4) + 4.0 * (A.n + 1) + 2.0 * A.n * sizeof(T);
 }
+// the same with x = p formed from r and q, and written
+double spmvFormBytes(const SellMatrix& A) { return spmvBytes<double>(A) + 16.0 * A.n; }
 // flexible CG's u = A z: FP64 matrix, z of zbytes, u written, q and r read for the dots
 double fcgSpmvBytes(const SellMatrix& A, int zbytes) {
     return (double)A.nnz_csr * 12.0 + 4.0 * (A.n + 1) + (zbytes + 24.0) * A.n;
@@ -877,7 +881,8 @@ void iterateEager(const SellMatrix& A, const T* M, Vecs<T> V, Amg* amg, T* y, T*
                 cycle(V.p, y);
                 dp = y;
             }
-            const int slot = sample ? profBegin(PROF_SPMV, sizeof(T) == 4, spmvBytes<T>(A), s) : -1;
+            const double bytes = formsDirection<T>(amg) ? spmvFormBytes(A) : spmvBytes<T>(A);
+            const int slot = sample ? profBegin(PROF_SPMV, sizeof(T) == 4, bytes, s) : -1;
             if constexpr (sizeof(T) == 8) {
                 if (formsDirection<T>(amg))
                     launchPdl(k1_form, sgf, BS, s, A.nslices, n, A.sl_off, A.col, M, V.r, V.t, V.p, V.v, V.r0,

@@ -40,11 +40,11 @@ struct KState {
     double ts, tt;
     double rr_update, delta2;  // mixed precision: |r|^2 at the last reliable update, trigger factor^2
     double dq, dr;             // flexible CG: d.(A d) and d.r of the last direction
-    double scale;              // of the FP32 vectors that an FP32 cycle is given (cycleScale)
     long long iter, maxit;
     int done;  // 0 running, 1 converged, 2 max iterations, 3 restart needed, 4 zero rhs, 5 non-finite,
                // 6 reliable update due (mixed precision)
     int reliable;
+    int shift;  // scale of the FP32 vectors that an FP32 cycle is given (cycleShift)
 };
 
 // Workspace owned by a mesh, sized on first use.

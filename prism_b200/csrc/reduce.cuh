@@ -77,9 +77,14 @@ __device__ bool reduceLast(double (&v)[NV], double* partials, unsigned int* coun
 // not depend on a factor in it, so the scale only has to keep the residual's entries, down to 1e-18
 // of its first norm, within FP32's 1e-38 to 3e38: 1 from 1e-18 to 1e24, else the power of two that
 // brings the norm near 1 (every bit of the results is then that of a system scaled so).
-__device__ __forceinline__ double cycleScale(double rr) {
-    if (!(rr > 0.0) || !isfinite(rr) || (rr >= 1e-36 && rr <= 1e48)) return 1.0;
-    return ldexp(1.0, -(ilogb(rr) / 2));
+// Kept as what it adds to a double's upper word.
+__device__ __forceinline__ int cycleShift(double rr) {
+    if (!(rr > 0.0) || !isfinite(rr) || (rr >= 1e-36 && rr <= 1e48)) return 0;
+    return -(ilogb(rr) / 2) * (1 << 20);
+}
+__device__ __forceinline__ float cycleCopy(double v, int shift) {
+    const int hi = __double2hiint(v);
+    return (float)__hiloint2double((hi & 0x7fffffff) ? hi + shift : hi, __double2loint(v));
 }
 
 }  // namespace pb
