@@ -661,7 +661,7 @@ class SIMPLEControls:
     pressure_residual: float = 1e-7
     p_ref_cell: Optional[int] = None
     p_ref_value: float = 0.0
-    batched_momentum: bool = False  # momentum components solved together in one persistent launch
+    batched_momentum: bool = False  # momentum components solved together in one persistent BiCGSTAB launch
 
     def to_c(self):
         c = A.SIMPLEControls()
@@ -791,7 +791,8 @@ def adjoint_backward(eqn: Transport, dJ_dphi, solver: Optional[_Solver] = None, 
 
 # ---- batched solves ------------------------------------------------------------------
 class BatchSolver:
-    """Independent equations solved together in one persistent launch
+    """Independent equations solved together in one launch (flexible CG over the block-diagonal
+    matrix where all are symmetric and hold 8,192 rows or more, else persistent BiCGSTAB)
     (prism_batch_solve): solve(eqns) ~ [solver.solve(e, n_iter=1) for e in eqns]."""
 
     def __init__(self, solver: Optional[_Solver] = None, lib=None):

@@ -1,4 +1,4 @@
-"""A batched diffusion solve (many independent systems in one persistent
+"""A batched diffusion solve (many independent systems in one
 launch), for profiling and timing the batched solver.
 
 Builds `count` problems of N^3 unit-cube hexes, N = round(exp(U(ln nmin,

@@ -1,4 +1,5 @@
-// batched.h -- many independent linear solves in one persistent launch.
+// batched.h -- many independent linear solves in one launch: flexible CG over the block-diagonal
+// matrix where all are symmetric (a graph with device-side loops), else persistent BiCGSTAB.
 #pragma once
 
 #include <memory>

@@ -842,7 +842,7 @@ void setURF(Transport& eq, double f) {  // transport.cpp:38-52: out-of-range val
 
 // solveImplicitMomentum, SIMPLE.cpp:19-41. With batched_momentum every component
 // is assembled and relaxed as usual and the systems are then solved together in
-// one persistent launch (one step each, to the Krylov tolerance).
+// one persistent BiCGSTAB launch (one step each, to the Krylov tolerance).
 void solveImplicitMomentum(const PrismSIMPLEControls& c, std::vector<Transport*>& mom, const PrismSolveOpts& so,
                            std::vector<Report>& rep) {
     if (c.batched_momentum) {

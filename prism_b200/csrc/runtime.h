@@ -137,14 +137,14 @@ struct Transport {
     DevBuf<double> store;  // A, b, bconv and bdiff in one allocation
     DevSlice<double> A, b, bconv, bdiff;
     std::shared_ptr<Amg> amg;  // AMG hierarchy (PRISM_PC_AMG), built on the first solve
-    // symmetric positive (semi-)definite matrix (the pressure correction): with AMG,
-    // FP64 solves run flexible CG with the K-cycle instead of BiCGSTAB
+    // symmetric positive (semi-)definite matrix (the pressure correction): with AMG, FP64 solves
+    // run flexible CG (smoothed aggregation's FP32 V-cycle, or amg's cycle) instead of BiCGSTAB
     bool spd = false;
     // PRISM_PC_AUTO at AMG sizes, decided on the equation's first solve: Jacobi when
     // its matrix is diagonally dominant enough (offDiagonalRatio), else AMG (0: not yet)
     int auto_pc = 0;
-    // the method standing in for BiCGSTAB with amg's cycle failed on this equation (kindFor):
-    // it keeps the latter
+    // smoothed aggregation failed on this equation where the solve in its place did not
+    // (standInGaveUp): BiCGSTAB or flexible CG with amg's cycle from then on (kindFor)
     bool no_stand_in = false;
     // the next solves assemble the same matrix as the last one (only b changes):
     // its AMG hierarchy keeps its values
@@ -213,8 +213,9 @@ struct FixedPointOut {
 FixedPointOut steadySolve(Transport& eq, const PrismSolveOpts& o, int max_outer, double outer_tol);
 
 // Batched ISolver::solve(eq, n_iter = 1): every equation is assembled and
-// relaxed on its mesh, then all systems are solved together in one persistent
-// launch (batched.h) and each field receives its solution.
+// relaxed on its mesh, then all systems are solved together in one launch (batched.h:
+// flexible CG over the block-diagonal matrix, or persistent BiCGSTAB) and each field
+// receives its solution.
 struct BatchHandle {
     double* host = nullptr;  // pinned: the parts of each system's scaled residual
     size_t host_n = 0;
