@@ -45,6 +45,12 @@ constexpr int MAX_LEVELS = 12;
 constexpr int MIS_ROUNDS = 24;   // 6-9 rounds leave nothing undecided on the meshes seen
 constexpr int MIS_BATCH = 8;     // rounds between two looks at the number left
 constexpr double STRONG = 0.25;
+// Coarse symmetric levels are smoothed (omega 1.1) and their prolongation is smoothed (0.95) as if
+// the spectrum of D^-1 A ended near 1.5, which holds for diffusion. With a time term it may reach 3 from
+// the third level on, where both amplify: 2.1M rows with off-diagonal sums of 0.9 of the diagonal took
+// 242 iterations, of 0.8 13. A diagonal raised to half of its row's sum keeps it below 2 (15 iterations, as
+// many as before without a time term; 1.8 costs 5-8% more there, for convection the bound only costs).
+constexpr double SPECTRUM = 2.0;
 // Products per entry (A P: of A; P^T A P: of P and A P) beyond which a row that does not fit its
 // table makes the hierarchy give way to one with a piecewise-constant prolongation: a row coupled to
 // all others fills A P. Meshes have 2 to 10; one such row among 26,000 has 740, whose structure and
@@ -67,14 +73,19 @@ __global__ void csr_pos_kernel(int n, const int* rowptr, const int* sl_off, int*
     for (int k = rowptr[r]; k < rowptr[r + 1]; ++k) csr_pos[k] = base + 32 * (k - rowptr[r]);
 }
 
-// D^-1 and omega D^-1 (0 for a zero diagonal)
+// D^-1 and omega D^-1 (0 for a zero diagonal). bound > 0: a diagonal below 1/bound of its row's sum of
+// magnitudes is taken as that, which keeps the spectrum of D^-1 A within it
 __global__ void scaling_kernel(int n, const int* rowptr, const int* col, const int* csr_pos, const double* vals,
-                               double omega, double* dinv, float* wd) {
+                               double omega, double bound, double* dinv, float* wd) {
     const int i = blockIdx.x * BS + threadIdx.x;
     if (i >= n) return;
-    double d = 0.0;
-    for (int k = rowptr[i]; k < rowptr[i + 1]; ++k)
-        if (col[k] == i) d = valueAt(vals, csr_pos, k);
+    double d = 0.0, sum = 0.0;
+    for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) {
+        const double a = valueAt(vals, csr_pos, k);
+        if (col[k] == i) d = a;
+        sum += fabs(a);
+    }
+    if (bound > 0.0 && d != 0.0 && sum > bound * fabs(d)) d = copysign(sum / bound, d);
     const double di = d != 0.0 ? 1.0 / d : 0.0;
     dinv[i] = di;
     wd[i] = (float)(omega * di);
@@ -1108,7 +1119,8 @@ void withLanes(int l, F&& f) {
 
 // D^-1 and the FP32 copy of A from the current values of level L
 void SaAmg::levelScaling(SaLevel& L, cudaStream_t s) {
-    scaling_kernel<<<grid(L.n), BS, 0, s>>>(L.n, L.rowptr, L.col, L.csr_pos, L.vals, L.omega, L.dinv.p, L.wd.p); countLaunch();
+    scaling_kernel<<<grid(L.n), BS, 0, s>>>(L.n, L.rowptr, L.col, L.csr_pos, L.vals, L.omega, L.csr_pos || L.tr_pos.p ? 0.0 : SPECTRUM,
+                                            L.dinv.p, L.wd.p); countLaunch();
     const int64_t m = L.csr_pos ? L.sell_nnz : L.nnz;
     const int* col = L.csr_pos ? L.sl_col : L.col;
     scaled_values_kernel<<<(int)std::min<int64_t>(grid(m), NUM_SMS * 32), BS, 0, s>>>(m, col, L.vals, L.dinv.p, L.omega,
