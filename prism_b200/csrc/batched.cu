@@ -1220,6 +1220,7 @@ FlexEnd runFlex(const std::vector<BatchSystem>& sys, BatchPlan& pl, double tol, 
         }
         pl.fstate.alloc(sizeof(FState) * pl.nprob);
         pl.sa = std::make_unique<SaAmg>();
+        pl.sa->max_fill = 100.0;  // as for single systems of these sizes: the other way is Jacobi
         pl.cs = std::make_unique<CaptureStreams>();
     }
     const bool fresh = !pl.sa->built;  // the structure is of this call's matrix

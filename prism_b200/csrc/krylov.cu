@@ -1149,6 +1149,14 @@ void setupCycle(Amg* amg, int mode, const SellMatrix& A, const int* rowptr, cons
         return;
     }
     if (!amg->sa) amg->sa = std::make_unique<SaAmg>();
+    // Coefficients that vary by orders of magnitude from cell to cell leave few strong couplings, so
+    // coarsening slows and the levels fill in. What their products cost goes with rows x (entries per
+    // row)^2: 1 to 4 times the matrix's for smooth coefficients, 30 to 700 for lognormal ones (sigma 2 to 3),
+    // where refreshing them takes longer than the solve with amg's own hierarchy: at 32 25.7 ms against 20.9
+    // (490,000 rows), at 42 26.5 against 17.7 (690,640), at 123 62.6 against 18.5 (357,911); but at 30 7.3
+    // against 8.9 (216,000), at 10 8.0 against 13 (690,640). Where the other way is the one-launch Jacobi
+    // solve more pays: at 89 6.6 ms against 21 (29,791 rows).
+    amg->sa->max_fill = smallSolveFits(A, 1) ? 100.0 : 25.0;
     amg->sa->setup(A, rowptr, col, mode == KM_FCG_SA, amg->values_current, s);
 }
 }  // namespace

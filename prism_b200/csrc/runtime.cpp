@@ -605,7 +605,7 @@ static bool jacobiInstead(const PrismSolveOpts& o, const SellMatrix& A) {
     return o.method == PRISM_SOLVER_BICGSTAB && o.preconditioner == PRISM_PC_AUTO && smallSolveFits(A, 1);
 }
 static bool gaveUpToJacobi(const Transport& eq, const PrismSolveOpts& o, const SellMatrix& A) {
-    return eq.no_stand_in && jacobiInstead(o, A);
+    return (eq.no_stand_in || (eq.amg && eq.amg->no_sa)) && jacobiInstead(o, A);
 }
 // the hierarchy of a solve of eq, as yet unbuilt on the first one (null: none)
 static Amg* hierarchyFor(Transport& eq, const PrismSolveOpts& o, const SellMatrix& A) {
@@ -711,7 +711,7 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o, b
             jacobiStep(A, eq.b.p, phi.v.p, m.kw, m.stream);
         } else {
             const HoldAmgValues hold(amg, eq.matrix_unchanged || iter > 0);  // A is fixed within one solve
-            if ((eq.no_stand_in || plain) && jacobiInstead(o, A)) amg = nullptr;  // since an earlier step
+            if (gaveUpToJacobi(eq, o, A) || (plain && jacobiInstead(o, A))) amg = nullptr;  // since an earlier step
             int kind = kindFor(eq, o, amg, A);
             if (plain && standsIn(eq, o, kind, amg, A)) kind = standsInFor(eq, o);
             const long long cap = iter == 0 && o.krylov_max_iter > 0 ? kmax - spent : kmax;
@@ -1142,7 +1142,7 @@ FixedPointOut adjointBackward(Transport& eq, const double* dJ, double* gk, doubl
         if (!eq.amg_adj) eq.amg_adj = std::make_shared<Amg>();
         amg = eq.amg_adj.get();
         lookAtDominance(amg, AT, m.kw, s);
-        if (amg->not_dominant && o.preconditioner == PRISM_PC_AUTO && smallSolveFits(AT, 1)) amg = nullptr;
+        if ((amg->not_dominant || amg->no_sa) && o.preconditioner == PRISM_PC_AUTO && smallSolveFits(AT, 1)) amg = nullptr;
     }
     const double ktol = o.krylov_tol > 0 ? o.krylov_tol : 1e-12;
     const long long kmax = o.krylov_max_iter > 0 ? o.krylov_max_iter : 2LL * m.nc;
@@ -1155,7 +1155,7 @@ FixedPointOut adjointBackward(Transport& eq, const double* dJ, double* gk, doubl
         adjointCorrection(P, lam.p, u.p, d.p, np, s);
         adjointRhs(P, d_dJ.p, lam.p, u.p, d.p, np, rhs.p, s);
         PB_CUDA(cudaMemcpyAsync(lam_prev.p, lam.p, m.nc * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        if (amg && eq.no_stand_in && o.preconditioner == PRISM_PC_AUTO && smallSolveFits(AT, 1)) amg = nullptr;
+        if (amg && (eq.no_stand_in || amg->no_sa) && o.preconditioner == PRISM_PC_AUTO && smallSolveFits(AT, 1)) amg = nullptr;
         const HoldAmgValues hold(amg, it > 0);
         KrylovOut k = amg && !eq.no_stand_in && smoothedFits(amg, AT) && !amg->not_dominant
                           ? standInStep(AT, rhs.p, lam.p, ktol, kmax, SOLVE_FLEXIBLE, fp64, m, amg, eq)

@@ -1205,6 +1205,7 @@ void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, bool s
     L0->sl_col = A.col;
     L0->diag_pos = A.diag_pos;
     levels.push_back(std::move(L0));
+    double filled = 0.0;
     while (true) {
         const size_t l = levels.size() - 1;
         SaLevel& L = *levels[l];
@@ -1290,6 +1291,8 @@ void SaAmg::build(const SellMatrix& A, const int* rowptr, const int* col, bool s
         C->vals = C->o_vals.p;
         C->lpr_a = lanesFor(nc, C->nnz);
         levels.push_back(std::move(C));
+        filled += (double)levels.back()->nnz * levels.back()->nnz / nc;
+        if (filled > max_fill * A.nnz_csr * A.nnz_csr / A.n) fail(PRISM_BAD_ARG, "multigrid levels too dense for smoothed aggregation");
         levelValues(l, s);
         PB_LAUNCH("smoothed aggregation: level");
     }

@@ -58,6 +58,8 @@ struct SaAmg {
     bool built = false, symmetric = true;
     bool fresh = false;  // the last setup built the structure: it belongs to the matrix of that call
     uint64_t generation = 0;
+    // rows x (entries per row)^2 of the coarse levels over the matrix's: beyond it setup throws
+    double max_fill = 25.0;
     int tail = -1;  // first level of the fused coarse tail (-1: none)
     int coarse_n = 0;
     ArenaBuf<double> coarse_a;
