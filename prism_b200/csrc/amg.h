@@ -96,6 +96,7 @@ struct Amg {
     std::unique_ptr<SaAmg> sa;
     // its symmetric form is for weakly diagonally dominant matrices (lookAtDominance)
     bool not_dominant = false;
+    int sa_pays = -1;  // its other form: for matrices that are far from dominant (standInPays; -1: not measured)
     bool no_sa = false;  // that hierarchy did not fit (memory, 32-bit indices): this struct's own from then on
 
     // Build the hierarchy (first call) or refresh its values (later calls) for

@@ -573,7 +573,17 @@ static int kindFor(const Transport& eq, const PrismSolveOpts& o, const Amg* amg,
     if (eq.spd) return o.precision == PRISM_PREC_FP64 ? flexible : SOLVE_PLAIN;
     if (eq.no_stand_in || g_in_step || !smoothedFits(amg, A)) return SOLVE_PLAIN;
     if (symmetricMatrix(eq)) return amg->not_dominant ? SOLVE_PLAIN : SOLVE_FLEXIBLE;
-    return SOLVE_SMOOTHED;
+    return amg->sa_pays == 0 ? SOLVE_PLAIN : SOLVE_SMOOTHED;
+}
+// Convection with a time term or relaxation that leaves off-diagonal row sums of at most 0.7 of
+// the diagonal: a few iterations do with any cycle, and refreshing the smoothed hierarchy costs more
+// than it saves (amg's own against it: hexahedra, 2.1M rows, 6.5 ms against 10.3 at 0.5, 13.0 against
+// 9.9 at 0.8; 216,000 1.7 / 1.9 and 2.8 / 1.9; 384,000 tetrahedra 1.8 / 3.2, 2.9 / 3.3 at 0.8 and
+// 3.7 / 3.3 at 0.9; 34,992 0.87 / 1.44 and 1.45 / 1.21). Looked at again while it does not pay: the time
+// step may grow.
+static void standInPays(Amg* amg, const SellMatrix& A, Mesh& m) {
+    constexpr double NEARLY_DIAGONAL = 0.7;
+    amg->sa_pays = offDiagonalRatio(A, m.kw, m.stream) > NEARLY_DIAGONAL;
 }
 // flexible CG is what an AMG solve of eq would be
 static bool flexibleFor(const Transport& eq, const PrismSolveOpts& o) {
@@ -686,6 +696,8 @@ static PrismSolveResult solveAssembled(Transport& eq, const PrismSolveOpts& o, b
     Amg* amg = hierarchyFor(eq, o, A);
     if (amg && flexibleFor(eq, o) && (amg->not_dominant || kindFor(eq, o, amg, A) == SOLVE_FLEXIBLE))
         lookAtDominance(amg, A, m.kw, m.stream);
+    if (amg && amg->sa_pays == 0 && !eq.matrix_unchanged) amg->sa_pays = -1;
+    if (amg && amg->sa_pays < 0 && kindFor(eq, o, amg, A) == SOLVE_SMOOTHED) standInPays(amg, A, m);
     if (amg && (plain || (flexibleFor(eq, o) && amg->not_dominant)) && jacobiInstead(o, A)) amg = nullptr;
     if (o.method == PRISM_SOLVER_BICGSTAB && !amg && spent == 0 && smallSolveFits(A, kmax, o.n_iter)) {
         const SolveCtl& c = runSmall(A, eq.b.p, phi.v.p, std::max<int64_t>(o.n_iter, 0), o.eps, ktol, kmax,

@@ -268,3 +268,42 @@ def test_filled_levels_of_a_small_matrix():
     k.set_values(np.random.default_rng(1).lognormal(0, 3, mesh.n_cells))
     res, t = repeated(api.BiCGSTAB(), mesh, T, eqn)
     assert all(r.status == 0 and r.krylov_iterations < 200 for r in res)
+
+
+
+WITH_TIME_TERM = """
+import sys
+import numpy as np
+import prism_b200
+from prism_b200 import api
+from tests import cases
+n, ratio = 40, float(sys.argv[1])
+mesh, T, U, keep = cases.transport_c3(n, prism_b200.lib(), conv="Upwind", jitter=0.0)
+T.set_history_size(1)
+T.update(np.zeros(mesh.n_cells))
+k = api.Scalar("k", mesh, 1.0)
+dt = 1.0 / n ** 2 / 6.0 * ratio / (1.0 - ratio)  # diffusion through six faces: V/dt = 6 h (1/ratio - 1)
+eqn = api.Transport(api.temporal.BackwardEuler(T, dt), api.convection.Upwind(U, T), api.diffusion.NonCorrected(k, T))
+eqn.set_time_step(dt)
+r = api.BiCGSTAB(preconditioner="amg").solve(eqn, 1, 0.0)
+assert r.status == 0 and r.krylov_rel_residual < 1e-11
+if len(sys.argv) > 2:  # the time step grows
+    eqn.set_time_step(100 * dt)
+    T.set_values(np.zeros(mesh.n_cells))
+    r = api.BiCGSTAB(preconditioner="amg").solve(eqn, 1, 0.0)
+    assert r.status == 0 and r.krylov_rel_residual < 1e-11
+"""
+
+
+@pytest.mark.parametrize("args, smoothed", [(["0.3"], False), (["0.6"], False), (["0.99"], True), (["0.6", "growing"], True)])
+def test_convection_with_a_time_term(args, smoothed):
+    """A nearly diagonal matrix keeps amg's own cycle: the smoothed one's refresh takes longer than what its
+    iterations save (64,000 rows; the walls' half distances put the largest ratio a little lower)."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", WITH_TIME_TERM, *args], cwd=root, capture_output=True, text=True, timeout=300,
+                       env={**os.environ, "PRISM_VERBOSE": "1"})
+    assert p.returncode == 0, p.stderr
+    assert ("[prism samg] hierarchy" in p.stderr) == smoothed
