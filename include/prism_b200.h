@@ -339,7 +339,8 @@ typedef struct {
     double ref_value;
     int32_t clear_coeffs;
     double krylov_tol;      /* BiCGSTAB step: stop at ||b-Ax||/||b|| <= krylov_tol (0: default 1e-12) */
-    int64_t krylov_max_iter; /* per step, restarts and fallbacks included (0: default 2*n_cells for each) */
+    int64_t krylov_max_iter; /* per step, restarts and fallbacks included; conjugate gradients in place of BiCGSTAB
+                                count two iterations as one (0: default 2*n_cells for each) */
     double inner_tol;        /* mixed precision: residual reduction between FP64 reliable updates (0: default 0.1) */
     int32_t preconditioner;  /* PRISM_PC_* (BiCGSTAB only) */
     int32_t graph;           /* 1: prism_solve, and the SIMPLE/PRIME/PISO steps given these options, run as
@@ -356,7 +357,7 @@ typedef struct {
     double final_residual;
     int32_t converged;
     int32_t status;           /* worst Krylov status met (PRISM_OK / NOT_CONVERGED / ...) */
-    int64_t krylov_iterations; /* total inner Krylov iterations */
+    int64_t krylov_iterations; /* total inner Krylov iterations, counted as for krylov_max_iter */
     double krylov_rel_residual; /* ||b-Ax||/||b|| after the last step */
 } PrismSolveResult;
 

@@ -1252,7 +1252,7 @@ FlexEnd runFlex(const std::vector<BatchSystem>& sys, BatchPlan& pl, double tol, 
     P.z = pl.fz32.p;
     P.st = reinterpret_cast<FState*>(pl.fstate.p);
     P.tol = tol;
-    P.maxit = std::min<long long>(maxit, FLEX_MAX_ITER);
+    P.maxit = std::min<long long>(2 * std::min<long long>(maxit, FLEX_MAX_ITER), FLEX_MAX_ITER);
 
     std::vector<CopyEntry> tab(sys.size());
     std::vector<uintptr_t> key = {2, (uintptr_t)P.maxit, 0};
@@ -1338,11 +1338,11 @@ FlexEnd runFlex(const std::vector<BatchSystem>& sys, BatchPlan& pl, double tol, 
     FlexEnd end = FLEX_OK;
     bool nonfinite = false;
     for (int i = 0; i < pl.nprob; ++i) {
-        out[i].iterations = hs[i].iter;
+        out[i].iterations = (hs[i].iter + 1) / 2;  // in place of BiCGSTAB, as for single systems (krylov.cu)
         out[i].passes = hs[i].pass + 1;
         out[i].rel_residual = hs[i].rel;
         out[i].status = hs[i].status;
-        const bool capped = own_cap && hs[i].status == PRISM_NOT_CONVERGED && hs[i].iter >= maxit;
+        const bool capped = own_cap && hs[i].status == PRISM_NOT_CONVERGED && out[i].iterations >= maxit;
         nonfinite = nonfinite || hs[i].status == PRISM_NONFINITE;
         if (hs[i].status == PRISM_OK || capped || hs[i].bad) continue;
         end = std::max(end, hs[i].done == 1 ? FLEX_SHORT : FLEX_FAILED);

@@ -1411,12 +1411,16 @@ KrylovOut standInSolve(const SellMatrix& A, const double* b, double* x, double t
                        double inner_tol, KrylovWork& w, cudaStream_t s, Amg* amg, const int* rowptr, const int* col,
                        int kind, int precision, const Instead& instead, int* instead_status) {
     *instead_status = -1;
+    // Flexible CG in place of BiCGSTAB: two of its iterations apply the matrix and the cycle as often as
+    // one asked for, and count as one (63,888 tetrahedra: 26 against 22 with amg's cycle). A cap that was enough stays so.
+    const int per = kind == SOLVE_FLEXIBLE && instead.kind == SOLVE_PLAIN ? 2 : 1;
     w.ensure(A.nslices * 32, A.nnz_padded, false);
     PB_CUDA(cudaMemcpyAsync(w.xs.p, x, A.n * sizeof(double), cudaMemcpyDeviceToDevice, s));
     long long left = maxit, used = 0;
     while (true) {
-        KrylovOut k = bicgstab(A, b, x, tol, std::min(left, STAND_IN_MAX),
+        KrylovOut k = bicgstab(A, b, x, tol, std::min(std::min(left, STAND_IN_MAX) * per, STAND_IN_MAX),
                                kind == SOLVE_FLEXIBLE ? PRISM_PREC_FP64 : precision, inner_tol, w, s, amg, rowptr, col, kind);
+        k.iterations = (k.iterations + per - 1) / per;
         used += k.iterations;
         if (cap > 0) left -= k.iterations;
         k.iterations = used;
@@ -1552,7 +1556,7 @@ constexpr int GRAPH_UNROLL = 4;  // BiCGSTAB iterations per pass of the device l
 __device__ __forceinline__ double nanValue() { return __longlong_as_double(0x7ff8000000000000LL); }
 
 __global__ void ctl_solve_begin_kernel(SolveCtl* c, long long n_iter, double eps, long long kmax, double tol,
-                                       int stand_in, cudaGraphConditionalHandle ho) {
+                                       int stand_in, int per, cudaGraphConditionalHandle ho) {
     if (threadIdx.x) return;
     cudaGraphSetConditional(ho, 1u);
     SolveCtl z{};
@@ -1561,6 +1565,7 @@ __global__ void ctl_solve_begin_kernel(SolveCtl* c, long long n_iter, double eps
     z.kmax = kmax;
     z.tol = tol;
     z.stand_in = stand_in;
+    z.per = per;
     z.status = PRISM_OK;
     z.kstatus = PRISM_OK;
     z.phase = PH_DONE;
@@ -1652,7 +1657,9 @@ __global__ void ctl_outer_step_kernel(SolveCtl* c, const double* scal, cudaGraph
     c->outer += 1;
     const bool conv = cur < c->eps;
     if (conv) c->converged = 1;
-    c->step_iterations = c->kmax - c->maxit_left;
+    const long long its = c->kmax - c->maxit_left;
+    c->step_iterations = (its + c->per - 1) / c->per;
+    c->krylov_iterations -= its - c->step_iterations;
     c->failed = c->stand_in && c->kstatus != PRISM_OK && !(c->stand_in == 2 && c->kstatus == PRISM_NOT_CONVERGED);
     cudaGraphSetConditional(ho, (!conv && !c->failed && c->outer < c->n_iter) ? 1u : 0u);
 }
@@ -1714,9 +1721,9 @@ void endConditional(cudaStream_t body) {
     PB_CUDA(cudaStreamEndCapture(body, &g));
 }
 
-void emitSolveBegin(SolveCtl* ctl, long long n_iter, double eps, long long kmax, double tol, int stand_in,
+void emitSolveBegin(SolveCtl* ctl, long long n_iter, double eps, long long kmax, double tol, int stand_in, int per,
                     cudaGraphConditionalHandle outer, cudaStream_t s) {
-    ctl_solve_begin_kernel<<<1, 32, 0, s>>>(ctl, n_iter, eps, kmax, tol, stand_in, outer); countLaunch();
+    ctl_solve_begin_kernel<<<1, 32, 0, s>>>(ctl, n_iter, eps, kmax, tol, stand_in, per, outer); countLaunch();
 }
 
 void emitResidual(const SellMatrix& A, const double* b, const double* x, KrylovWork& w, cudaStream_t s) {

@@ -169,6 +169,7 @@ struct SolveCtl {
     // a stand-in (runtime.cpp): its first failed step ends the solve (failed; its iterations in
     // step_iterations). stand_in 2: the iteration cap is the caller's, and reaching it no failure
     int stand_in, failed;
+    int per;  // iterations that count as one (standInSolve); kmax and maxit_left hold single ones
     long long step_iterations;
     int no_cg;  // one-launch solves: conjugate gradients broke down
 };
@@ -204,7 +205,7 @@ bool capturing(cudaStream_t s);
 // Device-controlled pieces of solve(), emitted into the capture on s:
 // ctl := ISolver::solve bookkeeping for n_iter steps, eps, kmax, tol
 // (and switches on the outer loop's condition)
-void emitSolveBegin(SolveCtl* ctl, long long n_iter, double eps, long long kmax, double tol, int stand_in,
+void emitSolveBegin(SolveCtl* ctl, long long n_iter, double eps, long long kmax, double tol, int stand_in, int per,
                     cudaGraphConditionalHandle outer, cudaStream_t s);
 // w.scal := max|A x - b|, max|diag(A) x|, non-finite flag (the scaled residual's parts)
 void emitResidual(const SellMatrix& A, const double* b, const double* x, KrylovWork& w, cudaStream_t s);

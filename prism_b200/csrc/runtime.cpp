@@ -1402,10 +1402,11 @@ PrismSolveResult solveCaptured(Transport& eq, const PrismSolveOpts& o) {
         r.iterations = -(slot + 1);
         return r;
     }
-    const long long cap = stand_in ? std::min(kmax, STAND_IN_MAX) : kmax;
+    const int per = stand_in && kind == SOLVE_FLEXIBLE && standsInFor(eq, o) == SOLVE_PLAIN ? 2 : 1;  // as in standInSolve
+    const long long cap = stand_in ? std::min(std::min(kmax, STAND_IN_MAX) * per, STAND_IN_MAX) : kmax;
     cudaGraphConditionalHandle outer = createConditional(s, 0);
-    const int stop = !stand_in ? 0 : o.krylov_max_iter > 0 && o.krylov_max_iter <= STAND_IN_MAX ? 2 : 1;
-    emitSolveBegin(ctl, n_iter, o.eps, cap, ktol, stop, outer, s);
+    const int stop = !stand_in ? 0 : o.krylov_max_iter > 0 && o.krylov_max_iter <= STAND_IN_MAX / per ? 2 : 1;
+    emitSolveBegin(ctl, n_iter, o.eps, cap, ktol, stop, per, outer, s);
     if (n_iter > 0) {
         ++phi.event;
         emitResidual(A, eq.b.p, phi.v.p, m.kw, s);
